@@ -220,7 +220,6 @@ struct lpp_engine {
     double* ex_block_sum = nullptr;
     int* ex_entry_count = nullptr;
     ExactEntry* ex_entries = nullptr;
-    float* ex_scalars = nullptr;
     float2* rope = nullptr;
     StepState* st = nullptr;
     int run_cap = 0;  // capacity of r_values / out_tokens
@@ -813,7 +812,6 @@ static cudaError_t launch_sampler(lpp_engine* e, cudaStream_t s, bool pdl, bool 
         ea.block_sum = e->ex_block_sum;
         ea.entry_count = e->ex_entry_count;
         ea.entries = e->ex_entries;
-        ea.scalars = e->ex_scalars;
         return launch_kernel(sample_exact_kernel, dim3(e->sample_blocks), dim3(kSampleThreads), 0, s, pdl, ea);
     }
     return launch_kernel(sample_kernel, dim3(e->sample_blocks), dim3(kSampleThreads), 0, s, pdl, a);
@@ -1343,9 +1341,8 @@ static lpp_status alloc_step_buffers(lpp_engine* e, size_t att_n, size_t hb_n) {
         CU(cudaMalloc(&e->ex_sync, 2 * sizeof(unsigned int)));
         CU(cudaMemsetAsync(e->ex_sync, 0, 2 * sizeof(unsigned int), e->stream));
         CU(cudaMalloc(&e->ex_block_sum, e->sample_blocks * sizeof(double)));
-        CU(cudaMalloc(&e->ex_entry_count, e->sample_blocks * sizeof(int)));
-        CU(cudaMalloc(&e->ex_entries, (size_t)e->sample_blocks * kExactMaxEntries * sizeof(ExactEntry)));
-        CU(cudaMalloc(&e->ex_scalars, 64 * sizeof(float)));
+        CU(cudaMalloc(&e->ex_entry_count, (size_t)kExactLists * e->sample_blocks * sizeof(int)));
+        CU(cudaMalloc(&e->ex_entries, (size_t)kExactLists * e->sample_blocks * kExactMaxEntries * sizeof(ExactEntry)));
     }
     e->run_cap = std::max<int>(4096, c.seq_len);
     CU(cudaMalloc(&e->r_values, (size_t)e->run_cap * 4));
@@ -1812,7 +1809,7 @@ extern "C" lpp_status lpp_engine_destroy(lpp_engine* e) {
                     e->rms_final, e->kcache, e->vcache, e->xa, e->xb, e->q, e->att_out, e->hb, e->logits,
                     e->attn_part, e->attn_counters, e->samp_max, e->samp_sum, e->samp_idx, e->samp_counter,
                     e->r_values, e->out_tokens, e->st, e->rope, e->stage, e->gtrace, e->pf_x, e->pf_q, e->pf_part, e->pf_xn, e->pf_att, e->pf_hb,
-                    e->pf_tokens, e->ex_sync, e->ex_block_sum, e->ex_entry_count, e->ex_entries, e->ex_scalars, e->final_b, e->lat_qplain,
+                    e->pf_tokens, e->ex_sync, e->ex_block_sum, e->ex_entry_count, e->ex_entries, e->final_b, e->lat_qplain,
                     e->lat_raw, e->lat_gate, e->lat_query, e->lat_part, e->pf_rows, e->pf_logits, e->pf_qn, e->pf_olat, e->pf_lq,
                     e->pf_lpart, e->pf_gate, e->loop_vec, e->scan_x, e->scan_z, e->scan_low, e->row_counters, e->pf_sx, e->pf_sz, e->pf_tail, e->pf_sxp, e->pf_low};
     for (void* p : bufs)
@@ -2977,16 +2974,6 @@ extern "C" int lpp_debug_gemv_trace(lpp_engine* e, unsigned long long* out, int 
     cudaStreamSynchronize(e->stream);
     if (cudaMemcpy(out, e->gtrace, n * sizeof(unsigned long long), cudaMemcpyDeviceToHost) != cudaSuccess) return -3;
     return e->num_sms;
-}
-
-// Debugging aid (not part of the public header): the exact sampler's entry lists of its last stage.
-extern "C" int lpp_debug_sampler_entries(lpp_engine* e, int* counts, void* entries, float* scalars) {
-    if (!e || !e->exact_sampler) return -1;
-    cudaStreamSynchronize(e->stream);
-    cudaMemcpy(counts, e->ex_entry_count, e->sample_blocks * sizeof(int), cudaMemcpyDeviceToHost);
-    cudaMemcpy(entries, e->ex_entries, (size_t)e->sample_blocks * kExactMaxEntries * sizeof(ExactEntry), cudaMemcpyDeviceToHost);
-    cudaMemcpy(scalars, e->ex_scalars, 64 * sizeof(float), cudaMemcpyDeviceToHost);
-    return e->sample_blocks;
 }
 
 #ifdef LPP_TIMING_AIDS

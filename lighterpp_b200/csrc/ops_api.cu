@@ -78,11 +78,11 @@ lpp_status op_gemv_t(float* out, const float* x, const void* w, int n, int d, cu
 }
 
 // ---- scratch layout of the stand-alone samplers: step state, per-block partials, ticket counter and barrier
-//      words, then what the exact-order kernel adds (block sums, entry counts, scalars, entry lists).
+//      words, then what the exact-order kernel adds (block sums, entry counts, entry lists).
 //      `cap_blocks` sizes the areas: the blocks of this call (stream-ordered scratch) or of the largest
 //      vocabulary the fixed array takes.
 struct SampleScratch {
-    size_t state, part, counters, sums, counts, scalars, entries, total;
+    size_t state, part, counters, sums, counts, entries, total;
 };
 constexpr SampleScratch sample_scratch_layout(int cap_blocks, bool exact) {
     SampleScratch L = {};
@@ -97,11 +97,9 @@ constexpr SampleScratch sample_scratch_layout(int cap_blocks, bool exact) {
         L.sums = o;
         o += ((size_t)cap_blocks * sizeof(double) + 255) & ~(size_t)255;
         L.counts = o;
-        o += ((size_t)cap_blocks * sizeof(int) + 255) & ~(size_t)255;
-        L.scalars = o;
-        o += 256;
+        o += ((size_t)kExactLists * cap_blocks * sizeof(int) + 255) & ~(size_t)255;
         L.entries = o;
-        o += (size_t)cap_blocks * kExactMaxEntries * sizeof(ExactEntry);
+        o += (size_t)kExactLists * cap_blocks * kExactMaxEntries * sizeof(ExactEntry);
     }
     L.total = o;
     return L;
@@ -127,7 +125,6 @@ void launch_sampler_on_scratch(char* scratch, const SampleScratch& L, bool exact
         ea.sync = (unsigned int*)(scratch + L.counters + 256);
         ea.block_sum = (double*)(scratch + L.sums);
         ea.entry_count = (int*)(scratch + L.counts);
-        ea.scalars = (float*)(scratch + L.scalars);
         ea.entries = (ExactEntry*)(scratch + L.entries);
         sample_exact_kernel<<<nb, kSampleThreads, 0, s>>>(ea);
     } else {

@@ -14,14 +14,21 @@
 //   "S -> S + d[parity of S]", and maps compose associatively: a run of elements collapses, with a
 //   parallel scan, into one pair (D0, D1).
 //
-//   Where the sum may change binade the emulation does not apply.  Every thread classifies its four
-//   consecutive elements from an approximate (double) prefix sum: if the prefix before and after the
-//   quad is safely inside one binade the quad is "plain" and contributes a map, otherwise it is a
-//   "window" whose elements are added one by one with real FP32 additions.  Blocks publish a short
-//   list of entries (map runs and windows); one warp then walks all entries in order.  A map entry
-//   is applied only after checking that s really is in the predicted binade and stays in it;
-//   otherwise its elements are added one by one as well, so the result never depends on the
-//   approximate prefix being accurate -- only the speed does.
+//   Where the sum may change binade one map does not do.  Every thread classifies its four consecutive
+//   elements from an approximate (double) prefix sum: if the prefix before and after the quad is safely
+//   inside one binade the quad is "plain" and contributes a map; near a power of two it is a "window"
+//   whose elements are added one by one with real FP32 additions; and where many quads of a block lie
+//   near one (a confident distribution: the sum sits at 1 + a little for the whole rest of the
+//   vocabulary) they are "dual" and contribute the maps of both binades, of which the walk takes the one
+//   that the exact sum is in.  Blocks publish a short list of entries (runs of maps and windows); one warp
+//   then walks all entries in order.  A map entry is applied only after checking that s really is in its
+//   binade and stays in it; a run that leaves it is done over by the whole block (resolve_range: parallel
+//   scan up to the element that leaves the binade, one real addition, and on from there), so the result
+//   never depends on the approximate prefix being accurate -- only the speed does.
+//
+//   Latency-bound: ceil(V/2048) blocks, a few microseconds per dependent stage.  A token of the
+//   Llama-3.2-1B shape whose distribution is confident (0.998 on one token): 3.35 ms with windows of
+//   whole blocks added one by one by one warp, of which this kernel took 2.7 ms; 0.66 ms now.
 //
 // exp() is exp_repro (common.cuh): IEEE double arithmetic only, identical on host and device; it
 // differs from libm's expf in the last bit for about 0.06 % of arguments, which is the only source
@@ -35,27 +42,32 @@
 
 namespace lpp {
 
-constexpr int kExactMaxEntries = 96;  // per block; a block that needs more becomes one "add one by one" entry
+constexpr int kExactMaxEntries = 48;  // per block and list; a block that needs more becomes one kEntrySeq entry
+constexpr int kExactLists = 2;        // of the denominator's sum and of the running distribution
 constexpr double kExactEps = 1.0 / 4096.0;  // safety margin of the binade prediction (speed only)
+// Quads near a power of two become dual runs when a block has more of them than this.  A window is the cheaper form where
+// the sum passes a power of two within a quad or two (flat distributions: some ten windows per vocabulary, nearly each of
+// which would leave its binade inside a dual run and be done over); a block that stays near one has hundreds.
+constexpr int kExactDualMin = 16;
 
-enum : int { kEntryMap = 0, kEntrySeq = 1, kEntryQuad = 2 };
+enum : int { kEntryMap = 0, kEntrySeq = 1, kEntryQuad = 2, kEntryDual = 3 };
 constexpr int kExactListCap = 512;  // entries the walking block stages in shared memory per round
 
 struct ExactEntry {
-    int kind;  // kEntryMap: apply (d0, d1) in binade e; kEntrySeq: add elements [lo, hi) one by one;
-               // kEntryQuad: add the four floats stored in (d0, d1), elements lo..lo+3, one by one
+    int kind;  // kEntryMap: elements [lo, hi) as the map d[0..1] of binade e; kEntryDual: also as the map d[2..3] of binade
+               // e + 1; kEntryQuad: add the four floats in d, elements lo..lo+3, one by one; kEntrySeq: elements [lo, hi)
+               // through resolve_range
     int lo, hi;
     int e;
-    unsigned long long d0, d1;
+    unsigned int d[4];
 };
 
 struct SampleExactArgs {
     SampleArgs base;
     unsigned int* sync;      // [0] grid-barrier counter, [1] exit ticket; zero between launches
     double* block_sum;       // [n_blocks] approximate sum of exp per block
-    int* entry_count;        // [n_blocks]
-    ExactEntry* entries;     // [n_blocks][kExactMaxEntries]
-    float* scalars;          // [0] exact softmax denominator
+    int* entry_count;        // [kExactLists][n_blocks]
+    ExactEntry* entries;     // [kExactLists][n_blocks][kExactMaxEntries]
 };
 
 // ---- the integer map of one element -------------------------------------------------------------
@@ -102,18 +114,13 @@ __device__ __forceinline__ int binade_of(double v) {  // floor(log2(v)) for v > 
     return (int)((__double_as_longlong(v) >> 52) & 0x7ff) - 1023;
 }
 
-// Exact fl(s + x) bookkeeping helpers for the walking warp.
-__device__ __forceinline__ bool apply_map(float& s, int E, unsigned long long d0, unsigned long long d1) {
-    const unsigned int bits = __float_as_uint(s);
-    const int es = (int)((bits >> 23) & 0xffu) - 127;
-    if (!(s > 0.f) || es != E || ((bits >> 23) & 0xffu) == 0u) return false;
-    const unsigned long long S = (bits & 0x7fffffu) | 0x800000u;
-    const unsigned long long R = S + ((S & 1ull) ? d1 : d0);
-    if (R > (1ull << 24)) return false;
-    // R in [2^23, 2^24]: the float with mantissa R in binade E (or exactly 2^(E+1))
-    s = (R == (1ull << 24)) ? __uint_as_float((unsigned int)(E + 128) << 23)
-                            : __uint_as_float(((unsigned int)(E + 127) << 23) | ((unsigned int)R & 0x7fffffu));
-    return true;
+// Increments of a valid run are at most 2^23; larger ones only have to stay invalid.
+__device__ __forceinline__ unsigned int map_word(unsigned long long d) { return (unsigned int)min(d, 0x7fffffffull); }
+
+// The float that S ulps of binade E are (S in [2^23, 2^24]).
+__device__ __forceinline__ float float_of_ulps(unsigned long long S, int E) {
+    return (S >= (1ull << 24)) ? __uint_as_float((unsigned int)(E + 128) << 23)
+                               : __uint_as_float(((unsigned int)(E + 127) << 23) | ((unsigned int)S & 0x7fffffu));
 }
 
 // ---- grid barrier for this kernel (all blocks co-resident; bounded wait) -------------------------
@@ -224,30 +231,44 @@ static __device__ __noinline__ void emit_entries(const float (&x)[4], double pre
     const int lane = tid & 31;
     const bool valid = tid < n_valid_quads;
     const double post = pre + (double)x[0] + (double)x[1] + (double)x[2] + (double)x[3];
-    // plain: the sum is provably inside one binade before, during and after this quad
-    bool plain = false;
+    // plain: the sum is provably inside one binade before, during and after this quad; near: inside one or the next
+    bool plain = false, near = false;
     int E = 0;
     if (valid && pre > 0.0) {
         const int e0 = binade_of(pre * (1.0 - kExactEps)), e1 = binade_of(post * (1.0 + kExactEps));
         E = e0;
         const float lim = __uint_as_float((unsigned int)((e0 > -120 && e0 < 120 ? e0 : 0) + 127) << 23);  // 2^e0
-        plain = (e0 == e1) && e0 > -120 && e0 < 120 && x[0] < lim && x[1] < lim && x[2] < lim && x[3] < lim;
+        const bool fits = e0 > -120 && e0 < 119 && x[0] < lim && x[1] < lim && x[2] < lim && x[3] < lim;
+        plain = fits && e0 == e1;
+        near = fits && e1 == e0 + 1;
     }
-    // runs: maximal sequences of threads of one class (plain runs also share E)
-    const int cls = !valid ? 2000 : (plain ? E : 1000);  // binades lie in (-120, 120): no clash with the markers
+    const bool use_dual = __syncthreads_count(near) > kExactDualMin;
+    const bool dual = near && use_dual;
+    const bool mapped = plain || dual;
+    const bool zero = valid && post == 0.0;  // nothing but zeros so far: no entry
+    // runs: maximal sequences of threads of one class (mapped runs also share E)
+    const int cls = !valid ? 5000 : zero ? 4000 : plain ? E : dual ? 1000 + E : 3000;  // binades lie in (-120, 119): no clash
     const int prev = __shfl_up_sync(0xffffffffu, cls, 1);
     __shared__ int s_cls_last[kSampleThreads / 32];
     if (lane == 31) s_cls_last[tid >> 5] = cls;
     __syncthreads();
-    const int before = (tid == 0) ? 3000 : (lane == 0 ? s_cls_last[(tid >> 5) - 1] : prev);
-    // a quad outside the plain class is an entry of its own: it travels with its four values
-    const bool start = valid && (cls != before || !plain);
-    Map2 mp = map_identity();
-    if (plain) {
+    const int before = (tid == 0) ? 6000 : (lane == 0 ? s_cls_last[(tid >> 5) - 1] : prev);
+    // a quad without a map is an entry of its own: it travels with its four values
+    const bool start = valid && !zero && (cls != before || !mapped);
+    Map2 mp = map_identity(), mp2 = map_identity();
+    if (mapped) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) mp = map_compose(mp, map_of(x[k], E));
     }
     const Map2 run = block_segscan(mp, start, s_wm, s_wf, tid);
+    Map2 run2 = map_identity();
+    if (use_dual) {  // the same for the whole block
+        if (dual) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) mp2 = map_compose(mp2, map_of(x[k], E + 1));
+        }
+        run2 = block_segscan(mp2, start, s_wm, s_wf, tid);
+    }
     // entry index = number of run starts up to and including this thread, minus one
     int cnt = start ? 1 : 0;
 #pragma unroll
@@ -268,25 +289,22 @@ static __device__ __noinline__ void emit_entries(const float (&x)[4], double pre
     const int nxt_cls = __shfl_down_sync(0xffffffffu, cls, 1);
     if (lane == 0) s_cls_last[tid >> 5] = cls;  // reuse as "first class of warp"
     __syncthreads();
-    const int after = (tid == kSampleThreads - 1) ? 3000 : (lane == 31 ? s_cls_last[(tid >> 5) + 1] : nxt_cls);
-    const bool last = valid && (cls != after || !plain);
+    const int after = (tid == kSampleThreads - 1) ? 6000 : (lane == 31 ? s_cls_last[(tid >> 5) + 1] : nxt_cls);
+    const bool last = valid && !zero && (cls != after || !mapped);
     if (!overflow) {
         if (start) {
-            out[idx].kind = plain ? kEntryMap : kEntrySeq;
+            out[idx].kind = plain ? kEntryMap : dual ? kEntryDual : kEntryQuad;
             out[idx].lo = first_elem + 4 * tid;
             out[idx].e = E;
         }
         if (last) {
             out[idx].hi = first_elem + 4 * tid + 4;
-            if (!plain && start) {
-                // a window of one quad (the usual case) carries its values, sparing the walker a memory round trip
-                out[idx].kind = kEntryQuad;
-                out[idx].d0 = (unsigned long long)__float_as_uint(x[0]) | ((unsigned long long)__float_as_uint(x[1]) << 32);
-                out[idx].d1 = (unsigned long long)__float_as_uint(x[2]) | ((unsigned long long)__float_as_uint(x[3]) << 32);
-            } else {
-                out[idx].d0 = run.d0;
-                out[idx].d1 = run.d1;
-            }
+            uint4 d;
+            if (mapped)
+                d = make_uint4(map_word(run.d0), map_word(run.d1), map_word(run2.d0), map_word(run2.d1));
+            else  // a window carries its values, sparing the walker a memory round trip
+                d = make_uint4(__float_as_uint(x[0]), __float_as_uint(x[1]), __float_as_uint(x[2]), __float_as_uint(x[3]));
+            *reinterpret_cast<uint4*>(out[idx].d) = d;
         }
         if (tid == 0) *out_count = total;
     } else if (tid == 0) {
@@ -294,99 +312,144 @@ static __device__ __noinline__ void emit_entries(const float (&x)[4], double pre
         out[0].lo = first_elem;
         out[0].hi = first_elem + 4 * n_valid_quads;
         out[0].e = 0;
-        out[0].d0 = out[0].d1 = 0ull;
+        *reinterpret_cast<uint4*>(out[0].d) = make_uint4(0u, 0u, 0u, 0u);
         *out_count = 1;
     }
     __syncthreads();
 }
 
-// State of the walk over all entries, kept by warp 0 of the walking block (identical on all lanes).
+// State of the walk over all entries (shared memory).
 struct WalkState {
-    float s;                    // exact running sum
-    int found;                  // >= 0: first element whose running sum exceeds r
-    int run_lo, run_hi, run_e;  // >= 0: the crossing lies inside this map run ...
-    float run_s0;               // ... which starts from this exact sum
+    float s;       // exact running sum
+    int found;     // >= 0: first element whose running sum exceeds r
+    int resolved;  // runs that were done over
+};
+struct ResolveScratch {
+    float s;
+    int brk, cross, found;
+    Map2 last_map[kSampleThreads / 32];
 };
 
-// Applies `count` entries (in shared memory) in order.  Returns true when the walk is over (stop
-// requested and the crossing was located).  A map moves the sum by an integer number of ulps inside
-// one binade (or exactly onto the next power of two), which on the bit pattern of a positive float
-// is a plain integer addition.
-static __device__ __noinline__ bool walk_list(const ExactEntry* list, int count, const float* x, int n_total,
-                                          const bool kStop, float r, int lane, WalkState& w) {
-    unsigned int bits = __float_as_uint(w.s);
-    int4 nh = *reinterpret_cast<const int4*>(&list[0]);
-    ulonglong2 nd = *reinterpret_cast<const ulonglong2*>(&list[0].d0);
-    for (int i = 0; i < count; ++i) {
-        const int4 h = nh;  // kind, lo, hi, e
-        const ulonglong2 d = nd;
-        const int nx = min(i + 1, count - 1);  // fetched while this entry is applied
-        nh = *reinterpret_cast<const int4*>(&list[nx]);
-        nd = *reinterpret_cast<const ulonglong2*>(&list[nx].d0);
-        if (h.x == kEntryMap) {
-            const unsigned int ebase = (unsigned int)(h.w + 127) << 23;
-            const unsigned long long dd = (bits & 1u) ? d.y : d.x;
-            const unsigned int nb = bits + (unsigned int)dd;
-            // sum inside binade e before, and inside it or exactly on its upper end after
-            if (bits - ebase < 0x800000u && dd <= 0x800000ull && nb - ebase <= 0x800000u) {
-                if (kStop && r < __uint_as_float(nb)) {  // the first crossing lies inside this run
-                    w.run_lo = h.y;
-                    w.run_hi = min(h.z, n_total);
-                    w.run_e = h.w;
-                    w.run_s0 = __uint_as_float(bits);
-                    w.s = __uint_as_float(bits);
-                    return true;
+// Adds elements [lo, hi) of x to w->s in order, exactly, by the whole block: while the sum stays in one binade E the
+// elements are maps and a block scan gives the sum before and after each; the first element that leaves the binade (or is
+// no map of it: x >= 2^E, or the sum is zero) is added with one FP32 addition, and the scan starts over behind it.  Sums
+// close to the subnormals go element by element.  With `stop`, ends at the first element after which the sum exceeds r.
+// Every pass leaves a binade for good or ends the range, so a range costs a few passes of about 1.5 us.  A sum that is no
+// number ends it at once: nothing changes it any more.
+static __device__ __noinline__ void resolve_range(const float* x, int lo, int hi, bool stop, float r, WalkState* w, ResolveScratch* z, Map2* s_wm,
+                                                  int* s_wf, int tid) {
+    const int lane = tid & 31, warp = tid >> 5;
+    constexpr int kNone = 0x7fffffff;
+    for (int c0 = lo; c0 < hi; c0 += kSampleChunk) {
+        const int end = min(hi - c0, kSampleChunk), i0 = 4 * tid;  // chunk-relative elements i0 .. i0 + 3 are this thread's
+        float y[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[k] = (i0 + k < end) ? __ldcg(x + c0 + i0 + k) : 0.f;
+        int from = 0;
+        while (from < end) {
+            const float s = w->s;
+            if (!(s < INFINITY)) return;
+            const unsigned int bits = __float_as_uint(s);
+            const int E = (int)((bits >> 23) & 0xffu) - 127;
+            const bool scan = s > 0.f && E > -120 && E < 119;
+            __syncthreads();
+            if (s > 0.f && !scan) {
+                if (warp == 0) {
+                    float sum = s;
+                    int at = from;
+                    bool hit = false;
+                    while (at < end && !hit && sum < 0x1p-118f) {
+                        const float v = (at + lane < end) ? __ldcg(x + c0 + at + lane) : 0.f;
+                        const int m = min(32, end - at);
+                        for (int j = 0; j < m && !hit; ++j, ++at) {
+                            sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, v, j));
+                            hit = stop && r < sum;
+                        }
+                    }
+                    if (lane == 0) {
+                        w->s = sum;
+                        if (hit) w->found = c0 + at - 1;
+                        z->brk = at;
+                    }
                 }
-                bits = nb;
+                __syncthreads();
+                if (w->found >= 0) return;
+                from = z->brk;
+                __syncthreads();
                 continue;
             }
-        } else if (h.x == kEntryQuad) {
-            const float v[4] = {__uint_as_float((unsigned int)d.x), __uint_as_float((unsigned int)(d.x >> 32)),
-                                __uint_as_float((unsigned int)d.y), __uint_as_float((unsigned int)(d.y >> 32))};
-            float s = __uint_as_float(bits);
+            if (tid == 0) z->brk = z->cross = z->found = kNone;
+            __syncthreads();
+            // the first element that is no map
+            const float lim = scan ? __uint_as_float((unsigned int)(E + 127) << 23) : 0.f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                s = __fadd_rn(s, v[j]);
-                if (kStop && r < s) {
-                    w.found = h.y + j;
-                    w.s = s;
-                    return true;
+            for (int k = 3; k >= 0; --k)
+                if (i0 + k >= from && i0 + k < end && (scan ? !(y[k] < lim) : y[k] != 0.f)) atomicMin(&z->brk, i0 + k);
+            __syncthreads();
+            const int brk = min(z->brk, end);
+            // maps of the elements before it
+            Map2 m[4], mp = map_identity();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                m[k] = (scan && i0 + k >= from && i0 + k < brk) ? map_of(y[k], E) : map_identity();
+                mp = map_compose(mp, m[k]);
+            }
+            const Map2 incl = block_segscan(mp, tid == 0, s_wm, s_wf, tid);
+            Map2 ex;  // everything before this thread's elements
+            ex.d0 = __shfl_up_sync(0xffffffffu, incl.d0, 1);
+            ex.d1 = __shfl_up_sync(0xffffffffu, incl.d1, 1);
+            if (lane == 31) z->last_map[warp] = incl;
+            __syncthreads();
+            if (lane == 0) ex = (warp == 0) ? map_identity() : z->last_map[warp - 1];
+            const unsigned long long S0 = (bits & 0x7fffffu) | 0x800000u;
+            unsigned long long S = S0 + ((S0 & 1ull) ? ex.d1 : ex.d0), before[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                before[k] = S;
+                S += (S & 1ull) ? m[k].d1 : m[k].d0;
+                if (scan && i0 + k >= from && i0 + k < brk) {
+                    if (S > (1ull << 24))
+                        atomicMin(&z->cross, i0 + k);
+                    else if (stop && r < float_of_ulps(S, E))
+                        atomicMin(&z->found, i0 + k);
                 }
             }
-            bits = __float_as_uint(s);
-            continue;
-        }
-        // one-by-one FP32 additions from global memory, 32 loads at a time (oversized blocks, failed predictions)
-        float s = __uint_as_float(bits);
-        const int hi = min(h.z, n_total);
-        for (int b = h.y; b < hi; b += 32) {
-            const float v = (b + lane < hi) ? __ldcg(x + b + lane) : 0.f;
-            const int m = min(32, hi - b);
-            for (int j = 0; j < m; ++j) {
-                s = __fadd_rn(s, __shfl_sync(0xffffffffu, v, j));
-                if (kStop && r < s) {
-                    w.found = b + j;
-                    w.s = s;
-                    return true;
-                }
+            __syncthreads();
+            const int cross = min(z->cross, brk), found = z->found;
+            if (found < cross) {
+                if (tid == 0) w->found = c0 + found;
+                __syncthreads();
+                return;
             }
+            // the element at `cross` is added on its own; at the end of the range there is none
+            if (cross < end) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (i0 + k == cross) z->s = __fadd_rn(scan ? float_of_ulps(before[k], E) : s, y[k]);
+            } else if (tid == kSampleThreads - 1) {
+                z->s = scan ? float_of_ulps(S, E) : s;
+            }
+            __syncthreads();
+            if (tid == 0) {
+                w->s = z->s;
+                if (stop && cross < end && r < z->s) w->found = c0 + cross;
+            }
+            __syncthreads();
+            if (w->found >= 0) return;
+            from = cross + 1;
         }
-        bits = __float_as_uint(s);
     }
-    w.s = __uint_as_float(bits);
-    return false;
 }
 
 // Whole-block walk.  The blocks' entry lists are concatenated in block order (a prefix sum of the
 // counts gives every entry its place), staged into shared memory kExactListCap at a time, and
-// applied by warp 0.  Returns the final state in *out (shared memory).
+// applied by warp 0.  Leaves the final state in *out (shared memory).
 static __device__ __noinline__ void walk_all(const ExactEntry* entries, const int* counts, int n_blocks, const float* x,
-                                         int n_total, bool stop, float r, ExactEntry* s_list, int* s_pref, int* s_i,
-                                         WalkState* out, int tid) {
+                                         int n_total, bool stop, float r, ExactEntry* s_list, int* s_pref, int* s_i, Map2* s_wm, int* s_wf,
+                                         ResolveScratch* z, WalkState* out, int tid) {
     static_assert(kSampleMaxBlocks <= kSampleThreads, "one thread per block's count");
     const int lane = tid & 31;
-    __shared__ int s_done;
-    __shared__ int s_ctl[2];                          // first failed entry, first crossing entry
+    __shared__ int s_ctl[2];                              // first entry that was not applied, first crossing entry
     __shared__ unsigned int s_before[kExactListCap + 1];  // bit pattern of the sum before every staged entry
     // inclusive prefix of the counts: thread t owns block t
     int c = (tid < n_blocks) ? __ldcg(counts + tid) : 0;
@@ -399,10 +462,7 @@ static __device__ __noinline__ void walk_all(const ExactEntry* entries, const in
     if (tid == 0) {
         out->s = 0.f;
         out->found = -1;
-        out->run_lo = -1;
-        out->run_hi = out->run_e = 0;
-        out->run_s0 = 0.f;
-        s_done = 0;
+        out->resolved = 0;
         s_pref[0] = 0;
     }
     __syncthreads();
@@ -430,87 +490,62 @@ static __device__ __noinline__ void walk_all(const ExactEntry* entries, const in
             dst[1] = v1;
         }
         __syncthreads();
-        // pass 1 (warp 0, every lane the same): apply the entries speculatively without a branch, keeping the
-        // sum before every entry; the first entry whose prediction fails (or that needs the one-by-one path)
-        // is remembered
-        if (tid < 32) {
-            unsigned int bits = __float_as_uint(out->s);
-            int bad = 0x7fffffff;
-#pragma unroll 4
-            for (int i = 0; i < m; ++i) {
-                const int4 h = *reinterpret_cast<const int4*>(&s_list[i]);  // kind, lo, hi, e
-                const ulonglong2 d = *reinterpret_cast<const ulonglong2*>(&s_list[i].d0);
-                s_before[i] = bits;
-                // as a map
-                const unsigned int ebase = (unsigned int)(h.w + 127) << 23;
-                const unsigned long long dd = (bits & 1u) ? d.y : d.x;
-                const unsigned int nb = bits + (unsigned int)dd;
-                const bool map_ok = bits - ebase < 0x800000u && dd <= 0x800000ull && nb - ebase <= 0x800000u;
-                // as four values
-                float q = __uint_as_float(bits);
-                q = __fadd_rn(q, __uint_as_float((unsigned int)d.x));
-                q = __fadd_rn(q, __uint_as_float((unsigned int)(d.x >> 32)));
-                q = __fadd_rn(q, __uint_as_float((unsigned int)d.y));
-                q = __fadd_rn(q, __uint_as_float((unsigned int)(d.y >> 32)));
-                const bool is_map = h.x == kEntryMap;
-                const bool fine = is_map ? map_ok : (h.x == kEntryQuad);
-                bad = (!fine && bad == 0x7fffffff) ? i : bad;
-                bits = is_map ? nb : __float_as_uint(q);
-            }
-            s_before[m] = bits;
-            if (lane == 0) {
-                s_ctl[0] = bad;
-                s_ctl[1] = 0x7fffffff;
-            }
-        }
-        __syncthreads();
-        const int bad = s_ctl[0];
-        const int good = min(m, bad);  // entries [0, good) were applied exactly
-        // pass 2: the first entry after which the running sum exceeds r (sums never decrease)
-        if (stop) {
-            for (int i = tid; i < good; i += kSampleThreads)
-                if (r < __uint_as_float(s_before[i + 1])) atomicMin(&s_ctl[1], i);
-            __syncthreads();
-        }
-        const int cross = stop ? s_ctl[1] : 0x7fffffff;
-        if (cross < good) {
-            if (tid == 0) {
-                const ExactEntry e = s_list[cross];
-                float sum = __uint_as_float(s_before[cross]);
-                if (e.kind == kEntryQuad) {
-                    const float v[4] = {__uint_as_float((unsigned int)e.d0), __uint_as_float((unsigned int)(e.d0 >> 32)),
-                                        __uint_as_float((unsigned int)e.d1), __uint_as_float((unsigned int)(e.d1 >> 32))};
-                    int j = 0;
-                    for (; j < 3; ++j) {
-                        sum = __fadd_rn(sum, v[j]);
-                        if (r < sum) break;
-                    }
-                    out->found = e.lo + j;
-                } else {  // inside a map run: the caller redoes the run element by element
-                    out->run_lo = e.lo;
-                    out->run_hi = min(e.hi, n_total);
-                    out->run_e = e.e;
-                    out->run_s0 = sum;
-                }
-                out->s = sum;
-                s_done = 1;
-            }
-        } else if (bad < m) {
-            // a prediction failed: warp 0 goes on from that entry with the checked walk
+        for (int i0 = 0; i0 < m;) {
+            // pass 1 (warp 0, every lane the same): apply the entries from i0 on speculatively without a branch, keeping
+            // the sum before every entry; the first entry whose map does not hold is remembered.  A map moves the sum by
+            // an integer number of ulps inside one binade (or exactly onto the next power of two), which on the bit
+            // pattern of a positive float is a plain integer addition.
             if (tid < 32) {
-                WalkState w = *out;
-                w.s = __uint_as_float(s_before[bad]);
-                const bool done = walk_list(s_list + bad, m - bad, x, n_total, stop, r, lane, w);
+                unsigned int bits = __float_as_uint(out->s);
+                int bad = 0x7fffffff;
+#pragma unroll 4
+                for (int i = i0; i < m; ++i) {
+                    const int4 h = *reinterpret_cast<const int4*>(&s_list[i]);  // kind, lo, hi, e
+                    const uint4 d = *reinterpret_cast<const uint4*>(s_list[i].d);
+                    s_before[i] = bits;
+                    // as a map: of binade e, or of the next one when the sum of a dual entry is there
+                    const unsigned int ebase = (unsigned int)(h.w + 127) << 23;
+                    const bool next = h.x == kEntryDual && bits - ebase >= 0x800000u;
+                    const unsigned int from = next ? ebase + 0x800000u : ebase;
+                    const unsigned int dd = next ? ((bits & 1u) ? d.w : d.z) : ((bits & 1u) ? d.y : d.x);
+                    const unsigned int nb = bits + dd;
+                    const bool map_ok = bits - from < 0x800000u && dd <= 0x800000u && nb - from <= 0x800000u;
+                    // as four values
+                    float q = __uint_as_float(bits);
+                    q = __fadd_rn(q, __uint_as_float(d.x));
+                    q = __fadd_rn(q, __uint_as_float(d.y));
+                    q = __fadd_rn(q, __uint_as_float(d.z));
+                    q = __fadd_rn(q, __uint_as_float(d.w));
+                    const bool is_quad = h.x == kEntryQuad;
+                    const bool fine = is_quad || (h.x != kEntrySeq && map_ok);
+                    bad = (!fine && bad == 0x7fffffff) ? i : bad;
+                    bits = is_quad ? __float_as_uint(q) : nb;
+                }
+                s_before[m] = bits;
                 if (lane == 0) {
-                    *out = w;
-                    if (done) s_done = 1;
+                    s_ctl[0] = bad;
+                    s_ctl[1] = 0x7fffffff;
                 }
             }
-        } else if (tid == 0) {
-            out->s = __uint_as_float(s_before[m]);
+            __syncthreads();
+            const int good = min(m, s_ctl[0]);  // entries [i0, good) were applied exactly
+            // pass 2: the first entry after which the running sum exceeds r (sums never decrease)
+            if (stop) {
+                for (int i = i0 + tid; i < good; i += kSampleThreads)
+                    if (r < __uint_as_float(s_before[i + 1])) atomicMin(&s_ctl[1], i);
+                __syncthreads();
+            }
+            const int redo = stop ? min(s_ctl[1], good) : good;  // entry to look at element by element, m = none
+            if (tid == 0) {
+                out->s = __uint_as_float(s_before[redo]);
+                if (redo == good && good < m) ++out->resolved;
+            }
+            __syncthreads();
+            if (redo == m) break;
+            resolve_range(x, s_list[redo].lo, min(s_list[redo].hi, n_total), stop, r, out, z, s_wm, s_wf, tid);
+            if (out->found >= 0 || !(out->s < INFINITY)) return;
+            i0 = redo + 1;
         }
-        __syncthreads();
-        if (s_done) break;
     }
 }
 
@@ -523,16 +558,16 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_exact_kernel(con
     __shared__ int s_wf[kSampleThreads / 32];
     __shared__ int s_i[kSampleThreads / 32];
     __shared__ int s_flag;
-    __shared__ int s_found;
     __shared__ __align__(16) ExactEntry s_list[kExactListCap];
     __shared__ int s_pref[kSampleThreads + 1];
     __shared__ WalkState s_walk;
+    __shared__ ResolveScratch s_res;
     __shared__ int s_hist[kHistoryMax];
 
     pdl_launch_dependents();
     pdl_wait();
     StepState* st = a.st;
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int tid = threadIdx.x;
     const int nb = gridDim.x;
     const int base = blockIdx.x * kSampleChunk;
     const int n = min(kSampleChunk, a.vocab - base);
@@ -614,18 +649,17 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_exact_kernel(con
         }
         alive = alive && sampler_grid_barrier(&ea.sync[0], ++bar * nb, st, &s_flag, tid);
 
-        // ---- stage 3: block 0, warp 0 walks the entries: the exact softmax denominator
-        if (alive && blockIdx.x == 0) {
-            walk_all(ea.entries, ea.entry_count, nb, a.logits, a.vocab, false, 0.f, s_list, s_pref, s_i, &s_walk, tid);
-            if (tid == 0) {
-                __stcg(ea.scalars, s_walk.s);
-                __threadfence();
-            }
+        // ---- stage 3: every block walks the entries itself: the exact softmax denominator (handing it out from one block
+        // would cost another grid barrier).  Runs that were done over read the e of other blocks, which these replace below:
+        // all blocks have come to the same end and wait for each other then.
+        float denom = 1.f;
+        if (alive) {
+            walk_all(ea.entries, ea.entry_count, nb, a.logits, a.vocab, false, 0.f, s_list, s_pref, s_i, s_wm, s_wf, &s_res, &s_walk, tid);
+            denom = s_walk.s;
+            if (s_walk.resolved > 0) alive = sampler_grid_barrier(&ea.sync[0], ++bar * nb, st, &s_flag, tid);
         }
-        alive = alive && sampler_grid_barrier(&ea.sync[0], ++bar * nb, st, &s_flag, tid);
 
         // ---- stage 4: p = e / sum (IEEE division), entry list of the running CDF
-        const float denom = __ldcg(ea.scalars);
         double locp = 0.0;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -637,9 +671,10 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_exact_kernel(con
         const double inclp = block_scan_double(locp, s_d, tid);
         // approximate prefix of p before this block = (approximate prefix of e) / denominator
         const double pre_p = before_blocks / (double)denom + (inclp - locp);
+        ExactEntry* cdf_entries = ea.entries + (size_t)nb * kExactMaxEntries;  // other blocks may still walk the first list
+        int* cdf_count = ea.entry_count + nb;
         if (alive) {
-            emit_entries(x, pre_p, base, n_quads, ea.entries + (size_t)blockIdx.x * kExactMaxEntries,
-                         ea.entry_count + blockIdx.x, s_wm, s_wf, s_i, tid);
+            emit_entries(x, pre_p, base, n_quads, cdf_entries + (size_t)blockIdx.x * kExactMaxEntries, cdf_count + blockIdx.x, s_wm, s_wf, s_i, tid);
             __threadfence();
         }
         alive = alive && sampler_grid_barrier(&ea.sync[0], ++bar * nb, st, &s_flag, tid);
@@ -647,46 +682,8 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_exact_kernel(con
         // ---- stage 5: block 0 finds the first index whose running sum exceeds r
         if (alive && blockIdx.x == 0) {
             const float r = st->advance ? a.r_values[st->step_idx] : st->r;
-            walk_all(ea.entries, ea.entry_count, nb, a.logits, a.vocab, true, r, s_list, s_pref, s_i, &s_walk, tid);
-            if (tid == 0) s_found = (s_walk.found >= 0) ? s_walk.found : 0x7fffffff;
-            __syncthreads();
-            const int run_lo = s_walk.run_lo, run_hi = s_walk.run_hi, E = s_walk.run_e;
-            if (run_lo >= 0) {
-                // the crossing lies inside a map run (<= 2048 elements, quads aligned): redo the run's scan
-                // with the exact starting sum and look at every element
-                const float s0 = s_walk.run_s0;
-                const unsigned int b0 = __float_as_uint(s0);
-                const unsigned long long S0 = (b0 & 0x7fffffu) | 0x800000u;
-                float y[4];
-                Map2 mp = map_identity();
-                const int q = run_lo + 4 * tid;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    y[k] = (q + k < run_hi) ? __ldcg(a.logits + q + k) : 0.f;
-                    mp = map_compose(mp, map_of(y[k], E));
-                }
-                const Map2 incl_m = block_segscan(mp, tid == 0, s_wm, s_wf, tid);
-                // exclusive prefix for this thread: shift by one thread
-                Map2 ex;
-                ex.d0 = __shfl_up_sync(0xffffffffu, incl_m.d0, 1);
-                ex.d1 = __shfl_up_sync(0xffffffffu, incl_m.d1, 1);
-                __shared__ Map2 s_last_map[kSampleThreads / 32];
-                if (lane == 31) s_last_map[tid >> 5] = incl_m;
-                __syncthreads();
-                if (lane == 0) ex = (tid == 0) ? map_identity() : s_last_map[(tid >> 5) - 1];
-                unsigned long long S = S0 + ((S0 & 1ull) ? ex.d1 : ex.d0);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const Map2 m1 = map_of(y[k], E);
-                    S += (S & 1ull) ? m1.d1 : m1.d0;
-                    const float cum = (S >= (1ull << 24))
-                                          ? __uint_as_float((unsigned int)(E + 128) << 23)
-                                          : __uint_as_float(((unsigned int)(E + 127) << 23) | ((unsigned int)S & 0x7fffffu));
-                    if (q + k < run_hi && r < cum) atomicMin(&s_found, q + k);
-                }
-                __syncthreads();
-            }
-            token = (s_found != 0x7fffffff) ? s_found : a.vocab - 1;
+            walk_all(cdf_entries, cdf_count, nb, a.logits, a.vocab, true, r, s_list, s_pref, s_i, s_wm, s_wf, &s_res, &s_walk, tid);
+            token = (s_walk.found >= 0) ? s_walk.found : a.vocab - 1;
         }
     }
 
