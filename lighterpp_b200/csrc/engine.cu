@@ -39,6 +39,7 @@
 #include "mamba.cuh"
 #include "ops.cuh"
 #include "prefill.cuh"
+#include "prefill_pair.cuh"
 #include "prefill_mixers.cuh"
 #include "sampler.cuh"
 #include "sampler_exact.cuh"
@@ -132,6 +133,10 @@ static bool load() {
 
 enum Kind { kQkv = 0, kAttn = 1, kOproj = 2, kGateUp = 3, kDown = 4, kLmHead = 5, kSampler = 6, kAllReduce = 7, kLatQuery = 8, kLatValue = 9, kScanIn = 10, kScan = 11, kKinds = 12 };
 
+// A matrix of the batched prompt path as the CTA kernel and as the pair kernel read it.
+struct PrefillMap {
+    CUtensorMap cta, pair;
+};
 // One layer of an engine described layer by layer.  Weight matrices: rows x pitch, pitch = inputs rounded up to 64, zero
 // padded; element type = weight_dtype.
 struct ModelLayer {
@@ -140,7 +145,7 @@ struct ModelLayer {
     int o_in, o_pitch, ff_pitch;  // inputs of the output projection, and of it and the down projection with padding
     void *w_in = nullptr, *wo = nullptr, *w13 = nullptr, *w2 = nullptr;
     float *n1w = nullptr, *n1b = nullptr, *n2w = nullptr, *n2b = nullptr, *o_b = nullptr;
-    CUtensorMap m_in, m_wo, m_w13, m_w2, x_att, x_hb;   // weights, activation blocks with this layer's widths (batched path)
+    PrefillMap m_in, m_wo, m_w13, m_w2, x_att, x_hb;    // weights, activation blocks with this layer's widths (batched path)
     // attention over shared rows (latent_attention.cuh): heads of a group, groups, value part and whole of a row
     int group_heads = 0, groups = 0, rank_pitch = 0, row_width = 0;
     const float2* rope = nullptr;
@@ -150,7 +155,7 @@ struct ModelLayer {
     int q_plain_rows, q_rot_rows, latent_rows;
     void *w_uk = nullptr, *w_uv = nullptr;
     float* lat_w = nullptr;
-    CUtensorMap m_uk, m_uv, x_qn, x_olat;
+    PrefillMap m_uk, m_uv, x_qn, x_olat;
     // attention whose values are its keys (shared_kv.cuh)
     int head_rows, q_rows, k_rows;
     float* qk_b = nullptr;
@@ -158,7 +163,7 @@ struct ModelLayer {
     int inner_rows, inner_pitch, low_rows, dt_pitch, state_pitch;
     void *w_low = nullptr, *w_dt = nullptr;
     float *conv_w = nullptr, *conv_b = nullptr, *dt_b = nullptr, *A = nullptr, *skip = nullptr;
-    CUtensorMap m_low, x_low;
+    PrefillMap m_low, x_low;
 };
 // A layer in its place in the order of execution, with what it keeps of the sequence.
 struct LayerRun {
@@ -241,20 +246,21 @@ struct lpp_engine {
     // graph variants by context length; only [0] is used at present
     cudaGraphExec_t g_full[2] = {nullptr, nullptr}, g_logits[2] = {nullptr, nullptr};
 
-    // batched prompt path (allocated by the first lpp_prefill)
+    // batched prompt path: one allocation for blocks of up to pf_cap tokens, made by the first call that needs them
+    void* pf_slab = nullptr;
+    int pf_cap = 0, pf_limit = kPfMaxTokens;  // the latter: largest block there was memory for
     float *pf_x = nullptr, *pf_q = nullptr, *pf_part = nullptr;
     void *pf_xn = nullptr, *pf_att = nullptr, *pf_hb = nullptr;
     int *pf_tokens = nullptr, *pf_rows = nullptr;
     float* pf_logits = nullptr;
-    CUtensorMap pf_map_cls;
+    PrefillMap pf_map_cls;
     void *pf_qn = nullptr, *pf_olat = nullptr;      // latent attention: plain queries, attended latents (hi + lo operands)
     __half* pf_lq = nullptr;                        // query rows
     float *pf_lpart = nullptr, *pf_gate = nullptr;  // attention partials, gates
     float *pf_sx = nullptr, *pf_sz = nullptr, *pf_tail = nullptr;  // selective scan: convolved x, z, last convolution inputs
     float* pf_low = nullptr;                                       // dt | B | C rows
     void* pf_sxp = nullptr;                                        // x as hi + lo operands
-    CUtensorMap pf_map_wqkv, pf_map_wo, pf_map_w13, pf_map_w2, pf_map_xn, pf_map_att, pf_map_hb;
-    bool pf_ready = false;
+    PrefillMap pf_map_wqkv, pf_map_wo, pf_map_w13, pf_map_w2, pf_map_xn, pf_map_att, pf_map_hb;
 
     bool finalized = false;
     int kernels_full = 0;
@@ -682,7 +688,7 @@ static cudaError_t launch_mamba_step(const MambaScanArgs& a, bool pdl, cudaStrea
 }
 template <int L, int NS>
 static cudaError_t launch_mamba_scan_t(const lpp_engine* e, MambaScanArgs a, cudaStream_t s) {
-    a.tile_tokens = kPrefillTokens;
+    a.tile_tokens = kPfTile;
     while (a.tile_tokens > 4 && (size_t)mamba_scan_smem<L>(a.dt_pitch, a.state_pitch, a.tile_tokens) > e->smem_optin) a.tile_tokens /= 2;
     const size_t smem = (size_t)mamba_scan_smem<L>(a.dt_pitch, a.state_pitch, a.tile_tokens);
     const cudaError_t r = cudaFuncSetAttribute(mamba_scan_kernel<L, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem_optin);
@@ -1808,10 +1814,8 @@ extern "C" lpp_status lpp_engine_destroy(lpp_engine* e) {
     void* bufs[] = {e->wqkv, e->wo, e->w13, e->w2, e->emb, e->wcls_owned ? e->wcls : nullptr, e->rms_att, e->rms_ffn,
                     e->rms_final, e->kcache, e->vcache, e->xa, e->xb, e->q, e->att_out, e->hb, e->logits,
                     e->attn_part, e->attn_counters, e->samp_max, e->samp_sum, e->samp_idx, e->samp_counter,
-                    e->r_values, e->out_tokens, e->st, e->rope, e->stage, e->gtrace, e->pf_x, e->pf_q, e->pf_part, e->pf_xn, e->pf_att, e->pf_hb,
-                    e->pf_tokens, e->ex_sync, e->ex_block_sum, e->ex_entry_count, e->ex_entries, e->final_b, e->lat_qplain,
-                    e->lat_raw, e->lat_gate, e->lat_query, e->lat_part, e->pf_rows, e->pf_logits, e->pf_qn, e->pf_olat, e->pf_lq,
-                    e->pf_lpart, e->pf_gate, e->loop_vec, e->scan_x, e->scan_z, e->scan_low, e->row_counters, e->pf_sx, e->pf_sz, e->pf_tail, e->pf_sxp, e->pf_low};
+                    e->r_values, e->out_tokens, e->st, e->rope, e->stage, e->gtrace, e->pf_slab, e->ex_sync, e->ex_block_sum, e->ex_entry_count, e->ex_entries, e->final_b, e->lat_qplain,
+                    e->lat_raw, e->lat_gate, e->lat_query, e->lat_part, e->pf_logits, e->loop_vec, e->scan_x, e->scan_z, e->scan_low, e->row_counters};
     for (void* p : bufs)
         if (p) cudaFree(p);
     for (const ModelLayer& y : e->layers)
@@ -2333,14 +2337,14 @@ static encode_tiled_fn tensor_map_encoder() {
 // the 128-byte swizzle: the K-major operand layout of the MMA descriptors).  cols must be a multiple of 64; elements
 // outside the matrix read as zero.
 //
-// Weights [rows][cols] seen as (64 inputs, rows, cols / 64): a box is 64 inputs x box_rows rows x 2 pieces, i.e. one
-// copy delivers both 64-input sub-tiles of a stage, sub-tile after sub-tile.
-static lpp_status make_weight_map(CUtensorMap* m, const void* base, size_t rows, size_t cols, int box_rows) {
+// Weights [rows][cols] seen as (64 inputs, rows, cols / 64): a box is 64 inputs x box_rows rows x `pieces` pieces,
+// i.e. one copy delivers the 64-input sub-tiles of a stage, sub-tile after sub-tile.
+static lpp_status encode_weight_map(CUtensorMap* m, const void* base, size_t rows, size_t cols, int box_rows, int pieces) {
     encode_tiled_fn encode = tensor_map_encoder();
     if (!encode) return fail(LPP_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     const cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)};
     const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, 128};
-    const cuuint32_t box[3] = {64u, (cuuint32_t)box_rows, 2u};
+    const cuuint32_t box[3] = {64u, (cuuint32_t)box_rows, (cuuint32_t)pieces};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -2348,21 +2352,33 @@ static lpp_status make_weight_map(CUtensorMap* m, const void* base, size_t rows,
     if (r != CUDA_SUCCESS) return fail(LPP_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for a %zu x %zu matrix", (int)r, rows, cols);
     return LPP_OK;
 }
-// Activations: hi plane [tokens][cols] followed by the lo plane, seen as (64 inputs, tokens, 2 planes, cols / 64): a
-// box is 64 inputs x box_tokens x 2 planes x 2 pieces, i.e. one copy delivers, per 64-input piece, the hi rows
-// followed by the lo rows: one K-major operand tile of 2 x box_tokens rows (the MMA's N) per piece.
-static lpp_status make_activation_map(CUtensorMap* m, const void* base, size_t tokens, size_t cols, int box_tokens) {
+// The CTA kernel takes two pieces of 128 rows at a time, the pair kernel one.
+static lpp_status make_weight_map(PrefillMap* m, const void* base, size_t rows, size_t cols) {
+    TRY(encode_weight_map(&m->cta, base, rows, cols, kUmmaM, 2));
+    return encode_weight_map(&m->pair, base, rows, cols, kPairM / 2, 1);
+}
+// Activations: hi plane [tokens][cols] followed by the lo plane, seen as (64 inputs, tokens, 2 planes, cols / 64).  CTA
+// kernel: a box is 64 inputs x 64 tokens x 2 planes x 2 pieces, i.e. one copy delivers, per 64-input piece, the hi rows
+// followed by the lo rows: one K-major operand tile of 128 rows (the MMA's N) per piece.  Pair kernel: 64 inputs x 128
+// tokens of one plane.
+static lpp_status encode_activation_map(CUtensorMap* m, const void* base, size_t tokens, size_t cols, int box_tokens, int planes, int pieces) {
     encode_tiled_fn encode = tensor_map_encoder();
     if (!encode) return fail(LPP_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     const cuuint64_t dims[4] = {64, (cuuint64_t)tokens, 2, (cuuint64_t)(cols / 64)};
     const cuuint64_t strides[3] = {(cuuint64_t)cols * 2, (cuuint64_t)tokens * cols * 2, 128};
-    const cuuint32_t box[4] = {64u, (cuuint32_t)box_tokens, 2u, 2u};
+    const cuuint32_t box[4] = {64u, (cuuint32_t)box_tokens, (cuuint32_t)planes, (cuuint32_t)pieces};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(LPP_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for a %zu x %zu activation block", (int)r, tokens, cols);
     return LPP_OK;
+}
+
+static lpp_status make_activation_map(PrefillMap* m, const void* base, size_t tokens, size_t cols) {
+    TRY(encode_activation_map(&m->cta, base, tokens, cols, kPfTile, 2, 2));
+    if (tokens < 128) return LPP_OK;  // blocks of one tile: the CTA kernel's
+    return encode_activation_map(&m->pair, base, tokens, cols, 128, 1, 1);
 }
 
 // The tensor-core path takes 16-bit weights, an FP16 cache and a single GPU; everything else is fed token by token.
@@ -2373,29 +2389,87 @@ static bool prefill_batched(const lpp_engine* e) {
            e->c.dim % 64 == 0 && e->Dq % 64 == 0 && e->Fl % 64 == 0;
 }
 
+template <typename T, int EPI>
+static lpp_status allow_pair_smem() {
+    CU(cudaFuncSetAttribute(prefill_gemm_pair_kernel<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));
+    return LPP_OK;
+}
 template <typename T>
 static lpp_status allow_gemm_smem() {
     CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<T, kPfResid>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
     CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<T, kPfSwiglu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
     CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<T, kPfStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
-    return LPP_OK;
+    TRY((allow_pair_smem<T, kPfResid>()));
+    TRY((allow_pair_smem<T, kPfSwiglu>()));
+    return allow_pair_smem<T, kPfStore>();
 }
 
-static lpp_status prefill_setup(lpp_engine* e) {
-    if (e->pf_ready) return LPP_OK;
-    const lpp_config& c = e->c;
-    const size_t D = e->Dp, L = c.n_layers, T = kPrefillTokens;
+// How a GEMM of n tokens is cut: tokens per item (64: prefill_gemm_umma_kernel, 128: prefill_gemm_pair_kernel) and ranges
+// of K.  Up to 64 tokens, and for grouped weights (whose matrices are few rows each), the CTA kernel; its row tiles (128
+// weight rows) are cut along K as often as fills the GPU.  Else the cheapest of the pair kernel's cuts by a model of its
+// time: waves of items over the SM pairs, each item 64 inputs at a time (0.45 us measured) plus a fixed part, plus the
+// traffic of partial sums through L2.
+struct PrefillPlan {
+    int tile, splits;
+};
+static PrefillPlan prefill_plan(const lpp_engine* e, int n_rows, int K, int n, int groups, int max_splits) {
+    if (n <= kPfTile || groups > 0) {
+        const int tiles = (n_rows + kUmmaM - 1) / kUmmaM * std::max(1, groups) * ((n + kPfTile - 1) / kPfTile), n_kc = (K + kPfKc - 1) / kPfKc;
+        return {kPfTile, tiles < e->num_sms ? std::max(1, std::min({max_splits, n_kc, (e->num_sms + tiles - 1) / tiles})) : 1};
+    }
+    const int row_tiles = (n_rows + kPairM - 1) / kPairM, n_kc = K / 64, units = std::max(1, e->num_sms / 2);
+    PrefillPlan best = {kPairTokens, 1};
+    double least = 0;
+    for (int s = 1; s <= std::min(max_splits, n_kc); ++s) {
+        const int items = row_tiles * ((n + kPairTokens - 1) / kPairTokens) * s, waves = (items + units - 1) / units;
+        const double us = waves * ((n_kc + s - 1) / s * 0.45 + 1.5) + (s > 1 ? s * (double)n * n_rows * 8 / 5e6 : 0.0);
+        if (s == 1 || us < least) best.splits = s, least = us;
+    }
+    return best;
+}
+// Token rows that one range of K takes in the partial sums of a block of n tokens.
+static int prefill_part_tokens(int n) { return (int)align_up((size_t)n, kPfTile); }
+
+// Hands out the parts of one allocation; without a base it only counts.
+struct SlabCarver {
+    char* base;
+    size_t used = 0;
+    template <typename T>
+    void take(T** p, size_t bytes) {
+        if (base) *p = reinterpret_cast<T*>(base + used);
+        used += align_up(std::max<size_t>(bytes, 16), 256);
+    }
+};
+// The workspace of blocks of up to `cap` tokens: its size, and with a base its parts.
+static size_t prefill_carve(lpp_engine* e, int cap, char* base) {
+    const size_t D = e->Dp, T = cap;
     const bool layered = !e->layers.empty();
-    size_t part_rows = D, att_n = e->Dq, hb_n = e->Fl, qn_n = 0, olat_n = 0, lq_n = 0, lpart_n = 0, gate_n = 0, scan_n = 0, tail_n = 0, low_n = 0;
-    const size_t qkv_rows = layered ? 0 : e->Dq + 2 * (size_t)e->KVd;
-    part_rows = std::max(part_rows, qkv_rows);
+    size_t part_n = 0, att_n = e->Dq, hb_n = e->Fl, qn_n = 0, olat_n = 0, lq_n = 0, lpart_n = 0, gate_n = 0, scan_n = 0, tail_n = 0, low_n = 0;
+    std::vector<std::pair<std::pair<int, int>, int>> seen;
+    auto partial_sums = [&](int n_rows, int K, int max_splits) {
+        if (std::find(seen.begin(), seen.end(), std::make_pair(std::make_pair(n_rows, K), max_splits)) != seen.end()) return;
+        seen.push_back({{n_rows, K}, max_splits});
+        for (int n = kPfTile; n <= cap; n += kPfTile)  // the plan depends on the number of tiles: their last tokens stand for all
+            for (int m : {n - kPfTile + 1, n})
+                part_n = std::max(part_n, (size_t)prefill_plan(e, n_rows, K, m, 0, max_splits).splits * prefill_part_tokens(m) * n_rows);
+    };
+    if (!layered) {
+        partial_sums(e->Dq + 2 * e->KVd, e->c.dim, kPfMaxSplits);
+        partial_sums((int)D, e->Dq, kPfMaxSplits);
+        partial_sums((int)D, e->Fl, kPfMaxSplits);
+    }
+    const ModelLayer* last = nullptr;
     for (const ModelLayer& y : e->layers) {
         const size_t H = y.d.heads;
-        part_rows = std::max(part_rows, (size_t)y.in_rows);
+        if (last && memcmp(&last->d, &y.d, sizeof(y.d)) == 0) continue;
+        last = &y;
+        partial_sums(y.in_rows, (int)D, kPfMaxSplits);
+        partial_sums((int)D, y.o_pitch, kPfMaxSplits);
+        if (y.d.ff > 0) partial_sums((int)D, y.ff_pitch, kPfMaxSplits);
         att_n = std::max(att_n, (size_t)y.o_pitch);
         hb_n = std::max(hb_n, (size_t)y.ff_pitch);
         if (y.d.mixer == LPP_MIXER_MAMBA) {
-            part_rows = std::max(part_rows, (size_t)y.low_rows * kLowMaxSplits / kPfMaxSplits);
+            partial_sums(y.low_rows, y.inner_pitch, kLowMaxSplits);
             low_n = std::max(low_n, (size_t)mamba_low_pitch(y.dt_pitch, y.state_pitch));
             scan_n = std::max(scan_n, (size_t)y.inner_pitch);
             tail_n = std::max(tail_n, (size_t)(y.d.conv - 1) * y.inner_rows);
@@ -2412,100 +2486,146 @@ static lpp_status prefill_setup(lpp_engine* e) {
         }
         gate_n = std::max(gate_n, y.d.mixer == LPP_MIXER_LATENT ? H : H * y.d.dim);
     }
-    TRY(zeroed(e, &e->pf_x, T * D * 4));
-    TRY(zeroed(e, &e->pf_xn, 2 * T * D * 2));      // hi plane, lo plane
-    TRY(zeroed(e, &e->pf_att, 2 * T * att_n * 2));  // hi plane, lo plane
-    TRY(zeroed(e, &e->pf_hb, 2 * T * hb_n * 2));    // hi plane, lo plane
-    TRY(zeroed(e, &e->pf_part, (size_t)kPfMaxSplits * T * part_rows * 4));
-    TRY(zeroed(e, &e->pf_tokens, T * sizeof(int)));
-    TRY(zeroed(e, &e->pf_rows, T * sizeof(int)));
+    SlabCarver c = {base};
+    c.take(&e->pf_x, T * D * 4);
+    c.take(&e->pf_xn, 2 * T * D * 2);      // hi plane, lo plane
+    c.take(&e->pf_att, 2 * T * att_n * 2);
+    c.take(&e->pf_hb, 2 * T * hb_n * 2);
+    c.take(&e->pf_part, part_n * 4);
+    c.take(&e->pf_tokens, T * sizeof(int));
+    c.take(&e->pf_rows, T * sizeof(int));
     if (layered) {
-        TRY(zeroed(e, &e->pf_qn, 2 * T * qn_n * 2));
-        TRY(zeroed(e, &e->pf_olat, 2 * T * olat_n * 2));
-        TRY(zeroed(e, &e->pf_lq, T * lq_n * 2));
-        TRY(zeroed(e, &e->pf_lpart, lpart_n * 4));
-        TRY(zeroed(e, &e->pf_gate, T * gate_n * 4));
-        TRY(zeroed(e, &e->pf_sx, T * scan_n * 4));
-        TRY(zeroed(e, &e->pf_sz, T * scan_n * 4));
-        TRY(zeroed(e, &e->pf_sxp, 2 * T * scan_n * 2));
-        TRY(zeroed(e, &e->pf_tail, tail_n * 4));
-        TRY(zeroed(e, &e->pf_low, T * low_n * 4));
+        c.take(&e->pf_qn, 2 * T * qn_n * 2);
+        c.take(&e->pf_olat, 2 * T * olat_n * 2);
+        c.take(&e->pf_lq, T * lq_n * 2);
+        c.take(&e->pf_lpart, lpart_n * 4);
+        c.take(&e->pf_gate, T * gate_n * 4);
+        c.take(&e->pf_sx, T * scan_n * 4);
+        c.take(&e->pf_sz, T * scan_n * 4);
+        c.take(&e->pf_sxp, 2 * T * scan_n * 2);
+        c.take(&e->pf_tail, tail_n * 4);
+        c.take(&e->pf_low, T * low_n * 4);
+    } else {
+        c.take(&e->pf_q, T * e->Dq * 4);
+    }
+    return c.used;
+}
+static lpp_status prefill_maps(lpp_engine* e) {
+    const lpp_config& c = e->c;
+    const size_t D = e->Dp, L = c.n_layers, T = e->pf_cap;
+    if (!e->layers.empty()) {
         for (ModelLayer& y : e->layers) {
             const size_t H = y.d.heads, D2 = align_up(c.dim, 2);
-            TRY(make_weight_map(&y.m_in, y.w_in, y.in_rows, D, kUmmaM));
+            TRY(make_weight_map(&y.m_in, y.w_in, y.in_rows, D));
             if (y.d.mixer == LPP_MIXER_LATENT) {
-                TRY(make_weight_map(&y.m_uk, y.w_uk, H * y.rank_pitch, y.dim_pitch, kUmmaM));
-                TRY(make_weight_map(&y.m_uv, y.w_uv, H * y.vdim_rows, y.val_pitch, kUmmaM));
-                TRY(make_activation_map(&y.x_qn, e->pf_qn, T, H * y.dim_pitch, kPrefillTokens));
-                TRY(make_activation_map(&y.x_olat, e->pf_olat, T, H * y.val_pitch, kPrefillTokens));
+                TRY(make_weight_map(&y.m_uk, y.w_uk, H * y.rank_pitch, y.dim_pitch));
+                TRY(make_weight_map(&y.m_uv, y.w_uv, H * y.vdim_rows, y.val_pitch));
+                TRY(make_activation_map(&y.x_qn, e->pf_qn, T, H * y.dim_pitch));
+                TRY(make_activation_map(&y.x_olat, e->pf_olat, T, H * y.val_pitch));
             } else if (y.d.mixer == LPP_MIXER_MAMBA) {
-                TRY(make_weight_map(&y.m_low, y.w_low, y.low_rows, y.inner_pitch, kUmmaM));
-                TRY(make_activation_map(&y.x_low, e->pf_sxp, T, y.inner_pitch, kPrefillTokens));
+                TRY(make_weight_map(&y.m_low, y.w_low, y.low_rows, y.inner_pitch));
+                TRY(make_activation_map(&y.x_low, e->pf_sxp, T, y.inner_pitch));
             }
-            TRY(make_weight_map(&y.m_wo, y.wo, D2, y.o_pitch, kUmmaM));
-            TRY(make_activation_map(&y.x_att, e->pf_att, T, y.o_pitch, kPrefillTokens));
+            TRY(make_weight_map(&y.m_wo, y.wo, D2, y.o_pitch));
+            TRY(make_activation_map(&y.x_att, e->pf_att, T, y.o_pitch));
             if (y.d.ff > 0) {
-                TRY(make_weight_map(&y.m_w13, y.w13, 2 * (size_t)y.d.ff, D, kUmmaM));
-                TRY(make_weight_map(&y.m_w2, y.w2, D2, y.ff_pitch, kUmmaM));
-                TRY(make_activation_map(&y.x_hb, e->pf_hb, T, y.ff_pitch, kPrefillTokens));
+                TRY(make_weight_map(&y.m_w13, y.w13, 2 * (size_t)y.d.ff, D));
+                TRY(make_weight_map(&y.m_w2, y.w2, D2, y.ff_pitch));
+                TRY(make_activation_map(&y.x_hb, e->pf_hb, T, y.ff_pitch));
             }
         }
         TRY(allow_gemm_smem<__nv_bfloat16>());
         CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<__nv_bfloat16, kPfLatentQuery>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
         CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<__nv_bfloat16, kPfLatentValue>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
     } else {
-        TRY(zeroed(e, &e->pf_q, T * e->Dq * 4));
-        TRY(make_weight_map(&e->pf_map_wqkv, e->wqkv, L * qkv_rows, D, kUmmaM));
-        TRY(make_weight_map(&e->pf_map_wo, e->wo, L * D, e->Dq, kUmmaM));
-        TRY(make_weight_map(&e->pf_map_w13, e->w13, L * 2 * e->Fl, D, kUmmaM));
-        TRY(make_weight_map(&e->pf_map_w2, e->w2, L * D, e->Fl, kUmmaM));
-        TRY(make_activation_map(&e->pf_map_att, e->pf_att, T, e->Dq, kPrefillTokens));
-        TRY(make_activation_map(&e->pf_map_hb, e->pf_hb, T, e->Fl, kPrefillTokens));
+        TRY(make_weight_map(&e->pf_map_wqkv, e->wqkv, L * (e->Dq + 2 * (size_t)e->KVd), D));
+        TRY(make_weight_map(&e->pf_map_wo, e->wo, L * D, e->Dq));
+        TRY(make_weight_map(&e->pf_map_w13, e->w13, L * 2 * e->Fl, D));
+        TRY(make_weight_map(&e->pf_map_w2, e->w2, L * D, e->Fl));
+        TRY(make_activation_map(&e->pf_map_att, e->pf_att, T, e->Dq));
+        TRY(make_activation_map(&e->pf_map_hb, e->pf_hb, T, e->Fl));
         TRY(allow_gemm_smem<__half>());
         CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<__half, kPfQkv>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
+        TRY((allow_pair_smem<__half, kPfQkv>()));
         CU(cudaFuncSetAttribute(prefill_attention_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_attn_smem<64>()));
         CU(cudaFuncSetAttribute(prefill_attention_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_attn_smem<128>()));
     }
-    TRY(make_activation_map(&e->pf_map_xn, e->pf_xn, T, D, kPrefillTokens));
-    TRY(make_weight_map(&e->pf_map_cls, e->wcls, e->Vp, D, kUmmaM));
-    e->pf_ready = true;
-    return LPP_OK;
+    TRY(make_activation_map(&e->pf_map_xn, e->pf_xn, T, D));
+    return make_weight_map(&e->pf_map_cls, e->wcls, e->Vp, D);
+}
+// Workspace for a portion of n tokens: room for one tile, or for the largest block that the cache has positions for.  Where
+// memory is short the blocks become smaller, down to one tile.
+static lpp_status prefill_setup(lpp_engine* e, int n) {
+    const int most = (int)std::min<size_t>(e->pf_limit, align_up((size_t)e->c.seq_len, kPfTile));
+    int cap = n <= kPfTile ? kPfTile : most;
+    if (e->pf_cap >= cap) return LPP_OK;
+    if (e->pf_slab) {
+        CU(cudaStreamSynchronize(e->stream));
+        CU(cudaFree(e->pf_slab));
+        e->pf_slab = nullptr;
+        e->pf_cap = 0;
+    }
+    size_t bytes = 0;
+    for (;; cap = std::max(kPfTile, cap / 2 / kPfTile * kPfTile)) {
+        bytes = prefill_carve(e, cap, nullptr);
+        const cudaError_t r = cudaMalloc(&e->pf_slab, bytes);
+        if (r == cudaSuccess) break;
+        e->pf_slab = nullptr;
+        if (r != cudaErrorMemoryAllocation || cap <= kPfTile) CU(r);
+        (void)cudaGetLastError();
+        e->pf_limit = std::max(kPfTile, cap / 2 / kPfTile * kPfTile);
+    }
+    CU(cudaMemsetAsync(e->pf_slab, 0, bytes, e->stream));
+    prefill_carve(e, cap, (char*)e->pf_slab);
+    e->pf_cap = cap;
+    const lpp_status st = prefill_maps(e);
+    if (st != LPP_OK) e->pf_cap = 0;
+    return st;
 }
 
-// Ranges of K a GEMM is cut into so that its row tiles (128 weight rows: the weight maps' box) fill the GPU.
-static int prefill_splits(const lpp_engine* e, int n_rows, int K, int max_splits = kPfMaxSplits) {
-    const int tiles = (n_rows + kUmmaM - 1) / kUmmaM, n_kc = (K + kPfKc - 1) / kPfKc;
-    return tiles < e->num_sms ? std::max(1, std::min({max_splits, n_kc, (e->num_sms + tiles - 1) / tiles})) : 1;
-}
-
-// A GEMM whose row tiles do not fill the GPU is also cut along K (a.splits); its partial sums go to pf_part and are added
-// up by the next prefill_norm_kernel (residual projections) or by a finishing kernel (input projections).
+// Partial sums of a GEMM that is cut along K go to pf_part and are added up by the next prefill_norm_kernel (residual
+// projections) or by a finishing kernel (input projections).
 template <typename T, int EPI>
-static cudaError_t launch_prefill_gemm_t(lpp_engine* e, const CUtensorMap& wm, const CUtensorMap& xm, const PrefillGemmArgs& a) {
-    const int tiles = (a.n_rows + kUmmaM - 1) / kUmmaM * std::max(1, a.groups);
-    return launch_kernel(prefill_gemm_umma_kernel<T, EPI>, dim3(std::min(tiles * a.splits, e->num_sms)), dim3(kUmmaThreads),
-                         (size_t)kPfSmemBytes, e->stream, true, wm, xm, a);
+static cudaError_t launch_prefill_gemm_t(lpp_engine* e, const PrefillMap& wm, const PrefillMap& xm, const PrefillGemmArgs& a) {
+    const int toks = (a.n_tokens + a.tile - 1) / a.tile;
+    if (a.tile == kPfTile) {
+        const int tiles = (a.n_rows + kUmmaM - 1) / kUmmaM * std::max(1, a.groups) * toks;
+        return launch_kernel(prefill_gemm_umma_kernel<T, EPI>, dim3(std::min(tiles * a.splits, e->num_sms)), dim3(kUmmaThreads), (size_t)kPfSmemBytes,
+                             e->stream, true, wm.cta, xm.cta, a);
+    }
+    if constexpr (EPI == kPfLatentQuery || EPI == kPfLatentValue) {
+        return cudaErrorInvalidValue;  // grouped weights: always the CTA kernel
+    } else {
+        const int items = (a.n_rows + kPairM - 1) / kPairM * toks * a.splits;
+        const dim3 grid(2 * std::min(items, std::max(1, e->num_sms / 2)));
+        return launch_clusters(prefill_gemm_pair_kernel<T, EPI>, grid, dim3(kUmmaThreads), (size_t)kPairSmemBytes, e->stream, true, 2, wm.pair, xm.pair, a);
+    }
 }
 template <int EPI>
-static cudaError_t launch_prefill_gemm(lpp_engine* e, const CUtensorMap& wm, const CUtensorMap& xm, const PrefillGemmArgs& a) {
+static cudaError_t launch_prefill_gemm(lpp_engine* e, const PrefillMap& wm, const PrefillMap& xm, const PrefillGemmArgs& a) {
     return e->c.weight_dtype == LPP_BF16 ? launch_prefill_gemm_t<__nv_bfloat16, EPI>(e, wm, xm, a)
                                          : launch_prefill_gemm_t<__half, EPI>(e, wm, xm, a);
 }
-static PrefillGemmArgs prefill_gemm_args(const lpp_engine* e, int n_rows, int K, int n_tokens, int start_pos) {
+static PrefillGemmArgs prefill_gemm_args(const lpp_engine* e, int n_rows, int K, int n_tokens, int start_pos, int max_splits = 1, int groups = 0) {
     PrefillGemmArgs a = {};
+    const PrefillPlan p = prefill_plan(e, n_rows, K, n_tokens, groups, max_splits);
+    a.tile = p.tile;
+    a.splits = p.splits;
+    a.groups = groups;
+    a.cap = e->pf_cap;
+    a.part_tokens = prefill_part_tokens(n_tokens);
     a.n_rows = n_rows;
     a.K = K;
     a.n_tokens = n_tokens;
     a.start_pos = start_pos;
-    a.splits = 1;
     a.part = e->pf_part;
     a.st = e->st;
     return a;
 }
 
-// x_rows -> normalised operands; `parts` > 1: the previous residual GEMM's partial sums are added to x first, and so is `add`
+// n rows of x (of a block of block_n tokens) -> normalised operands; `parts` > 1: the previous residual GEMM's partial sums are added to x first, and so is `add`
 // (nullptr = nothing).
-static lpp_status prefill_norm(lpp_engine* e, int n, const float* w, const float* b, bool embed, const float* add, int parts, const int* rows, bool pdl) {
+static lpp_status prefill_norm(lpp_engine* e, int n, int block_n, const float* w, const float* b, bool embed, const float* add, int parts, const int* rows, bool pdl) {
     PrefillNormArgs a = {};
     a.x = e->pf_x;
     a.tokens = e->pf_tokens;
@@ -2521,6 +2641,8 @@ static lpp_status prefill_norm(lpp_engine* e, int n, const float* w, const float
     a.out = e->pf_xn;
     a.D = e->Dp;
     a.part = e->pf_part;
+    a.cap = e->pf_cap;
+    a.part_tokens = prefill_part_tokens(block_n);
     a.splits = embed ? 1 : parts;
     a.st = e->st;
     if (e->c.weight_dtype == LPP_BF16)
@@ -2531,13 +2653,13 @@ static lpp_status prefill_norm(lpp_engine* e, int n, const float* w, const float
 }
 
 // x += W . in  for the block: output and down projection.  Returns the number of partial sums the next norm adds.
-static lpp_status prefill_resid(lpp_engine* e, const CUtensorMap& wm, int row0, const CUtensorMap& xm, int K, int n, int start_pos, int* parts) {
+static lpp_status prefill_resid(lpp_engine* e, const PrefillMap& wm, int row0, const PrefillMap& xm, int K, int n, int start_pos, int* parts) {
     // all Dp columns: beyond dim the products are zero (rows outside the map), and so are the partial sums that the norm adds
-    PrefillGemmArgs g = prefill_gemm_args(e, e->Dp, K, n, start_pos);
+    PrefillGemmArgs g = prefill_gemm_args(e, e->Dp, K, n, start_pos, kPfMaxSplits);
     g.row0 = row0;
     g.x = e->pf_x;
     g.x_pitch = e->Dp;
-    g.splits = *parts = prefill_splits(e, g.n_rows, K);
+    *parts = g.splits;
     CU(launch_prefill_gemm<kPfResid>(e, wm, xm, g));
     return LPP_OK;
 }
@@ -2548,7 +2670,7 @@ static lpp_status prefill_gqa_mixer(lpp_engine* e, int l, int n, int start_pos, 
     const lpp_config& c = e->c;
     const int D = c.dim, qkv_rows = e->Dq + 2 * e->KVd;
     const size_t lofs = (size_t)l * e->KVHl * c.seq_len * e->hs;
-    PrefillGemmArgs g = prefill_gemm_args(e, qkv_rows, D, n, start_pos);
+    PrefillGemmArgs g = prefill_gemm_args(e, qkv_rows, D, n, start_pos, kPfMaxSplits);
     g.row0 = l * qkv_rows;
     g.epi = kPfQkv;
     g.q = e->pf_q;
@@ -2559,7 +2681,6 @@ static lpp_status prefill_gqa_mixer(lpp_engine* e, int l, int n, int start_pos, 
     g.rope = e->rope;
     g.k_cache = (__half*)e->kcache + lofs;
     g.v_cache = (__half*)e->vcache + lofs;
-    g.splits = prefill_splits(e, qkv_rows, D);
     const cudaError_t ge = launch_prefill_gemm_t<__half, kPfQkv>(e, e->pf_map_wqkv, e->pf_map_xn, g);
     CU(ge);
     if (g.splits > 1)
@@ -2571,26 +2692,26 @@ static lpp_status prefill_gqa_mixer(lpp_engine* e, int l, int n, int start_pos, 
     if (pf_mma && e->hs == 64 && e->gqa <= 8)
         CU(launch_kernel(prefill_attention_mma_kernel<64>, agrid, dim3(32 * e->gqa), pf_attn_smem<64>(), e->stream, true,
                          (const float*)e->pf_q, (const __half*)g.k_cache, (const __half*)g.v_cache, att, n, start_pos,
-                         c.seq_len, e->gqa, e->Dq));
+                         c.seq_len, e->gqa, e->Dq, e->pf_cap));
     else if (pf_mma && e->hs == 128 && e->gqa <= 8)
         CU(launch_kernel(prefill_attention_mma_kernel<128>, agrid, dim3(32 * e->gqa), pf_attn_smem<128>(), e->stream, true,
                          (const float*)e->pf_q, (const __half*)g.k_cache, (const __half*)g.v_cache, att, n, start_pos,
-                         c.seq_len, e->gqa, e->Dq));
+                         c.seq_len, e->gqa, e->Dq, e->pf_cap));
     else
         CU(launch_kernel(prefill_attention_kernel, dim3(n, e->KVHl), dim3(32 * e->gqa),
                          (size_t)e->gqa * e->hs * sizeof(float), e->stream, true, (const float*)e->pf_q,
                          (const __half*)g.k_cache, (const __half*)g.v_cache, att, n, start_pos, c.seq_len, e->hs,
-                         e->gqa, e->Dq));
+                         e->gqa, e->Dq, e->pf_cap));
     return LPP_OK;
 }
 
 // W . in of a block as partial sums over ranges of K, [range][token][row] in pf_part; *splits = the number of ranges.
-static lpp_status prefill_partial_sums(lpp_engine* e, const CUtensorMap& wm, const CUtensorMap& xm, int n_rows, int K, int n, int start_pos, int* splits,
+static lpp_status prefill_partial_sums(lpp_engine* e, const PrefillMap& wm, const PrefillMap& xm, int n_rows, int K, int n, int start_pos, int* splits,
                                        int max_splits = kPfMaxSplits) {
-    PrefillGemmArgs g = prefill_gemm_args(e, n_rows, K, n, start_pos);
+    PrefillGemmArgs g = prefill_gemm_args(e, n_rows, K, n, start_pos, max_splits);
     g.out = e->pf_part;
     g.out_pitch = n_rows;
-    g.splits = *splits = prefill_splits(e, n_rows, K, max_splits);
+    *splits = g.splits;
     CU((launch_prefill_gemm_t<__nv_bfloat16, kPfStore>(e, wm, xm, g)));
     return LPP_OK;
 }
@@ -2604,6 +2725,7 @@ static lpp_status prefill_row_attention(lpp_engine* e, const ModelLayer& y, cons
     a.start_pos = start_pos;
     a.n_tokens = n;
     a.planes = (__nv_bfloat16*)planes;
+    a.cap = e->pf_cap;
     a.out = nullptr;
     if (a.gate) a.gate = e->pf_gate;
     CU(launch_latent_attn(e, p, a, y.d.mixer == LPP_MIXER_SHARED_KV, true, e->stream));
@@ -2622,10 +2744,12 @@ static lpp_status prefill_latent_mixer(lpp_engine* e, int l, int n, int start_po
     PrefillLatentFinishArgs f = {};
     TRY(prefill_partial_sums(e, y.m_in, e->pf_map_xn, y.in_rows, e->Dp, n, start_pos, &f.splits));
     f.part = e->pf_part;
+    f.part_tokens = prefill_part_tokens(n);
     f.n_rows = y.in_rows;
     f.start_pos = start_pos;
     f.seq_len = e->c.seq_len;
     f.qn = e->pf_qn;
+    f.cap = e->pf_cap;
     f.gate = e->pf_gate;
     f.st = e->st;
     f.lat = latent_args(e, y, r);
@@ -2634,16 +2758,14 @@ static lpp_status prefill_latent_mixer(lpp_engine* e, int l, int n, int start_po
     CU(launch_kernel(prefill_latent_finish_kernel<T>, dim3(n, 1 + q_sections), dim3(kLatFinishThreads), (size_t)y.latent_rows * 4, e->stream,
                      true, f));
     if (cache_only) return LPP_OK;
-    PrefillGemmArgs q = prefill_gemm_args(e, y.rank_pitch, y.dim_pitch, n, start_pos);
-    q.groups = H;
+    PrefillGemmArgs q = prefill_gemm_args(e, y.rank_pitch, y.dim_pitch, n, start_pos, 1, H);
     q.group_stride = y.rank_pitch;
     q.group_pieces = y.dim_pitch / 64;
     q.lat_query = e->pf_lq;
     q.lat_pitch = y.row_width;
     CU((launch_prefill_gemm_t<T, kPfLatentQuery>(e, y.m_uk, y.x_qn, q)));
     TRY(prefill_row_attention(e, y, r, n, start_pos, e->pf_olat));
-    PrefillGemmArgs v = prefill_gemm_args(e, y.vdim_rows, y.val_pitch, n, start_pos);
-    v.groups = H;
+    PrefillGemmArgs v = prefill_gemm_args(e, y.vdim_rows, y.val_pitch, n, start_pos, 1, H);
     v.group_stride = y.vdim_rows;
     v.group_pieces = y.val_pitch / 64;
     v.hb = e->pf_att;
@@ -2661,6 +2783,7 @@ static lpp_status prefill_shared_kv_mixer(lpp_engine* e, int l, int n, int start
     PrefillSharedKvArgs f = {};
     TRY(prefill_partial_sums(e, y.m_in, e->pf_map_xn, y.in_rows, e->Dp, n, start_pos, &f.splits));
     f.part = e->pf_part;
+    f.part_tokens = prefill_part_tokens(n);
     f.n_rows = y.in_rows;
     f.start_pos = start_pos;
     f.seq_len = e->c.seq_len;
@@ -2680,6 +2803,8 @@ static lpp_status prefill_mamba_mixer(lpp_engine* e, int l, int n, int start_pos
     MambaConvArgs v = {};
     TRY(prefill_partial_sums(e, y.m_in, e->pf_map_xn, y.in_rows, e->Dp, n, start_pos, &v.splits));
     v.part = e->pf_part;
+    v.part_tokens = prefill_part_tokens(n);
+    v.cap = e->pf_cap;
     v.n_tokens = n;
     v.start_pos = start_pos;
     v.seq_len = e->c.seq_len;
@@ -2700,7 +2825,7 @@ static lpp_status prefill_mamba_mixer(lpp_engine* e, int l, int n, int start_pos
     int splits;
     TRY(prefill_partial_sums(e, y.m_low, y.x_low, y.low_rows, y.inner_pitch, n, start_pos, &splits, kLowMaxSplits));
     CU(launch_kernel(mamba_low_kernel, dim3(n, (y.dt_pitch + 2 * y.state_pitch + kLowColumns - 1) / kLowColumns), dim3(kLowThreads), 0, e->stream, true,
-                     a, (const float*)e->pf_part, splits, e->pf_low));
+                     a, (const float*)e->pf_part, prefill_part_tokens(n), splits, e->pf_low));
     a.low = e->pf_low;
     a.n_tokens = n;
     a.start_pos = start_pos;
@@ -2710,11 +2835,12 @@ static lpp_status prefill_mamba_mixer(lpp_engine* e, int l, int n, int start_pos
     a.tail = e->pf_tail;
     a.planes = (__nv_bfloat16*)e->pf_att;
     a.plane_row = y.o_pitch;
+    a.cap = e->pf_cap;
     CU(launch_mamba_scan(e, a, e->stream));
     return LPP_OK;
 }
 
-// One block of n <= kPrefillTokens prompt tokens at positions start_pos ...  Without wanted logits the last layer stops
+// One block of n <= pf_cap prompt tokens at positions start_pos ...  Without wanted logits the last layer stops
 // after its cache rows are written (nothing downstream of them is needed); otherwise the n_want rows `want` of the block go
 // through the final norm and the classifier and their logits are copied to h_logits.
 static lpp_status prefill_block(lpp_engine* e, const int* h_tokens, int n, int start_pos, const int* want, int n_want, float* h_logits) {
@@ -2730,7 +2856,7 @@ static lpp_status prefill_block(lpp_engine* e, const int* h_tokens, int n, int s
         const LayerView v = layer_view(e, l);
         const ModelLayer* y = layered ? &e->layers[e->runs[l].layer] : nullptr;
         // layer 0 takes the embedding rows; later layers first add the previous residual GEMM's partial sums
-        TRY(prefill_norm(e, n, layered ? y->n1w : e->rms_att + (size_t)l * c.dim, layered ? y->n1b : nullptr, l == 0, add, parts, nullptr, l > 0));
+        TRY(prefill_norm(e, n, n, layered ? y->n1w : e->rms_att + (size_t)l * c.dim, layered ? y->n1b : nullptr, l == 0, add, parts, nullptr, l > 0));
         if (!layered)
             TRY(prefill_gqa_mixer(e, l, n, start_pos, cache_only));
         else if (y->d.mixer == LPP_MIXER_LATENT)
@@ -2744,7 +2870,7 @@ static lpp_status prefill_block(lpp_engine* e, const int* h_tokens, int n, int s
                           &parts));
         add = v.o_add;
         if (v.ff == 0) continue;  // a layer without a feed-forward
-        TRY(prefill_norm(e, n, v.norm2_w, v.norm2_b, false, add, parts, nullptr, true));
+        TRY(prefill_norm(e, n, n, v.norm2_w, v.norm2_b, false, add, parts, nullptr, true));
         PrefillGemmArgs u = prefill_gemm_args(e, 2 * v.ff, e->Dp, n, start_pos);
         u.row0 = layered ? 0 : l * 2 * v.ff;
         u.hb = e->pf_hb;
@@ -2755,14 +2881,17 @@ static lpp_status prefill_block(lpp_engine* e, const int* h_tokens, int n, int s
                           &parts));
         add = v.down_add;
     }
-    if (!e->pf_logits) CU(cudaMalloc(&e->pf_logits, (size_t)kPrefillTokens * e->Vp * 4));
-    TRY(prefill_norm(e, n_want, e->rms_final, e->final_b, false, add, parts, e->pf_rows, true));
-    PrefillGemmArgs g = prefill_gemm_args(e, e->Vp, e->Dp, n_want, start_pos);
-    g.out = e->pf_logits;
-    g.out_pitch = e->Vp;
-    CU(launch_prefill_gemm<kPfStore>(e, e->pf_map_cls, e->pf_map_xn, g));
-    CU(cudaMemcpy2DAsync(h_logits, (size_t)c.vocab_size * 4, e->pf_logits, (size_t)e->Vp * 4, (size_t)c.vocab_size * 4, n_want,
-                         cudaMemcpyDeviceToHost, e->stream));
+    if (!e->pf_logits) CU(cudaMalloc(&e->pf_logits, (size_t)kPfTile * e->Vp * 4));
+    for (int i = 0; i < n_want; i += kPfTile) {
+        const int m = std::min(kPfTile, n_want - i);
+        TRY(prefill_norm(e, m, n, e->rms_final, e->final_b, false, add, parts, e->pf_rows + i, true));
+        PrefillGemmArgs g = prefill_gemm_args(e, e->Vp, e->Dp, m, start_pos);
+        g.out = e->pf_logits;
+        g.out_pitch = e->Vp;
+        CU(launch_prefill_gemm<kPfStore>(e, e->pf_map_cls, e->pf_map_xn, g));
+        CU(cudaMemcpy2DAsync(h_logits + (size_t)i * c.vocab_size, (size_t)c.vocab_size * 4, e->pf_logits, (size_t)e->Vp * 4, (size_t)c.vocab_size * 4, m,
+                             cudaMemcpyDeviceToHost, e->stream));
+    }
     return LPP_OK;
 }
 
@@ -2780,13 +2909,18 @@ extern "C" lpp_status lpp_extend(lpp_engine* e, const int* h_tokens, int n, int 
     TRY(push_state(e, h_tokens[0], start_pos, nullptr, nullptr, 0, 0.f, 0, 0));  // clears the device status
     TRY(state_runs(e, start_pos));
     if (prefill_batched(e) && n > 1) {
-        TRY(prefill_setup(e));
+        TRY(prefill_setup(e, n));
         CU(cudaEventRecord(e->ev0, e->stream));
-        for (int i = 0; i < n; i += kPrefillTokens) {
-            const int m = std::min(kPrefillTokens, n - i);
-            int rows[kPrefillTokens], k = 0;
+        // blocks of about the same size, whole token tiles of the pair kernel where they are larger than one
+        const int blocks = (n + e->pf_cap - 1) / e->pf_cap;
+        const int per = std::min<int>(e->pf_cap, (int)align_up((size_t)(n + blocks - 1) / blocks, kPairTokens));
+        std::vector<int> rows;
+        for (int i = 0; i < n; i += per) {
+            const int m = std::min(per, n - i);
+            int k = 0;
+            rows.resize(m);
             while (w + k < n_want && want[w + k] < i + m) rows[k] = want[w + k] - i, ++k;
-            TRY(prefill_block(e, h_tokens + i, m, start_pos + i, rows, k, h_logits + (size_t)w * V));
+            TRY(prefill_block(e, h_tokens + i, m, start_pos + i, rows.data(), k, h_logits + (size_t)w * V));
             w += k;
         }
         CU(cudaEventRecord(e->ev1, e->stream));

@@ -37,10 +37,10 @@ struct LatentAttnArgs {
     unsigned int* counters;  // one per row tile (or head), zero between launches
     // Tensor-core kernel: the splits of a row tile form a cluster and put themselves together
     int cluster;             // 0 = partial results to `part`
-    // A prompt block's finished rows, hi + lo: [2 planes][kPrefillTokens][plane_row], head after head of plane_pitch
+    // A prompt block's finished rows, hi + lo: [2 planes][cap][plane_row], head after head of plane_pitch
     // columns, of which the first plane_cols are written
     __nv_bfloat16* planes;
-    int plane_pitch, plane_cols, plane_row;
+    int plane_pitch, plane_cols, plane_row, cap;
 };
 
 // Global query row of a group's row r.
@@ -267,7 +267,7 @@ __device__ __forceinline__ void latent_planes4(const LatentAttnArgs& a, int t, i
             if (col + c < a.plane_cols) y[c] *= __ldcg(g + c);
     }
     __nv_bfloat16* d = a.planes + (size_t)t * a.plane_row + (size_t)h * a.plane_pitch + col;
-    __nv_bfloat16* d_lo = d + (size_t)kPrefillTokens * a.plane_row;
+    __nv_bfloat16* d_lo = d + (size_t)a.cap * a.plane_row;
     __align__(8) __nv_bfloat16 hi[4], lo[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) split_pair(y[c], hi[c], lo[c]);
@@ -632,13 +632,13 @@ static __global__ void __launch_bounds__(128) prefill_latent_combine_kernel(cons
 // grid: (tokens, 1 + query sections): y = 0 takes latent, rotated key part and gates, y >= 1 512 query rows each.
 constexpr int kLatFinishThreads = 256;
 struct PrefillLatentFinishArgs {
-    const float* part;  // [splits][kPrefillTokens][n_rows]
-    int n_rows, splits;
+    const float* part;  // [splits][part_tokens][n_rows]
+    int part_tokens, cap, n_rows, splits;
     int start_pos, seq_len;
-    void* qn;           // plain queries: [2 planes][kPrefillTokens][heads * dim_pitch]
-    float* gate;        // [kPrefillTokens][heads]
+    void* qn;           // plain queries: [2 planes][cap][heads * dim_pitch]
+    float* gate;        // [tokens][heads]
     StepState* st;
-    LatentArgs lat;     // query: [kPrefillTokens * heads][row_width]
+    LatentArgs lat;     // query: [tokens * heads][row_width]
 };
 template <typename T>
 static __global__ void __launch_bounds__(kLatFinishThreads) prefill_latent_finish_kernel(const PrefillLatentFinishArgs a) {
@@ -656,7 +656,7 @@ static __global__ void __launch_bounds__(kLatFinishThreads) prefill_latent_finis
         float2 p[kPfMaxSplits], v = make_float2(0.f, 0.f);
 #pragma unroll
         for (int s = 0; s < kPfMaxSplits; ++s)
-            if (s < a.splits) p[s] = *reinterpret_cast<const float2*>(a.part + ((size_t)s * kPrefillTokens + t) * a.n_rows + row);
+            if (s < a.splits) p[s] = *reinterpret_cast<const float2*>(a.part + ((size_t)s * a.part_tokens + t) * a.n_rows + row);
 #pragma unroll
         for (int s = 0; s < kPfMaxSplits; ++s)
             if (s < a.splits) {
@@ -676,7 +676,7 @@ static __global__ void __launch_bounds__(kLatFinishThreads) prefill_latent_finis
         float2 v = sum2(row);
         if (row < L.q_plain_rows) {
             T* qn = reinterpret_cast<T*>(a.qn) + (size_t)t * L.heads * L.dim_pitch;
-            const size_t plane = (size_t)kPrefillTokens * L.heads * L.dim_pitch;
+            const size_t plane = (size_t)a.cap * L.heads * L.dim_pitch;
             const float x[2] = {v.x, v.y};
 #pragma unroll
             for (int i = 0; i < 2; ++i) {

@@ -65,11 +65,11 @@ struct MambaScanArgs {
     int inner, state, dt_rank;
     int state_pitch, dt_pitch;  // elements per channel of S and A (4 L NS), of w_dt (multiple of 8)
     int low_rows;               // row of `low`: dt | B | C, even
-    const float* low;           // step: [low_rows]; prompt block: [kPrefillTokens][mamba_low_pitch], padded
+    const float* low;           // step: [low_rows]; prompt block: [tokens][mamba_low_pitch], padded
     const void* w_dt;           // [inner][dt_pitch], weight type
     const float *dt_b, *A, *D;  // [inner], [inner][state_pitch] (negative), [inner]
     float* S;                   // [inner][state_pitch]
-    const float *x, *z;         // step: [inner]; prompt block: [kPrefillTokens][x_pitch]
+    const float *x, *z;         // step: [inner]; prompt block: [tokens][x_pitch]
     float* out;                 // step: [inner]
     StepState* st;
     int seq_len;
@@ -77,8 +77,8 @@ struct MambaScanArgs {
     // prompt block
     int n_tokens, start_pos, x_pitch;
     int tile_tokens;            // tokens whose rows fit shared memory together (a multiple of 4)
-    __nv_bfloat16* planes;      // [2 planes][kPrefillTokens][plane_row]
-    int plane_row;
+    __nv_bfloat16* planes;      // [2 planes][cap][plane_row]
+    int plane_row, cap;
     const float* tail;          // convolution inputs of the block's last tokens, laid out like the ring
     float* ring;
     int taps, ring_pitch;

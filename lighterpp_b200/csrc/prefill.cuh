@@ -1,4 +1,4 @@
-// Batched prompt path ("prefill"): the K/V cache rows of up to kPrefillTokens prompt positions in one pass over
+// Batched prompt path ("prefill"): the K/V cache rows of a block of prompt positions in one pass over
 // the weights, instead of one pass per token.
 //
 // The reference feeds a prompt through forward() token by token (src/main.cpp:163-179): every prompt token
@@ -29,9 +29,10 @@
 
 namespace lpp {
 
-constexpr int kPrefillTokens = 64;   // tokens per pass (rows of the activation tiles)
+constexpr int kPfTile = 64;          // tokens of an item of the CTA kernel (rows of its activation tiles)
+constexpr int kPfMaxTokens = 1024;   // most tokens of a block
 constexpr int kPfKc = 128;           // inputs per stage: two 64-wide (128-byte) swizzled sub-tiles per operand
-constexpr int kPfSubBytesX = kPrefillTokens * 128;  // one activation sub-tile: 64 tokens x 64 inputs
+constexpr int kPfSubBytesX = kPfTile * 128;  // one activation sub-tile: 64 tokens x 64 inputs
 constexpr int kPfMaxSplits = 8;
 constexpr int kPfRingBytes = 192 * 1024;
 constexpr int kPfSmemBytes = 1024 /*barriers*/ + 1024 /*alignment slack*/ + kPfRingBytes;
@@ -48,7 +49,8 @@ enum PfEpi : int {
 // An activation x is handed to the tensor cores as two numbers of the weights' 16-bit type, hi = round(x) and
 // lo = round(x - hi): the MMA accumulates W.hi + W.lo in FP32, which keeps about 22 bits of x with FP16 (17 with BF16),
 // so the batched pass carries FP32 activations through 16-bit-operand MMAs like the token loop carries them through its
-// FP32 arithmetic.  Every activation buffer holds the hi plane [kPrefillTokens][cols] followed by the lo plane; one
+// FP32 arithmetic.  Every activation buffer holds the hi plane [cap][cols] (cap: the tokens the buffers have room
+// for) followed by the lo plane; one
 // 4-D tensor map covers both.
 template <typename T>
 __device__ __forceinline__ void split_pair(float x, T& hi, T& lo) {
@@ -60,17 +62,20 @@ __device__ __forceinline__ void split_half(float x, __half& hi, __half& lo) { sp
 struct PrefillGemmArgs {
     int n_rows, K;        // rows of the weight matrix, inputs per row
     int row0;             // first row of this layer's matrix inside the tensor map (layers are stacked)
-    int n_tokens;         // valid tokens (<= kPrefillTokens)
+    int n_tokens;         // valid tokens
+    int cap;              // token rows of a plane of the activation buffers
+    int part_tokens;      // token rows of one range of K in part and out
     int start_pos;        // position of token 0
+    int tile;             // tokens of an item: kPfTile (this file's kernel) or kPairTokens (prefill_pair.cuh)
     int epi;
-    int splits;           // K is cut into this many ranges (kPfResid and kPfQkv): work item = (row tile, range)
+    int splits;           // K is cut into this many ranges: work item = (row tile, token tile, range)
     StepState* st;
-    // kPfResid: x[t][row] += c (x: [kPrefillTokens][n_rows] FP32) when splits == 1; else the partial sums go to
+    // kPfResid: x[t][row] += c (x: [tokens][n_rows] FP32) when splits == 1; else the partial sums go to
     // part[split][t][row] and the next kernel (prefill_norm_kernel) adds them to x in split order
     float* x;
     float* part;
     int x_pitch;          // row pitch of x and part (kPfResid)
-    // kPfSwiglu: hb[t][row/2] = act(gate) * up   (rows interleaved gate, up; hb: hi and lo plane [kPrefillTokens][hb_pitch])
+    // kPfSwiglu: hb[t][row/2] = act(gate) * up   (rows interleaved gate, up; hb: hi and lo plane [cap][hb_pitch])
     void* hb;
     int hb_pitch;
     int act;
@@ -86,7 +91,7 @@ struct PrefillGemmArgs {
     // kPfLatentValue: column group * n_valid + row of hb (rows below n_valid), times gate[t][group]
     const float* gate;
     int n_valid;
-    // kPfQkv: rows are q | k | v; RoPE on q and k, q -> FP32 [kPrefillTokens][q_rows], k/v -> cache at start_pos + t
+    // kPfQkv: rows are q | k | v; RoPE on q and k, q -> FP32 [tokens][q_rows], k/v -> cache at start_pos + t
     float* q;
     int q_rows, kv_rows, head_size, seq_len;
     const float2* rope;   // [seq_len][head_size/2]
@@ -168,7 +173,7 @@ constexpr int kUmmaStage = 2 * kUmmaSubW + 4 * kPfSubBytesX;       // 64 KiB: we
 constexpr int kUmmaStages = kPfRingBytes / kUmmaStage;             // 3
 constexpr int kUmmaEpiWarps = 8;                                   // two per tensor-memory lane quarter: 32 tokens each
 constexpr int kUmmaThreads = (2 + kUmmaEpiWarps) * 32;
-constexpr int kUmmaN = 2 * kPrefillTokens;                         // MMA N: the 64 hi rows and the 64 lo rows of the activation tile
+constexpr int kUmmaN = 2 * kPfTile;                                // MMA N: the 64 hi rows and the 64 lo rows of the activation tile
 constexpr int kUmmaAccCols = kUmmaN;                               // FP32 columns of one accumulator: W.hi | W.lo
 constexpr int kUmmaTmemCols = 2 * kUmmaAccCols;                    // power of two >= 32
 // Instruction descriptor: D = F32 (bits 4-5 = 1), A and B of the same 16-bit type (bits 7-9 and 10-12: 0 = FP16,
@@ -234,21 +239,24 @@ __device__ __forceinline__ void umma_epilogue(const PrefillGemmArgs& a, int spli
     const int nt = min(32, a.n_tokens - t0);  // valid tokens of this half (may be <= 0)
     if constexpr (EPI == kPfResid) {
         if (a.splits > 1) {
-            float* p = a.part + ((size_t)split * kPrefillTokens + t0) * a.x_pitch + row;
+            float* p = a.part + ((size_t)split * a.part_tokens + t0) * a.x_pitch + row;
 #pragma unroll
             for (int i = 0; i < 32; ++i)
                 if (row_ok && i < nt) p[(size_t)i * a.x_pitch] = v[i];
         } else {
             float* p = a.x + (size_t)t0 * a.x_pitch + row;
-            float old[32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) old[i] = (row_ok && i < nt) ? p[(size_t)i * a.x_pitch] : 0.f;
+            for (int i0 = 0; i0 < 32; i0 += 8) {  // eight loads in flight: the pair kernel has no registers for more
+                float old[8];
 #pragma unroll
-            for (int i = 0; i < 32; ++i)
-                if (row_ok && i < nt) p[(size_t)i * a.x_pitch] = old[i] + v[i];  // x += W.xb (src/model.cpp:232, 239)
+                for (int i = 0; i < 8; ++i) old[i] = (row_ok && i0 + i < nt) ? p[(size_t)(i0 + i) * a.x_pitch] : 0.f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (row_ok && i0 + i < nt) p[(size_t)(i0 + i) * a.x_pitch] = old[i] + v[i0 + i];  // x += W.xb (src/model.cpp:232, 239)
+            }
         }
     } else if constexpr (EPI == kPfStore) {
-        float* p = a.out + ((size_t)split * kPrefillTokens + t0) * a.out_pitch + row;
+        float* p = a.out + ((size_t)split * a.part_tokens + t0) * a.out_pitch + row;
 #pragma unroll
         for (int i = 0; i < 32; ++i)
             if (row_ok && i < nt) p[(size_t)i * a.out_pitch] = v[i];
@@ -269,7 +277,7 @@ __device__ __forceinline__ void umma_epilogue(const PrefillGemmArgs& a, int spli
                 T hi, lo;
                 split_pair(v[i] * gt[i], hi, lo);
                 p[(size_t)i * a.hb_pitch] = hi;
-                p[(size_t)(kPrefillTokens + i) * a.hb_pitch] = lo;
+                p[(size_t)(a.cap + i) * a.hb_pitch] = lo;
             }
     } else if constexpr (EPI == kPfSwiglu) {
         // rows interleaved (gate_i, up_i): the even lane finishes tokens 0..15 of the pair, the odd lane tokens 16..31;
@@ -289,11 +297,11 @@ __device__ __forceinline__ void umma_epilogue(const PrefillGemmArgs& a, int spli
             split_pair(r, hi, lo);
             if (row_ok && k < nt_mine) {
                 hb[(size_t)k * a.hb_pitch] = hi;
-                hb[(size_t)(kPrefillTokens + k) * a.hb_pitch] = lo;
+                hb[(size_t)(a.cap + k) * a.hb_pitch] = lo;
             }
         }
     } else if (a.splits > 1) {  // kPfQkv cut along K: partial sums, finished by prefill_qkv_finish_kernel
-        float* p = a.part + ((size_t)split * kPrefillTokens + t0) * a.n_rows + row;
+        float* p = a.part + ((size_t)split * a.part_tokens + t0) * a.n_rows + row;
 #pragma unroll
         for (int i = 0; i < 32; ++i)
             if (row_ok && i < nt) p[(size_t)i * a.n_rows] = v[i];
@@ -365,8 +373,8 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
     const int group_tiles = (a.n_rows + kUmmaM - 1) / kUmmaM;  // row tiles of one matrix
     const int n_tiles = group_tiles * max(1, a.groups);        // items along the rows
     const int n_kc = (a.K + kPfKc - 1) / kPfKc;
-    const int S = a.splits;
-    const int n_items = n_tiles * S;
+    const int S = a.splits, tok_tiles = (a.n_tokens + kPfTile - 1) / kPfTile;
+    const int n_items = n_tiles * tok_tiles * S;  // item = (row tile, token tile, K range)
     pdl_launch_dependents();
     if (tid == 0) {
         *s_fail = 0;
@@ -400,10 +408,11 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
             int early = 0;  // stages whose weights are already in flight
             // one copy per operand and stage: both 64-input weight sub-tiles / the four activation sub-tiles (hi, lo)
             auto load_w = [&](uint32_t dst, int kc, int wrow, int sl) { tma_load_3d(dst, &w_map, 0, wrow, 2 * kc, smem_u32(&full[sl])); };
-            auto load_x = [&](uint32_t dst, int piece, int sl) { tma_load_4d(dst, &x_map, 0, 0, 0, piece, smem_u32(&full[sl])); };
+            auto load_x = [&](uint32_t dst, int tok0, int piece, int sl) { tma_load_4d(dst, &x_map, 0, tok0, 0, piece, smem_u32(&full[sl])); };
             auto expect = [&](int sl) { mbar_arrive_expect_tx(&full[sl], kStage); };
             for (int item = unit; item < n_items && ok; item += n_units) {
-                const int tile = item / S, split = item - tile * S;
+                const int unsplit = item / S, split = item - unsplit * S, tile = unsplit / tok_tiles;
+                const int tok0 = (unsplit - tile * tok_tiles) * kPfTile;
                 const int kc0 = (split * n_kc) / S, kc1 = ((split + 1) * n_kc) / S;
                 const int group = tile / group_tiles, piece0 = group * a.group_pieces;
                 const int wrow = a.row0 + group * a.group_stride + (tile - group * group_tiles) * kUmmaM;
@@ -432,7 +441,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
                         load_w(dst, kc, wrow, slot);
                     }
                     PF_STAMP(2 + kc - kc0);
-                    load_x(dst + 2 * kUmmaSubW, piece0 + 2 * kc, slot);
+                    load_x(dst + 2 * kUmmaSubW, tok0, piece0 + 2 * kc, slot);
                     if (++slot == kStages) {
                         slot = 0;
                         ++pass;
@@ -449,10 +458,9 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
             bool ok = true;
             int it = 0;
             for (int item = unit; item < n_items && ok; item += n_units, ++it) {
-                const int tile = item / S, split = item - tile * S;
+                const int split = item % S;
                 const int kc0 = (split * n_kc) / S, kc1 = ((split + 1) * n_kc) / S;
                 const int b = it & 1, use = it >> 1;
-                (void)tile;
                 if (use > 0 && !mbar_wait_bounded(&acc_empty[b], (uint32_t)(use - 1) & 1u, a.st)) {
                     *s_fail = 1;
                     break;
@@ -493,7 +501,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         int it = 0;
         for (int item = unit; item < n_items; item += n_units, ++it) {
-            const int tile = item / S, split = item - tile * S;
+            const int unsplit = item / S, split = item - unsplit * S, tile = unsplit / tok_tiles;
             const int b = it & 1, use = it >> 1;
             if (!__all_sync(0xffffffffu, mbar_wait_bounded(&acc_full[b], (uint32_t)use & 1u, a.st))) {
                 *s_fail = 1;
@@ -504,7 +512,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
             float v[32], vlo[32];
             const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * kUmmaAccCols);
             tc_ld32(taddr + half * 32, v);                     // W.hi of this warp's 32 tokens
-            tc_ld32(taddr + kPrefillTokens + half * 32, vlo);  // W.lo
+            tc_ld32(taddr + kPfTile + half * 32, vlo);  // W.lo
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] += vlo[i];
             tc_fence_before();
@@ -512,7 +520,8 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
             if (lane == 0) mbar_arrive(&acc_empty[b]);
             if (tid == 64) PF_STAMP(35);
             const int group = tile / group_tiles;
-            umma_epilogue<T, EPI>(a, split, group, (tile - group * group_tiles) * kUmmaM + quarter * 32 + lane, half * 32, v, lane);
+            umma_epilogue<T, EPI>(a, split, group, (tile - group * group_tiles) * kUmmaM + quarter * 32 + lane,
+                                  (unsplit - tile * tok_tiles) * kPfTile + half * 32, v, lane);
             if (tid == 64) PF_STAMP(36);
         }
     }
@@ -544,7 +553,7 @@ static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const Pr
     float2 p[kPfMaxSplits];
 #pragma unroll
     for (int s0 = 0; s0 < kPfMaxSplits; ++s0)
-        if (s0 < a.splits) p[s0] = *reinterpret_cast<const float2*>(a.part + ((size_t)s0 * kPrefillTokens + t) * a.n_rows + row);
+        if (s0 < a.splits) p[s0] = *reinterpret_cast<const float2*>(a.part + ((size_t)s0 * a.part_tokens + t) * a.n_rows + row);
 #pragma unroll
     for (int s0 = 0; s0 < kPfMaxSplits; ++s0)
         if (s0 < a.splits) {
@@ -561,7 +570,7 @@ static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const Pr
 // statistics cover the first norm_n inputs, the rest is zero padding with zero weights.  grid: rows.
 constexpr int kPfNormThreads = 512;
 struct PrefillNormArgs {
-    float* x;            // [kPrefillTokens][D]
+    float* x;            // [tokens][D]
     const int* tokens;   // with emb
     const void* emb;     // [vocab][D], nullptr = the rows of x
     float emb_scale;     // factor of the embedding rows
@@ -572,9 +581,10 @@ struct PrefillNormArgs {
     const float* norm_b; // nullptr = RMSNorm
     float norm_eps;
     int norm_n;
-    void* out;           // [2 planes][kPrefillTokens][D]
+    void* out;           // [2 planes][cap][D]
     int D;
-    const float* part;   // [splits][kPrefillTokens][D], added to x in order when splits > 1
+    const float* part;   // [splits][part_tokens][D], added to x in order when splits > 1
+    int cap, part_tokens;
     int splits;
     StepState* st;
 };
@@ -623,7 +633,7 @@ static __global__ void __launch_bounds__(kPfNormThreads) prefill_norm_kernel(con
         if (add_parts) {
 #pragma unroll
             for (int s0 = 0; s0 < kPfMaxSplits; ++s0)
-                if (s0 < splits) p[s0] = reinterpret_cast<const float4*>(a.part + ((size_t)s0 * kPrefillTokens + t) * D)[i];
+                if (s0 < splits) p[s0] = reinterpret_cast<const float4*>(a.part + ((size_t)s0 * a.part_tokens + t) * D)[i];
 #pragma unroll
             for (int s0 = 0; s0 < kPfMaxSplits; ++s0)
                 if (s0 < splits) {
@@ -692,7 +702,7 @@ static __global__ void __launch_bounds__(kPfNormThreads) prefill_norm_kernel(con
 #pragma unroll
         for (int c = 0; c < 4; ++c) split_pair(y[c], hi[c], lo[c]);
         *reinterpret_cast<uint2*>(out + 4 * (size_t)i) = *reinterpret_cast<const uint2*>(hi);
-        *reinterpret_cast<uint2*>(out + (size_t)kPrefillTokens * D + 4 * (size_t)i) = *reinterpret_cast<const uint2*>(lo);
+        *reinterpret_cast<uint2*>(out + (size_t)a.cap * D + 4 * (size_t)i) = *reinterpret_cast<const uint2*>(lo);
     };
 #pragma unroll
     for (int k = 0; k < kMaxPer; ++k) {
@@ -707,7 +717,7 @@ static __global__ void __launch_bounds__(kPfNormThreads) prefill_norm_kernel(con
 // lanes over positions with an online softmax, FP32 throughout.  grid: (tokens, kv heads), block: gqa warps.
 static __global__ void __launch_bounds__(256) prefill_attention_kernel(const float* q, const __half* k_cache, const __half* v_cache,
                                                                        __half* out, int n_tokens, int start_pos, int seq_len,
-                                                                       int head_size, int gqa, int q_rows) {
+                                                                       int head_size, int gqa, int q_rows, int cap) {
     extern __shared__ float sm[];  // [gqa][head_size] query rows, then [gqa warps][32 lanes][head_size] is too much: V sums go through registers
     pdl_launch_dependents();
     pdl_wait();
@@ -779,7 +789,7 @@ static __global__ void __launch_bounds__(256) prefill_attention_kernel(const flo
             __half hi, lo;
             split_half(__fdiv_rn(acc[c], l), hi, lo);
             out[(size_t)t * q_rows + (size_t)h * hs + lane + 32 * c] = hi;
-            out[(size_t)(kPrefillTokens + t) * q_rows + (size_t)h * hs + lane + 32 * c] = lo;
+            out[(size_t)(cap + t) * q_rows + (size_t)h * hs + lane + 32 * c] = lo;
         }
 }
 
@@ -815,7 +825,8 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t add
 template <int HS>
 static __global__ void __launch_bounds__(256) prefill_attention_mma_kernel(const float* q, const __half* k_cache,
                                                                            const __half* v_cache, __half* out, int n_tokens,
-                                                                           int start_pos, int seq_len, int gqa, int q_rows) {
+                                                                           int start_pos, int seq_len, int gqa, int q_rows,
+                                                                           int cap) {
     constexpr int kStride = HS * 2 + 16;              // bytes per padded row
     constexpr int kMat = kPfAttnTile * kStride;       // bytes of one K or V tile
     constexpr int kChunks = kPfAttnTile * (HS / 8);   // 16-byte pieces of one tile
@@ -970,7 +981,7 @@ static __global__ void __launch_bounds__(256) prefill_attention_mma_kernel(const
             split_half(a0, hi[0], lo[0]);
             split_half(a1, hi[1], lo[1]);
             *reinterpret_cast<uint32_t*>(out + (size_t)r * q_rows + (size_t)h * HS + d) = *reinterpret_cast<const uint32_t*>(hi);
-            *reinterpret_cast<uint32_t*>(out + (size_t)(kPrefillTokens + r) * q_rows + (size_t)h * HS + d) =
+            *reinterpret_cast<uint32_t*>(out + (size_t)(cap + r) * q_rows + (size_t)h * HS + d) =
                 *reinterpret_cast<const uint32_t*>(lo);
         };
         if (r0 < n_tokens) put(r0, __fdiv_rn(o[i][0], l0), __fdiv_rn(o[i][1], l0));

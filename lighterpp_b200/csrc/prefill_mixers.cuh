@@ -6,12 +6,12 @@
 
 namespace lpp {
 
-// The sum, in range order, of the partial sums of two neighbouring rows (n_rows apart: tokens, kPrefillTokens apart: ranges).
-__device__ __forceinline__ float2 prefill_sum2(const float* part, int n_rows, int splits, int t, int row) {
+// The sum, in range order, of the partial sums of two neighbouring rows (n_rows apart: tokens, part_tokens tokens apart: ranges).
+__device__ __forceinline__ float2 prefill_sum2(const float* part, int part_tokens, int n_rows, int splits, int t, int row) {
     float2 p[kPfMaxSplits], v = make_float2(0.f, 0.f);
 #pragma unroll
     for (int s = 0; s < kPfMaxSplits; ++s)
-        if (s < splits) p[s] = *reinterpret_cast<const float2*>(part + ((size_t)s * kPrefillTokens + t) * n_rows + row);
+        if (s < splits) p[s] = *reinterpret_cast<const float2*>(part + ((size_t)s * part_tokens + t) * n_rows + row);
 #pragma unroll
     for (int s = 0; s < kPfMaxSplits; ++s)
         if (s < splits) {
@@ -25,12 +25,12 @@ __device__ __forceinline__ float2 prefill_sum2(const float* part, int n_rows, in
 // range order), one row pair per thread.
 // grid: (tokens, ceil(row pairs / 256))
 struct PrefillSharedKvArgs {
-    const float* part;  // [splits][kPrefillTokens][n_rows]
-    int n_rows, splits;
+    const float* part;  // [splits][part_tokens][n_rows]
+    int part_tokens, n_rows, splits;
     int start_pos, seq_len;
     int keys_only;      // only the cache rows are wanted
     StepState* st;
-    SharedKvArgs kv;    // query: [kPrefillTokens][heads][row_width] FP16, gate: [kPrefillTokens][heads * dim]
+    SharedKvArgs kv;    // query: [tokens][heads][row_width] FP16, gate: [tokens][heads * dim]
 };
 static __global__ void __launch_bounds__(256) prefill_shared_kv_finish_kernel(const PrefillSharedKvArgs a) {
     pdl_launch_dependents();
@@ -46,7 +46,7 @@ static __global__ void __launch_bounds__(256) prefill_shared_kv_finish_kernel(co
     pdl_wait();
     if (!pos_ok && threadIdx.x == 0) atomicOr(&a.st->status, kStatusBadPos);
     if (!mine) return;
-    const float2 v = prefill_sum2(a.part, a.n_rows, a.splits, t, row);
+    const float2 v = prefill_sum2(a.part, a.part_tokens, a.n_rows, a.splits, t, row);
     void* query = reinterpret_cast<__half*>(s.query) + (size_t)t * s.heads * s.row_width;
     float* gate = s.gate + (size_t)t * s.heads * s.dim;
     shared_kv_row(s, query, gate, a.seq_len, pos, row, v.x, v.y, p0);
@@ -62,20 +62,20 @@ static __global__ void __launch_bounds__(256) prefill_shared_kv_finish_kernel(co
 // grid: (ceil(inner / 256), ceil(tokens / kConvTokens), 2: x, z); shared memory (TAPS 0): (kConvTokens + taps - 1) * 256 floats
 constexpr int kConvThreads = 64, kConvTokens = 4;
 struct MambaConvArgs {
-    const float* part;  // [splits][kPrefillTokens][2 * inner_rows]
-    int splits, n_tokens, start_pos, seq_len;
+    const float* part;  // [splits][part_tokens][2 * inner_rows]
+    int part_tokens, cap, splits, n_tokens, start_pos, seq_len;
     int inner, inner_rows, taps;
     const float *conv_w, *conv_b;
     const float* ring;
-    float *tail, *x, *z;    // x, z: [kPrefillTokens][x_pitch]
+    float *tail, *x, *z;    // x, z: [tokens][x_pitch]
     int x_pitch;
-    __nv_bfloat16* planes;  // [2 planes][kPrefillTokens][x_pitch]
+    __nv_bfloat16* planes;  // [2 planes][cap][x_pitch]
     StepState* st;
 };
 // N tokens' sums of the partial sums of rows row .. row + 3, tokens t0 .. (clamped to the block: no branches, so the loads of
 // a range of K are in flight together), in range order.
 template <int N>
-__device__ __forceinline__ void prefill_sums(const float* part, int n_rows, int splits, int n_tokens, int t0, int row, float4 (&v)[N]) {
+__device__ __forceinline__ void prefill_sums(const float* part, int part_tokens, int n_rows, int splits, int n_tokens, int t0, int row, float4 (&v)[N]) {
     const float4* p[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -86,7 +86,7 @@ __device__ __forceinline__ void prefill_sums(const float* part, int n_rows, int 
     for (int s = 1; s < splits; ++s)
 #pragma unroll
         for (int i = 0; i < N; ++i) {
-            const float4 w = p[i][(size_t)s * kPrefillTokens * n_rows / 4];
+            const float4 w = p[i][(size_t)s * part_tokens * n_rows / 4];
             v[i].x += w.x; v[i].y += w.y; v[i].z += w.z; v[i].w += w.w;
         }
 }
@@ -117,7 +117,7 @@ static __global__ void __launch_bounds__(kConvThreads) mamba_conv_kernel(const M
     if (!ok || !in) return;
     if (blockIdx.z == 1) {
         float4 v[kConvTokens];
-        prefill_sums(a.part, n_rows, a.splits, a.n_tokens, t0, a.inner_rows + c, v);
+        prefill_sums(a.part, a.part_tokens, n_rows, a.splits, a.n_tokens, t0, a.inner_rows + c, v);
 #pragma unroll
         for (int i = 0; i < kConvTokens; ++i)
             if (t0 + i < a.n_tokens) *reinterpret_cast<float4*>(a.z + (size_t)(t0 + i) * a.x_pitch + c) = silu4(v[i]);
@@ -144,12 +144,12 @@ static __global__ void __launch_bounds__(kConvThreads) mamba_conv_kernel(const M
 #pragma unroll
         for (int k = 0; k < 4; ++k) split_pair(x[k], hi[k], lo[k]);
         *reinterpret_cast<uint2*>(a.planes + (size_t)t * a.x_pitch + c) = *reinterpret_cast<const uint2*>(hi);
-        *reinterpret_cast<uint2*>(a.planes + (size_t)(kPrefillTokens + t) * a.x_pitch + c) = *reinterpret_cast<const uint2*>(lo);
+        *reinterpret_cast<uint2*>(a.planes + (size_t)(a.cap + t) * a.x_pitch + c) = *reinterpret_cast<const uint2*>(lo);
     };
     if constexpr (TAPS > 0) {
         constexpr int N = kConvTokens + TAPS - 1;
         float4 v[N];
-        prefill_sums(a.part, n_rows, a.splits, a.n_tokens, t0 - slots, c, v);
+        prefill_sums(a.part, a.part_tokens, n_rows, a.splits, a.n_tokens, t0 - slots, c, v);
         if constexpr (TAPS > 1) {
             if (t0 < slots)
 #pragma unroll
@@ -168,7 +168,7 @@ static __global__ void __launch_bounds__(kConvThreads) mamba_conv_kernel(const M
     } else {
         for (int i = 0; i < kConvTokens + slots; ++i) {
             float4 v[1];
-            prefill_sums(a.part, n_rows, a.splits, a.n_tokens, t0 - slots + i, c, v);
+            prefill_sums(a.part, a.part_tokens, n_rows, a.splits, a.n_tokens, t0 - slots + i, c, v);
             v[0] = earlier(i, v[0]);
             if (slots > 0) keep(i, v[0]);
             cv_in[i * kConvThreads + tid] = v[0];
@@ -191,7 +191,7 @@ __host__ __device__ inline int mamba_low_pitch(int dt_pitch, int state_pitch) {
     const int n = dt_pitch + 2 * state_pitch;
     return (n / 4) % 2 ? n : n + 4;
 }
-static __global__ void __launch_bounds__(kLowThreads) mamba_low_kernel(const MambaScanArgs a, const float* part, int splits, float* out) {
+static __global__ void __launch_bounds__(kLowThreads) mamba_low_kernel(const MambaScanArgs a, const float* part, int part_tokens, int splits, float* out) {
     __shared__ float group_sum[kLowGroups][kLowColumns];
     pdl_launch_dependents();
     const int t = blockIdx.x, tid = threadIdx.x, col = tid % kLowColumns, group = tid / kLowColumns, i = (int)blockIdx.y * kLowColumns + col;
@@ -199,10 +199,10 @@ static __global__ void __launch_bounds__(kLowThreads) mamba_low_kernel(const Mam
     constexpr int N = kLowMaxSplits / kLowGroups;
     const int per = (splits + kLowGroups - 1) / kLowGroups, s0 = group * per, n = min(per, splits - s0);
     pdl_wait();
-    const float* p = part + ((size_t)s0 * kPrefillTokens + t) * a.low_rows + max(src, 0);
+    const float* p = part + ((size_t)s0 * part_tokens + t) * a.low_rows + max(src, 0);
     float v[N], sum = 0.f;
 #pragma unroll
-    for (int s = 0; s < N; ++s) v[s] = s < n ? __ldcg(p + (size_t)s * kPrefillTokens * a.low_rows) : 0.f;
+    for (int s = 0; s < N; ++s) v[s] = s < n ? __ldcg(p + (size_t)s * part_tokens * a.low_rows) : 0.f;
 #pragma unroll
     for (int s = 0; s < N; ++s) sum += v[s];
     group_sum[group][col] = sum;
@@ -361,7 +361,7 @@ static __global__ void __launch_bounds__(kScanThreads) mamba_scan_kernel(const M
             split_pair(c0 + ch + 1 < a.inner ? xs[t * CH + ch + 1] * zs[t * CH + ch + 1] : 0.f, hi[1], lo[1]);
             __nv_bfloat16* d = a.planes + (size_t)(t0 + t) * a.plane_row + c0 + ch;
             *reinterpret_cast<uint32_t*>(d) = *reinterpret_cast<const uint32_t*>(hi);
-            *reinterpret_cast<uint32_t*>(d + (size_t)kPrefillTokens * a.plane_row) = *reinterpret_cast<const uint32_t*>(lo);
+            *reinterpret_cast<uint32_t*>(d + (size_t)a.cap * a.plane_row) = *reinterpret_cast<const uint32_t*>(lo);
         }
     }
     if (!in) return;

@@ -1,0 +1,104 @@
+"""Prompt blocks of more than one 64-token tile (GEMMs on pairs of SMs): the logits of token counts around the tiles and the
+block against the token-by-token loop, for every kind of layer; less memory than the largest block's workspace takes."""
+import numpy as np
+import pytest
+
+from lighterpp_b200 import synth
+from lighterpp_b200.formats import ModelConfig
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def E():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from lighterpp_b200 import engine
+    return engine
+
+
+def pair(E, name, seq_len):
+    c, dt, tied, seed = synth.SHAPES[name]
+    c = ModelConfig(**{**c.asdict(), "seq_len": seq_len})
+    T = synth.gen_model(c, seed, dt, tied)
+    engines = E.Engine(c, dt, "f16"), E.Engine(c, dt, "f16", flags=E.FLAG_NO_PREFILL_GEMM)
+    for e in engines:
+        e.load_weights(T)
+    return c, synth.prompt_tokens(c.vocab_size, seq_len, seed), engines
+
+
+def check(a, b, rel):
+    assert np.isfinite(a).all() and np.linalg.norm(a - b) <= rel * np.linalg.norm(b), np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+# row tiles of 256: 512 (q, k and v of 256 + 2 x 64 rows: a ragged tile), 704-wide feed-forward: K of eleven 64-input pieces
+@pytest.mark.parametrize("name", ["tiny-gqa-f16", "mini-8b-f16"])
+def test_llama_blocks_match_token_loop(E, name):
+    c, toks, (batched, loop) = pair(E, name, 1200)
+    sizes = (65, 127, 128, 129, 191, 257, 1024, 1025, 1153)
+    want = sorted({n - 1 for n in sizes} | {0, 63, 64})
+    ref = loop.extend(toks[:1153], 0, want)
+    for n in sizes:
+        at = [w for w in want if w < n]
+        # FP16 cache rows may differ by their last bit: 2^-11 of values that the scores see through 1/sqrt(64..128)
+        check(batched.extend(toks[:n], 0, at), ref[:len(at)], 2e-3)
+    many = batched.extend(toks[:200], 0, range(200))  # more wanted rows than one classifier tile
+    check(many, loop.extend(toks[:200], 0, range(200)), 2e-3)
+    batched.extend(toks[:70], 0)  # a block behind a cache
+    check(batched.extend(toks[70:330], 70, [259]), loop.extend(toks[:330], 0, [329]), 2e-3)
+    for e in (batched, loop):
+        e.close()
+
+
+@pytest.mark.parametrize("which", ["rutenex", "kolatar"])
+def test_layered_blocks_match_token_loop(E, which):
+    from oracle import kolatar, rutenex
+    from lighterpp_b200.models import ARCHITECTURES
+    rot = {"base": 1e4, "dims": 16, "scaling": {"factor": 4.0, "original": 64, "fast": 8.0, "slow": 1.0}}
+    if which == "rutenex":
+        mix = {"heads": 5, "dim": 40, "rot_dim": 16, "vdim": 24, "kv_rank": 72, "scale": 56 ** -0.5, "mask": {"size": 200}, "rot": rot}
+        cfg = {"architecture": "Rutenex", "width": 136, "vocab": 320, "norm": {"eps": 1e-5},
+               "layers": [{"type": "latent_attention", "mixer": mix, "mlp": {"kind": "dense", "ff": 200}}] * 2}
+        W = rutenex.random_weights(cfg, 3)
+    else:
+        scan = {"type": "mamba1", "mixer": {"inner": 264, "state": 16, "conv": 4, "dt_rank": 8}, "mlp": None}
+        attn = {"type": "attention", "mlp": {"kind": "dense", "ff": 200},
+                "mixer": {"heads": 4, "kv_heads": 2, "dim": 48, "vdim": 48, "scale": 48 ** -0.5, "softcap": 15.0, "mask": {"size": 130}, "rot": rot}}
+        cfg = {"architecture": "Kolatar", "width": 112, "vocab": 300, "norm": {"eps": 1e-5}, "embedding": {"scale": 10.0}, "logit_scale": 1.5,
+               "loop": {"start": 0, "stop": 1, "times": 2}, "layers": [scan, attn]}
+        W = kolatar.random_weights(cfg, 3)
+    arch = ARCHITECTURES[cfg["architecture"]]
+    c = arch.configure(cfg, 1200)
+    engines = [E.Engine(c, "bf16", "f16", flags=f) for f in (0, E.FLAG_NO_PREFILL_GEMM)]
+    for e in engines:
+        for ours, layer, name, _ in arch.tensors(c):
+            e.upload(ours, (np.ascontiguousarray(W[name], dtype=np.float32).view(np.uint32) >> 16).astype(np.uint16), layer)
+        e.finalize()
+    toks = np.random.default_rng(4).integers(0, cfg["vocab"], 1153)
+    sizes = (65, 128, 129, 321, 1025, 1153)
+    want = [0, 63, 64] + [n - 1 for n in sizes if n != 65]
+    ref = engines[1].extend(toks, 0, want)
+    for n in sizes:
+        at = [w for w in want if w < n]
+        check(engines[0].extend(toks[:n], 0, at), ref[:len(at)], 4e-3)  # the bound of these models' other tests
+    for e in engines:
+        e.close()
+
+
+def test_workspace_shrinks_when_memory_is_short(E):
+    import torch
+    c, toks, (batched, loop) = pair(E, "mini-8b-f16", 1200)
+    ref = loop.extend(toks[:700], 0, [699])
+    batched.extend(toks[:10], 0)
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    hog = torch.empty(free - (30 << 20), dtype=torch.uint8, device="cuda")  # the workspace of 1200 tokens takes over 50 MB
+    try:
+        got = batched.extend(toks[:700], 0, [699])
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    check(got, ref, 2e-3)
+    for e in (batched, loop):
+        e.close()
