@@ -40,6 +40,7 @@
 #include "ops.cuh"
 #include "prefill.cuh"
 #include "prefill_pair.cuh"
+#include "prefill_f32.cuh"
 #include "prefill_mixers.cuh"
 #include "sampler.cuh"
 #include "sampler_exact.cuh"
@@ -252,6 +253,7 @@ struct lpp_engine {
     float *pf_x = nullptr, *pf_q = nullptr, *pf_part = nullptr;
     void *pf_xn = nullptr, *pf_att = nullptr, *pf_hb = nullptr;
     int *pf_tokens = nullptr, *pf_rows = nullptr;
+    unsigned int* pf_counters = nullptr;
     float* pf_logits = nullptr;
     PrefillMap pf_map_cls;
     void *pf_qn = nullptr, *pf_olat = nullptr;      // latent attention: plain queries, attended latents (hi + lo operands)
@@ -2381,9 +2383,14 @@ static lpp_status make_activation_map(PrefillMap* m, const void* base, size_t to
     return encode_activation_map(&m->pair, base, tokens, cols, 128, 1, 1);
 }
 
-// The tensor-core path takes 16-bit weights, an FP16 cache and a single GPU; everything else is fed token by token.
+// Prompts in blocks: the tensor-core path takes 16-bit weights, an FP16 cache and a single GPU, the FP32 path FP32 weights and
+// an FP32 cache of the reference's architecture; everything else is fed token by token.
+static bool prefill_f32(const lpp_engine* e) {
+    return e->layers.empty() && e->c.weight_dtype == LPP_F32 && e->c.kv_dtype == LPP_F32 && e->c.tp_size == 1;
+}
 static bool prefill_batched(const lpp_engine* e) {
     if (e->c.flags & LPP_FLAG_NO_PREFILL_GEMM) return false;
+    if (prefill_f32(e)) return true;
     if (!e->layers.empty()) return e->c.weight_dtype == LPP_BF16 && e->c.kv_dtype == LPP_F16;
     return e->c.tp_size == 1 && e->c.weight_dtype == LPP_F16 && e->c.kv_dtype == LPP_F16 && e->hs <= 128 && e->gqa <= 8 &&
            e->c.dim % 64 == 0 && e->Dq % 64 == 0 && e->Fl % 64 == 0;
@@ -2422,7 +2429,7 @@ static PrefillPlan prefill_plan(const lpp_engine* e, int n_rows, int K, int n, i
     double least = 0;
     for (int s = 1; s <= std::min(max_splits, n_kc); ++s) {
         const int items = row_tiles * ((n + kPairTokens - 1) / kPairTokens) * s, waves = (items + units - 1) / units;
-        const double us = waves * ((n_kc + s - 1) / s * 0.45 + 1.5) + (s > 1 ? s * (double)n * n_rows * 8 / 5e6 : 0.0);
+        const double us = waves * ((n_kc + s - 1) / s * 0.45 + 1.5) + s * (double)n * n_rows * 8 / 5e6;
         if (s == 1 || us < least) best.splits = s, least = us;
     }
     return best;
@@ -2440,8 +2447,25 @@ struct SlabCarver {
         used += align_up(std::max<size_t>(bytes, 16), 256);
     }
 };
+// Floats of partial results that the attention splits of one token leave.
+static size_t prefill_f32_part_row(const lpp_engine* e) { return (size_t)e->Hl * e->attn_splits * (e->hs + 2); }
+static size_t prefill_carve_f32(lpp_engine* e, int cap, char* base) {
+    const size_t D = e->Dp, T = cap;
+    SlabCarver c = {base};
+    c.take(&e->pf_x, T * D * 4);
+    c.take(&e->pf_xn, T * D * 4);
+    c.take(&e->pf_att, T * e->Dq * 4);
+    c.take(&e->pf_hb, T * e->Fl * 4);
+    c.take(&e->pf_q, T * e->Dq * 4);
+    c.take(&e->pf_part, kPfTile * prefill_f32_part_row(e) * 4);
+    c.take(&e->pf_counters, (size_t)kPfTile * e->KVHl * e->attn_z * 4);  // zero between launches
+    c.take(&e->pf_tokens, T * sizeof(int));
+    c.take(&e->pf_rows, T * sizeof(int));
+    return c.used;
+}
 // The workspace of blocks of up to `cap` tokens: its size, and with a base its parts.
 static size_t prefill_carve(lpp_engine* e, int cap, char* base) {
+    if (prefill_f32(e)) return prefill_carve_f32(e, cap, base);
     const size_t D = e->Dp, T = cap;
     const bool layered = !e->layers.empty();
     size_t part_n = 0, att_n = e->Dq, hb_n = e->Fl, qn_n = 0, olat_n = 0, lq_n = 0, lpart_n = 0, gate_n = 0, scan_n = 0, tail_n = 0, low_n = 0;
@@ -2512,6 +2536,7 @@ static size_t prefill_carve(lpp_engine* e, int cap, char* base) {
 }
 static lpp_status prefill_maps(lpp_engine* e) {
     const lpp_config& c = e->c;
+    if (prefill_f32(e)) return LPP_OK;
     const size_t D = e->Dp, L = c.n_layers, T = e->pf_cap;
     if (!e->layers.empty()) {
         for (ModelLayer& y : e->layers) {
@@ -2664,27 +2689,31 @@ static lpp_status prefill_resid(lpp_engine* e, const PrefillMap& wm, int row0, c
     return LPP_OK;
 }
 
+// What the QKV rows' finishing kernel needs beside the sums.
+static void prefill_qkv_args(const lpp_engine* e, int l, PrefillGemmArgs& g) {
+    const size_t lofs = (size_t)l * e->KVHl * e->c.seq_len * e->hs * e->kvesz;
+    g.q = e->pf_q;
+    g.q_rows = e->Dq;
+    g.kv_rows = e->KVd;
+    g.head_size = e->hs;
+    g.seq_len = e->c.seq_len;
+    g.rope = e->rope;
+    g.k_cache = (char*)e->kcache + lofs;
+    g.v_cache = (char*)e->vcache + lofs;
+}
+
 // Grouped-query attention of a prompt block: K/V rows to the cache and, unless only those are wanted, the attended values
 // to pf_att.
 static lpp_status prefill_gqa_mixer(lpp_engine* e, int l, int n, int start_pos, bool cache_only) {
     const lpp_config& c = e->c;
     const int D = c.dim, qkv_rows = e->Dq + 2 * e->KVd;
-    const size_t lofs = (size_t)l * e->KVHl * c.seq_len * e->hs;
     PrefillGemmArgs g = prefill_gemm_args(e, qkv_rows, D, n, start_pos, kPfMaxSplits);
     g.row0 = l * qkv_rows;
     g.epi = kPfQkv;
-    g.q = e->pf_q;
-    g.q_rows = e->Dq;
-    g.kv_rows = e->KVd;
-    g.head_size = e->hs;
-    g.seq_len = c.seq_len;
-    g.rope = e->rope;
-    g.k_cache = (__half*)e->kcache + lofs;
-    g.v_cache = (__half*)e->vcache + lofs;
+    prefill_qkv_args(e, l, g);
     const cudaError_t ge = launch_prefill_gemm_t<__half, kPfQkv>(e, e->pf_map_wqkv, e->pf_map_xn, g);
     CU(ge);
-    if (g.splits > 1)
-        CU(launch_kernel(prefill_qkv_finish_kernel, dim3(n, (qkv_rows / 2 + 255) / 256), dim3(256), 0, e->stream, true, g));
+    CU(launch_kernel(prefill_qkv_finish_kernel<__half>, dim3(n, (qkv_rows / 2 + 255) / 256), dim3(256), 0, e->stream, true, g));
     if (cache_only) return LPP_OK;
     const dim3 agrid((n + kPfAttnRows - 1) / kPfAttnRows, e->KVHl);
     __half* att = (__half*)e->pf_att;
@@ -2840,6 +2869,112 @@ static lpp_status prefill_mamba_mixer(lpp_engine* e, int l, int n, int start_pos
     return LPP_OK;
 }
 
+// ---- FP32 path: every kernel repeats the arithmetic of its counterpart in the decode step (prefill_f32.cuh)
+
+template <int EPI>
+static lpp_status prefill_gemm_f32(lpp_engine* e, const void* w, const void* x, int n_rows, int K, int n, float* out, int out_pitch, const PrefillGemmArgs* qkv = nullptr) {
+    PrefillF32Args a = {};
+    a.w = (const float*)w;
+    a.x = (const float*)x;
+    a.n_rows = n_rows;
+    a.K = K;
+    a.n_tokens = n;
+    a.out = out;
+    a.out_pitch = out_pitch;
+    a.act = kActSilu;
+    if (qkv) a.qkv = *qkv;
+    GemvArgs g = {};  // the inputs that the step's GEMV sums up at a time
+    g.K = K;
+    gemv_geometry(g, 4, kStageTarget);
+    a.kc = (e->c.flags & LPP_FLAG_GEMV_LDG) ? K : g.kc;
+    const dim3 grid((n_rows + kF32Rows - 1) / kF32Rows, (n + kF32Tokens - 1) / kF32Tokens);
+    CU(launch_kernel(a.kc < K ? prefill_f32_gemm_kernel<EPI, true> : prefill_f32_gemm_kernel<EPI, false>, grid, dim3(kF32Threads), 0, e->stream, true, a));
+    return LPP_OK;
+}
+static lpp_status prefill_f32_norm(lpp_engine* e, int n, const float* w, bool embed, const int* rows) {
+    PrefillF32NormArgs a = {};
+    a.x = e->pf_x;
+    a.tokens = e->pf_tokens;
+    a.emb = embed ? (const float*)e->emb : nullptr;
+    a.emb_scale = e->emb_scale;
+    a.vocab = e->c.vocab_size;
+    a.rows = rows;
+    a.norm_w = w;
+    a.norm_eps = e->norm_eps;
+    a.out = (float*)e->pf_xn;
+    a.D = e->c.dim;
+    a.st = e->st;
+    CU(launch_kernel(prefill_f32_norm_kernel, dim3(n), dim3(kF32NormThreads), 0, e->stream, !embed, a));
+    return LPP_OK;
+}
+template <int DPL>
+static cudaError_t launch_f32_attn_d(lpp_engine* e, const AttnArgs& a, dim3 grid, int start_pos, int block_pos) {
+    const int part_row = (int)prefill_f32_part_row(e);
+    return launch_kernel(e->attn_gb == 4   ? prefill_f32_attn_kernel<DPL, 4>
+                         : e->attn_gb == 2 ? prefill_f32_attn_kernel<DPL, 2>
+                                           : prefill_f32_attn_kernel<DPL, 1>,
+                         grid, dim3(kAttnKernelThreads), 0, e->stream, true, a, start_pos, block_pos, e->attn_z, e->Dq, part_row);
+}
+// Attention of a block, a tile of tokens at a time (what the splits of their partial results take).
+static lpp_status prefill_f32_attention(lpp_engine* e, const PrefillGemmArgs& g, int n, int start_pos) {
+    for (int i = 0; i < n; i += kPfTile) {
+        const int m = std::min(kPfTile, n - i);
+        AttnArgs a = {};
+        a.q = e->pf_q + (size_t)i * e->Dq;
+        a.k_cache = g.k_cache;
+        a.v_cache = g.v_cache;
+        a.out = (float*)e->pf_att + (size_t)i * e->Dq;
+        a.part = e->pf_part;
+        a.counters = e->pf_counters;
+        a.st = e->st;
+        a.seq_len = e->c.seq_len;
+        a.head_size = e->hs;
+        a.gqa = e->gqa;
+        a.n_splits = e->attn_splits;
+        a.n_kv_heads = e->KVHl;
+        const dim3 grid(attn_effective_splits(start_pos + i + m, a.n_splits, a.min_chunk), e->KVHl, m * e->attn_z);
+        cudaError_t r = cudaErrorInvalidValue;
+        switch (e->hs / 8) {
+            case 2: r = launch_f32_attn_d<2>(e, a, grid, start_pos + i, start_pos); break;
+            case 4: r = launch_f32_attn_d<4>(e, a, grid, start_pos + i, start_pos); break;
+            case 6: r = launch_f32_attn_d<6>(e, a, grid, start_pos + i, start_pos); break;
+            case 8: r = launch_f32_attn_d<8>(e, a, grid, start_pos + i, start_pos); break;
+            case 12: r = launch_f32_attn_d<12>(e, a, grid, start_pos + i, start_pos); break;
+            case 16: r = launch_f32_attn_d<16>(e, a, grid, start_pos + i, start_pos); break;
+        }
+        CU(r);
+    }
+    return LPP_OK;
+}
+// prefill_block for engines with FP32 weights.
+static lpp_status prefill_block_f32(lpp_engine* e, int n, int start_pos, int n_want, float* h_logits) {
+    const lpp_config& c = e->c;
+    const size_t D = c.dim, qkv = e->Dq + 2 * (size_t)e->KVd, F = e->Fl;
+    for (int l = 0; l < c.n_layers; ++l) {
+        TRY(prefill_f32_norm(e, n, e->rms_att + l * D, l == 0, nullptr));
+        PrefillGemmArgs g = {};
+        g.n_rows = (int)qkv;
+        g.n_tokens = n;
+        g.start_pos = start_pos;
+        g.st = e->st;
+        prefill_qkv_args(e, l, g);
+        TRY((prefill_gemm_f32<kPfQkv>(e, (const float*)e->wqkv + l * qkv * D, e->pf_xn, (int)qkv, (int)D, n, nullptr, 0, &g)));
+        if (l == c.n_layers - 1 && n_want == 0) return LPP_OK;
+        TRY(prefill_f32_attention(e, g, n, start_pos));
+        TRY((prefill_gemm_f32<kPfResid>(e, (const float*)e->wo + l * D * e->Dq, e->pf_att, (int)D, e->Dq, n, e->pf_x, (int)D)));
+        TRY(prefill_f32_norm(e, n, e->rms_ffn + l * D, false, nullptr));
+        TRY((prefill_gemm_f32<kPfSwiglu>(e, (const float*)e->w13 + l * 2 * F * D, e->pf_xn, 2 * (int)F, (int)D, n, (float*)e->pf_hb, (int)F)));
+        TRY((prefill_gemm_f32<kPfResid>(e, (const float*)e->w2 + l * D * F, e->pf_hb, (int)D, (int)F, n, e->pf_x, (int)D)));
+    }
+    for (int i = 0; i < n_want; i += kPfTile) {
+        const int m = std::min(kPfTile, n_want - i);
+        TRY(prefill_f32_norm(e, m, e->rms_final, false, e->pf_rows + i));
+        TRY((prefill_gemm_f32<kPfStore>(e, e->wcls, e->pf_xn, c.vocab_size, (int)D, m, e->pf_logits, c.vocab_size)));
+        CU(cudaMemcpyAsync(h_logits + (size_t)i * c.vocab_size, e->pf_logits, (size_t)m * c.vocab_size * 4, cudaMemcpyDeviceToHost, e->stream));
+    }
+    return LPP_OK;
+}
+
 // One block of n <= pf_cap prompt tokens at positions start_pos ...  Without wanted logits the last layer stops
 // after its cache rows are written (nothing downstream of them is needed); otherwise the n_want rows `want` of the block go
 // through the final norm and the classifier and their logits are copied to h_logits.
@@ -2849,6 +2984,8 @@ static lpp_status prefill_block(lpp_engine* e, const int* h_tokens, int n, int s
     const bool layered = !e->layers.empty();
     CU(cudaMemcpyAsync(e->pf_tokens, h_tokens, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, e->stream));
     if (n_want > 0) CU(cudaMemcpyAsync(e->pf_rows, want, (size_t)n_want * sizeof(int), cudaMemcpyHostToDevice, e->stream));
+    if (n_want > 0 && !e->pf_logits) CU(cudaMalloc(&e->pf_logits, (size_t)kPfTile * e->Vp * 4));
+    if (prefill_f32(e)) return prefill_block_f32(e, n, start_pos, n_want, h_logits);
     int parts = 1;
     const float* add = first_add(e);  // what the next norm adds to the residual stream first
     for (int l = 0; l < L; ++l) {
@@ -2881,7 +3018,6 @@ static lpp_status prefill_block(lpp_engine* e, const int* h_tokens, int n, int s
                           &parts));
         add = v.down_add;
     }
-    if (!e->pf_logits) CU(cudaMalloc(&e->pf_logits, (size_t)kPfTile * e->Vp * 4));
     for (int i = 0; i < n_want; i += kPfTile) {
         const int m = std::min(kPfTile, n_want - i);
         TRY(prefill_norm(e, m, n, e->rms_final, e->final_b, false, add, parts, e->pf_rows + i, true));

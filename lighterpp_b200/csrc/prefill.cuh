@@ -91,12 +91,12 @@ struct PrefillGemmArgs {
     // kPfLatentValue: column group * n_valid + row of hb (rows below n_valid), times gate[t][group]
     const float* gate;
     int n_valid;
-    // kPfQkv: rows are q | k | v; RoPE on q and k, q -> FP32 [tokens][q_rows], k/v -> cache at start_pos + t
+    // kPfQkv: partial sums like kPfResid, also of one range; prefill_qkv_finish_kernel: rows are q | k | v; RoPE on q and k, q -> FP32 [tokens][q_rows], k/v -> cache at start_pos + t
     float* q;
     int q_rows, kv_rows, head_size, seq_len;
     const float2* rope;   // [seq_len][head_size/2]
-    __half* k_cache;      // this layer: [kv_heads][seq_len][head_size]
-    __half* v_cache;
+    void* k_cache;        // this layer: [kv_heads][seq_len][head_size], FP16 (FP32 weights: FP32)
+    void* v_cache;
 };
 
 __device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar_addr) {
@@ -120,34 +120,33 @@ __device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
 }
-// QKV epilogue of one value: row `row` (and its pair partner `other`, the value of row ^ 1), token t: rotation of
-// q and k pairs, q -> FP32 rows, k / v -> cache rows at the reference index.
+// One value of the QKV rows: row `row` (and its pair partner `other`, the value of row ^ 1), token t: rotation of q and k
+// pairs, q -> FP32 rows, k / v -> cache rows at the reference index.
+template <typename CT>
 __device__ __forceinline__ void pf_qkv_store(const PrefillGemmArgs& a, int row, int t, float v, float other) {
+    const int pos = a.start_pos + t;
     if (row >= a.n_rows || t >= a.n_tokens) return;
-    {  // (one scope: the body reads like the decode epilogue it mirrors, gemv.cuh)
-        const int pos = a.start_pos + t;
-        if (pos < 0 || pos >= a.seq_len) {
-            atomicOr(&a.st->status, kStatusBadPos);
-            return;
-        }
-        const int hs = a.head_size;
-        float r = v;
-        if (row < a.q_rows + a.kv_rows) {
-            // adjacent-pair rotation with the table entry for (pos, (row % hs)/2) (src/ops.cpp:34-54)
-            const float2 cs = __ldg(a.rope + (size_t)pos * (hs >> 1) + ((row % hs) >> 1));
-            r = (row & 1) ? __fadd_rn(__fmul_rn(other, cs.y), __fmul_rn(v, cs.x))   // v1' = v0*sin + v1*cos
-                          : __fsub_rn(__fmul_rn(v, cs.x), __fmul_rn(other, cs.y));  // v0' = v0*cos - v1*sin
-        }
-        if (row < a.q_rows) {
-            a.q[(size_t)t * a.q_rows + row] = r;
-        } else {
-            const bool is_k = row < a.q_rows + a.kv_rows;
-            const int rr = row - a.q_rows - (is_k ? 0 : a.kv_rows);
-            const int h = rr / hs, off = rr % hs;
-            // cache index within the layer: h*(seq_len*hs) + pos*hs + off (src/scatter_kv.cu:15-16)
-            const size_t idx = (size_t)h * ((size_t)a.seq_len * hs) + (size_t)pos * hs + off;
-            (is_k ? a.k_cache : a.v_cache)[idx] = __float2half_rn(r);
-        }
+    if (pos < 0 || pos >= a.seq_len) {
+        atomicOr(&a.st->status, kStatusBadPos);
+        return;
+    }
+    const int hs = a.head_size;
+    float r = v;
+    if (row < a.q_rows + a.kv_rows) {
+        // adjacent-pair rotation with the table entry for (pos, (row % hs)/2) (src/ops.cpp:34-54)
+        const float2 cs = __ldg(a.rope + (size_t)pos * (hs >> 1) + ((row % hs) >> 1));
+        r = (row & 1) ? __fadd_rn(__fmul_rn(other, cs.y), __fmul_rn(v, cs.x))   // v1' = v0*sin + v1*cos
+                      : __fsub_rn(__fmul_rn(v, cs.x), __fmul_rn(other, cs.y));  // v0' = v0*cos - v1*sin
+    }
+    if (row < a.q_rows) {
+        a.q[(size_t)t * a.q_rows + row] = r;
+    } else {
+        const bool is_k = row < a.q_rows + a.kv_rows;
+        const int rr = row - a.q_rows - (is_k ? 0 : a.kv_rows);
+        const int h = rr / hs, off = rr % hs;
+        // cache index within the layer: h*(seq_len*hs) + pos*hs + off (src/scatter_kv.cu:15-16)
+        const size_t idx = (size_t)h * ((size_t)a.seq_len * hs) + (size_t)pos * hs + off;
+        reinterpret_cast<CT*>(is_k ? a.k_cache : a.v_cache)[idx] = from_float<CT>(r);
     }
 }
 
@@ -163,8 +162,7 @@ __device__ __forceinline__ void pf_qkv_store(const PrefillGemmArgs& a, int row, 
 // run the epilogue from registers while the next item's MMAs already fill the other accumulator.  Warp roles: 0
 // producer, 1 MMA issue and tensor-memory allocation, 2..9 epilogue (a warp may only read the tensor-memory lanes
 // of its quarter, warp index modulo 4; two warps share a quarter and take 32 tokens each).  An epilogue thread owns
-// one weight row and walks its tokens, so everything that depends on the row alone (which of q/k/v, head,
-// rotation-table column) is computed once.
+// one weight row and walks its tokens, so what depends on the row alone is computed once.
 // Every wait is bounded; every path, also a failed one, reaches the common exit, which lets copies in flight land
 // (bounded) and frees the tensor memory.
 constexpr int kUmmaM = 128;
@@ -231,7 +229,7 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
 
 // Epilogue of one thread: weight row `row`, tokens t0 .. t0+31 with the sums v[0..31].  Lanes are consecutive rows,
 // so for a fixed token a warp's stores are contiguous; the partner row (row ^ 1) of the rotation and SwiGLU pairs
-// is the neighbouring lane.  The rotation rounds like pf_qkv_store.
+// is the neighbouring lane.
 template <typename T, int EPI>
 __device__ __forceinline__ void umma_epilogue(const PrefillGemmArgs& a, int split, int group, int row, int t0, const float (&v)[32],
                                               int lane) {
@@ -300,41 +298,12 @@ __device__ __forceinline__ void umma_epilogue(const PrefillGemmArgs& a, int spli
                 hb[(size_t)(a.cap + k) * a.hb_pitch] = lo;
             }
         }
-    } else if (a.splits > 1) {  // kPfQkv cut along K: partial sums, finished by prefill_qkv_finish_kernel
+    } else {  // kPfQkv: partial sums (also of one range: the rotation's table and the cache rows want another layout), finished
+              // by prefill_qkv_finish_kernel
         float* p = a.part + ((size_t)split * a.part_tokens + t0) * a.n_rows + row;
 #pragma unroll
         for (int i = 0; i < 32; ++i)
             if (row_ok && i < nt) p[(size_t)i * a.n_rows] = v[i];
-    } else {  // kPfQkv
-        const int hs = a.head_size;
-        const bool pos_ok = a.start_pos >= 0 && a.start_pos + a.n_tokens <= a.seq_len;
-        if (!pos_ok && lane == 0) atomicOr(&a.st->status, kStatusBadPos);
-        const bool rot = row < a.q_rows + a.kv_rows;   // q and k rows rotate, v rows do not
-        const bool is_q = row < a.q_rows, is_k = rot && !is_q;
-        const int rr = is_q ? row : row - a.q_rows - (is_k ? 0 : a.kv_rows);
-        const int head = rr / hs, off = rr - head * hs;
-        const float2* rope = a.rope + (off >> 1);       // + pos * (hs / 2)
-        float* qp = a.q + row;                          // + t * q_rows
-        // cache index within the layer: h*(seq_len*hs) + pos*hs + off (src/scatter_kv.cu:15-16)
-        __half* cp = (is_k ? a.k_cache : a.v_cache) + (size_t)head * ((size_t)a.seq_len * hs) + off;
-        const bool odd = row & 1;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const float other = __shfl_xor_sync(0xffffffffu, v[i], 1);
-            if (!(row_ok && pos_ok && i < nt)) continue;
-            const int t = t0 + i, pos = a.start_pos + t;
-            float r = v[i];
-            if (rot) {
-                // adjacent-pair rotation with the table entry for (pos, off/2) (src/ops.cpp:34-54)
-                const float2 cs = __ldg(rope + (size_t)pos * (hs >> 1));
-                r = odd ? __fadd_rn(__fmul_rn(other, cs.y), __fmul_rn(v[i], cs.x))   // v1' = v0*sin + v1*cos
-                        : __fsub_rn(__fmul_rn(v[i], cs.x), __fmul_rn(other, cs.y));  // v0' = v0*cos - v1*sin
-            }
-            if (is_q)
-                qp[(size_t)t * a.q_rows] = r;
-            else
-                cp[(size_t)pos * hs] = __float2half_rn(r);
-        }
     }
 }
 
@@ -540,9 +509,10 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
     if (warp == 1) tc_dealloc(tmem, kUmmaTmemCols);
 }
 
-// Finishes a QKV GEMM that was cut along K: adds the partial sums of a row pair in range order and applies the
+// Finishes a QKV GEMM: adds the partial sums of a row pair in range order and applies the
 // QKV epilogue (rotation of q and k pairs, q -> FP32 rows, k/v -> cache rows at the reference index).
 // grid: (tokens, ceil(row pairs / 256)).
+template <typename CT>
 static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const PrefillGemmArgs a) {
     pdl_launch_dependents();
     pdl_wait();
@@ -560,8 +530,8 @@ static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const Pr
             v.x += p[s0].x;
             v.y += p[s0].y;
         }
-    pf_qkv_store(a, row, t, v.x, v.y);
-    pf_qkv_store(a, row + 1, t, v.y, v.x);
+    pf_qkv_store<CT>(a, row, t, v.x, v.y);
+    pf_qkv_store<CT>(a, row + 1, t, v.y, v.x);
 }
 
 // Rows of the residual stream -> normalised rows (hi + lo MMA operands): RMSNorm, or LayerNorm when a bias is given.

@@ -51,6 +51,31 @@ def test_llama_blocks_match_token_loop(E, name):
         e.close()
 
 
+# every head size's kernel, one to four query heads a CTA, K of one and several chunks (2080 = 2048 + 32, 1100 = 1096 + 4) and odd row tiles
+@pytest.mark.parametrize("cfg,flags", [(ModelConfig(96, 256, 2, 2, 2, 320, 1200), 0), (ModelConfig(336, 704, 2, 7, 7, 502, 1200), 0),
+                                       (ModelConfig(512, 1100, 2, 4, 1, 1000, 1200), 0), (ModelConfig(128, 68, 1, 8, 4, 302, 1200), 0),
+                                       (ModelConfig(192, 2080, 1, 2, 1, 320, 1200), 0), (ModelConfig(256, 4100, 1, 8, 8, 320, 1200), 0),
+                                       (ModelConfig(512, 2080, 1, 8, 2, 320, 1200), 1)], ids=str)
+def test_fp32_blocks_equal_the_token_loop(E, cfg, flags):
+    """Bit for bit: logits around every tile, and behind a cache of earlier portions."""
+    T = synth.gen_model(cfg, 5, "f32", True)
+    toks = synth.prompt_tokens(cfg.vocab_size, 1153, 5)
+    batched, loop = [E.Engine(cfg, "f32", "f32", flags=f | flags) for f in (0, E.FLAG_NO_PREFILL_GEMM)]
+    for e in (batched, loop):
+        e.load_weights(T)
+    sizes = (2, 15, 16, 17, 63, 64, 65, 129, 1024, 1153)
+    want = sorted({n - 1 for n in sizes} | {0})
+    ref = loop.extend(toks, 0, want)
+    for n in sizes:
+        at = [w for w in want if w < n]
+        assert np.array_equal(batched.extend(toks[:n], 0, at), ref[:len(at)]), n
+    batched.extend(toks[:70], 0)
+    assert np.array_equal(batched.extend(toks[70:1153], 70, [1082]), ref[-1:])
+    assert np.array_equal(batched.extend(toks[:130], 0, range(130))[128:129], ref[want.index(128):][:1])
+    for e in (batched, loop):
+        e.close()
+
+
 @pytest.mark.parametrize("which", ["rutenex", "kolatar"])
 def test_layered_blocks_match_token_loop(E, which):
     from oracle import kolatar, rutenex
