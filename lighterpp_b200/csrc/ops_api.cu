@@ -22,9 +22,34 @@ inline lpp_status chk() { return cudaGetLastError() == cudaSuccess ? LPP_OK : LP
 inline cudaStream_t S(void* s) { return (cudaStream_t)s; }
 inline int blocks(long long n, int t) { return (int)std::max<long long>(1, (n + t - 1) / t); }
 
+// Launches an operator kernel.  It may start while the kernel before it in the stream ends (it waits for it in op_begin):
+// 18 operators of a layer one after the other take about a microsecond less each.  A stream that is being captured gets a plain
+// launch, because what comes before it in the graph need not be a kernel.
+template <typename... KArgs, typename... Args>
+lpp_status launch_op(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) {
+        (void)cudaGetLastError();
+        capturing = cudaStreamCaptureStatusActive;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = capturing == cudaStreamCaptureStatusNone ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, ((KArgs)args)...);
+    return chk();
+}
+
 // Any-shape fallback for the stand-alone GEMV: one warp per row, scalar loads.
 template <typename WT>
 __global__ void gemv_generic_kernel(float* out, const float* x, const WT* w, int n, int d) {
+    op_begin();
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= n) return;
@@ -42,39 +67,27 @@ __global__ void gemv_generic_kernel(float* out, const float* x, const WT* w, int
     if (lane == 0) out[row] = acc;
 }
 
-// Status word for stand-alone GEMV launches (their bounded waits need somewhere to report).
-__device__ StepState g_op_state;
-
 template <typename WT>
 lpp_status op_gemv_t(float* out, const float* x, const void* w, int n, int d, cudaStream_t s) {
     const int vec = 16 / (int)sizeof(WT);
-    const size_t smem = 128 + (((size_t)d * 4 + 127) & ~(size_t)127);
-    // the vector kernel stages x with 16-byte loads, reads the rows with 16-byte loads and stores row pairs
-    // with 8-byte stores: anything else (an offset sub-vector, say) takes the scalar kernel
-    if ((n & 1) || (d % vec) || (((uintptr_t)w) & 15) || (((uintptr_t)x) & 15) || (((uintptr_t)out) & 7) ||
-        smem > 200 * 1024) {
-        gemv_generic_kernel<WT><<<blocks(n, 8), 256, 0, s>>>(out, x, (const WT*)w, n, d);
-        return chk();
-    }
-    StepState* st = nullptr;
-    if (cudaGetSymbolAddress((void**)&st, g_op_state) != cudaSuccess) return LPP_ERR_CUDA;
+    const size_t smem = (size_t)d * 4;
+    // the vector kernel stages x and reads the rows with 16-byte loads: anything else (an offset sub-vector, say) takes the
+    // scalar kernel
+    if ((d % vec) || (((uintptr_t)w) & 15) || (((uintptr_t)x) & 15) || smem > 200 * 1024)
+        return launch_op(gemv_generic_kernel<WT>, dim3(blocks(n, 8)), 256, 0, s, out, x, (const WT*)w, n, d);
     if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(gemv_ldg_kernel<WT, kEpiStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess)
+        cudaFuncSetAttribute(op_gemv_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return LPP_ERR_CUDA;
-    GemvArgs a = {};
-    a.W = w;
-    a.n_rows = n;
-    a.K = d;
-    a.x = x;
-    a.out = out;
-    a.st = st;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = std::max(1, std::min(n / kRowsPerGroup, sms * 4));
-    gemv_ldg_kernel<WT, kEpiStore><<<grid, kGemvLdgThreads, smem, s>>>(a);
-    return chk();
+    // two CTAs per SM; as many warps on a row as leave every warp something to do in one round, and a row of less than a
+    // batch per warp to one
+    const int warps = kOpGemvThreads / 32, ctas = 2 * sms;
+    int split = 1;
+    while (split < warps && (long long)n * split * 2 <= (long long)ctas * warps && d / vec >= split * 2 * 32 * kOpGemvU) split *= 2;
+    const int grid = std::min(ctas, blocks((long long)n * split, warps));
+    return launch_op(op_gemv_kernel<WT>, dim3(grid), kOpGemvThreads, smem, s, out, x, (const WT*)w, n, d, split);
 }
 
 // ---- scratch layout of the stand-alone samplers: step state, per-block partials, ticket counter and barrier
@@ -177,9 +190,7 @@ extern "C" {
 lpp_status lpp_op_convert_f32_to_f16(void* d_dst, const float* d_src, int64_t n, void* stream) {
     if (!d_dst || !d_src || n < 0) return LPP_ERR_INVALID_ARG;
     if (n == 0) return LPP_OK;
-    convert_f32_to_f16_kernel<<<(int)std::min<long long>(blocks(n, 256), 148 * 16), 256, 0, S(stream)>>>(
-        (__half*)d_dst, d_src, n);
-    return chk();
+    return launch_op(convert_f32_to_f16_kernel, dim3(std::min(blocks(n, 256), 148 * 16)), 256, 0, S(stream), (__half*)d_dst, d_src, (long long)n);
 }
 
 lpp_status lpp_op_gemv(float* d_out, const float* d_x, const void* d_w, int n, int d, int w_dtype, void* stream) {
@@ -191,35 +202,29 @@ lpp_status lpp_op_gemv(float* d_out, const float* d_x, const void* d_w, int n, i
 
 lpp_status lpp_op_rmsnorm(float* d_out, const float* d_x, const float* d_w, int n, void* stream) {
     if (!d_out || !d_x || !d_w || n <= 0) return LPP_ERR_INVALID_ARG;
-    rmsnorm_kernel<<<1, 256, 0, S(stream)>>>(d_out, d_x, d_w, n);
-    return chk();
+    return launch_op(rmsnorm_kernel, dim3(1), kOpNormThreads, 0, S(stream), d_out, d_x, d_w, n);
 }
 
 lpp_status lpp_op_rope(float* d_q, float* d_k, int pos, int dim, int kv_dim, int head_size, float rope_base,
                        void* stream) {
     if (!d_q || !d_k || dim <= 0 || (dim & 1) || head_size <= 0 || (head_size & 1)) return LPP_ERR_INVALID_ARG;
-    rope_kernel<<<blocks(dim / 2, 256), 256, 0, S(stream)>>>(d_q, d_k, pos, dim, kv_dim, head_size, rope_base);
-    return chk();
+    return launch_op(rope_kernel, dim3(blocks(dim / 2, 256)), 256, 0, S(stream), d_q, d_k, pos, dim, kv_dim, head_size, rope_base);
 }
 
 lpp_status lpp_op_swiglu(float* d_hb, const float* d_h1, const float* d_h3, int size, void* stream) {
     if (!d_hb || !d_h1 || !d_h3 || size <= 0) return LPP_ERR_INVALID_ARG;
-    swiglu_kernel<<<blocks(size, 256), 256, 0, S(stream)>>>(d_hb, d_h1, d_h3, size);
-    return chk();
+    return launch_op(swiglu_kernel, dim3(blocks(size, 256)), 256, 0, S(stream), d_hb, d_h1, d_h3, size);
 }
 
 lpp_status lpp_op_softmax_multihead(float* d_out, const float* d_x, int n_heads, int seq_len, int att_stride,
                                     void* stream) {
     if (!d_out || !d_x || n_heads <= 0 || seq_len <= 0) return LPP_ERR_INVALID_ARG;
-    softmax_multihead_kernel<<<n_heads, 256, 0, S(stream)>>>(d_out, d_x, seq_len, att_stride);
-    return chk();
+    return launch_op(softmax_multihead_kernel, dim3(n_heads), 256, 0, S(stream), d_out, d_x, seq_len, att_stride);
 }
 
 lpp_status lpp_op_scale_multihead(float* d_att, float scale, int n_heads, int seq_len, int att_stride, void* stream) {
     if (!d_att || n_heads <= 0 || seq_len <= 0) return LPP_ERR_INVALID_ARG;
-    scale_multihead_kernel<<<dim3(blocks(seq_len, 256), n_heads), 256, 0, S(stream)>>>(d_att, scale, seq_len,
-                                                                                        att_stride);
-    return chk();
+    return launch_op(scale_multihead_kernel, dim3(blocks(seq_len, 256), n_heads), 256, 0, S(stream), d_att, scale, seq_len, att_stride);
 }
 
 lpp_status lpp_op_aggregation_multihead(float* d_out, const void* d_v_f16, const float* d_att, int n_heads,
@@ -227,15 +232,16 @@ lpp_status lpp_op_aggregation_multihead(float* d_out, const void* d_v_f16, const
     if (!d_out || !d_v_f16 || !d_att || n_heads <= 0 || seq_len <= 0 || head_size <= 0 || head_size > 128 ||
         gqa_factor <= 0)
         return LPP_ERR_INVALID_ARG;
-    aggregation_multihead_kernel<<<n_heads, 128, 0, S(stream)>>>(d_out, (const __half*)d_v_f16, d_att, seq_len,
-                                                                 head_size, gqa_factor, att_stride);
-    return chk();
+    const __half* v = (const __half*)d_v_f16;
+    if (head_size % 8 || ((uintptr_t)v & 15))
+        return launch_op(aggregation_any_kernel, dim3(n_heads), 128, 0, S(stream), d_out, v, d_att, seq_len, head_size, gqa_factor, att_stride);
+    return launch_op(aggregation_kernel, dim3(n_heads * kAggCtas), kAggThreads, 0, S(stream), d_out, v, d_att, seq_len, head_size, gqa_factor,
+                     att_stride);
 }
 
 lpp_status lpp_op_residual_add(float* d_out, const float* d_a, const float* d_b, int n, void* stream) {
     if (!d_out || !d_a || !d_b || n <= 0) return LPP_ERR_INVALID_ARG;
-    residual_add_kernel<<<blocks(n, 256), 256, 0, S(stream)>>>(d_out, d_a, d_b, n);
-    return chk();
+    return launch_op(residual_add_kernel, dim3(blocks(n, 256)), 256, 0, S(stream), d_out, d_a, d_b, n);
 }
 
 lpp_status lpp_op_scatter_kv(void* d_kc_f16, void* d_vc_f16, const float* d_k, const float* d_v, int layer, int pos,
@@ -243,9 +249,8 @@ lpp_status lpp_op_scatter_kv(void* d_kc_f16, void* d_vc_f16, const float* d_k, c
     if (!d_kc_f16 || !d_vc_f16 || !d_k || !d_v || layer < 0 || pos < 0 || pos >= seq_len || n_kv_heads <= 0 ||
         head_size <= 0)
         return LPP_ERR_INVALID_ARG;
-    scatter_kv_kernel<<<blocks(n_kv_heads * head_size, 256), 256, 0, S(stream)>>>(
-        (__half*)d_kc_f16, (__half*)d_vc_f16, d_k, d_v, layer, pos, n_kv_heads, head_size, seq_len);
-    return chk();
+    return launch_op(scatter_kv_kernel, dim3(blocks(n_kv_heads * head_size, 256)), 256, 0, S(stream), (__half*)d_kc_f16, (__half*)d_vc_f16, d_k,
+                     d_v, layer, pos, n_kv_heads, head_size, seq_len);
 }
 
 lpp_status lpp_op_multihead_gemv(float* d_out, const float* d_q, const void* d_k_cache_f16, int layer, int pos,
@@ -253,9 +258,23 @@ lpp_status lpp_op_multihead_gemv(float* d_out, const float* d_q, const void* d_k
     if (!d_out || !d_q || !d_k_cache_f16 || layer < 0 || pos < 0 || pos >= seq_len || n_heads <= 0 ||
         n_kv_heads <= 0 || n_heads % n_kv_heads)
         return LPP_ERR_INVALID_ARG;
-    multihead_gemv_kernel<<<dim3(blocks(pos + 1, 4), n_heads), 128, 0, S(stream)>>>(
-        d_out, d_q, (const __half*)d_k_cache_f16, layer, pos, n_heads, n_kv_heads, head_size, seq_len);
-    return chk();
+    const __half* kc = (const __half*)d_k_cache_f16;
+    auto dot = [&](auto kernel, int lanes) {  // lanes of a cache row
+        const int rows = kDotThreads / lanes * kDotRows;
+        return launch_op(kernel, dim3(blocks(pos + 1, rows), n_heads), kDotThreads, 0, S(stream), d_out, d_q, kc, layer, pos, n_heads, n_kv_heads,
+                         seq_len);
+    };
+    if (((uintptr_t)kc & 15) == 0) {
+        switch (head_size) {
+            case 16: return dot(multihead_gemv_kernel<2>, 2);
+            case 32: return dot(multihead_gemv_kernel<4>, 4);
+            case 64: return dot(multihead_gemv_kernel<8>, 8);
+            case 128: return dot(multihead_gemv_kernel<16>, 16);
+            case 256: return dot(multihead_gemv_kernel<32>, 32);
+        }
+    }
+    return launch_op(multihead_gemv_any_kernel, dim3(blocks(pos + 1, 4), n_heads), 128, 0, S(stream), d_out, d_q, kc, layer, pos, n_heads,
+                     n_kv_heads, head_size, seq_len);
 }
 
 lpp_status lpp_op_rope_scatter(float* d_q, const float* d_k, const float* d_v, void* d_kc_f16, void* d_vc_f16,
@@ -264,10 +283,8 @@ lpp_status lpp_op_rope_scatter(float* d_q, const float* d_k, const float* d_v, v
     if (!d_q || !d_k || !d_v || !d_kc_f16 || !d_vc_f16 || layer < 0 || pos < 0 || pos >= seq_len || dim <= 0 ||
         (dim & 1) || (head_size & 1) || head_size <= 0)
         return LPP_ERR_INVALID_ARG;
-    rope_scatter_kernel<<<blocks(dim / 2, 256), 256, 0, S(stream)>>>(d_q, d_k, d_v, (__half*)d_kc_f16,
-                                                                    (__half*)d_vc_f16, layer, pos, dim, n_kv_heads,
-                                                                    head_size, seq_len, rope_base);
-    return chk();
+    return launch_op(rope_scatter_kernel, dim3(blocks(dim / 2, 256)), 256, 0, S(stream), d_q, d_k, d_v, (__half*)d_kc_f16, (__half*)d_vc_f16,
+                     layer, pos, dim, n_kv_heads, head_size, seq_len, rope_base);
 }
 
 lpp_status lpp_op_sample(float* d_logits, int vocab_size, float temperature, float penalty, const int* d_history,
