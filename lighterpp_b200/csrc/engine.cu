@@ -40,6 +40,7 @@
 #include "ops.cuh"
 #include "prefill.cuh"
 #include "prefill_pair.cuh"
+#include "prefill_attention.cuh"
 #include "prefill_f32.cuh"
 #include "prefill_mixers.cuh"
 #include "sampler.cuh"
@@ -263,6 +264,7 @@ struct lpp_engine {
     float* pf_low = nullptr;                                       // dt | B | C rows
     void* pf_sxp = nullptr;                                        // x as hi + lo operands
     PrefillMap pf_map_wqkv, pf_map_wo, pf_map_w13, pf_map_w2, pf_map_xn, pf_map_att, pf_map_hb;
+    CUtensorMap pf_map_k, pf_map_v;  // the caches as (64 columns, rows, head size / 64)
 
     bool finalized = false;
     int kernels_full = 0;
@@ -2572,8 +2574,13 @@ static lpp_status prefill_maps(lpp_engine* e) {
         TRY(allow_gemm_smem<__half>());
         CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<__half, kPfQkv>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
         TRY((allow_pair_smem<__half, kPfQkv>()));
-        CU(cudaFuncSetAttribute(prefill_attention_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_attn_smem<64>()));
-        CU(cudaFuncSetAttribute(prefill_attention_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_attn_smem<128>()));
+        if (e->hs == 64 || e->hs == 128) {
+            const size_t rows = L * e->KVHl * (size_t)c.seq_len;
+            TRY(encode_weight_map(&e->pf_map_k, e->kcache, rows, e->hs, kFaKeys, e->hs / 64));
+            TRY(encode_weight_map(&e->pf_map_v, e->vcache, rows, e->hs, kFaKeys, e->hs / 64));
+            CU(cudaFuncSetAttribute(prefill_attention_umma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, fa_smem<64>()));
+            CU(cudaFuncSetAttribute(prefill_attention_umma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, fa_smem<128>()));
+        }
     }
     TRY(make_activation_map(&e->pf_map_xn, e->pf_xn, T, D));
     return make_weight_map(&e->pf_map_cls, e->wcls, e->Vp, D);
@@ -2715,22 +2722,34 @@ static lpp_status prefill_gqa_mixer(lpp_engine* e, int l, int n, int start_pos, 
     CU(ge);
     CU(launch_kernel(prefill_qkv_finish_kernel<__half>, dim3(n, (qkv_rows / 2 + 255) / 256), dim3(256), 0, e->stream, true, g));
     if (cache_only) return LPP_OK;
-    const dim3 agrid((n + kPfAttnRows - 1) / kPfAttnRows, e->KVHl);
     __half* att = (__half*)e->pf_att;
-    const bool pf_mma = !aid_env("LPP_ATTN_CUDA_CORES");
-    if (pf_mma && e->hs == 64 && e->gqa <= 8)
-        CU(launch_kernel(prefill_attention_mma_kernel<64>, agrid, dim3(32 * e->gqa), pf_attn_smem<64>(), e->stream, true,
-                         (const float*)e->pf_q, (const __half*)g.k_cache, (const __half*)g.v_cache, att, n, start_pos,
-                         c.seq_len, e->gqa, e->Dq, e->pf_cap));
-    else if (pf_mma && e->hs == 128 && e->gqa <= 8)
-        CU(launch_kernel(prefill_attention_mma_kernel<128>, agrid, dim3(32 * e->gqa), pf_attn_smem<128>(), e->stream, true,
-                         (const float*)e->pf_q, (const __half*)g.k_cache, (const __half*)g.v_cache, att, n, start_pos,
-                         c.seq_len, e->gqa, e->Dq, e->pf_cap));
+    if (e->hs != 64 && e->hs != 128) {
+        CU(launch_kernel(prefill_attention_kernel, dim3(n, e->KVHl), dim3(32 * e->gqa), (size_t)e->gqa * e->hs * sizeof(float), e->stream, true,
+                         (const float*)e->pf_q, (const __half*)g.k_cache, (const __half*)g.v_cache, att, n, start_pos, c.seq_len, e->hs, e->gqa, e->Dq,
+                         e->pf_cap));
+        return LPP_OK;
+    }
+    PrefillAttnArgs a = {};
+    a.q = e->pf_q;
+    a.out = att;
+    a.st = e->st;
+    a.n_tokens = n;
+    a.start_pos = start_pos;
+    a.gqa = e->gqa;
+    a.kv_heads = e->KVHl;
+    a.q_rows = e->Dq;
+    a.cap = e->pf_cap;
+    a.row0 = l * e->KVHl * c.seq_len;
+    a.seq_len = c.seq_len;
+    // CTAs on the keys of a row tile: as many as leave one CTA per SM and each a tile of keys
+    const int tile_tokens = kFaRows / e->gqa, tiles = (n + tile_tokens - 1) / tile_tokens * e->KVHl, key_tiles = (start_pos + n + kFaKeys - 1) / kFaKeys;
+    a.cluster = 1;
+    while (a.cluster < kFaMaxCluster && tiles * a.cluster * 2 <= e->num_sms && a.cluster * 2 <= key_tiles) a.cluster *= 2;
+    const dim3 grid(tiles * a.cluster), block(kFaThreads);
+    if (e->hs == 64)
+        CU(launch_clusters(prefill_attention_umma_kernel<64>, grid, block, (size_t)fa_smem<64>(), e->stream, true, a.cluster, e->pf_map_k, e->pf_map_v, a));
     else
-        CU(launch_kernel(prefill_attention_kernel, dim3(n, e->KVHl), dim3(32 * e->gqa),
-                         (size_t)e->gqa * e->hs * sizeof(float), e->stream, true, (const float*)e->pf_q,
-                         (const __half*)g.k_cache, (const __half*)g.v_cache, att, n, start_pos, c.seq_len, e->hs,
-                         e->gqa, e->Dq, e->pf_cap));
+        CU(launch_clusters(prefill_attention_umma_kernel<128>, grid, block, (size_t)fa_smem<128>(), e->stream, true, a.cluster, e->pf_map_k, e->pf_map_v, a));
     return LPP_OK;
 }
 

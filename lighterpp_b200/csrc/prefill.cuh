@@ -18,8 +18,8 @@
 // a share; partial sums are added in a fixed order by the next kernel (the norm kernel for the residual
 // projections, prefill_qkv_finish_kernel for QKV).  Activations reach the MMAs as hi + lo FP16 pairs (see
 // split_half); everything between the GEMMs (residual stream, RMSNorm, RoPE, softmax) stays FP32, following
-// src/ops.cpp like the decode path.  The causal attention of the block (prefill_attention_mma_kernel) is a
-// tensor-core flash attention over the cache.
+// src/ops.cpp like the decode path.  The causal attention of the block is a tensor-core
+// flash attention over the cache (prefill_attention.cuh; other head sizes: prefill_attention_kernel).
 //
 // Tensor maps cover this GPU's own memory only; no cluster multicast is used anywhere.
 #pragma once
@@ -763,20 +763,6 @@ static __global__ void __launch_bounds__(256) prefill_attention_kernel(const flo
         }
 }
 
-// Causal attention of the prompt block on the tensor cores: CTA (query tile of 16 tokens, KV head), one warp per
-// query head of the group.  K and V rows stream through shared memory 64 positions at a time (16-byte asynchronous
-// copies, double buffered, rows padded by 16 bytes so that the 8-row matrix loads do not collide on banks); every
-// warp keeps its 16 x head_size query tile as A fragments, forms the 16 x 64 scores with mma.sync m16n8k16, masks
-// them causally, runs the online softmax in FP32 on the accumulator layout, and feeds the probabilities back as A
-// fragments of the P x V product (V read through transposing matrix loads).  Same mathematics as
-// prefill_attention_kernel (src/model.cpp:178-199), FP16 operands with FP32 accumulation.
-constexpr int kPfAttnTile = 64;   // positions per shared-memory tile
-constexpr int kPfAttnRows = 16;   // query tokens per CTA
-template <int HS>
-constexpr int pf_attn_smem() {
-    return 2 /*buffers*/ * 2 /*K, V*/ * kPfAttnTile * (HS * 2 + 16);
-}
-
 __device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src, bool valid) {
     const uint32_t d = smem_u32(dst_smem);
     const int n = valid ? 16 : 0;  // 0 source bytes: the 16 destination bytes are filled with zeros
@@ -791,172 +777,6 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t add
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(addr));
-}
-template <int HS>
-static __global__ void __launch_bounds__(256) prefill_attention_mma_kernel(const float* q, const __half* k_cache,
-                                                                           const __half* v_cache, __half* out, int n_tokens,
-                                                                           int start_pos, int seq_len, int gqa, int q_rows,
-                                                                           int cap) {
-    constexpr int kStride = HS * 2 + 16;              // bytes per padded row
-    constexpr int kMat = kPfAttnTile * kStride;       // bytes of one K or V tile
-    constexpr int kChunks = kPfAttnTile * (HS / 8);   // 16-byte pieces of one tile
-    extern __shared__ __align__(128) unsigned char at_smem[];
-    pdl_launch_dependents();
-    pdl_wait();
-    const int t0 = blockIdx.x * kPfAttnRows, kvh = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, tq = lane & 3;
-    const int h = kvh * gqa + warp;
-    const int rows_here = min(kPfAttnRows, n_tokens - t0);
-    const int t_max = start_pos + t0 + rows_here;  // positions 0 .. t_max - 1 are visible to the last token of the tile
-    const int n_tiles = (t_max + kPfAttnTile - 1) / kPfAttnTile;
-    const unsigned char* kb = reinterpret_cast<const unsigned char*>(k_cache + (size_t)kvh * seq_len * HS);
-    const unsigned char* vb = reinterpret_cast<const unsigned char*>(v_cache + (size_t)kvh * seq_len * HS);
-
-    auto load_tile = [&](int tile, int buf) {
-        unsigned char* ks = at_smem + (size_t)buf * 2 * kMat;
-        unsigned char* vs = ks + kMat;
-        const int p0 = tile * kPfAttnTile;
-        for (int c = threadIdx.x; c < kChunks; c += blockDim.x) {
-            const int row = c / (HS / 8), col = c % (HS / 8);
-            const bool ok = p0 + row < t_max;
-            const size_t src = ok ? ((size_t)(p0 + row) * HS * 2 + (size_t)col * 16) : 0;
-            cp_async_16(ks + row * kStride + col * 16, kb + src, ok);
-            cp_async_16(vs + row * kStride + col * 16, vb + src, ok);
-        }
-    };
-
-    // the query tile of this warp's head as A fragments
-    uint32_t qa[HS / 16][4];
-    {
-        const int r0 = t0 + g, r1 = t0 + g + 8;
-        const float* q0 = q + (size_t)r0 * q_rows + (size_t)h * HS;
-        const float* q1 = q + (size_t)r1 * q_rows + (size_t)h * HS;
-#pragma unroll
-        for (int kk = 0; kk < HS / 16; ++kk) {
-            const int c0 = kk * 16 + 2 * tq;
-            const float2 z = make_float2(0.f, 0.f);
-            const float2 a0 = (r0 < n_tokens) ? *reinterpret_cast<const float2*>(q0 + c0) : z;
-            const float2 a1 = (r1 < n_tokens) ? *reinterpret_cast<const float2*>(q1 + c0) : z;
-            const float2 a2 = (r0 < n_tokens) ? *reinterpret_cast<const float2*>(q0 + c0 + 8) : z;
-            const float2 a3 = (r1 < n_tokens) ? *reinterpret_cast<const float2*>(q1 + c0 + 8) : z;
-            qa[kk][0] = pack_half2(a0.x, a0.y);
-            qa[kk][1] = pack_half2(a1.x, a1.y);
-            qa[kk][2] = pack_half2(a2.x, a2.y);
-            qa[kk][3] = pack_half2(a3.x, a3.y);
-        }
-    }
-    const float scale = __fdiv_rn(1.0f, __fsqrt_rn((float)HS));
-    const int lim0 = (t0 + g < n_tokens) ? start_pos + t0 + g : -1;          // last visible position of row g
-    const int lim1 = (t0 + g + 8 < n_tokens) ? start_pos + t0 + g + 8 : -1;  // ... of row g + 8
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-    float o[HS / 8][4];
-#pragma unroll
-    for (int i = 0; i < HS / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-
-    load_tile(0, 0);
-    cp_async_commit();
-    for (int tile = 0; tile < n_tiles; ++tile) {
-        const int buf = tile & 1;
-        if (tile + 1 < n_tiles) {
-            load_tile(tile + 1, buf ^ 1);
-            cp_async_commit();
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        const uint32_t ks = smem_u32(at_smem + (size_t)buf * 2 * kMat);
-        const uint32_t vs = ks + kMat;
-        const int p0 = tile * kPfAttnTile;
-        // scores of 16 rows x 64 positions
-        float c[kPfAttnTile / 8][4];
-#pragma unroll
-        for (int j = 0; j < kPfAttnTile / 8; ++j) c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.f;
-        const int mi = lane >> 3, mr = lane & 7;
-#pragma unroll
-        for (int jp = 0; jp < kPfAttnTile / 16; ++jp) {
-#pragma unroll
-            for (int kk = 0; kk < HS / 16; ++kk) {
-                uint32_t b[4];
-                ldmatrix_x4(ks + (uint32_t)((jp * 16 + (mi >> 1) * 8 + mr) * kStride + (kk * 16 + (mi & 1) * 8) * 2), b[0], b[1],
-                            b[2], b[3]);
-                mma_f16_16816(c[2 * jp], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], b[0], b[1]);
-                mma_f16_16816(c[2 * jp + 1], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], b[2], b[3]);
-            }
-        }
-        // scale, causal mask, online softmax (rows g and g + 8; a row's 64 scores lie on the four lanes of a quad)
-        float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < kPfAttnTile / 8; ++j) {
-            const int p = p0 + 8 * j + 2 * tq;
-            c[j][0] = (p <= lim0) ? c[j][0] * scale : -INFINITY;
-            c[j][1] = (p + 1 <= lim0) ? c[j][1] * scale : -INFINITY;
-            c[j][2] = (p <= lim1) ? c[j][2] * scale : -INFINITY;
-            c[j][3] = (p + 1 <= lim1) ? c[j][3] * scale : -INFINITY;
-            mx0 = fmaxf(mx0, fmaxf(c[j][0], c[j][1]));
-            mx1 = fmaxf(mx1, fmaxf(c[j][2], c[j][3]));
-        }
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1);
-        const float u0 = (n0 == -INFINITY) ? 0.f : n0, u1 = (n1 == -INFINITY) ? 0.f : n1;  // nothing visible yet
-        const float f0 = __expf(m0 - u0), f1 = __expf(m1 - u1);  // exp(-inf) = 0 on the first visible tile
-        m0 = n0;
-        m1 = n1;
-        l0 *= f0;
-        l1 *= f1;
-#pragma unroll
-        for (int i = 0; i < HS / 8; ++i) {
-            o[i][0] *= f0;
-            o[i][1] *= f0;
-            o[i][2] *= f1;
-            o[i][3] *= f1;
-        }
-        uint32_t pa[kPfAttnTile / 16][4];
-#pragma unroll
-        for (int j = 0; j < kPfAttnTile / 8; ++j) {
-            const float e0 = __expf(c[j][0] - u0), e1 = __expf(c[j][1] - u0);
-            const float e2 = __expf(c[j][2] - u1), e3 = __expf(c[j][3] - u1);
-            l0 += e0 + e1;
-            l1 += e2 + e3;
-            pa[j >> 1][(j & 1) * 2 + 0] = pack_half2(e0, e1);
-            pa[j >> 1][(j & 1) * 2 + 1] = pack_half2(e2, e3);
-        }
-        // o += P x V
-#pragma unroll
-        for (int kk = 0; kk < kPfAttnTile / 16; ++kk) {
-#pragma unroll
-            for (int dp = 0; dp < HS / 16; ++dp) {
-                uint32_t b[4];
-                ldmatrix_x4_trans(b, vs + (uint32_t)((kk * 16 + (mi & 1) * 8 + mr) * kStride + (dp * 16 + (mi >> 1) * 8) * 2));
-                mma_f16_16816(o[2 * dp], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b[0], b[1]);
-                mma_f16_16816(o[2 * dp + 1], pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3], b[2], b[3]);
-            }
-        }
-        __syncthreads();  // the buffer is refilled two iterations from now, by the copy issued in the next one
-    }
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    const int r0 = t0 + g, r1 = t0 + g + 8;
-#pragma unroll
-    for (int i = 0; i < HS / 8; ++i) {
-        const int d = 8 * i + 2 * tq;
-        auto put = [&](int r, float a0, float a1) {
-            __align__(4) __half hi[2], lo[2];
-            split_half(a0, hi[0], lo[0]);
-            split_half(a1, hi[1], lo[1]);
-            *reinterpret_cast<uint32_t*>(out + (size_t)r * q_rows + (size_t)h * HS + d) = *reinterpret_cast<const uint32_t*>(hi);
-            *reinterpret_cast<uint32_t*>(out + (size_t)(cap + r) * q_rows + (size_t)h * HS + d) =
-                *reinterpret_cast<const uint32_t*>(lo);
-        };
-        if (r0 < n_tokens) put(r0, __fdiv_rn(o[i][0], l0), __fdiv_rn(o[i][1], l0));
-        if (r1 < n_tokens) put(r1, __fdiv_rn(o[i][2], l1), __fdiv_rn(o[i][3], l1));
-    }
 }
 
 }  // namespace lpp
