@@ -2677,10 +2677,11 @@ static lpp_status prefill_norm(lpp_engine* e, int n, int block_n, const float* w
     a.part_tokens = prefill_part_tokens(block_n);
     a.splits = embed ? 1 : parts;
     a.st = e->st;
+    const dim3 threads(prefill_norm_threads(a.D, a.splits > 1));
     if (e->c.weight_dtype == LPP_BF16)
-        CU(launch_kernel(prefill_norm_kernel<__nv_bfloat16>, dim3(n), dim3(kPfNormThreads), 0, e->stream, pdl, a));
+        CU(launch_kernel(a.splits > 1 ? prefill_norm_kernel<__nv_bfloat16, true> : prefill_norm_kernel<__nv_bfloat16, false>, dim3(n), threads, 0, e->stream, pdl, a));
     else
-        CU(launch_kernel(prefill_norm_kernel<__half>, dim3(n), dim3(kPfNormThreads), 0, e->stream, pdl, a));
+        CU(launch_kernel(a.splits > 1 ? prefill_norm_kernel<__half, true> : prefill_norm_kernel<__half, false>, dim3(n), threads, 0, e->stream, pdl, a));
     return LPP_OK;
 }
 
@@ -2720,7 +2721,7 @@ static lpp_status prefill_gqa_mixer(lpp_engine* e, int l, int n, int start_pos, 
     prefill_qkv_args(e, l, g);
     const cudaError_t ge = launch_prefill_gemm_t<__half, kPfQkv>(e, e->pf_map_wqkv, e->pf_map_xn, g);
     CU(ge);
-    CU(launch_kernel(prefill_qkv_finish_kernel<__half>, dim3(n, (qkv_rows / 2 + 255) / 256), dim3(256), 0, e->stream, true, g));
+    CU(launch_kernel(prefill_qkv_finish_kernel<__half>, dim3((n + kFinishTokens - 1) / kFinishTokens, (qkv_rows + 1023) / 1024), dim3(256), 0, e->stream, true, g));
     if (cache_only) return LPP_OK;
     __half* att = (__half*)e->pf_att;
     if (e->hs != 64 && e->hs != 128) {

@@ -509,36 +509,107 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
     if (warp == 1) tc_dealloc(tmem, kUmmaTmemCols);
 }
 
-// Finishes a QKV GEMM: adds the partial sums of a row pair in range order and applies the
-// QKV epilogue (rotation of q and k pairs, q -> FP32 rows, k/v -> cache rows at the reference index).
-// grid: (tokens, ceil(row pairs / 256)).
+// N tokens' sums of the partial sums of rows row .. row + 3, tokens t0 .. (clamped to the block: no branches, so the loads of
+// a range of K are in flight together), in range order.
+template <int N>
+__device__ __forceinline__ void prefill_sums(const float* part, int part_tokens, int n_rows, int splits, int n_tokens, int t0, int row, float4 (&v)[N]) {
+    const float4* p[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        p[i] = reinterpret_cast<const float4*>(part + (size_t)min(max(t0 + i, 0), n_tokens - 1) * n_rows + row);
+        v[i] = *p[i];
+    }
+#pragma unroll 2
+    for (int s = 1; s < splits; ++s)
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float4 w = p[i][(size_t)s * part_tokens * n_rows / 4];
+            v[i].x += w.x; v[i].y += w.y; v[i].z += w.z; v[i].w += w.w;
+        }
+}
+
+// Finishes a QKV GEMM: adds the partial sums of the rows in range order and applies the QKV epilogue (rotation of q and k
+// pairs, q -> FP32 rows, k/v -> cache rows at the reference index).  A thread takes four rows (two pairs; there are always whole
+// quads: q rows come in multiples of 64, k and v rows are even and equally many) of kFinishTokens tokens, so that 64 bytes per
+// range of K are in flight and the rotation's table is there before the sums are.  Bound by the traffic through L2.  One pair of
+// one token per thread took 17 us for 1023 tokens of 3072 rows and 40 us for 1000 tokens of 6144 rows (one range).
+// grid: (ceil(tokens / kFinishTokens), ceil(rows / 1024)).
+constexpr int kFinishTokens = 4;
 template <typename CT>
 static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const PrefillGemmArgs a) {
     pdl_launch_dependents();
-    pdl_wait();
-    const int t = blockIdx.x, pr = blockIdx.y * 256 + threadIdx.x;
-    const int row = 2 * pr;
-    if (row >= a.n_rows) return;
-    float2 v = make_float2(0.f, 0.f);
-    float2 p[kPfMaxSplits];
+    const int t0 = blockIdx.x * kFinishTokens, row = 4 * ((int)blockIdx.y * 256 + (int)threadIdx.x), hs = a.head_size;
+    const bool mine = row < a.n_rows;
+    float2 cs[kFinishTokens][2];
+    size_t at[2] = {0, 0};  // in the cache: position 0 of the pair's row
+    const bool is_q = row < a.q_rows;
+    if (mine) {  // constants: ahead of the dependency wait
 #pragma unroll
-    for (int s0 = 0; s0 < kPfMaxSplits; ++s0)
-        if (s0 < a.splits) p[s0] = *reinterpret_cast<const float2*>(a.part + ((size_t)s0 * a.part_tokens + t) * a.n_rows + row);
+        for (int j = 0; j < 2; ++j) {
+            const int r = row + 2 * j;
+            const bool turned = r < a.q_rows + a.kv_rows;
+            const int rr = is_q ? r : r - a.q_rows - (turned ? 0 : a.kv_rows);  // within q, k or v
+            const int h = rr / hs, off = rr - h * hs;
+            at[j] = (size_t)h * ((size_t)a.seq_len * hs) + off;  // h*(seq_len*hs) + pos*hs + off (src/scatter_kv.cu:15-16)
 #pragma unroll
-    for (int s0 = 0; s0 < kPfMaxSplits; ++s0)
-        if (s0 < a.splits) {
-            v.x += p[s0].x;
-            v.y += p[s0].y;
+            for (int i = 0; i < kFinishTokens; ++i) {
+                const int pos = a.start_pos + t0 + i;
+                // adjacent-pair rotation with the table entry for (pos, (row % hs)/2) (src/ops.cpp:34-54)
+                cs[i][j] = turned && pos >= 0 && pos < a.seq_len ? __ldg(a.rope + (size_t)pos * (hs >> 1) + (off >> 1)) : make_float2(1.f, 0.f);
+            }
         }
-    pf_qkv_store<CT>(a, row, t, v.x, v.y);
-    pf_qkv_store<CT>(a, row + 1, t, v.y, v.x);
+    }
+    pdl_wait();
+    if (!mine) return;
+    float4 v[kFinishTokens];
+    prefill_sums<kFinishTokens>(a.part, a.part_tokens, a.n_rows, a.splits, a.n_tokens, t0, row, v);
+#pragma unroll
+    for (int i = 0; i < kFinishTokens; ++i) {
+        const int t = t0 + i, pos = a.start_pos + t;
+        if (t >= a.n_tokens) break;
+        if (pos < 0 || pos >= a.seq_len) {
+            atomicOr(&a.st->status, kStatusBadPos);
+            break;
+        }
+        auto turn = [&](float x, float y, int j) -> float2 {
+            if (row + 2 * j >= a.q_rows + a.kv_rows) return make_float2(x, y);  // v
+            const float2 c = cs[i][j];
+            return make_float2(__fsub_rn(__fmul_rn(x, c.x), __fmul_rn(y, c.y)), __fadd_rn(__fmul_rn(x, c.y), __fmul_rn(y, c.x)));
+        };
+        const float2 p0 = turn(v[i].x, v[i].y, 0), p1 = turn(v[i].z, v[i].w, 1);
+        if (is_q) {
+            *reinterpret_cast<float4*>(a.q + (size_t)t * a.q_rows + row) = make_float4(p0.x, p0.y, p1.x, p1.y);
+        } else {
+            auto put = [&](float2 p, int j) {
+                __align__(8) CT pair[2] = {from_float<CT>(p.x), from_float<CT>(p.y)};
+                CT* dst = reinterpret_cast<CT*>(row + 2 * j < a.q_rows + a.kv_rows ? a.k_cache : a.v_cache) + at[j] + (size_t)pos * hs;
+                if constexpr (sizeof(CT) == 2)
+                    *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(pair);
+                else
+                    *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(pair);
+            };
+            put(p0, 0);
+            put(p1, 1);
+        }
+    }
 }
 
 // Rows of the residual stream -> normalised rows (hi + lo MMA operands): RMSNorm, or LayerNorm when a bias is given.
 // Layer 0 takes the embedding rows of the prompt tokens, times their factor, and also writes them out as the FP32 residual
 // stream.  With a row list, block i takes row rows[i] (the positions whose logits are wanted).  D is the row pitch; the
-// statistics cover the first norm_n inputs, the rest is zero padding with zero weights.  grid: rows.
-constexpr int kPfNormThreads = 512;
+// statistics cover the first norm_n inputs, the rest is zero padding with zero weights.  grid: rows; prefill_norm_threads
+// threads.  Without partial sums there are many rows: a thread has four pieces of four floats, few enough threads and registers
+// that the rows of a block are all resident at once (one or two pieces on 512 threads, two or three rows an SM: 13 us for 1023
+// rows of 2048 and 22 us for 1000 of 4096; now 6 and 11).  With partial sums there are few rows and the latency counts: one
+// or two pieces a thread, all ranges in flight (47 rows of 2048 with 8 ranges: 4.5 us, four pieces a thread 8.3).
+template <bool PARTS>
+struct PfNorm {
+    static constexpr int kPer = PARTS ? 2 : 4, kMaxThreads = PARTS ? 512 : 256;
+};
+static int prefill_norm_threads(int D, bool parts) {
+    const int pieces = parts ? D / 4 : (D / 4 + PfNorm<false>::kPer - 1) / PfNorm<false>::kPer;
+    return std::min(parts ? PfNorm<true>::kMaxThreads : PfNorm<false>::kMaxThreads, std::max(64, (pieces + 31) / 32 * 32));
+}
 struct PrefillNormArgs {
     float* x;            // [tokens][D]
     const int* tokens;   // with emb
@@ -562,24 +633,21 @@ __device__ __forceinline__ float norm_block_sum(float v, float* red, int tid) {
     v = warp_sum(v);
     if ((tid & 31) == 0) red[tid >> 5] = v;
     __syncthreads();
-    float tot = 0.f;
-#pragma unroll
-    for (int k = 0; k < kPfNormThreads / 32; ++k) tot += red[k];
-    return tot;
+    return warp_sum((tid & 31) < (int)(blockDim.x >> 5) ? red[tid & 31] : 0.f);
 }
-// Only the weights (emb, norm_w, norm_b) are loaded as read-only data: a load of what the preceding kernel produced must
-// not become an invariant one, which the compiler may move above the dependency wait.
-template <typename T>
-static __global__ void __launch_bounds__(kPfNormThreads) prefill_norm_kernel(const PrefillNormArgs a) {
-    __shared__ float red[2][kPfNormThreads / 32];
+// PARTS: partial sums are added first.  Only the weights (emb, norm_w, norm_b) are loaded as read-only data: a load of what
+// the preceding kernel produced must not become an invariant one, which the compiler may move above the dependency wait.
+template <typename T, bool PARTS>
+static __global__ void __launch_bounds__(PfNorm<PARTS>::kMaxThreads, PARTS ? 1 : 5) prefill_norm_kernel(const PrefillNormArgs a) {
+    constexpr int kPfNormPer = PfNorm<PARTS>::kPer;
+    __shared__ float red[2][PfNorm<PARTS>::kMaxThreads / 32];
     pdl_launch_dependents();
+    const int tid = threadIdx.x, D = a.D, nt = blockDim.x;
+    const int nv4 = D >> 2;  // D is a multiple of 8
+    float4 v[kPfNormPer];
     pdl_wait();
-    const int tid = threadIdx.x, D = a.D, splits = a.splits;
     const int t = a.rows ? *reinterpret_cast<const volatile int*>(a.rows + blockIdx.x) : (int)blockIdx.x;
     float4* xr = reinterpret_cast<float4*>(a.x + (size_t)t * D);
-    const int nv4 = D >> 2;  // D is a multiple of 8
-    constexpr int kMaxPer = 4;  // float4 per thread kept in registers for the second pass: rows up to 8192 wide
-    float4 v[kMaxPer];
     int tok = 0;
     if (a.emb) {
         tok = *reinterpret_cast<const volatile int*>(a.tokens + t);
@@ -588,85 +656,81 @@ static __global__ void __launch_bounds__(kPfNormThreads) prefill_norm_kernel(con
             tok = 0;
         }
     }
-    const bool add_parts = !a.emb && splits > 1;
-    // one piece of the row: the embedding, or the residual plus all partial sums in range order (every load issued
-    // before the first is used)
-    auto fetch = [&](int i) -> float4 {
-        float4 w, p[kPfMaxSplits];
-        if (a.emb) {
-            const uint2 h = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(a.emb) + (size_t)tok * D + 4 * (size_t)i));
-            const float2 lo = unpack2<T>(h.x), hi = unpack2<T>(h.y);
-            w = make_float4(lo.x * a.emb_scale, lo.y * a.emb_scale, hi.x * a.emb_scale, hi.y * a.emb_scale);
-        } else {
-            w = xr[i];
-        }
-        if (add_parts) {
-#pragma unroll
-            for (int s0 = 0; s0 < kPfMaxSplits; ++s0)
-                if (s0 < splits) p[s0] = reinterpret_cast<const float4*>(a.part + ((size_t)s0 * a.part_tokens + t) * D)[i];
-#pragma unroll
-            for (int s0 = 0; s0 < kPfMaxSplits; ++s0)
-                if (s0 < splits) {
-                    w.x += p[s0].x; w.y += p[s0].y; w.z += p[s0].z; w.w += p[s0].w;
-                }
-        }
-        if (a.add) {
-            const float4 p = __ldg(reinterpret_cast<const float4*>(a.add) + i);
-            w.x += p.x; w.y += p.y; w.z += p.z; w.w += p.w;
-        }
-        if (a.emb || a.add || add_parts) xr[i] = w;  // the residual stream as the next residual GEMM reads it
-        return w;
+    auto load = [&](int i) -> float4 {  // the embedding, or the residual stream
+        if (!a.emb) return xr[i];
+        const uint2 h = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(a.emb) + (size_t)tok * D + 4 * (size_t)i));
+        const float2 lo = unpack2<T>(h.x), hi = unpack2<T>(h.y);
+        return make_float4(lo.x * a.emb_scale, lo.y * a.emb_scale, hi.x * a.emb_scale, hi.y * a.emb_scale);
     };
+    auto part = [&](int s, int i) -> float4 { return reinterpret_cast<const float4*>(a.part + ((size_t)s * a.part_tokens + t) * D)[i]; };
+    auto plus = [](float4& x, const float4& y) { x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w; };
+    const bool store = a.emb || a.add || PARTS;  // the residual stream as the next residual GEMM reads it
     const bool ln = a.norm_b != nullptr;
     const float n = (float)a.norm_n;
     float ss = 0.f;  // RMSNorm: sum of squares; LayerNorm: sum
-    auto first = [&](const float4& w) {
-        ss = ln ? ss + ((w.x + w.y) + (w.z + w.w)) : fmaf(w.x, w.x, fmaf(w.y, w.y, fmaf(w.z, w.z, fmaf(w.w, w.w, ss))));
+    auto first = [&](int i, float4& x) {
+        if (a.add) plus(x, __ldg(reinterpret_cast<const float4*>(a.add) + i));
+        if (store) xr[i] = x;
+        ss = ln ? ss + ((x.x + x.y) + (x.z + x.w)) : fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, ss))));
     };
 #pragma unroll
-    for (int k = 0; k < kMaxPer; ++k) {
-        const int i = tid + k * kPfNormThreads;
-        if (i < nv4) {
-            v[k] = fetch(i);
-            first(v[k]);
+    for (int k = 0; k < kPfNormPer; ++k)
+        if (tid + k * nt < nv4) v[k] = load(tid + k * nt);
+    if constexpr (PARTS) {
+#pragma unroll
+        for (int k = 0; k < kPfNormPer; ++k) {
+            if (tid + k * nt >= nv4) continue;
+            float4 p[kPfMaxSplits];
+#pragma unroll
+            for (int s = 0; s < kPfMaxSplits; ++s)
+                if (s < a.splits) p[s] = part(s, tid + k * nt);
+#pragma unroll
+            for (int s = 0; s < kPfMaxSplits; ++s)  // in range order
+                if (s < a.splits) plus(v[k], p[s]);
         }
     }
-    // rows wider than kMaxPer * kPfNormThreads * 4: the rest without register caching
-    for (int i = tid + kMaxPer * kPfNormThreads; i < nv4; i += kPfNormThreads) first(fetch(i));
+#pragma unroll
+    for (int k = 0; k < kPfNormPer; ++k)
+        if (tid + k * nt < nv4) first(tid + k * nt, v[k]);
+    // rows wider than what the threads keep: the rest without register caching
+    for (int i = tid + kPfNormPer * nt; i < nv4; i += nt) {
+        float4 x = load(i);
+        if constexpr (PARTS)
+            for (int s = 0; s < a.splits; ++s) plus(x, part(s, i));
+        first(i, x);
+    }
     float tot = norm_block_sum(ss, red[0], tid), mean = 0.f;
     if (ln) {
         mean = __fdiv_rn(tot, n);
         float q = 0.f;
-        auto second = [&](int i, const float4& w) {
-            const float d[4] = {w.x - mean, w.y - mean, w.z - mean, w.w - mean};
+        auto second = [&](int i, const float4& x) {
+            const float d[4] = {x.x - mean, x.y - mean, x.z - mean, x.w - mean};
 #pragma unroll
             for (int c = 0; c < 4; ++c)
                 if (4 * i + c < a.norm_n) q = fmaf(d[c], d[c], q);
         };
 #pragma unroll
-        for (int k = 0; k < kMaxPer; ++k) {
-            const int i = tid + k * kPfNormThreads;
-            if (i < nv4) second(i, v[k]);
-        }
-        for (int i = tid + kMaxPer * kPfNormThreads; i < nv4; i += kPfNormThreads) second(i, xr[i]);
+        for (int k = 0; k < kPfNormPer; ++k)
+            if (tid + k * nt < nv4) second(tid + k * nt, v[k]);
+        for (int i = tid + kPfNormPer * nt; i < nv4; i += nt) second(i, xr[i]);
         tot = norm_block_sum(q, red[1], tid);
     }
     const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(tot, n), a.norm_eps)));
     T* out = reinterpret_cast<T*>(a.out) + (size_t)blockIdx.x * D;
     auto emit = [&](int i, const float4& xv) {
-        const float4 w = __ldg(reinterpret_cast<const float4*>(a.norm_w) + i);
+        const float4 wv = __ldg(reinterpret_cast<const float4*>(a.norm_w) + i);
         float y[4];
         if (ln) {
             const float4 b = __ldg(reinterpret_cast<const float4*>(a.norm_b) + i);
-            y[0] = fmaf(__fmul_rn(xv.x - mean, scale), w.x, b.x);
-            y[1] = fmaf(__fmul_rn(xv.y - mean, scale), w.y, b.y);
-            y[2] = fmaf(__fmul_rn(xv.z - mean, scale), w.z, b.z);
-            y[3] = fmaf(__fmul_rn(xv.w - mean, scale), w.w, b.w);
+            y[0] = fmaf(__fmul_rn(xv.x - mean, scale), wv.x, b.x);
+            y[1] = fmaf(__fmul_rn(xv.y - mean, scale), wv.y, b.y);
+            y[2] = fmaf(__fmul_rn(xv.z - mean, scale), wv.z, b.z);
+            y[3] = fmaf(__fmul_rn(xv.w - mean, scale), wv.w, b.w);
         } else {
-            y[0] = __fmul_rn(__fmul_rn(xv.x, scale), w.x);
-            y[1] = __fmul_rn(__fmul_rn(xv.y, scale), w.y);
-            y[2] = __fmul_rn(__fmul_rn(xv.z, scale), w.z);
-            y[3] = __fmul_rn(__fmul_rn(xv.w, scale), w.w);
+            y[0] = __fmul_rn(__fmul_rn(xv.x, scale), wv.x);
+            y[1] = __fmul_rn(__fmul_rn(xv.y, scale), wv.y);
+            y[2] = __fmul_rn(__fmul_rn(xv.z, scale), wv.z);
+            y[3] = __fmul_rn(__fmul_rn(xv.w, scale), wv.w);
         }
         __align__(8) T hi[4], lo[4];
 #pragma unroll
@@ -675,11 +739,9 @@ static __global__ void __launch_bounds__(kPfNormThreads) prefill_norm_kernel(con
         *reinterpret_cast<uint2*>(out + (size_t)a.cap * D + 4 * (size_t)i) = *reinterpret_cast<const uint2*>(lo);
     };
 #pragma unroll
-    for (int k = 0; k < kMaxPer; ++k) {
-        const int i = tid + k * kPfNormThreads;
-        if (i < nv4) emit(i, v[k]);
-    }
-    for (int i = tid + kMaxPer * kPfNormThreads; i < nv4; i += kPfNormThreads) emit(i, xr[i]);  // re-read what this thread wrote
+    for (int k = 0; k < kPfNormPer; ++k)
+        if (tid + k * nt < nv4) emit(tid + k * nt, v[k]);
+    for (int i = tid + kPfNormPer * nt; i < nv4; i += nt) emit(i, xr[i]);  // re-read what this thread wrote
 }
 
 // Causal attention of the prompt block: query token t (position start_pos + t) over cache rows 0..start_pos + t,

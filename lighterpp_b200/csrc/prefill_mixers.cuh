@@ -72,24 +72,6 @@ struct MambaConvArgs {
     __nv_bfloat16* planes;  // [2 planes][cap][x_pitch]
     StepState* st;
 };
-// N tokens' sums of the partial sums of rows row .. row + 3, tokens t0 .. (clamped to the block: no branches, so the loads of
-// a range of K are in flight together), in range order.
-template <int N>
-__device__ __forceinline__ void prefill_sums(const float* part, int part_tokens, int n_rows, int splits, int n_tokens, int t0, int row, float4 (&v)[N]) {
-    const float4* p[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        p[i] = reinterpret_cast<const float4*>(part + (size_t)min(max(t0 + i, 0), n_tokens - 1) * n_rows + row);
-        v[i] = *p[i];
-    }
-#pragma unroll 2
-    for (int s = 1; s < splits; ++s)
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const float4 w = p[i][(size_t)s * part_tokens * n_rows / 4];
-            v[i].x += w.x; v[i].y += w.y; v[i].z += w.z; v[i].w += w.w;
-        }
-}
 // With the fast exponential and division, like the gated feed-forward's activation on this path.
 __device__ __forceinline__ float4 silu4(const float4& v) {
     return make_float4(__fdividef(v.x, 1.f + __expf(-v.x)), __fdividef(v.y, 1.f + __expf(-v.y)), __fdividef(v.z, 1.f + __expf(-v.z)),
