@@ -41,6 +41,7 @@
 #include "prefill.cuh"
 #include "prefill_pair.cuh"
 #include "prefill_attention.cuh"
+#include "row_attention.cuh"
 #include "prefill_f32.cuh"
 #include "prefill_mixers.cuh"
 #include "sampler.cuh"
@@ -150,6 +151,7 @@ struct ModelLayer {
     PrefillMap m_in, m_wo, m_w13, m_w2, x_att, x_hb;    // weights, activation blocks with this layer's widths (batched path)
     // attention over shared rows (latent_attention.cuh): heads of a group, groups, value part and whole of a row
     int group_heads = 0, groups = 0, rank_pitch = 0, row_width = 0;
+    CUtensorMap x_rows;         // query rows of a prompt block (row_attention.cuh)
     const float2* rope = nullptr;
     // latent attention (latent.cuh)
     int dim_pitch, val_pitch;   // inputs per head of the query and of the value matrix
@@ -172,6 +174,7 @@ struct LayerRun {
     int layer;
     int step_row = -1;          // row of the loop's vectors that is added before this run, -1 = none
     void* cache = nullptr;      // [groups][seq_len][row_width]
+    CUtensorMap m_rows;         // the same as (columns, rows)
     float* ring = nullptr;      // convolution inputs [taps - 1][inner_rows]
     float* S = nullptr;         // recurrent state [inner][state_pitch]
     // vectors added with the output and with the down projection: the output's bias, and the loop's vector that comes before
@@ -2536,6 +2539,31 @@ static size_t prefill_carve(lpp_engine* e, int cap, char* base) {
     }
     return c.used;
 }
+// FP16 rows of `cols` elements as (columns, `inner` rows, `outer` times as many), boxes of 64 columns x box_inner x box_outer
+// rows; columns beyond `cols` read as zero.
+static lpp_status encode_row_map(CUtensorMap* m, const void* base, size_t cols, size_t inner, size_t outer, int box_inner, int box_outer) {
+    encode_tiled_fn encode = tensor_map_encoder();
+    if (!encode) return fail(LPP_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+    const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)inner, (cuuint64_t)outer};
+    const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)(cols * inner) * 2};
+    const cuuint32_t box[3] = {64u, (cuuint32_t)box_inner, (cuuint32_t)box_outer};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, outer > 0 ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(LPP_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for rows of %zu", (int)r, cols);
+    return LPP_OK;
+}
+// Attention over shared rows of n tokens on tcgen05: the sizes it takes, and how many CTAs it makes.
+static bool row_attention_fits(const lpp_engine* e, const ModelLayer& y) {
+    return latent_mma_supported(e, y) && y.row_width >= 64 && y.group_heads <= kRaRows &&
+           (size_t)ra_fixed(y.row_width) + kRaMinSlots * kRaPiece + kRaStatic <= e->smem_optin;
+}
+static int row_attention_halves(const ModelLayer& y) { return y.rank_pitch > 256 ? 2 : 1; }
+static int row_attention_ctas(const ModelLayer& y, int n) {
+    const int tokens = kRaRows / y.group_heads;
+    return (n + tokens - 1) / tokens * row_attention_halves(y) * y.groups;
+}
 static lpp_status prefill_maps(lpp_engine* e) {
     const lpp_config& c = e->c;
     if (prefill_f32(e)) return LPP_OK;
@@ -2561,6 +2589,14 @@ static lpp_status prefill_maps(lpp_engine* e) {
                 TRY(make_activation_map(&y.x_hb, e->pf_hb, T, y.ff_pitch));
             }
         }
+        for (LayerRun& r : e->runs) {
+            ModelLayer& y = e->layers[r.layer];
+            if (y.d.mixer == LPP_MIXER_MAMBA || !row_attention_fits(e, y)) continue;
+            TRY(encode_row_map(&y.x_rows, e->pf_lq, y.row_width, y.group_heads * y.groups, T, y.group_heads, kRaRows / y.group_heads));
+            TRY(encode_row_map(&r.m_rows, r.cache, y.row_width, (size_t)y.groups * c.seq_len, 0, kRaKeys, 1));
+        }
+        CU(cudaFuncSetAttribute(row_attention_umma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem_optin - kRaStatic));
+        CU(cudaFuncSetAttribute(row_attention_umma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem_optin - kRaStatic));
         TRY(allow_gemm_smem<__nv_bfloat16>());
         CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<__nv_bfloat16, kPfLatentQuery>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
         CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<__nv_bfloat16, kPfLatentValue>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
@@ -2777,7 +2813,20 @@ static lpp_status prefill_row_attention(lpp_engine* e, const ModelLayer& y, cons
     a.cap = e->pf_cap;
     a.out = nullptr;
     if (a.gate) a.gate = e->pf_gate;
-    CU(launch_latent_attn(e, p, a, y.d.mixer == LPP_MIXER_SHARED_KV, true, e->stream));
+    const bool skv = y.d.mixer == LPP_MIXER_SHARED_KV;
+    const int ctas = row_attention_ctas(y, n);
+    if (row_attention_fits(e, y) && 2 * ctas >= e->num_sms) {
+        RowAttnArgs ra = {};
+        ra.a = a;
+        ra.halves = row_attention_halves(y);
+        ra.pieces = (ra_pieces(y.rank_pitch) + ra.halves - 1) / ra.halves;
+        ra.slots = (int)std::min<size_t>(kRaMaxSlots, (e->smem_optin - kRaStatic - ra_fixed(y.row_width)) / kRaPiece);
+        const size_t smem = (size_t)ra_fixed(y.row_width) + ra.slots * kRaPiece;
+        CU(launch_kernel(skv ? row_attention_umma_kernel<true> : row_attention_umma_kernel<false>, dim3(ctas), dim3(kFaThreads), smem, e->stream, true,
+                         y.x_rows, r.m_rows, ra));
+        return LPP_OK;
+    }
+    CU(launch_latent_attn(e, p, a, skv, true, e->stream));
     if (!p.cluster)
         CU(launch_kernel(prefill_latent_combine_kernel, dim3(n * a.all_heads), dim3(128), 0, e->stream, true, a, p.tile_rows));
     return LPP_OK;

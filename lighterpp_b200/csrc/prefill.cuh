@@ -202,6 +202,13 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// True in one thread of a converged warp, the same one every time.  The MMA and commit instructions take their operands from
+// the warp's uniform registers; behind a branch on the lane number the compiler has to assume several threads.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -337,7 +344,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     int* s_fail = reinterpret_cast<int*>(tmem_slot + 1);  // set by a role whose wait ran out
     const uint32_t ring = (smem_u32(smem) + 1024u + 1023u) & ~1023u;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int unit = blockIdx.x, n_units = gridDim.x;
     const int group_tiles = (a.n_rows + kUmmaM - 1) / kUmmaM;  // row tiles of one matrix
     const int n_tiles = group_tiles * max(1, a.groups);        // items along the rows
@@ -421,7 +428,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
         }
     } else if (warp == 1) {
         // ---------------- MMA issue
-        if (lane == 0) {
+        {
             int slot = 0;
             uint32_t par = 0;
             bool ok = true;
@@ -445,23 +452,27 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
                     tc_fence_after();
                     PF_STAMP(18 + kc - kc0);
                     const uint32_t st = ring + (uint32_t)slot * kStage;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int sub = 0; sub < 2; ++sub) {
-                        // the activation sub-tile holds the hi rows followed by the lo rows: one MMA covers both (N = 128)
-                        const uint32_t wt = st + sub * kUmmaSubW, xt = st + 2 * kUmmaSubW + sub * 2 * kSubX;
+                        for (int sub = 0; sub < 2; ++sub) {
+                            // the activation sub-tile holds the hi rows followed by the lo rows: one MMA covers both (N = 128)
+                            const uint32_t wt = st + sub * kUmmaSubW, xt = st + 2 * kUmmaSubW + sub * 2 * kSubX;
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {  // 16 inputs = 32 bytes along the swizzled row per step
-                            const uint32_t acc = (kc > kc0 || sub > 0 || ks > 0) ? 1u : 0u;
-                            tc_mma_f16(d_tmem, umma_desc(wt + ks * 32), umma_desc(xt + ks * 32), umma_idesc<T>(), acc);
+                            for (int ks = 0; ks < 4; ++ks) {  // 16 inputs = 32 bytes along the swizzled row per step
+                                const uint32_t acc = (kc > kc0 || sub > 0 || ks > 0) ? 1u : 0u;
+                                tc_mma_f16(d_tmem, umma_desc(wt + ks * 32), umma_desc(xt + ks * 32), umma_idesc<T>(), acc);
+                            }
                         }
+                        tc_commit(&empty[slot]);  // arrives once the MMAs issued so far have read this stage
                     }
-                    tc_commit(&empty[slot]);  // arrives once the MMAs issued so far have read this stage
+                    __syncwarp();
                     if (++slot == kStages) {
                         slot = 0;
                         par ^= 1u;
                     }
                 }
-                if (ok) tc_commit(&acc_full[b]);
+                if (ok && elect_one()) tc_commit(&acc_full[b]);
+                __syncwarp();
             }
         }
     } else {

@@ -76,7 +76,7 @@ static __global__ void __launch_bounds__(kFaThreads, 1) prefill_attention_umma_k
     int* s_fail = reinterpret_cast<int*>(tmem_slot + 1);
     const uint32_t base = (smem_u32(smem) + 1024u + 1023u) & ~1023u;
     const uint32_t sq = base, sk = sq + kTile, sv = sk + 2 * kTile, sp = sv + 2 * kTile;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int rank = a.cluster > 1 ? (int)cluster_rank() : 0, work = blockIdx.x / a.cluster;
     const int kvh = work % a.kv_heads, tile_tokens = kFaRows / a.gqa;
     const int row_tile = (a.n_tokens + tile_tokens - 1) / tile_tokens - 1 - work / a.kv_heads;
@@ -145,7 +145,7 @@ static __global__ void __launch_bounds__(kFaThreads, 1) prefill_attention_umma_k
             if (!mbar_wait_bounded(&k_full[b], (uint32_t)(it >> 1) & 1u, a.st)) return false;
             if (it >= 2 && !mbar_wait_bounded(&s_free[b], (uint32_t)((it >> 1) - 1) & 1u, a.st)) return false;
             tc_fence_after();
-            if (lane == 0) {
+            if (elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < HS / 16; ++ks) {
                     const uint32_t off = (uint32_t)((ks >> 2) * kFaSub + (ks & 3) * 32);
@@ -174,7 +174,7 @@ static __global__ void __launch_bounds__(kFaThreads, 1) prefill_attention_umma_k
             ok = mbar_wait_bounded(p_ready, (uint32_t)it & 1u, a.st) && (it < 2 || mbar_wait_bounded(&pv_free[b], (uint32_t)((it >> 1) - 1) & 1u, a.st));
             if (!ok) break;
             tc_fence_after();
-            if (lane == 0) {
+            if (elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < kFaKeys / 16; ++ks)
                     tc_mma_f16(tmem + 256 + b * 128, umma_desc(sp + (uint32_t)((ks >> 2) * kFaSub + (ks & 3) * 32)), fa_desc_mn(sv + b * kTile + ks * 2048),

@@ -117,7 +117,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_pair_kern
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     int* s_fail = reinterpret_cast<int*>(tmem_slot + 1);  // set by a role whose wait ran out
     const uint32_t ring = (smem_u32(smem) + 1024u + 1023u) & ~1023u;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int rank = (int)cluster_rank(), unit = blockIdx.x >> 1, n_units = gridDim.x >> 1;
     const int row_tiles = (a.n_rows + kPairM - 1) / kPairM, tok_tiles = (a.n_tokens + kPairTokens - 1) / kPairTokens;
     const int n_kc = a.K / 64, S = a.splits;
@@ -193,7 +193,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_pair_kern
         }
     } else if (warp == 1) {
         // ---------------- MMA issue for the pair
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             int slot = 0, it = 0;
             uint32_t par = 0;
             bool ok = true;
@@ -217,16 +217,20 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_pair_kern
                         }
                         tc_fence_after();
                         const uint32_t wt = ring + (uint32_t)slot * kStage, xt = wt + kPairSub;
+                        if (elect_one()) {
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks)  // 16 inputs = 32 bytes along the swizzled row per step
-                            pair_mma(d_tmem, umma_desc(wt + ks * 32), umma_desc(xt + ks * 32), pair_idesc<T>(), (kc > k0 || ks > 0) ? 1u : 0u);
-                        pair_commit(&empty[slot]);  // arrives in both CTAs once the MMAs issued so far have read this stage
+                            for (int ks = 0; ks < 4; ++ks)  // 16 inputs = 32 bytes along the swizzled row per step
+                                pair_mma(d_tmem, umma_desc(wt + ks * 32), umma_desc(xt + ks * 32), pair_idesc<T>(), (kc > k0 || ks > 0) ? 1u : 0u);
+                            pair_commit(&empty[slot]);  // arrives in both CTAs once the MMAs issued so far have read this stage
+                        }
+                        __syncwarp();
                         if (++slot == kStages) {
                             slot = 0;
                             par ^= 1u;
                         }
                     }
-                    if (ok) pair_commit(&acc_full[b]);
+                    if (ok && elect_one()) pair_commit(&acc_full[b]);
+                    __syncwarp();
                 }
             }
         }
