@@ -324,6 +324,14 @@ lpp_status lpp_op_rope_scatter(float* d_q, const float* d_k, const float* d_v, v
 lpp_status lpp_op_sample(float* d_logits, int vocab_size, float temperature, float penalty, const int* d_history,
                          int history_len, float r, int* d_sampled_token, void* stream);
 
+/* lpp_op_sample with scratch of the caller's: at least lpp_op_sample_scratch_bytes(vocab_size) bytes of device memory (-1: no
+ * such vocabulary, or no device) on a 256-byte boundary, which the call uses in stream order and leaves to the caller.  A caching
+ * allocator serves it at once, where the stream-ordered allocator of lpp_op_sample gives its memory back to the system at the
+ * next synchronisation and takes 0.4 ms to get it again. */
+int64_t lpp_op_sample_scratch_bytes(int vocab_size);
+lpp_status lpp_op_sample_on(void* scratch, int64_t scratch_bytes, float* d_logits, int vocab_size, float temperature, float penalty,
+                            const int* d_history, int history_len, float r, int* d_sampled_token, void* stream);
+
 /* lpp_op_sample for callers that must not allocate.  No counterpart in the reference: its
  * cuda_sample works in place with shared memory only, while this library's multi-block sampler needs
  * global scratch (step state, per-block partials, counters, the entry lists of the exact-order kernel)

@@ -118,46 +118,11 @@ constexpr SampleScratch sample_scratch_layout(int cap_blocks, bool exact) {
     return L;
 }
 
-// Launches the sampler on logits with its scratch at `scratch` (laid out by sample_scratch_layout for
-// cap_blocks >= the blocks of this vocabulary).  The step state at the head of the scratch and the zeroed
-// counters are the caller's business.  The exact-order kernel (ids equal to the reference's sequential CPU
-// sample()) needs all its blocks co-resident; a vocabulary beyond that takes the tree-sum kernel.
-void launch_sampler_on_scratch(char* scratch, const SampleScratch& L, bool exact, float* d_logits, int vocab_size,
-                               int nb, cudaStream_t s) {
-    SampleArgs a = {};
-    a.logits = d_logits;
-    a.vocab = vocab_size;
-    a.st = (StepState*)(scratch + L.state);
-    a.part_max = (float*)(scratch + L.part);
-    a.part_idx = (int*)(scratch + L.part + (size_t)nb * 4);
-    a.part_sum = (float*)(scratch + L.part + (size_t)nb * 8);
-    a.counter = (unsigned int*)(scratch + L.counters);
-    if (exact) {
-        SampleExactArgs ea = {};
-        ea.base = a;
-        ea.sync = (unsigned int*)(scratch + L.counters + 256);
-        ea.block_sum = (double*)(scratch + L.sums);
-        ea.entry_count = (int*)(scratch + L.counts);
-        ea.entries = (ExactEntry*)(scratch + L.entries);
-        sample_exact_kernel<<<nb, kSampleThreads, 0, s>>>(ea);
-    } else {
-        sample_kernel<<<nb, kSampleThreads, 0, s>>>(a);
-    }
-}
-
-// ---- scratch for lpp_op_sample_static: lives in the library image, one copy per GPU that loads it
-constexpr int kStaticSampleMaxVocab = 262144;  // 128 blocks of kSampleChunk logits
-constexpr int kStaticSampleBlocks = kStaticSampleMaxVocab / kSampleChunk;
-constexpr SampleScratch kStaticLayout = sample_scratch_layout(kStaticSampleBlocks, true);
-static __device__ __align__(256) unsigned char g_sample_scratch[kStaticLayout.total];
-// Device addresses of g_sample_scratch, one per CUDA device, filled in on first use.  In host code
-// the name g_sample_scratch is only a handle for cudaGetSymbolAddress, never a pointer to pass on.
-static unsigned char* g_sample_scratch_addr[64];
-
 // Writes the step-state header the sampler reads, copies the history device-to-device and zeroes
-// the ticket counter -- everything in the shared scratch that must not survive from the last call.
-static __global__ void sample_static_setup_kernel(StepState* st, unsigned int* counters, float temperature,
-                                                  float penalty, float r, const int* history, int history_len) {
+// the counters -- everything in the scratch that has to start clean.
+__global__ void __launch_bounds__(256) sample_setup_kernel(StepState* st, unsigned int* counters, float temperature, float penalty, float r,
+                                                           const int* history, int history_len) {
+    op_begin();
     if (threadIdx.x == 0) {
         st->token = 0;
         st->pos = 0;
@@ -175,11 +140,59 @@ static __global__ void sample_static_setup_kernel(StepState* st, unsigned int* c
         st->tp_wait_cycles = 0;
     }
     if (threadIdx.x < 128) counters[threadIdx.x] = 0u;  // ticket counter, barrier counter, exit ticket
-    if (threadIdx.x == 0) {
-    }
     for (int i = threadIdx.x; i < history_len; i += blockDim.x) st->history[i] = history[i];
 }
-static __global__ void sample_static_publish_kernel(const StepState* st, int* dst) { *dst = st->out_token; }
+
+// What a call on a vocabulary of this size launches.
+struct SamplePlan {
+    int blocks;
+    bool exact;  // the exact-order kernel (ids equal to the reference's sequential CPU sample()) needs all its blocks co-resident
+};
+lpp_status sample_plan(int vocab_size, SamplePlan* p) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return LPP_ERR_CUDA;
+    p->blocks = (vocab_size + kSampleChunk - 1) / kSampleChunk;
+    p->exact = p->blocks <= sms;
+    return p->blocks > kSampleMaxBlocks ? LPP_ERR_TOO_LARGE : LPP_OK;
+}
+
+// Runs the sampler on logits with its scratch at `scratch` (laid out by sample_scratch_layout for at least the blocks of this
+// vocabulary): two launches, everything that a call needs travels as kernel arguments.  (Header and counters as copies and a
+// memset, the token as another copy: four more operations of the stream between the launches.)
+lpp_status run_sampler(char* scratch, const SampleScratch& L, const SamplePlan& plan, float* d_logits, int vocab_size, float temperature, float penalty,
+                       const int* d_history, int history_len, float r, int* d_token, cudaStream_t s) {
+    const int nb = plan.blocks;
+    const bool use_hist = penalty > 1.0f && d_history && history_len > 0;
+    const lpp_status st = launch_op(sample_setup_kernel, dim3(1), 256, 0, s, (StepState*)(scratch + L.state), (unsigned int*)(scratch + L.counters),
+                                    temperature, penalty, r, use_hist ? d_history : nullptr, use_hist ? history_len : 0);
+    if (st != LPP_OK) return st;
+    SampleArgs a = {};
+    a.logits = d_logits;
+    a.vocab = vocab_size;
+    a.st = (StepState*)(scratch + L.state);
+    a.part_max = (float*)(scratch + L.part);
+    a.part_idx = (int*)(scratch + L.part + (size_t)nb * 4);
+    a.part_sum = (float*)(scratch + L.part + (size_t)nb * 8);
+    a.counter = (unsigned int*)(scratch + L.counters);
+    a.token_out = d_token;
+    if (!plan.exact) return launch_op(sample_kernel, dim3(nb), kSampleThreads, 0, s, a);
+    SampleExactArgs ea = {};
+    ea.base = a;
+    ea.sync = (unsigned int*)(scratch + L.counters + 256);
+    ea.block_sum = (double*)(scratch + L.sums);
+    ea.entry_count = (int*)(scratch + L.counts);
+    ea.entries = (ExactEntry*)(scratch + L.entries);
+    return launch_op(sample_exact_kernel, dim3(nb), kSampleThreads, 0, s, ea);
+}
+
+// ---- scratch for lpp_op_sample_static: lives in the library image, one copy per GPU that loads it
+constexpr int kStaticSampleMaxVocab = 262144;  // 128 blocks of kSampleChunk logits
+constexpr int kStaticSampleBlocks = kStaticSampleMaxVocab / kSampleChunk;
+constexpr SampleScratch kStaticLayout = sample_scratch_layout(kStaticSampleBlocks, true);
+static __device__ __align__(256) unsigned char g_sample_scratch[kStaticLayout.total];
+// Device addresses of g_sample_scratch, one per CUDA device, filled in on first use.  In host code
+// the name g_sample_scratch is only a handle for cudaGetSymbolAddress, never a pointer to pass on.
+static unsigned char* g_sample_scratch_addr[64];
 
 }  // namespace
 
@@ -287,35 +300,38 @@ lpp_status lpp_op_rope_scatter(float* d_q, const float* d_k, const float* d_v, v
                      layer, pos, dim, n_kv_heads, head_size, seq_len, rope_base);
 }
 
+int64_t lpp_op_sample_scratch_bytes(int vocab_size) {
+    SamplePlan p = {};
+    if (vocab_size <= 0 || sample_plan(vocab_size, &p) != LPP_OK) return -1;
+    return (int64_t)sample_scratch_layout(p.blocks, p.exact).total;
+}
+
+lpp_status lpp_op_sample_on(void* scratch, int64_t scratch_bytes, float* d_logits, int vocab_size, float temperature, float penalty,
+                            const int* d_history, int history_len, float r, int* d_sampled_token, void* stream) {
+    if (!scratch || ((uintptr_t)scratch & 255) || !d_logits || !d_sampled_token || vocab_size <= 0 || history_len < 0 || history_len > kHistoryMax)
+        return LPP_ERR_INVALID_ARG;
+    SamplePlan p = {};
+    const lpp_status st = sample_plan(vocab_size, &p);
+    if (st != LPP_OK) return st;
+    const SampleScratch L = sample_scratch_layout(p.blocks, p.exact);
+    if (scratch_bytes < (int64_t)L.total) return LPP_ERR_INVALID_ARG;
+    return run_sampler((char*)scratch, L, p, d_logits, vocab_size, temperature, penalty, d_history, history_len, r, d_sampled_token, S(stream));
+}
+
 lpp_status lpp_op_sample(float* d_logits, int vocab_size, float temperature, float penalty, const int* d_history,
                          int history_len, float r, int* d_sampled_token, void* stream) {
     if (!d_logits || !d_sampled_token || vocab_size <= 0 || history_len < 0 || history_len > kHistoryMax)
         return LPP_ERR_INVALID_ARG;
     cudaStream_t s = S(stream);
-    const int nb = (vocab_size + kSampleChunk - 1) / kSampleChunk;
-    if (nb > kSampleMaxBlocks) return LPP_ERR_TOO_LARGE;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return LPP_ERR_CUDA;
-    const bool exact = nb <= sms;  // see launch_sampler_on_scratch
-    const SampleScratch L = sample_scratch_layout(nb, exact);  // stream-ordered scratch, sized for this call
+    SamplePlan p = {};
+    lpp_status st = sample_plan(vocab_size, &p);
+    if (st != LPP_OK) return st;
+    const SampleScratch L = sample_scratch_layout(p.blocks, p.exact);  // stream-ordered scratch, sized for this call
     char* scratch = nullptr;
     if (cudaMallocAsync((void**)&scratch, L.total, s) != cudaSuccess) return LPP_ERR_CUDA;
-    StepState h = {};
-    h.temperature = temperature;
-    h.penalty = penalty;
-    h.r = r;
-    const bool use_hist = penalty > 1.0f && d_history && history_len > 0;
-    h.history_len = use_hist ? history_len : 0;
-    cudaMemcpyAsync(scratch + L.state, &h, offsetof(StepState, history), cudaMemcpyHostToDevice, s);
-    if (use_hist)
-        cudaMemcpyAsync(scratch + L.state + offsetof(StepState, history), d_history, (size_t)history_len * sizeof(int),
-                        cudaMemcpyDeviceToDevice, s);
-    cudaMemsetAsync(scratch + L.counters, 0, 512, s);
-    launch_sampler_on_scratch(scratch, L, exact, d_logits, vocab_size, nb, s);
-    cudaMemcpyAsync(d_sampled_token, scratch + offsetof(StepState, out_token), sizeof(int), cudaMemcpyDeviceToDevice, s);
+    st = run_sampler(scratch, L, p, d_logits, vocab_size, temperature, penalty, d_history, history_len, r, d_sampled_token, s);
     cudaFreeAsync(scratch, s);
-    return chk();
+    return st != LPP_OK ? st : chk();
 }
 
 lpp_status lpp_op_sample_static(float* d_logits, int vocab_size, float temperature, float penalty,
@@ -346,17 +362,10 @@ lpp_status lpp_op_sample_static(float* d_logits, int vocab_size, float temperatu
     }
     unsigned char* scratch = g_sample_scratch_addr[dev];
     cudaStream_t s = S(stream);
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return LPP_ERR_CUDA;
-    const int nb = (vocab_size + kSampleChunk - 1) / kSampleChunk;
-    const bool exact = nb <= sms;  // the same choice of kernel as lpp_op_sample
-    const bool use_hist = penalty > 1.0f && d_history && history_len > 0;
-    sample_static_setup_kernel<<<1, 256, 0, s>>>((StepState*)(scratch + kStaticLayout.state),
-                                                 (unsigned int*)(scratch + kStaticLayout.counters), temperature, penalty, r,
-                                                 use_hist ? d_history : nullptr, use_hist ? history_len : 0);
-    launch_sampler_on_scratch((char*)scratch, kStaticLayout, exact, d_logits, vocab_size, nb, s);
-    sample_static_publish_kernel<<<1, 1, 0, s>>>((const StepState*)(scratch + kStaticLayout.state), d_sampled_token);
-    return chk();
+    SamplePlan p = {};
+    const lpp_status st = sample_plan(vocab_size, &p);  // the same choice of kernel as lpp_op_sample
+    if (st != LPP_OK) return st;
+    return run_sampler((char*)scratch, kStaticLayout, p, d_logits, vocab_size, temperature, penalty, d_history, history_len, r, d_sampled_token, s);
 }
 
 }  // extern "C"

@@ -36,6 +36,7 @@ struct SampleArgs {
     unsigned int* counter;  // zero between launches
     const float* r_values;  // free-running mode: one uniform draw per step
     int* out_tokens;        // free-running mode: sampled token per step
+    int* token_out;         // where the token goes besides the step state (nullptr = nowhere)
     unsigned int* zero;     // counters to clear once the step is over (grid-barrier tickets), may be null
     int zero_n;
     unsigned int* bump;     // word to increment once the step is over (tensor-parallel exchange epoch), may be null
@@ -229,6 +230,7 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const Sam
 
     if (tid == 0) {
         st->out_token = token;
+        if (a.token_out) *a.token_out = token;
         if (st->advance) {
             const int k = st->step_idx;
             a.out_tokens[k] = token;

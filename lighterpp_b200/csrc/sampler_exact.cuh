@@ -691,6 +691,7 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_exact_kernel(con
     __syncthreads();
     if (blockIdx.x == 0 && tid == 0) {
         st->out_token = token;
+        if (a.token_out) *a.token_out = token;
         if (st->advance) {
             const int k = st->step_idx;
             a.out_tokens[k] = token;

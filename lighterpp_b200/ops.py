@@ -41,6 +41,9 @@ def _lib():
         lib.lpp_op_multihead_gemv.argtypes = [vp, vp, vp, i, i, i, i, i, i, vp]
         lib.lpp_op_rope_scatter.argtypes = [vp, vp, vp, vp, vp, i, i, i, i, i, i, f, vp]
         lib.lpp_op_sample.argtypes = [vp, i, f, f, vp, i, f, vp, vp]
+        lib.lpp_op_sample_on.argtypes = [vp, i64, vp, i, f, f, vp, i, f, vp, vp]
+        lib.lpp_op_sample_scratch_bytes.argtypes = [i]
+        lib.lpp_op_sample_scratch_bytes.restype = i64
         lib._ops_bound = True
     return lib
 
@@ -107,6 +110,11 @@ def cuda_rope_scatter(d_q, d_k, d_v, d_key_cache, d_value_cache, layer, pos, dim
 
 def cuda_sample(d_logits, vocab_size, temperature, penalty, d_history, history_len, r, d_sampled_token):
     """``r`` is passed in (the reference wrapper draws it from rand(), src/sample.cu:211)."""
+    lib = _lib()
     hp = _p(d_history) if d_history is not None and history_len > 0 else C.c_void_p(None)
-    _check(_lib().lpp_op_sample(_p(d_logits), int(vocab_size), float(temperature), float(penalty), hp, int(history_len),
-                                float(r), _p(d_sampled_token), _s()), "cuda_sample")
+    logits, token = _p(d_logits), _p(d_sampled_token)
+    n = lib.lpp_op_sample_scratch_bytes(int(vocab_size))
+    # torch's allocator hands blocks on in stream order, so the scratch may be let go as soon as the work is queued
+    scratch = torch.empty(max(n, 1), dtype=torch.uint8, device=d_logits.device)
+    _check(lib.lpp_op_sample_on(_p(scratch), n, logits, int(vocab_size), float(temperature), float(penalty), hp, int(history_len),
+                                float(r), token, _s()), "cuda_sample")
