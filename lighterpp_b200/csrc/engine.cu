@@ -2815,7 +2815,10 @@ static lpp_status prefill_row_attention(lpp_engine* e, const ModelLayer& y, cons
     if (a.gate) a.gate = e->pf_gate;
     const bool skv = y.d.mixer == LPP_MIXER_SHARED_KV;
     const int ctas = row_attention_ctas(y, n);
-    if (row_attention_fits(e, y) && 2 * ctas >= e->num_sms) {
+    // A quarter of the SMs is where the two meet (whole prompts, us, tcgen05 / mma.sync with clusters): rutenex-1b with 128 tokens
+    // (32 CTAs) 2228 / 1972, 192 (48) 2479 / 2744, 320 (80) 2909 / 4278; rutenex-300m 128 (16) 2063 / 1894, 384 (48) 2343 / 3315;
+    // kolatar-1b 128 (32) 1589 / 1570, 192 (48) 1969 / 2025, 512 (128) 3238 / 3672; kolatar-300m 256 (32) 2358 / 2331, 512 (64) 3698 / 3927.
+    if (row_attention_fits(e, y) && 4 * ctas >= e->num_sms) {
         RowAttnArgs ra = {};
         ra.a = a;
         ra.halves = row_attention_halves(y);
