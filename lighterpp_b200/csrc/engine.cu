@@ -139,6 +139,7 @@ enum Kind { kQkv = 0, kAttn = 1, kOproj = 2, kGateUp = 3, kDown = 4, kLmHead = 5
 // A matrix of the batched prompt path as the CTA kernel and as the pair kernel read it.
 struct PrefillMap {
     CUtensorMap cta, pair;
+    CUtensorMap cta_small[3];  // activations: boxes of 16, 32 and 48 tokens (cta: 64)
 };
 // One layer of an engine described layer by layer.  Weight matrices: rows x pitch, pitch = inputs rounded up to 64, zero
 // padded; element type = weight_dtype.
@@ -2384,6 +2385,7 @@ static lpp_status encode_activation_map(CUtensorMap* m, const void* base, size_t
 
 static lpp_status make_activation_map(PrefillMap* m, const void* base, size_t tokens, size_t cols) {
     TRY(encode_activation_map(&m->cta, base, tokens, cols, kPfTile, 2, 2));
+    for (int i = 0; i < 3; ++i) TRY(encode_activation_map(&m->cta_small[i], base, tokens, cols, 16 * (i + 1), 2, 2));
     if (tokens < 128) return LPP_OK;  // blocks of one tile: the CTA kernel's
     return encode_activation_map(&m->pair, base, tokens, cols, 128, 1, 1);
 }
@@ -2657,9 +2659,11 @@ template <typename T, int EPI>
 static cudaError_t launch_prefill_gemm_t(lpp_engine* e, const PrefillMap& wm, const PrefillMap& xm, const PrefillGemmArgs& a) {
     const int toks = (a.n_tokens + a.tile - 1) / a.tile;
     if (a.tile == kPfTile) {
+        PrefillGemmArgs g = a;
+        g.box_tokens = a.n_tokens > 48 ? kPfTile : (a.n_tokens + 15) / 16 * 16;
         const int tiles = (a.n_rows + kUmmaM - 1) / kUmmaM * std::max(1, a.groups) * toks;
         return launch_kernel(prefill_gemm_umma_kernel<T, EPI>, dim3(std::min(tiles * a.splits, e->num_sms)), dim3(kUmmaThreads), (size_t)kPfSmemBytes,
-                             e->stream, true, wm.cta, xm.cta, a);
+                             e->stream, true, wm.cta, g.box_tokens == kPfTile ? xm.cta : xm.cta_small[g.box_tokens / 16 - 1], g);
     }
     if constexpr (EPI == kPfLatentQuery || EPI == kPfLatentValue) {
         return cudaErrorInvalidValue;  // grouped weights: always the CTA kernel

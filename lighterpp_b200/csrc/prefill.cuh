@@ -67,6 +67,7 @@ struct PrefillGemmArgs {
     int part_tokens;      // token rows of one range of K in part and out
     int start_pos;        // position of token 0
     int tile;             // tokens of an item: kPfTile (this file's kernel) or kPairTokens (prefill_pair.cuh)
+    int box_tokens;       // this file's kernel: token rows of an activation tile, a multiple of 16 up to kPfTile
     int epi;
     int splits;           // K is cut into this many ranges: work item = (row tile, token tile, range)
     StepState* st;
@@ -163,12 +164,16 @@ __device__ __forceinline__ void pf_qkv_store(const PrefillGemmArgs& a, int row, 
 // producer, 1 MMA issue and tensor-memory allocation, 2..9 epilogue (a warp may only read the tensor-memory lanes
 // of its quarter, warp index modulo 4; two warps share a quarter and take 32 tokens each).  An epilogue thread owns
 // one weight row and walks its tokens, so what depends on the row alone is computed once.
+// Every CTA reads all activations of its K range through L2, which for 128 weight rows x 64 tokens weighs as much as the weights:
+// the token rows of a tile follow the block (16, 32, 48 or 64; hi and lo rows are one N of twice that), and smaller tiles leave
+// room for more stages.  Whole prompts with 64-token tiles for all / now: 8 tokens, 8B 4.19 / 3.77 ms; 16 tokens, TinyLlama 1.250 /
+// 1.177; 4 tokens, 1B 1.020 / 0.987; 30 tokens, rutenex-1b 1.289 / 1.254.  (Fewer weight rows an item where 128 leave SMs
+// idle, 80 or 112: within 1.5 % either way at 64 tokens, not kept: the activations are read the more often.)
 // Every wait is bounded; every path, also a failed one, reaches the common exit, which lets copies in flight land
 // (bounded) and frees the tensor memory.
 constexpr int kUmmaM = 128;
 constexpr int kUmmaSubW = kUmmaM * 128;                            // 16 KiB
-constexpr int kUmmaStage = 2 * kUmmaSubW + 4 * kPfSubBytesX;       // 64 KiB: weights, activations hi, activations lo
-constexpr int kUmmaStages = kPfRingBytes / kUmmaStage;             // 3
+constexpr int kUmmaMaxStages = 8;
 constexpr int kUmmaEpiWarps = 8;                                   // two per tensor-memory lane quarter: 32 tokens each
 constexpr int kUmmaThreads = (2 + kUmmaEpiWarps) * 32;
 constexpr int kUmmaN = 2 * kPfTile;                                // MMA N: the 64 hi rows and the 64 lo rows of the activation tile
@@ -177,8 +182,8 @@ constexpr int kUmmaTmemCols = 2 * kUmmaAccCols;                    // power of t
 // Instruction descriptor: D = F32 (bits 4-5 = 1), A and B of the same 16-bit type (bits 7-9 and 10-12: 0 = FP16,
 // 1 = BF16), both K-major (bits 15, 16 = 0), N / 8 in bits 17-22, M / 16 in bits 24-28.
 template <typename T>
-__host__ __device__ constexpr uint32_t umma_idesc() {
-    return (1u << 4) | (std::is_same<T, __nv_bfloat16>::value ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(kUmmaN >> 3) << 17) |
+__host__ __device__ constexpr uint32_t umma_idesc(int n = kUmmaN) {
+    return (1u << 4) | (std::is_same<T, __nv_bfloat16>::value ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(n >> 3) << 17) |
            ((uint32_t)(kUmmaM >> 4) << 24);
 }
 
@@ -335,11 +340,13 @@ template <typename T, int EPI>
 static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kernel(const __grid_constant__ CUtensorMap w_map,
                                                                                    const __grid_constant__ CUtensorMap x_map,
                                                                                    const PrefillGemmArgs a) {
-    constexpr int kStages = kUmmaStages, kStage = kUmmaStage, kSubX = kPfSubBytesX;
+    constexpr int kMaxStages = kUmmaMaxStages;
+    const int kSubX = a.box_tokens * 128, kStage = 2 * kUmmaSubW + 4 * kSubX;
+    const int kStages = min(kMaxStages, kPfRingBytes / kStage);
     extern __shared__ __align__(128) unsigned char smem[];
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem);  // [kStages]
-    uint64_t* empty = full + kStages;                    // [kStages]
-    uint64_t* acc_full = empty + kStages;                // [2]
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem);  // [kMaxStages]
+    uint64_t* empty = full + kMaxStages;                 // [kMaxStages]
+    uint64_t* acc_full = empty + kMaxStages;             // [2]
     uint64_t* acc_empty = acc_full + 2;                  // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     int* s_fail = reinterpret_cast<int*>(tmem_slot + 1);  // set by a role whose wait ran out
@@ -429,6 +436,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
     } else if (warp == 1) {
         // ---------------- MMA issue
         {
+            const uint32_t idesc = umma_idesc<T>(2 * a.box_tokens);
             int slot = 0;
             uint32_t par = 0;
             bool ok = true;
@@ -455,12 +463,12 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
                     if (elect_one()) {
 #pragma unroll
                         for (int sub = 0; sub < 2; ++sub) {
-                            // the activation sub-tile holds the hi rows followed by the lo rows: one MMA covers both (N = 128)
+                            // the activation sub-tile holds the hi rows followed by the lo rows: one MMA covers both
                             const uint32_t wt = st + sub * kUmmaSubW, xt = st + 2 * kUmmaSubW + sub * 2 * kSubX;
 #pragma unroll
                             for (int ks = 0; ks < 4; ++ks) {  // 16 inputs = 32 bytes along the swizzled row per step
                                 const uint32_t acc = (kc > kc0 || sub > 0 || ks > 0) ? 1u : 0u;
-                                tc_mma_f16(d_tmem, umma_desc(wt + ks * 32), umma_desc(xt + ks * 32), umma_idesc<T>(), acc);
+                                tc_mma_f16(d_tmem, umma_desc(wt + ks * 32), umma_desc(xt + ks * 32), idesc, acc);
                             }
                         }
                         tc_commit(&empty[slot]);  // arrives once the MMAs issued so far have read this stage
@@ -492,7 +500,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
             float v[32], vlo[32];
             const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * kUmmaAccCols);
             tc_ld32(taddr + half * 32, v);                     // W.hi of this warp's 32 tokens
-            tc_ld32(taddr + kPfTile + half * 32, vlo);  // W.lo
+            tc_ld32(taddr + a.box_tokens + half * 32, vlo);  // W.lo
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] += vlo[i];
             tc_fence_before();
