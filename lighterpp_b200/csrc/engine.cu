@@ -2404,15 +2404,21 @@ static bool prefill_batched(const lpp_engine* e) {
 }
 
 template <typename T, int EPI>
+static lpp_status allow_cta_smem() {
+    CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<T, EPI, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
+    CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<T, EPI, kPfTile>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
+    return LPP_OK;
+}
+template <typename T, int EPI>
 static lpp_status allow_pair_smem() {
     CU(cudaFuncSetAttribute(prefill_gemm_pair_kernel<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));
     return LPP_OK;
 }
 template <typename T>
 static lpp_status allow_gemm_smem() {
-    CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<T, kPfResid>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
-    CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<T, kPfSwiglu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
-    CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<T, kPfStore>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
+    TRY((allow_cta_smem<T, kPfResid>()));
+    TRY((allow_cta_smem<T, kPfSwiglu>()));
+    TRY((allow_cta_smem<T, kPfStore>()));
     TRY((allow_pair_smem<T, kPfResid>()));
     TRY((allow_pair_smem<T, kPfSwiglu>()));
     return allow_pair_smem<T, kPfStore>();
@@ -2600,8 +2606,8 @@ static lpp_status prefill_maps(lpp_engine* e) {
         CU(cudaFuncSetAttribute(row_attention_umma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem_optin - kRaStatic));
         CU(cudaFuncSetAttribute(row_attention_umma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem_optin - kRaStatic));
         TRY(allow_gemm_smem<__nv_bfloat16>());
-        CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<__nv_bfloat16, kPfLatentQuery>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
-        CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<__nv_bfloat16, kPfLatentValue>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
+        TRY((allow_cta_smem<__nv_bfloat16, kPfLatentQuery>()));
+        TRY((allow_cta_smem<__nv_bfloat16, kPfLatentValue>()));
     } else {
         TRY(make_weight_map(&e->pf_map_wqkv, e->wqkv, L * (e->Dq + 2 * (size_t)e->KVd), D));
         TRY(make_weight_map(&e->pf_map_wo, e->wo, L * D, e->Dq));
@@ -2610,7 +2616,7 @@ static lpp_status prefill_maps(lpp_engine* e) {
         TRY(make_activation_map(&e->pf_map_att, e->pf_att, T, e->Dq));
         TRY(make_activation_map(&e->pf_map_hb, e->pf_hb, T, e->Fl));
         TRY(allow_gemm_smem<__half>());
-        CU(cudaFuncSetAttribute(prefill_gemm_umma_kernel<__half, kPfQkv>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes));
+        TRY((allow_cta_smem<__half, kPfQkv>()));
         TRY((allow_pair_smem<__half, kPfQkv>()));
         if (e->hs == 64 || e->hs == 128) {
             const size_t rows = L * e->KVHl * (size_t)c.seq_len;
@@ -2662,8 +2668,10 @@ static cudaError_t launch_prefill_gemm_t(lpp_engine* e, const PrefillMap& wm, co
         PrefillGemmArgs g = a;
         g.box_tokens = a.n_tokens > 48 ? kPfTile : (a.n_tokens + 15) / 16 * 16;
         const int tiles = (a.n_rows + kUmmaM - 1) / kUmmaM * std::max(1, a.groups) * toks;
-        return launch_kernel(prefill_gemm_umma_kernel<T, EPI>, dim3(std::min(tiles * a.splits, e->num_sms)), dim3(kUmmaThreads), (size_t)kPfSmemBytes,
-                             e->stream, true, wm.cta, g.box_tokens == kPfTile ? xm.cta : xm.cta_small[g.box_tokens / 16 - 1], g);
+        const bool whole = g.box_tokens == kPfTile;
+        return launch_kernel(whole ? prefill_gemm_umma_kernel<T, EPI, kPfTile> : prefill_gemm_umma_kernel<T, EPI, 0>,
+                             dim3(std::min(tiles * a.splits, e->num_sms)), dim3(kUmmaThreads), (size_t)kPfSmemBytes, e->stream, true, wm.cta,
+                             whole ? xm.cta : xm.cta_small[g.box_tokens / 16 - 1], g);
     }
     if constexpr (EPI == kPfLatentQuery || EPI == kPfLatentValue) {
         return cudaErrorInvalidValue;  // grouped weights: always the CTA kernel

@@ -336,12 +336,13 @@ __device__ unsigned long long g_pf_trace[160][48];
     } while (0)
 #endif
 
-template <typename T, int EPI>
+// BOX: token rows of an activation tile, 0 = a.box_tokens (whole tiles of 64 keep their sizes as constants).
+template <typename T, int EPI, int BOX>
 static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kernel(const __grid_constant__ CUtensorMap w_map,
                                                                                    const __grid_constant__ CUtensorMap x_map,
                                                                                    const PrefillGemmArgs a) {
     constexpr int kMaxStages = kUmmaMaxStages;
-    const int kSubX = a.box_tokens * 128, kStage = 2 * kUmmaSubW + 4 * kSubX;
+    const int box_tokens = BOX ? BOX : a.box_tokens, kSubX = box_tokens * 128, kStage = 2 * kUmmaSubW + 4 * kSubX;
     const int kStages = min(kMaxStages, kPfRingBytes / kStage);
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);  // [kMaxStages]
@@ -436,7 +437,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
     } else if (warp == 1) {
         // ---------------- MMA issue
         {
-            const uint32_t idesc = umma_idesc<T>(2 * a.box_tokens);
+            const uint32_t idesc = umma_idesc<T>(2 * box_tokens);
             int slot = 0;
             uint32_t par = 0;
             bool ok = true;
@@ -500,7 +501,7 @@ static __global__ void __launch_bounds__(kUmmaThreads, 1) prefill_gemm_umma_kern
             float v[32], vlo[32];
             const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * kUmmaAccCols);
             tc_ld32(taddr + half * 32, v);                     // W.hi of this warp's 32 tokens
-            tc_ld32(taddr + a.box_tokens + half * 32, vlo);  // W.lo
+            tc_ld32(taddr + box_tokens + half * 32, vlo);  // W.lo
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] += vlo[i];
             tc_fence_before();
