@@ -261,6 +261,8 @@ static __global__ void __launch_bounds__(kAggThreads) __cluster_dims__(kAggCtas,
     aggregation_kernel(float* out, const __half* v, const float* att, int seq_len, int head_size, int gqa_factor, int att_stride) {
     __shared__ float part[kAggThreads * 8];  // [position row][head_size]
     __shared__ float sums[kAggCtas][128];    // of the first CTA: what every CTA of the cluster found
+    // The first CTA has to run before its shared memory is written: everybody reports, and waits only ahead of the store.
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     op_begin();
     const int rank = blockIdx.x % kAggCtas, h = blockIdx.x / kAggCtas, tid = threadIdx.x;
     const int pieces = head_size >> 3, rows = kAggThreads / pieces;
@@ -296,6 +298,7 @@ static __global__ void __launch_bounds__(kAggThreads) __cluster_dims__(kAggCtas,
         for (int i = 0; i < 8; ++i) part[row * head_size + piece * 8 + i] = acc[i];
     }
     __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // all CTAs of the cluster have started
     if (tid < head_size) {
         float s = 0.f;
         for (int r = 0; r < rows; ++r) s += part[r * head_size + tid];

@@ -97,3 +97,22 @@ def test_operators_captured_in_a_graph(T):
         h = X / T.sqrt((X * X).mean() + 1e-5)
         ref = h + w.double() @ h
         assert (a.double() - ref).abs().max() <= 600 * 2.0 ** -24 * (w.double().abs() @ h.abs()).max()
+
+
+@pytest.mark.parametrize("positions", [1, 2, 7, 9])
+def test_aggregation_of_few_positions_in_a_graph(T, positions):
+    """Most CTAs of a cluster have no position and go straight to handing over their (empty) sums, 64 launches one behind the other."""
+    from lighterpp_b200 import ops
+    heads, hs, rows = 32, 128, 16
+    v = T.randn((heads, rows, hs), device="cuda", dtype=T.float16)
+    att, out = T.rand((64, heads, rows), device="cuda"), T.zeros((64, heads * hs), device="cuda")
+    graph = T.cuda.CUDAGraph()
+    with T.cuda.graph(graph):
+        for k in range(64):
+            ops.cuda_aggregation_multihead(out[k], v, att[k], heads, positions, hs, 1, rows)
+    for _ in range(3):
+        att.uniform_()
+        out.zero_()
+        graph.replay()
+        P, V = att[:, :, :positions].double(), v[:, :positions].double()
+        close(out.view(64, heads, hs).cpu().numpy(), T.einsum("kht,htd->khd", P, V).cpu().numpy(), T.einsum("kht,htd->khd", P, V.abs()).cpu().numpy(), positions)
