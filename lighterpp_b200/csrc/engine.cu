@@ -2629,26 +2629,44 @@ static lpp_status prefill_maps(lpp_engine* e) {
     TRY(make_activation_map(&e->pf_map_xn, e->pf_xn, T, D));
     return make_weight_map(&e->pf_map_cls, e->wcls, e->Vp, D);
 }
+static lpp_status prefill_release(lpp_engine* e) {
+    if (!e->pf_slab) return LPP_OK;
+    CU(cudaStreamSynchronize(e->stream));
+    CU(cudaFree(e->pf_slab));
+    e->pf_slab = nullptr;
+    e->pf_cap = 0;
+    return LPP_OK;
+}
 // Workspace for a portion of n tokens: room for one tile, or for the largest block that the cache has positions for.  Where
-// memory is short the blocks become smaller, down to one tile.
-static lpp_status prefill_setup(lpp_engine* e, int n) {
+// memory is short the blocks become smaller, down to one tile.  Logits, where the portion wants any, come first (and push out a
+// workspace of earlier portions): the blocks get what they leave.
+static lpp_status prefill_setup(lpp_engine* e, int n, bool logits) {
+    if (logits && !e->pf_logits) {
+        const size_t bytes = (size_t)kPfTile * e->Vp * 4;
+        cudaError_t r = cudaMalloc(&e->pf_logits, bytes);
+        if (r == cudaErrorMemoryAllocation && e->pf_slab) {
+            (void)cudaGetLastError();
+            TRY(prefill_release(e));
+            r = cudaMalloc(&e->pf_logits, bytes);
+        }
+        if (r != cudaSuccess) {
+            e->pf_logits = nullptr;
+            (void)cudaGetLastError();
+            return fail(LPP_ERR_CUDA, "no memory for a tile of logits (%zu bytes): %s", bytes, cudaGetErrorString(r));
+        }
+    }
     const int most = (int)std::min<size_t>(e->pf_limit, align_up((size_t)e->c.seq_len, kPfTile));
     int cap = n <= kPfTile ? kPfTile : most;
     if (e->pf_cap >= cap) return LPP_OK;
-    if (e->pf_slab) {
-        CU(cudaStreamSynchronize(e->stream));
-        CU(cudaFree(e->pf_slab));
-        e->pf_slab = nullptr;
-        e->pf_cap = 0;
-    }
+    TRY(prefill_release(e));
     size_t bytes = 0;
     for (;; cap = std::max(kPfTile, cap / 2 / kPfTile * kPfTile)) {
         bytes = prefill_carve(e, cap, nullptr);
         const cudaError_t r = cudaMalloc(&e->pf_slab, bytes);
         if (r == cudaSuccess) break;
         e->pf_slab = nullptr;
-        if (r != cudaErrorMemoryAllocation || cap <= kPfTile) CU(r);
         (void)cudaGetLastError();
+        if (r != cudaErrorMemoryAllocation || cap <= kPfTile) CU(r);
         e->pf_limit = std::max(kPfTile, cap / 2 / kPfTile * kPfTile);
     }
     CU(cudaMemsetAsync(e->pf_slab, 0, bytes, e->stream));
@@ -3068,7 +3086,6 @@ static lpp_status prefill_block(lpp_engine* e, const int* h_tokens, int n, int s
     const bool layered = !e->layers.empty();
     CU(cudaMemcpyAsync(e->pf_tokens, h_tokens, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, e->stream));
     if (n_want > 0) CU(cudaMemcpyAsync(e->pf_rows, want, (size_t)n_want * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    if (n_want > 0 && !e->pf_logits) CU(cudaMalloc(&e->pf_logits, (size_t)kPfTile * e->Vp * 4));
     if (prefill_f32(e)) return prefill_block_f32(e, n, start_pos, n_want, h_logits);
     int parts = 1;
     const float* add = first_add(e);  // what the next norm adds to the residual stream first
@@ -3129,7 +3146,7 @@ extern "C" lpp_status lpp_extend(lpp_engine* e, const int* h_tokens, int n, int 
     TRY(push_state(e, h_tokens[0], start_pos, nullptr, nullptr, 0, 0.f, 0, 0));  // clears the device status
     TRY(state_runs(e, start_pos));
     if (prefill_batched(e) && n > 1) {
-        TRY(prefill_setup(e, n));
+        TRY(prefill_setup(e, n, n_want > 0));
         CU(cudaEventRecord(e->ev0, e->stream));
         // blocks of about the same size, whole token tiles of the pair kernel where they are larger than one
         const int blocks = (n + e->pf_cap - 1) / e->pf_cap;

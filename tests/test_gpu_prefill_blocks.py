@@ -127,3 +127,41 @@ def test_workspace_shrinks_when_memory_is_short(E):
     check(got, ref, 2e-3)
     for e in (batched, loop):
         e.close()
+
+
+def free_bytes(torch):
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+
+@pytest.mark.parametrize("workspace_first", [False, True])
+def test_logits_and_workspace_share_short_memory(E, workspace_first):
+    """A vocabulary whose tile of logits (31 MiB) does not fit beside the largest workspace: blocks become smaller, whichever of the
+    two the engine made first."""
+    import torch
+    c = ModelConfig(512, 2048, 2, 8, 2, 128256, 1200, 10000.0)
+    T = synth.gen_model(c, 3, "f16", True)
+    toks = synth.prompt_tokens(c.vocab_size, 700, 3)
+    roomy, tight = E.Engine(c, "f16", "f16"), E.Engine(c, "f16", "f16")
+    for e in (roomy, tight):
+        e.load_weights(T)
+    before = free_bytes(torch)
+    roomy.extend(toks, 0)
+    whole, logits = before - free_bytes(torch), 64 * c.vocab_size * 4
+    ref = roomy.extend(toks, 0, [5, 699])
+    left = whole + logits * 3 // 4
+    assert left > logits + (8 << 20)
+    if workspace_first:
+        tight.extend(toks, 0)
+        left -= whole
+    hog = torch.empty(free_bytes(torch) - left, dtype=torch.uint8, device="cuda")
+    try:
+        got = [tight.extend(toks, 0, [5, 699]) for _ in range(2)]
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    for g in got:
+        check(g, ref, 2e-3)
+    for e in (roomy, tight):
+        e.close()
