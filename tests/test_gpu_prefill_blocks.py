@@ -111,28 +111,35 @@ def test_layered_blocks_match_token_loop(E, which):
         e.close()
 
 
+def free_bytes(torch):
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+
 def test_workspace_shrinks_when_memory_is_short(E):
+    """Half of what the largest block's workspace takes beyond the one of a tile, which an engine with enough memory shows."""
     import torch
     c, toks, (batched, loop) = pair(E, "mini-8b-f16", 1200)
+    T = synth.gen_model(c, synth.SHAPES["mini-8b-f16"][3], "f16", synth.SHAPES["mini-8b-f16"][2])
+    roomy = E.Engine(c, "f16", "f16")
+    roomy.load_weights(T)
     ref = loop.extend(toks[:700], 0, [699])
-    batched.extend(toks[:10], 0)
-    torch.cuda.empty_cache()
-    free, _ = torch.cuda.mem_get_info()
-    hog = torch.empty(free - (30 << 20), dtype=torch.uint8, device="cuda")  # the workspace of 1200 tokens takes over 50 MB
+    for e in (roomy, batched):
+        e.extend(toks[:10], 0, [9])
+    before = free_bytes(torch)
+    roomy.extend(toks[:700], 0, [699])
+    whole = before - free_bytes(torch)
+    assert whole > 8 << 20
+    hog = torch.empty(free_bytes(torch) - whole // 2, dtype=torch.uint8, device="cuda")
     try:
         got = batched.extend(toks[:700], 0, [699])
     finally:
         del hog
         torch.cuda.empty_cache()
     check(got, ref, 2e-3)
-    for e in (batched, loop):
+    for e in (batched, loop, roomy):
         e.close()
-
-
-def free_bytes(torch):
-    torch.cuda.synchronize()
-    torch.cuda.empty_cache()
-    return torch.cuda.mem_get_info()[0]
 
 
 @pytest.mark.parametrize("workspace_first", [False, True])
