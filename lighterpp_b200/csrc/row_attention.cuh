@@ -4,15 +4,16 @@
 // columns, 160 KiB), and keys and values pass through a ring of 64 rows x 64 columns (8 KiB) that the tensor memory
 // accelerator fills: first the pieces whose scores S = Q . K^T add up, then, once the probabilities are there, the pieces of
 // the value part again (the same cache rows; a tile of keys does not fit beside the queries, and re-reading a half of it costs
-// less than the smaller row tile would).  Results of up to 256 value columns stay in tensor memory, so wider rows are
-// shared by two CTAs that both form the scores.  Sixteen warps are the softmax, four threads a row.  The running maximum
-// that the results refer to moves only when a row's true maximum has passed it by 2^8 (probabilities then reach 256, exact in
-// FP16 as below 1); results are rescaled in tensor memory at those few tiles.
+// less than the smaller row tile would).  A CTA takes up to 256 value columns, so wider rows are shared by two CTAs that both
+// form the scores.  Sixteen warps are the softmax, four threads a row.  P . V of a tile starts from zero in tensor memory and is
+// added to FP32 registers, rescaled by the running maximum, while the scores of the next tile are formed: the tensor cores add with
+// truncation, and results of a whole window in one accumulator came out too small (3000 alike rows: by 1.9e-5, now 1.5e-7).
 //
-// Measured 8000 clocks a tile of keys, most of it MMAs of 64 keys (150 clocks each where 32 are arithmetic).  1023 tokens of the
-// rutenex-1b shape (16 heads, rows of 512 + 64, window 1024): 61 us a launch, mma.sync 170.  mma.sync tiles of 32 rows (latent_attn_mma_kernel)
-// fetch every key four times as often; they remain for blocks whose row tiles leave most of the GPU idle, because
-// there a cluster shares the keys (row_attention_umma, engine.cu).
+// Bound by the MMAs, 52 of 64 keys a tile at the widest (about 150 clocks each where 32 are arithmetic), and the hand-overs between
+// them and the softmax.  1023 tokens of the rutenex-1b shape (16 heads, rows of 512 + 64, window 1024): 71 us a launch (64 with results
+// that stay in tensor memory, mma.sync 170), rutenex-300m (rows of 256 + 32, window 512) 34 us (29).  mma.sync tiles of 32 rows
+// (latent_attn_mma_kernel) fetch every key four times as often; they remain for blocks whose row tiles leave most of the GPU idle,
+// because there a cluster shares the keys (prefill_row_attention in engine.cu draws the line).
 // Rows outside the tile's span of keys are masked, and as values zeroed in shared memory.  Waits are bounded; every path
 // reaches the common exit.
 #pragma once
@@ -25,6 +26,7 @@ constexpr int kRaRows = 128, kRaKeys = 64;
 constexpr int kRaPiece = kRaKeys * 128;       // a ring slot: 64 keys x 64 columns
 constexpr int kRaQueryPiece = kRaRows * 128;  // 128 query rows x 64 columns
 constexpr int kRaMaxSlots = 16, kRaMinSlots = 5;
+constexpr int kRaMaxPieces = 4;               // value columns of a CTA / 64
 constexpr int kRaStatic = 7 * 1024;           // static shared memory and what the driver keeps, at most
 __host__ __device__ constexpr int ra_pieces(int cols) { return (cols + 63) / 64; }
 constexpr int ra_fixed(int row_width) { return 1024 /*barriers*/ + 1024 /*alignment slack*/ + ra_pieces(row_width) * kRaQueryPiece + kRaRows * 128 /*P*/; }
@@ -41,18 +43,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap
                  "r"(x), "r"(y), "r"(bar_addr)
                  : "memory");
 }
-// 32 lanes x 16 consecutive columns back to tensor memory (see tc_ld16)
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const float (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-        "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])),
-        "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])), "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])),
-        "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])), "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])),
-        "r"(__float_as_uint(v[15]))
-        : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-
 // grid: groups x halves x row tiles, the last tokens first.  q_map: queries as (columns, heads, tokens), boxes of 64 columns x
 // a group's heads x the tile's tokens; c_map: the layer's cache as (columns, rows), boxes of 64 x 64.
 template <bool SKV>
@@ -177,7 +167,7 @@ static __global__ void __launch_bounds__(kFaThreads, 1) row_attention_umma_kerne
 #pragma unroll
                     for (int ks = 0; ks < kRaKeys / 16; ++ks)
                         tc_mma_f16(tmem + p * 64, umma_desc(sp + ks * 32), fa_desc_mn(ring + slot * kRaPiece + ks * 2048), fa_idesc(64, true),
-                                   it > 0 || ks > 0 ? 1u : 0u);
+                                   ks > 0 ? 1u : 0u);
                 }
                 taken();
             }
@@ -195,7 +185,25 @@ static __global__ void __launch_bounds__(kFaThreads, 1) row_attention_umma_kerne
         pdl_wait();  // (gates, and what still reads the finished rows of the layer before)
         constexpr float kLog2e = 1.4426950408889634f;
         const float rate = a.scale * kLog2e;
-        float ref = -INFINITY, l = 0.f;  // the maximum that results refer to
+        float m = -INFINITY, l = 0.f, f_before = 0.f;
+        float o[kRaMaxPieces][16];
+#pragma unroll
+        for (int c = 0; c < kRaMaxPieces; ++c)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[c][i] = 0.f;
+        auto products_done = [&](int it) -> bool { return __all_sync(0xffffffffu, mbar_wait_bounded(pv_done, (uint32_t)it & 1u, st)); };
+        auto add_values = [&]() {  // o = o * (rescaling) + P . V of the tile whose products are done
+            tc_fence_after();
+#pragma unroll
+            for (int c = 0; c < kRaMaxPieces; ++c) {
+                if (c >= P) break;
+                float v[16];
+                tc_ld16(results + c * 16, v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) o[c][i] = fmaf(o[c][i], f_before, v[i]);
+            }
+            tc_fence_before();
+        };
         bool ok = true;
         for (int it = 0; it < n_tiles && ok; ++it) {
             const int b = it & 1, p0 = k_begin + it * kRaKeys + part * 16;
@@ -229,10 +237,10 @@ static __global__ void __launch_bounds__(kFaThreads, 1) row_attention_umma_kerne
             float top = s_max[b][0][row];
 #pragma unroll
             for (int i = 1; i < kFaParts; ++i) top = fmaxf(top, s_max[b][i][row]);
-            const bool moves = top > ref + 8.f;  // (from minus infinity: at the first visible key)
-            const float f = moves ? ex2(ref - top) : 1.f;
-            if (moves) ref = top;
-            const float u = ref == -INFINITY ? 0.f : ref;  // nothing visible yet
+            const float m_new = fmaxf(m, top);
+            const float u = m_new == -INFINITY ? 0.f : m_new;  // nothing visible yet
+            const float f = ex2(m - u);
+            m = m_new;
             uint32_t p[8];
             float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
@@ -244,20 +252,9 @@ static __global__ void __launch_bounds__(kFaThreads, 1) row_attention_umma_kerne
             }
             l = fmaf(l, f, sum0 + sum1);
             // the probabilities of the tile before have been read, and its results are there, when its products are done
-            if (it > 0) {
-                ok = __all_sync(0xffffffffu, mbar_wait_bounded(pv_done, (uint32_t)(it - 1) & 1u, st));
-                if (!ok) break;
-                if (__any_sync(0xffffffffu, moves)) {
-                    tc_fence_after();
-                    for (int c = 0; c < P * 16; c += 16) {
-                        float o[16];
-                        tc_ld16(results + c, o);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] *= f;
-                        tc_st16(results + c, o);
-                    }
-                    tc_fence_before();
-                }
+            if (it > 0 && !products_done(it - 1)) {
+                ok = false;
+                break;
             }
 #pragma unroll
             for (int c = 0; c < 2; ++c)
@@ -265,28 +262,33 @@ static __global__ void __launch_bounds__(kFaThreads, 1) row_attention_umma_kerne
                              "r"(p[4 * c + 1]), "r"(p[4 * c + 2]), "r"(p[4 * c + 3])
                              : "memory");
             fence_async_smem();
+            if (it > 0) add_values();  // (the next products replace them)
+            f_before = f;
             __syncwarp();
             if (lane == 0) mbar_arrive(p_ready);
         }
-        if (ok && n_tiles > 0) ok = __all_sync(0xffffffffu, mbar_wait_bounded(pv_done, (uint32_t)(n_tiles - 1) & 1u, st));
+        if (ok && n_tiles > 0) {
+            ok = products_done(n_tiles - 1);
+            if (ok) add_values();
+        }
         if (!ok) *s_fail = 1;
         s_l[part][row] = l;
         asm volatile("bar.sync %0, %1;" ::"r"(1 + quarter), "n"(32 * kFaParts) : "memory");  // (every warp gets here)
         if (n_tiles > 0) {  // (also after a wait that ran out: the warps of these rows meet once more below)
-            tc_fence_after();
             float total = s_l[0][row];
 #pragma unroll
             for (int i = 1; i < kFaParts; ++i) total += s_l[i][row];
             // finished rows over the operands (every copy has landed and been read), so that a warp stores whole pieces of a row
-            const float inv = __fdiv_rn(1.f, total);
             const int pitch = P * 64 + 4;
             float* rows = reinterpret_cast<float*>(smem + (sq - smem_u32(smem)));
             float* mine = rows + row * pitch + part * P * 16;
-            for (int c = 0; c < P * 16; c += 16) {
-                float o[16];
-                tc_ld16(results + c, o);
 #pragma unroll
-                for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(mine + c + i) = make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
+            for (int c = 0; c < kRaMaxPieces; ++c) {
+                if (c >= P) break;
+#pragma unroll
+                for (int i = 0; i < 16; i += 4)
+                    *reinterpret_cast<float4*>(mine + c * 16 + i) =
+                        make_float4(__fdiv_rn(o[c][i], total), __fdiv_rn(o[c][i + 1], total), __fdiv_rn(o[c][i + 2], total), __fdiv_rn(o[c][i + 3], total));
             }
             asm volatile("bar.sync %0, %1;" ::"r"(1 + quarter), "n"(32 * kFaParts) : "memory");  // rows of this quarter
             for (int r = part; r < 32; r += kFaParts) {

@@ -66,3 +66,28 @@ def test_blocks_match_token_loop(E, cfg, first):
     check(batched.extend(toks[197:197 + first], 197, range(first)), list(range(197, 197 + first)))
     for e in engines:
         e.close()
+
+
+def test_sums_over_many_keys_are_not_truncated(E):
+    """The tensor cores add with truncation: 3000 alike rows in one accumulator (190 additions of 16 rows, each of which loses half of
+    2^-23 of the sum so far on average) come out (190 / 2) 2^-24 = 6e-6 too small.  Rounding errors have no direction, so the error of the
+    last 64 tokens' logits is laid onto what a larger attention output would change in them.  64 keys in one accumulator and the value
+    and output matrices (64 and 128 inputs) leave 16 additions, 1e-6 at most."""
+    from oracle import rutenex
+    from rutenex_util import engine
+    cfg = latent(8, 64, 16, 0)
+    cfg["layers"] = cfg["layers"][:1]
+    cfg["layers"][0]["mixer"]["vdim"] = 16
+    W = rutenex.random_weights(cfg, 5)
+    rng = np.random.default_rng(6)
+    W["embed"] = rutenex.bf16_round(rng.standard_normal(136) + 0.2 * rng.standard_normal((320, 136)))
+    W["l0.mix.o"] = rutenex.bf16_round(4 * W["l0.mix.o"])
+    toks = rng.integers(0, 320, 3072)
+    e = engine(E, cfg, W, "bfloat16", 3072)
+    got = e.extend(toks, 0, range(3008, 3072)).astype(np.float64)
+    e.close()
+    want = rutenex.forward(cfg, W, toks)[-64:]
+    more = (rutenex.forward(cfg, {**W, "l0.mix.o": W["l0.mix.o"].astype(np.float64) * 1.001}, toks)[-64:] - want) / 1e-3
+    short = float(((got - want) * more).sum() / (more * more).sum())
+    print("attention output off by", short)
+    assert np.linalg.norm(got - want) <= 2e-3 * np.linalg.norm(want) and abs(short) <= 1.5e-6, short
