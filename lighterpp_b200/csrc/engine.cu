@@ -2395,6 +2395,15 @@ static lpp_status make_activation_map(PrefillMap* m, const void* base, size_t to
 static bool prefill_f32(const lpp_engine* e) {
     return e->layers.empty() && e->c.weight_dtype == LPP_F32 && e->c.kv_dtype == LPP_F32 && e->c.tp_size == 1;
 }
+// Portions of up to this many tokens go through the step graph all the same: FP32 engines, where a block reads the weights slower
+// than the step does.  Whole portions, block / step by step (same results, us): 24 MB of layers, 2 tokens 246 / 236, 3 245 / 337; 101 MB, 3 530 /
+// 450, 4 541 / 597; 340 MB, 4 1045 / 945, 5 1049 / 1154; 487 MB, 4 974 / 823, 5 973 / 1022; 1.2 GB, 5 2700 / 2676, 6 2660 / 3153; 3.9 GB, 5 5467 /
+// 4720, 6 5469 / 5656.
+static int prefill_loop_tokens(const lpp_engine* e) {
+    if (!prefill_f32(e)) return 1;
+    const size_t D = e->c.dim, bytes = e->c.n_layers * D * (2 * (size_t)e->Dq + 2 * (size_t)e->KVd + 3 * (size_t)e->Fl) * 4;
+    return 2 + (bytes > (64u << 20)) + (bytes > (256u << 20)) + (bytes > (1024u << 20));
+}
 static bool prefill_batched(const lpp_engine* e) {
     if (e->c.flags & LPP_FLAG_NO_PREFILL_GEMM) return false;
     if (prefill_f32(e)) return true;
@@ -3145,7 +3154,7 @@ extern "C" lpp_status lpp_extend(lpp_engine* e, const int* h_tokens, int n, int 
     int w = 0;  // wanted tokens served so far
     TRY(push_state(e, h_tokens[0], start_pos, nullptr, nullptr, 0, 0.f, 0, 0));  // clears the device status
     TRY(state_runs(e, start_pos));
-    if (prefill_batched(e) && n > 1) {
+    if (prefill_batched(e) && n > prefill_loop_tokens(e)) {
         TRY(prefill_setup(e, n, n_want > 0));
         CU(cudaEventRecord(e->ev0, e->stream));
         // blocks of about the same size, whole token tiles of the pair kernel where they are larger than one
