@@ -2796,7 +2796,9 @@ static lpp_status prefill_gqa_mixer(lpp_engine* e, int l, int n, int start_pos, 
     prefill_qkv_args(e, l, g);
     const cudaError_t ge = launch_prefill_gemm_t<__half, kPfQkv>(e, e->pf_map_wqkv, e->pf_map_xn, g);
     CU(ge);
-    CU(launch_kernel(prefill_qkv_finish_kernel<__half>, dim3((n + kFinishTokens - 1) / kFinishTokens, (qkv_rows + 1023) / 1024), dim3(256), 0, e->stream, true, g));
+    const int per = n > kPfTile ? kFinishTokens : 1;  // tokens of a thread: a tile's ranges of K are many, beyond it they are one or two
+    CU(launch_kernel(per == 1 ? prefill_qkv_finish_kernel<1> : prefill_qkv_finish_kernel<kFinishTokens>, dim3((n + per - 1) / per, (qkv_rows + 1023) / 1024), dim3(256),
+                     0, e->stream, true, g));
     if (cache_only) return LPP_OK;
     __half* att = (__half*)e->pf_att;
     if (e->hs != 64 && e->hs != 128) {

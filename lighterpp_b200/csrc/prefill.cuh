@@ -552,15 +552,17 @@ __device__ __forceinline__ void prefill_sums(const float* part, int part_tokens,
 // pairs, q -> FP32 rows, k/v -> cache rows at the reference index).  A thread takes four rows (two pairs; there are always whole
 // quads: q rows come in multiples of 64, k and v rows are even and equally many) of kFinishTokens tokens, so that 64 bytes per
 // range of K are in flight and the rotation's table is there before the sums are.  Bound by the traffic through L2.  One pair of
-// one token per thread took 17 us for 1023 tokens of 3072 rows and 40 us for 1000 tokens of 6144 rows (one range).
-// grid: (ceil(tokens / kFinishTokens), ceil(rows / 1024)).
+// one token per thread took 17 us for 1023 tokens of 3072 rows and 40 us for 1000 tokens of 6144 rows (one range).  Few tokens are
+// bound by the latency of their up to eight ranges instead: TOKENS 1, all ranges in flight.  Whole prompts with four tokens a thread /
+// with one: 47 tokens of the TinyLlama shape 1169 / 1116 us, 33 of the Llama-3.2-1B shape 1031 / 1000, 64 of it 1042 / 1002.
+// grid: (ceil(tokens / TOKENS), ceil(rows / 1024)).
 constexpr int kFinishTokens = 4;
-template <typename CT>
+template <int TOKENS>
 static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const PrefillGemmArgs a) {
     pdl_launch_dependents();
-    const int t0 = blockIdx.x * kFinishTokens, row = 4 * ((int)blockIdx.y * 256 + (int)threadIdx.x), hs = a.head_size;
+    const int t0 = blockIdx.x * TOKENS, row = 4 * ((int)blockIdx.y * 256 + (int)threadIdx.x), hs = a.head_size;
     const bool mine = row < a.n_rows;
-    float2 cs[kFinishTokens][2];
+    float2 cs[TOKENS][2];
     size_t at[2] = {0, 0};  // in the cache: position 0 of the pair's row
     const bool is_q = row < a.q_rows;
     if (mine) {  // constants: ahead of the dependency wait
@@ -572,7 +574,7 @@ static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const Pr
             const int h = rr / hs, off = rr - h * hs;
             at[j] = (size_t)h * ((size_t)a.seq_len * hs) + off;  // h*(seq_len*hs) + pos*hs + off (src/scatter_kv.cu:15-16)
 #pragma unroll
-            for (int i = 0; i < kFinishTokens; ++i) {
+            for (int i = 0; i < TOKENS; ++i) {
                 const int pos = a.start_pos + t0 + i;
                 // adjacent-pair rotation with the table entry for (pos, (row % hs)/2) (src/ops.cpp:34-54)
                 cs[i][j] = turned && pos >= 0 && pos < a.seq_len ? __ldg(a.rope + (size_t)pos * (hs >> 1) + (off >> 1)) : make_float2(1.f, 0.f);
@@ -581,10 +583,24 @@ static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const Pr
     }
     pdl_wait();
     if (!mine) return;
-    float4 v[kFinishTokens];
-    prefill_sums<kFinishTokens>(a.part, a.part_tokens, a.n_rows, a.splits, a.n_tokens, t0, row, v);
+    float4 v[TOKENS];
+    if constexpr (TOKENS == 1) {
+        float4 p[kPfMaxSplits];
+        const float4* at0 = reinterpret_cast<const float4*>(a.part + (size_t)t0 * a.n_rows + row);
 #pragma unroll
-    for (int i = 0; i < kFinishTokens; ++i) {
+        for (int s = 0; s < kPfMaxSplits; ++s)
+            if (s < a.splits) p[s] = at0[(size_t)s * a.part_tokens * a.n_rows / 4];
+        v[0] = p[0];
+#pragma unroll
+        for (int s = 1; s < kPfMaxSplits; ++s)  // in range order
+            if (s < a.splits) {
+                v[0].x += p[s].x; v[0].y += p[s].y; v[0].z += p[s].z; v[0].w += p[s].w;
+            }
+    } else {
+        prefill_sums<TOKENS>(a.part, a.part_tokens, a.n_rows, a.splits, a.n_tokens, t0, row, v);
+    }
+#pragma unroll
+    for (int i = 0; i < TOKENS; ++i) {
         const int t = t0 + i, pos = a.start_pos + t;
         if (t >= a.n_tokens) break;
         if (pos < 0 || pos >= a.seq_len) {
@@ -601,12 +617,8 @@ static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const Pr
             *reinterpret_cast<float4*>(a.q + (size_t)t * a.q_rows + row) = make_float4(p0.x, p0.y, p1.x, p1.y);
         } else {
             auto put = [&](float2 p, int j) {
-                __align__(8) CT pair[2] = {from_float<CT>(p.x), from_float<CT>(p.y)};
-                CT* dst = reinterpret_cast<CT*>(row + 2 * j < a.q_rows + a.kv_rows ? a.k_cache : a.v_cache) + at[j] + (size_t)pos * hs;
-                if constexpr (sizeof(CT) == 2)
-                    *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(pair);
-                else
-                    *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(pair);
+                __half* dst = reinterpret_cast<__half*>(row + 2 * j < a.q_rows + a.kv_rows ? a.k_cache : a.v_cache) + at[j] + (size_t)pos * hs;
+                *reinterpret_cast<uint32_t*>(dst) = pack_half2(p.x, p.y);
             };
             put(p0, 0);
             put(p1, 1);
