@@ -251,6 +251,7 @@ struct lpp_engine {
     // graphs
     // graph variants by context length; only [0] is used at present
     cudaGraphExec_t g_full[2] = {nullptr, nullptr}, g_logits[2] = {nullptr, nullptr};
+    bool g_logits_there = false;  // g_logits is on the device: its first launch need not bring it there
 
     // batched prompt path: one allocation for blocks of up to pf_cap tokens, made by the first call that needs them
     void* pf_slab = nullptr;
@@ -1303,6 +1304,7 @@ static lpp_status run_step(lpp_engine* e, bool with_sampler, int pos) {
         return LPP_OK;
     }
     CU(cudaGraphLaunch(with_sampler ? e->g_full[v] : e->g_logits[v], e->stream));
+    if (!with_sampler) e->g_logits_there = true;
     return LPP_OK;
 }
 
@@ -2187,6 +2189,7 @@ extern "C" lpp_status lpp_finalize(lpp_engine* e) {
         if (e->g_full[v]) cudaGraphExecDestroy(e->g_full[v]), e->g_full[v] = nullptr;
         if (e->g_logits[v]) cudaGraphExecDestroy(e->g_logits[v]), e->g_logits[v] = nullptr;
     }
+    e->g_logits_there = false;
     TRACE("finalize: weights complete");
     if (aid_env("LPP_GEMV_TRACE") && !e->gtrace) {
         CU(cudaMalloc(&e->gtrace, (size_t)256 * e->num_sms * 8 * sizeof(unsigned long long)));
@@ -3172,6 +3175,11 @@ extern "C" lpp_status lpp_extend(lpp_engine* e, const int* h_tokens, int n, int 
             w += k;
         }
         CU(cudaEventRecord(e->ev1, e->stream));
+        // a host loop that samples goes on with single steps: their graph goes to the device while the prompt runs
+        if (prefill_f32(e) && e->g_logits[0] && !e->g_logits_there) {
+            CU(cudaGraphUpload(e->g_logits[0], e->stream));
+            e->g_logits_there = true;
+        }
     } else {
         // token by token through the step graph without its sampler, like the reference's prompt loop
         CU(cudaEventRecord(e->ev0, e->stream));
