@@ -229,10 +229,12 @@ lpp_status lpp_decode(lpp_engine* e, int first_token, int start_pos, int n, cons
 
 /* The prompt loop of src/main.cpp:163-179 without its n calls of forward(): fills the K/V cache rows of positions
  * start_pos .. start_pos + n - 1 for the n prompt tokens and produces no logits (feed the LAST prompt token to
- * lpp_step / lpp_step_logits as usual, and only the tokens before it to this call).  With FP16 weights, an FP16
- * cache and one GPU the tokens go through the layers in blocks of 64: every matrix is streamed once per block by a
- * TMA-fed tensor-core GEMM (activations rounded to FP16 as operands, FP32 accumulation), followed by causal
- * attention inside the block; other engines (or LPP_FLAG_NO_PREFILL_GEMM) run the step graph once per token.
+ * lpp_step / lpp_step_logits as usual, and only the tokens before it to this call).  With 16-bit weights, an FP16 cache
+ * and one GPU (FP16: widths in multiples of 64) the tokens go through the layers in blocks of up to 1024, fewer where device
+ * memory is short: every matrix is streamed once per block by a TMA-fed tensor-core GEMM (activations as the sum of two 16-bit
+ * operands, FP32 accumulation), followed by attention inside the block.  With FP32 weights and an FP32 cache on one GPU (engines
+ * that are not described layer by layer) the blocks repeat the step's own arithmetic: cache rows and logits are the same bits.
+ * Other engines (or LPP_FLAG_NO_PREFILL_GEMM) run the step graph once per token, and so do portions of a few FP32 tokens.
  * *device_ms (optional) receives the CUDA-event time. */
 lpp_status lpp_prefill(lpp_engine* e, const int* h_tokens, int n, int start_pos, float* device_ms);
 

@@ -2363,10 +2363,11 @@ static lpp_status encode_weight_map(CUtensorMap* m, const void* base, size_t row
     if (r != CUDA_SUCCESS) return fail(LPP_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for a %zu x %zu matrix", (int)r, rows, cols);
     return LPP_OK;
 }
-// The CTA kernel takes two pieces of 128 rows at a time, the pair kernel one.
-static lpp_status make_weight_map(PrefillMap* m, const void* base, size_t rows, size_t cols) {
+// The CTA kernel takes two pieces of 128 rows at a time, the pair kernel one.  pair false: matrices that only the CTA kernel reads
+// (grouped ones, the classifier's).
+static lpp_status make_weight_map(PrefillMap* m, const void* base, size_t rows, size_t cols, bool pair = true) {
     TRY(encode_weight_map(&m->cta, base, rows, cols, kUmmaM, 2));
-    return encode_weight_map(&m->pair, base, rows, cols, kPairM / 2, 1);
+    return pair ? encode_weight_map(&m->pair, base, rows, cols, kPairM / 2, 1) : LPP_OK;
 }
 // Activations: hi plane [tokens][cols] followed by the lo plane, seen as (64 inputs, tokens, 2 planes, cols / 64).  CTA
 // kernel: a box is 64 inputs x 64 tokens x 2 planes x 2 pieces, i.e. one copy delivers, per 64-input piece, the hi rows
@@ -2386,11 +2387,11 @@ static lpp_status encode_activation_map(CUtensorMap* m, const void* base, size_t
     return LPP_OK;
 }
 
-static lpp_status make_activation_map(PrefillMap* m, const void* base, size_t tokens, size_t cols) {
+static lpp_status make_activation_map(PrefillMap* m, const void* base, size_t tokens, size_t cols, bool pair = true) {
     TRY(encode_activation_map(&m->cta, base, tokens, cols, kPfTile, 2, 2));
     for (int i = 0; i < 3; ++i) TRY(encode_activation_map(&m->cta_small[i], base, tokens, cols, 16 * (i + 1), 2, 2));
-    if (tokens < 128) return LPP_OK;  // blocks of one tile: the CTA kernel's
-    return encode_activation_map(&m->pair, base, tokens, cols, 128, 1, 1);
+    if (tokens < kPairTokens) return LPP_OK;  // blocks of one tile: the CTA kernel's
+    return pair ? encode_activation_map(&m->pair, base, tokens, cols, kPairTokens, 1, 1) : LPP_OK;
 }
 
 // Prompts in blocks: the tensor-core path takes 16-bit weights, an FP16 cache and a single GPU, the FP32 path FP32 weights and
@@ -2441,6 +2442,11 @@ static lpp_status allow_gemm_smem() {
 // weight rows) are cut along K as often as fills the GPU.  Else the cheapest of the pair kernel's cuts by a model of its
 // time: waves of items over the SM pairs, each item 64 inputs at a time (0.45 us measured) plus a fixed part, plus the
 // traffic of partial sums through L2.
+// Between 65 and 127 tokens two tiles of the CTA kernel are the faster ones for narrow matrices and the slower ones for wide ones
+// (whole prompts, us, pair kernel / two tiles): rutenex-300m 65 1588 / 1302, 127 1621 / 1360; kolatar-300m 96 1439 / 1200; TinyLlama 65
+// 1557 / 1491, 127 1539 / 1541; Llama-3.2-1B 65 1319 / 1270, 127 1296 / 1309; rutenex-1b 1478 / 1485, 1559 / 1551; Llama-3-8B 4544 / 5679,
+// 5152 / 6320 (every tile of tokens reads the weights again).  Neither side wins for all widths; the pair kernel's worst case is the
+// smaller loss.
 struct PrefillPlan {
     int tile, splits;
 };
@@ -2593,10 +2599,10 @@ static lpp_status prefill_maps(lpp_engine* e) {
             const size_t H = y.d.heads, D2 = align_up(c.dim, 2);
             TRY(make_weight_map(&y.m_in, y.w_in, y.in_rows, D));
             if (y.d.mixer == LPP_MIXER_LATENT) {
-                TRY(make_weight_map(&y.m_uk, y.w_uk, H * y.rank_pitch, y.dim_pitch));
-                TRY(make_weight_map(&y.m_uv, y.w_uv, H * y.vdim_rows, y.val_pitch));
-                TRY(make_activation_map(&y.x_qn, e->pf_qn, T, H * y.dim_pitch));
-                TRY(make_activation_map(&y.x_olat, e->pf_olat, T, H * y.val_pitch));
+                TRY(make_weight_map(&y.m_uk, y.w_uk, H * y.rank_pitch, y.dim_pitch, false));
+                TRY(make_weight_map(&y.m_uv, y.w_uv, H * y.vdim_rows, y.val_pitch, false));
+                TRY(make_activation_map(&y.x_qn, e->pf_qn, T, H * y.dim_pitch, false));
+                TRY(make_activation_map(&y.x_olat, e->pf_olat, T, H * y.val_pitch, false));
             } else if (y.d.mixer == LPP_MIXER_MAMBA) {
                 TRY(make_weight_map(&y.m_low, y.w_low, y.low_rows, y.inner_pitch));
                 TRY(make_activation_map(&y.x_low, e->pf_sxp, T, y.inner_pitch));
@@ -2639,7 +2645,7 @@ static lpp_status prefill_maps(lpp_engine* e) {
         }
     }
     TRY(make_activation_map(&e->pf_map_xn, e->pf_xn, T, D));
-    return make_weight_map(&e->pf_map_cls, e->wcls, e->Vp, D);
+    return make_weight_map(&e->pf_map_cls, e->wcls, e->Vp, D, false);
 }
 static lpp_status prefill_release(lpp_engine* e) {
     if (!e->pf_slab) return LPP_OK;
@@ -2795,7 +2801,6 @@ static lpp_status prefill_gqa_mixer(lpp_engine* e, int l, int n, int start_pos, 
     const int D = c.dim, qkv_rows = e->Dq + 2 * e->KVd;
     PrefillGemmArgs g = prefill_gemm_args(e, qkv_rows, D, n, start_pos, kPfMaxSplits);
     g.row0 = l * qkv_rows;
-    g.epi = kPfQkv;
     prefill_qkv_args(e, l, g);
     const cudaError_t ge = launch_prefill_gemm_t<__half, kPfQkv>(e, e->pf_map_wqkv, e->pf_map_xn, g);
     CU(ge);

@@ -21,7 +21,7 @@
 // src/ops.cpp like the decode path.  The causal attention of the block is a tensor-core
 // flash attention over the cache (prefill_attention.cuh; other head sizes: prefill_attention_kernel).
 //
-// Tensor maps cover this GPU's own memory only; no cluster multicast is used anywhere.
+// Tensor maps cover this GPU's own memory only, and no copy is a multicast one.
 #pragma once
 #include <cuda.h>
 
@@ -32,7 +32,6 @@ namespace lpp {
 constexpr int kPfTile = 64;          // tokens of an item of the CTA kernel (rows of its activation tiles)
 constexpr int kPfMaxTokens = 1024;   // most tokens of a block
 constexpr int kPfKc = 128;           // inputs per stage: two 64-wide (128-byte) swizzled sub-tiles per operand
-constexpr int kPfSubBytesX = kPfTile * 128;  // one activation sub-tile: 64 tokens x 64 inputs
 constexpr int kPfMaxSplits = 8;
 constexpr int kPfRingBytes = 192 * 1024;
 constexpr int kPfSmemBytes = 1024 /*barriers*/ + 1024 /*alignment slack*/ + kPfRingBytes;
@@ -68,7 +67,6 @@ struct PrefillGemmArgs {
     int start_pos;        // position of token 0
     int tile;             // tokens of an item: kPfTile (this file's kernel) or kPairTokens (prefill_pair.cuh)
     int box_tokens;       // this file's kernel: token rows of an activation tile, a multiple of 16 up to kPfTile
-    int epi;
     int splits;           // K is cut into this many ranges: work item = (row tile, token tile, range)
     StepState* st;
     // kPfResid: x[t][row] += c (x: [tokens][n_rows] FP32) when splits == 1; else the partial sums go to
@@ -121,9 +119,8 @@ __device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
 }
-// One value of the QKV rows: row `row` (and its pair partner `other`, the value of row ^ 1), token t: rotation of q and k
+// One value of the QKV rows of the FP32 path: row `row` (and its pair partner `other`, the value of row ^ 1), token t: rotation of q and k
 // pairs, q -> FP32 rows, k / v -> cache rows at the reference index.
-template <typename CT>
 __device__ __forceinline__ void pf_qkv_store(const PrefillGemmArgs& a, int row, int t, float v, float other) {
     const int pos = a.start_pos + t;
     if (row >= a.n_rows || t >= a.n_tokens) return;
@@ -147,7 +144,7 @@ __device__ __forceinline__ void pf_qkv_store(const PrefillGemmArgs& a, int row, 
         const int h = rr / hs, off = rr % hs;
         // cache index within the layer: h*(seq_len*hs) + pos*hs + off (src/scatter_kv.cu:15-16)
         const size_t idx = (size_t)h * ((size_t)a.seq_len * hs) + (size_t)pos * hs + off;
-        reinterpret_cast<CT*>(is_k ? a.k_cache : a.v_cache)[idx] = from_float<CT>(r);
+        reinterpret_cast<float*>(is_k ? a.k_cache : a.v_cache)[idx] = r;
     }
 }
 
@@ -173,7 +170,7 @@ __device__ __forceinline__ void pf_qkv_store(const PrefillGemmArgs& a, int row, 
 // (bounded) and frees the tensor memory.
 constexpr int kUmmaM = 128;
 constexpr int kUmmaSubW = kUmmaM * 128;                            // 16 KiB
-constexpr int kUmmaMaxStages = 8;
+constexpr int kUmmaMaxStages = 4;                                  // tiles of 16 tokens: 40 KiB a stage
 constexpr int kUmmaEpiWarps = 8;                                   // two per tensor-memory lane quarter: 32 tokens each
 constexpr int kUmmaThreads = (2 + kUmmaEpiWarps) * 32;
 constexpr int kUmmaN = 2 * kPfTile;                                // MMA N: the 64 hi rows and the 64 lo rows of the activation tile

@@ -159,7 +159,7 @@ static __global__ void __launch_bounds__(kF32Threads) prefill_f32_gemm_kernel(co
             a.out[(size_t)t * a.out_pitch + (row >> 1)] = __fmul_rn(__fmul_rn(s, sig), other);
         }
     } else {
-        pf_qkv_store<float>(a.qkv, row, t, s, other);
+        pf_qkv_store(a.qkv, row, t, s, other);
     }
 }
 
