@@ -2647,6 +2647,7 @@ static lpp_status prefill_maps(lpp_engine* e) {
     TRY(make_activation_map(&e->pf_map_xn, e->pf_xn, T, D));
     return make_weight_map(&e->pf_map_cls, e->wcls, e->Vp, D, false);
 }
+constexpr int kPfShort = 256;
 static lpp_status prefill_release(lpp_engine* e) {
     if (!e->pf_slab) return LPP_OK;
     CU(cudaStreamSynchronize(e->stream));
@@ -2655,7 +2656,8 @@ static lpp_status prefill_release(lpp_engine* e) {
     e->pf_cap = 0;
     return LPP_OK;
 }
-// Workspace for a portion of n tokens: room for one tile, or for the largest block that the cache has positions for.  Where
+// Workspace for a portion of n tokens: room for one tile, for a short block, or for the largest block that the cache has positions for
+// (a turn of a chat of the Llama-3-8B shape need not hold the workspace of a document).  Where
 // memory is short the blocks become smaller, down to one tile.  Logits, where the portion wants any, come first (and push out a
 // workspace of earlier portions): the blocks get what they leave.
 static lpp_status prefill_setup(lpp_engine* e, int n, bool logits) {
@@ -2674,7 +2676,7 @@ static lpp_status prefill_setup(lpp_engine* e, int n, bool logits) {
         }
     }
     const int most = (int)std::min<size_t>(e->pf_limit, align_up((size_t)e->c.seq_len, kPfTile));
-    int cap = n <= kPfTile ? kPfTile : most;
+    int cap = n <= kPfTile ? kPfTile : n <= kPfShort ? std::min(kPfShort, most) : most;
     if (e->pf_cap >= cap) return LPP_OK;
     TRY(prefill_release(e));
     size_t bytes = 0;

@@ -233,3 +233,19 @@ def test_first_step_behind_an_fp32_prompt(E):
         if ratios[-1] <= 1.25:
             break
     assert min(ratios) <= 1.25, ratios
+
+
+def test_short_prompts_take_a_short_workspace(E):
+    """65 to 256 tokens: a quarter of the largest block's rows; a longer portion behind them takes the rest."""
+    import torch
+    c, toks, (batched, loop) = pair(E, "mini-8b-f16", 1200)
+    ref = loop.extend(toks[:700], 0, [199, 699])
+    batched.extend(toks[:10], 0, [9])
+    before = free_bytes(torch)
+    check(batched.extend(toks[:200], 0, [199]), ref[:1], 2e-3)
+    short = before - free_bytes(torch)
+    check(batched.extend(toks[:700], 0, [699]), ref[1:], 2e-3)
+    assert 2 * short < before - free_bytes(torch)
+    check(batched.extend(toks[200:700], 200, [499]), ref[1:], 2e-3)
+    for e in (batched, loop):
+        e.close()
