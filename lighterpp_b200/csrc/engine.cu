@@ -2478,8 +2478,8 @@ struct SlabCarver {
         used += align_up(std::max<size_t>(bytes, 16), 256);
     }
 };
-// Floats of partial results that the attention splits of one token leave.
-static size_t prefill_f32_part_row(const lpp_engine* e) { return (size_t)e->Hl * e->attn_splits * (e->hs + 2); }
+// Floats of partial results that `splits` attention splits of one token leave.
+static size_t prefill_f32_part_row(const lpp_engine* e, int splits) { return (size_t)e->Hl * splits * (e->hs + 2); }
 static size_t prefill_carve_f32(lpp_engine* e, int cap, char* base) {
     const size_t D = e->Dp, T = cap;
     SlabCarver c = {base};
@@ -2488,8 +2488,8 @@ static size_t prefill_carve_f32(lpp_engine* e, int cap, char* base) {
     c.take(&e->pf_att, T * e->Dq * 4);
     c.take(&e->pf_hb, T * e->Fl * 4);
     c.take(&e->pf_q, T * e->Dq * 4);
-    c.take(&e->pf_part, kPfTile * prefill_f32_part_row(e) * 4);
-    c.take(&e->pf_counters, (size_t)kPfTile * e->KVHl * e->attn_z * 4);  // zero between launches
+    c.take(&e->pf_part, kPfTile * prefill_f32_part_row(e, e->attn_splits) * 4);
+    c.take(&e->pf_counters, T * e->KVHl * e->attn_z * 4);  // zero between launches
     c.take(&e->pf_tokens, T * sizeof(int));
     c.take(&e->pf_rows, T * sizeof(int));
     return c.used;
@@ -2590,9 +2590,20 @@ static int row_attention_ctas(const ModelLayer& y, int n) {
     const int tokens = kRaRows / y.group_heads;
     return (n + tokens - 1) / tokens * row_attention_halves(y) * y.groups;
 }
+template <int EPI>
+static lpp_status allow_tile_smem(const lpp_engine* e) {
+    CU(cudaFuncSetAttribute(prefill_f32_tile_kernel<EPI, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem_optin));
+    CU(cudaFuncSetAttribute(prefill_f32_tile_kernel<EPI, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem_optin));
+    return LPP_OK;
+}
 static lpp_status prefill_maps(lpp_engine* e) {
     const lpp_config& c = e->c;
-    if (prefill_f32(e)) return LPP_OK;
+    if (prefill_f32(e)) {
+        TRY(allow_tile_smem<kPfQkv>(e));
+        TRY(allow_tile_smem<kPfResid>(e));
+        TRY(allow_tile_smem<kPfSwiglu>(e));
+        return allow_tile_smem<kPfStore>(e);
+    }
     const size_t D = e->Dp, L = c.n_layers, T = e->pf_cap;
     if (!e->layers.empty()) {
         for (ModelLayer& y : e->layers) {
@@ -3010,6 +3021,22 @@ static lpp_status prefill_gemm_f32(lpp_engine* e, const void* w, const void* x, 
     g.K = K;
     gemv_geometry(g, 4, kStageTarget);
     a.kc = (e->c.flags & LPP_FLAG_GEMV_LDG) ? K : g.kc;
+    a.st = e->st;
+    // Tiles in shared memory where the step sums a row up in one go (so that its order can be kept), they fit, and half of the SMs get
+    // a CTA; else the kernel that reads both operands through L1, whose CTAs are smaller (whole prompts, tiles always / by this rule, us:
+    // stories15M 17 tokens 238 / 227, 33 255 / 249; 4 layers of 512 x 1024 17 tokens 203 / 189, 64 236 / 210).  Four lanes to 16 outputs (32 rows a CTA) where that
+    // gives every SM a CTA, else eight (16 rows): half as many steps for a warp.
+    const int tiles = (n + kTileTokens - 1) / kTileTokens;
+    if (a.kc >= K && n > kF32Tokens && (n_rows + kTileRows<8> - 1) / kTileRows<8> * tiles >= e->num_sms / 2) {
+        const bool wide = (n_rows + kTileRows<4> - 1) / kTileRows<4> * tiles >= e->num_sms;
+        const int rows = wide ? kTileRows<4> : kTileRows<8>;
+        const size_t smem = f32_tile_smem(K, rows);
+        if (smem <= e->smem_optin) {
+            CU(launch_kernel(wide ? prefill_f32_tile_kernel<EPI, 4> : prefill_f32_tile_kernel<EPI, 8>, dim3((n_rows + rows - 1) / rows, tiles), dim3(32 * kTileWarps), smem,
+                             e->stream, true, a));
+            return LPP_OK;
+        }
+    }
     const dim3 grid((n_rows + kF32Rows - 1) / kF32Rows, (n + kF32Tokens - 1) / kF32Tokens);
     CU(launch_kernel(a.kc < K ? prefill_f32_gemm_kernel<EPI, true> : prefill_f32_gemm_kernel<EPI, false>, grid, dim3(kF32Threads), 0, e->stream, true, a));
     return LPP_OK;
@@ -3032,16 +3059,19 @@ static lpp_status prefill_f32_norm(lpp_engine* e, int n, const float* w, bool em
 }
 template <int DPL>
 static cudaError_t launch_f32_attn_d(lpp_engine* e, const AttnArgs& a, dim3 grid, int start_pos, int block_pos) {
-    const int part_row = (int)prefill_f32_part_row(e);
     return launch_kernel(e->attn_gb == 4   ? prefill_f32_attn_kernel<DPL, 4>
                          : e->attn_gb == 2 ? prefill_f32_attn_kernel<DPL, 2>
                                            : prefill_f32_attn_kernel<DPL, 1>,
-                         grid, dim3(kAttnKernelThreads), 0, e->stream, true, a, start_pos, block_pos, e->attn_z, e->Dq, part_row);
+                         grid, dim3(kAttnKernelThreads), 0, e->stream, true, a, start_pos, block_pos, e->attn_z, e->Dq, (int)prefill_f32_part_row(e, a.n_splits));
 }
-// Attention of a block, a tile of tokens at a time (what the splits of their partial results take).
+// Attention of a block: as many tokens a launch as there is room for the partial results of their splits, all of them where one split does
+// (201 tokens of the stories15M shape: one launch instead of four that each take a launch's latency, 47 -> 28 us a layer; 23 with a third CTA an SM).
 static lpp_status prefill_f32_attention(lpp_engine* e, const PrefillGemmArgs& g, int n, int start_pos) {
-    for (int i = 0; i < n; i += kPfTile) {
-        const int m = std::min(kPfTile, n - i);
+    const int splits = attn_effective_splits(start_pos + n, e->attn_splits);
+    const size_t room = kPfTile * prefill_f32_part_row(e, e->attn_splits) / prefill_f32_part_row(e, splits);
+    const int tile = splits == 1 ? n : (int)std::min<size_t>(n, room);
+    for (int i = 0; i < n; i += tile) {
+        const int m = std::min(tile, n - i);
         AttnArgs a = {};
         a.q = e->pf_q + (size_t)i * e->Dq;
         a.k_cache = g.k_cache;
@@ -3053,7 +3083,7 @@ static lpp_status prefill_f32_attention(lpp_engine* e, const PrefillGemmArgs& g,
         a.seq_len = e->c.seq_len;
         a.head_size = e->hs;
         a.gqa = e->gqa;
-        a.n_splits = e->attn_splits;
+        a.n_splits = splits;
         a.n_kv_heads = e->KVHl;
         const dim3 grid(attn_effective_splits(start_pos + i + m, a.n_splits, a.min_chunk), e->KVHl, m * e->attn_z);
         cudaError_t r = cudaErrorInvalidValue;
@@ -3069,6 +3099,9 @@ static lpp_status prefill_f32_attention(lpp_engine* e, const PrefillGemmArgs& g,
     }
     return LPP_OK;
 }
+// Logits of up to this many tokens go through the step's classifier GEMV one by one: it streams the matrix where the block kernel, whose
+// warps take eight tokens whether there are as many or not, is bound by the loads of its tiles (32 000 x 288, one token: 69 us -> 10).
+constexpr int kF32GemvRows = 4;
 // prefill_block for engines with FP32 weights.
 static lpp_status prefill_block_f32(lpp_engine* e, int n, int start_pos, int n_want, float* h_logits) {
     const lpp_config& c = e->c;
@@ -3092,6 +3125,23 @@ static lpp_status prefill_block_f32(lpp_engine* e, int n, int start_pos, int n_w
     for (int i = 0; i < n_want; i += kPfTile) {
         const int m = std::min(kPfTile, n_want - i);
         TRY(prefill_f32_norm(e, m, e->rms_final, false, e->pf_rows + i));
+        if (m <= kF32GemvRows) {
+            for (int r = 0; r < m; ++r) {
+                GemvArgs a = {};
+                a.W = e->wcls;
+                a.n_rows = e->Vp;
+                a.K = (int)D;
+                a.x = (const float*)e->pf_xn + (size_t)r * D;
+                a.st = e->st;
+                a.vocab = c.vocab_size;
+                a.seq_len = c.seq_len;
+                a.out = e->pf_logits + (size_t)r * e->Vp;
+                CU(launch_gemv(e, kEpiStore, LPP_F32, a, true, e->stream));
+            }
+            CU(cudaMemcpy2DAsync(h_logits + (size_t)i * c.vocab_size, (size_t)c.vocab_size * 4, e->pf_logits, (size_t)e->Vp * 4, (size_t)c.vocab_size * 4, m,
+                                 cudaMemcpyDeviceToHost, e->stream));
+            continue;
+        }
         TRY((prefill_gemm_f32<kPfStore>(e, e->wcls, e->pf_xn, c.vocab_size, (int)D, m, e->pf_logits, c.vocab_size)));
         CU(cudaMemcpyAsync(h_logits + (size_t)i * c.vocab_size, e->pf_logits, (size_t)m * c.vocab_size * 4, cudaMemcpyDeviceToHost, e->stream));
     }

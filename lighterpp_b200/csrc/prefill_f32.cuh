@@ -3,9 +3,10 @@
 // The same arithmetic as the decode step, operation by operation and in the same order, only that every weight row is used
 // for a block of tokens: a prompt's cache rows and logits are bit for bit those of the token-by-token loop, which streams
 // all weights and pays a step's launches and host round trip for every token.  Bound by FP32 FMAs for large shapes, by the
-// launches for small ones.  201 tokens of the stories15M shape: 20.9 ms token by token, 0.77 ms here.
+// launches for small ones.
 #pragma once
 #include "attention.cuh"
+#include "mamba.cuh"
 #include "prefill.cuh"
 
 namespace lpp {
@@ -81,6 +82,7 @@ struct PrefillF32Args {
     int n_rows, K, kc, n_tokens;
     float* out;          // kPfResid: [tokens][out_pitch] += ; kPfSwiglu: [tokens][out_pitch], column row / 2; kPfStore: [tokens][out_pitch]
     int out_pitch, act;
+    StepState* st;
     PrefillGemmArgs qkv; // kPfQkv: what pf_qkv_store takes
 };
 template <int EPI, bool CHUNKS>
@@ -163,10 +165,164 @@ static __global__ void __launch_bounds__(kF32Threads) prefill_f32_gemm_kernel(co
     }
 }
 
+// The same products for rows short enough that a tile of weight rows and of tokens fits shared memory.  KS (4 or 8) lanes share four
+// rows x four tokens: lane c forms, one after the other, the partial sums that lanes c, c + KS, .. of the step's warp have (two FMA
+// chains, here one pair: fma.rn.f32x2 rounds both halves like fmaf) and adds them up in the order in which warp_sum's tree takes
+// them (lanes 16, 8, 4 apart); the last two or three levels are shuffles.  The kernel above needs 12 global vector loads and the
+// transposing tree for a warp's 32 outputs, on one CTA an SM.  Bound by the instructions issued; a warp has 8 vector loads from shared
+// memory and 32 pair FMAs for 16 rows x 8 tokens x 16 inputs.  201 tokens of the stories15M shape, us a launch above -> here: gate|up 30.1 ->
+// 16.9, q|k|v 21.1 -> 12.4, output and down projection 13.6 -> 8.6.  (Lanes as tokens, weights read as broadcasts: 18.5, 15.6, 16.6: a vector
+// load from shared memory keeps its pipe for four clocks also where all lanes read the same address.)
+constexpr int kTileTokens = 32, kTileWarps = 8;  // four warps side by side cover the tokens, 8 each
+template <int KS>
+constexpr int kTileRows = 2 * 64 / KS;  // of a CTA: two warps of 4 (32 / KS / 2) rows each
+__host__ __device__ inline int f32_tile_pitch(int K) { return ((K >> 2) | 1) << 2; }  // odd number of 16-byte pieces: no bank conflicts
+__host__ __device__ inline size_t f32_tile_smem(int K, int rows) { return (size_t)(rows + kTileTokens) * f32_tile_pitch(K) * 4; }
+template <int EPI, int KS>
+static __global__ void __launch_bounds__(kTileWarps * 32, 2) prefill_f32_tile_kernel(const PrefillF32Args a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    constexpr int kRows = kTileRows<KS>, kGroups = 32 / KS / 2;  // row groups of a warp
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K = a.K, nv = K >> 2, pitch = f32_tile_pitch(K) >> 2;
+    uint4* ws = reinterpret_cast<uint4*>(smem);
+    uint4* xs = ws + (size_t)kRows * pitch;
+    const int row0 = blockIdx.x * kRows, tok0 = blockIdx.y * kTileTokens;
+    pdl_launch_dependents();
+    // A warp fetches row after row.  Rows and tokens beyond the end are neither fetched nor stored: what lies in their place only
+    // reaches their own sums (to repeat the last token made every CTA read that row 32 times: 33 tokens 384 us, 64 tokens 280).
+    for (int r = warp; r < min(kRows, a.n_rows - row0); r += kTileWarps) {
+        const uint4* src = reinterpret_cast<const uint4*>(a.w + (size_t)(row0 + r) * K);
+        for (int v = lane; v < nv; v += 32) cp_async_16(ws + r * pitch + v, src + v, true);  // constants: ahead of the dependency wait
+    }
+    pdl_wait();
+    for (int r = warp; r < min(kTileTokens, a.n_tokens - tok0); r += kTileWarps) {
+        const uint4* src = reinterpret_cast<const uint4*>(a.x + (size_t)(tok0 + r) * K);
+        for (int v = lane; v < nv; v += 32) cp_async_16(xs + r * pitch + v, src + v, true);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    const int c = lane % KS, group = lane / KS;
+    const int r0 = ((warp >> 2) * kGroups + group % kGroups) * 4, t0 = (warp & 3) * 8 + (group / kGroups) * 4;  // within the tile
+    uint32_t wa[4], xa[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        wa[i] = smem_u32(ws + (r0 + i) * pitch);
+        xa[i] = smem_u32(xs + (t0 + i) * pitch);
+    }
+    auto lds = [](uint32_t at) -> ulonglong2 {
+        ulonglong2 v;
+        asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(at));
+        return v;
+    };
+    // Partial sums of lane l of the step's warp, as pairs of tokens.  (A chain that starts with a product instead of a sum with +0, and p + q
+    // without the sum with +0 it goes into there, differ from the step's in the sign of a zero only: the last line makes up for that.)
+    auto chain = [&](int l, f32x2 (&s)[4][2]) {
+        f32x2 pq[4][4];
+        auto step = [&](uint32_t v, bool first) {
+            ulonglong2 wv[4], xv[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                wv[i] = lds(wa[i] + v);
+                xv[i] = lds(xa[i] + v);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) pq[i][j] = first ? mul2(wv[i].x, xv[j].x) : fma2(wv[i].x, xv[j].x, pq[i][j]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) pq[i][j] = fma2(wv[i].y, xv[j].y, pq[i][j]);
+        };
+        const uint32_t end = 16u * (uint32_t)nv;
+        uint32_t v = 16u * (uint32_t)l;
+        if (v < end) {
+            step(v, true);
+#pragma unroll 1
+            for (v += 512u; v < end; v += 512u) step(v, false);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) pq[i][j] = 0ull;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) s[i][j] = pack_f2(pair_sum(pq[i][2 * j]), pair_sum(pq[i][2 * j + 1]));
+    };
+    auto add = [](f32x2 (&s)[4][2], const f32x2 (&o)[4][2]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) s[i][j] = add2(s[i][j], o[i][j]);
+    };
+    f32x2 total[4][2];
+#pragma unroll
+    for (int b = 0; b < 8 / KS; ++b) {  // KS 4: lanes c, then c + 4
+        f32x2 s8[4][2], s16[4][2], s[4][2];
+        chain(c + 4 * b, s8);
+        chain(c + 4 * b + 16, s);
+        add(s8, s);
+        chain(c + 4 * b + 8, s16);
+        chain(c + 4 * b + 24, s);
+        add(s16, s);
+        add(s8, s16);
+        if (b == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) total[i][j] = s8[i][j];
+        } else {
+            add(total, s8);
+        }
+    }
+    float sum[4];  // lane c goes on with token c of the four
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 two = unpack_f2(total[i][j >> 1]);
+            float v = j & 1 ? two.y : two.x;
+            if constexpr (KS == 8) v += __shfl_xor_sync(0xffffffffu, v, 4);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            if (j == 0 || c == j) sum[i] = v + 0.f;
+        }
+    if (c >= 4) return;
+    const int row = row0 + r0, t = tok0 + t0 + c;
+    if (t >= a.n_tokens) return;
+    if constexpr (EPI == kPfStore) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (row + i < a.n_rows) a.out[(size_t)t * a.out_pitch + row + i] = sum[i];
+    } else if constexpr (EPI == kPfResid) {
+        float* p = a.out + (size_t)t * a.out_pitch + row;
+        float old[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) old[i] = row + i < a.n_rows ? p[i] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (row + i < a.n_rows) p[i] = sum[i] + old[i];  // x += W.xb (src/model.cpp:232, 239)
+    } else if constexpr (EPI == kPfSwiglu) {
+        // rows interleaved (gate, up): hb = (h1*sigmoid(h1))*h3 (src/ops.cpp:78-87)
+#pragma unroll
+        for (int i = 0; i < 4; i += 2)
+            if (row + i < a.n_rows) {
+                const float sig = __fdiv_rn(1.0f, 1.0f + expf(-act_gate_arg(a.act, sum[i])));
+                a.out[(size_t)t * a.out_pitch + ((row + i) >> 1)] = __fmul_rn(__fmul_rn(sum[i], sig), sum[i + 1]);
+            }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) pf_qkv_store(a.qkv, row + i, t, sum[i], sum[i ^ 1]);
+    }
+}
+
 // The decode attention of attn_decode_kernel for a block of tokens: token t attends to positions 0 .. start_pos + t with the
-// splits that a step at its position uses; rows before block_pos are complete before the block's first kernel starts.  grid: (splits of the last token, kv heads, tokens x head batches)
+// splits that a step at its position uses (a.n_splits: at least as many as the last token's); rows before block_pos are complete before the block's first kernel starts.  grid: (splits of the last token, kv heads, tokens x head batches)
+// (Bound by the latency of its stages: small head sizes give up registers for a third CTA an SM.)
 template <int DPL, int GB>
-static __global__ void __launch_bounds__(kAttnKernelThreads) prefill_f32_attn_kernel(AttnArgs a, int start_pos, int block_pos, int n_z, int q_rows,
+static __global__ void __launch_bounds__(kAttnKernelThreads, DPL * GB <= 8 ? 3 : 1) prefill_f32_attn_kernel(AttnArgs a, int start_pos, int block_pos, int n_z, int q_rows,
                                                                                       int part_row) {
     __shared__ float s_scratch[(kAttnKernelThreads / 32) * GB * (DPL * 8 + 2)];
     __shared__ int s_last;

@@ -1,0 +1,31 @@
+"""FP32 prompts through tiles in shared memory, the attention of a block in one launch and the classifier of a few tokens: bit for bit
+the token loop's logits around the tiles' edges (tokens 32, rows 16 and 32, rows of fewer inputs than a warp has lanes and of every
+remainder of 128), with one and several splits of the positions, and for one, four, five and more wanted tokens."""
+import numpy as np
+import pytest
+
+from lighterpp_b200 import synth
+from lighterpp_b200.formats import ModelConfig
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("cfg", [ModelConfig(96, 1192, 2, 6, 6, 1210, 400), ModelConfig(288, 768, 2, 6, 2, 1026, 400), ModelConfig(384, 1020, 1, 8, 8, 1202, 400),
+                                 ModelConfig(768, 100, 1, 12, 4, 1190, 400)], ids=str)
+def test_bits_equal_the_token_loop(cfg):
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from lighterpp_b200 import engine as E
+    T = synth.gen_model(cfg, 7, "f32", True)
+    toks = synth.prompt_tokens(cfg.vocab_size, 400, 7)
+    batched, loop = [E.Engine(cfg, "f32", "f32", flags=f) for f in (0, E.FLAG_NO_PREFILL_GEMM)]
+    for e in (batched, loop):
+        e.load_weights(T)
+    ref = loop.extend(toks, 0, range(400))
+    for n, want in ((17, 4), (31, 1), (32, 5), (33, 17), (63, 1), (97, 64), (128, 4), (129, 70), (257, 3), (400, 33)):
+        assert np.array_equal(batched.extend(toks[:n], 0, range(n - want, n)), ref[n - want:n]), (n, want)
+    batched.extend(toks[:130], 0)  # behind a cache
+    assert np.array_equal(batched.extend(toks[130:], 130, range(270)), ref[130:])
+    for e in (batched, loop):
+        e.close()
