@@ -2774,11 +2774,18 @@ static lpp_status prefill_norm(lpp_engine* e, int n, int block_n, const float* w
     a.part_tokens = prefill_part_tokens(block_n);
     a.splits = embed ? 1 : parts;
     a.st = e->st;
-    const dim3 threads(prefill_norm_threads(a.D, a.splits > 1));
+    const int mode = a.splits <= 1 ? kNormPlain : n * prefill_norm_threads(a.D, kNormFewParts) < kPfNormManyThreads ? kNormFewParts : kNormManyParts;
+    const dim3 threads(prefill_norm_threads(a.D, mode));
+#define LPP_NORM(T)                                                                                                                        \
+    CU(launch_kernel(mode == kNormPlain      ? prefill_norm_kernel<T, kNormPlain>                                                           \
+                     : mode == kNormFewParts ? prefill_norm_kernel<T, kNormFewParts>                                                        \
+                                             : prefill_norm_kernel<T, kNormManyParts>,                                                      \
+                     dim3(n), threads, 0, e->stream, pdl, a))
     if (e->c.weight_dtype == LPP_BF16)
-        CU(launch_kernel(a.splits > 1 ? prefill_norm_kernel<__nv_bfloat16, true> : prefill_norm_kernel<__nv_bfloat16, false>, dim3(n), threads, 0, e->stream, pdl, a));
+        LPP_NORM(__nv_bfloat16);
     else
-        CU(launch_kernel(a.splits > 1 ? prefill_norm_kernel<__half, true> : prefill_norm_kernel<__half, false>, dim3(n), threads, 0, e->stream, pdl, a));
+        LPP_NORM(__half);
+#undef LPP_NORM
     return LPP_OK;
 }
 

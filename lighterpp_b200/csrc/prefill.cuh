@@ -629,15 +629,21 @@ static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const Pr
 // statistics cover the first norm_n inputs, the rest is zero padding with zero weights.  grid: rows; prefill_norm_threads
 // threads.  Without partial sums there are many rows: a thread has four pieces of four floats, few enough threads and registers
 // that the rows of a block are all resident at once (one or two pieces on 512 threads, two or three rows an SM: 13 us for 1023
-// rows of 2048 and 22 us for 1000 of 4096; now 6 and 11).  With partial sums there are few rows and the latency counts: one
-// or two pieces a thread, all ranges in flight (47 rows of 2048 with 8 ranges: 4.5 us, four pieces a thread 8.3).
-template <bool PARTS>
+// rows of 2048 and 22 us for 1000 of 4096; now 6 and 11).  With partial sums of a few rows the latency counts: one
+// or two pieces a thread, all ranges in flight (47 rows of 2048 with 8 ranges: 4.5 us, four pieces a thread 8.3), one row an SM.  Many
+// rows become waves that way: half the threads and registers for four rows an SM instead (517 rows of 2048 with partial sums: 12.3 -> 7.9
+// us), from 384 rows of 512 threads on (whole prompts of the TinyLlama shape, few / many rows' kernel: 200 tokens 1878 / 1946 us, 350
+// 2127 / 2169, 400 2554 / 2501; kolatar-300m, rows of 256 threads: 400 tokens 2739 / 2788, 900 4080 / 3938).
+enum PfNormMode : int { kNormPlain = 0, kNormFewParts = 1, kNormManyParts = 2 };
+constexpr int kPfNormManyThreads = 384 * 512;
+template <int MODE>
 struct PfNorm {
-    static constexpr int kPer = PARTS ? 2 : 4, kMaxThreads = PARTS ? 512 : 256;
+    static constexpr int kPer = MODE == kNormFewParts ? 2 : 4, kMaxThreads = MODE == kNormFewParts ? 512 : 256;
+    static constexpr int kResident = MODE == kNormPlain ? 5 : MODE == kNormManyParts ? 4 : 1;
 };
-static int prefill_norm_threads(int D, bool parts) {
-    const int pieces = parts ? D / 4 : (D / 4 + PfNorm<false>::kPer - 1) / PfNorm<false>::kPer;
-    return std::min(parts ? PfNorm<true>::kMaxThreads : PfNorm<false>::kMaxThreads, std::max(64, (pieces + 31) / 32 * 32));
+static int prefill_norm_threads(int D, int mode) {
+    const int per = mode == kNormPlain ? PfNorm<kNormPlain>::kPer : mode == kNormManyParts ? 2 : 1, pieces = (D / 4 + per - 1) / per;
+    return std::min(mode == kNormFewParts ? PfNorm<kNormFewParts>::kMaxThreads : PfNorm<kNormPlain>::kMaxThreads, std::max(64, (pieces + 31) / 32 * 32));
 }
 struct PrefillNormArgs {
     float* x;            // [tokens][D]
@@ -664,12 +670,13 @@ __device__ __forceinline__ float norm_block_sum(float v, float* red, int tid) {
     __syncthreads();
     return warp_sum((tid & 31) < (int)(blockDim.x >> 5) ? red[tid & 31] : 0.f);
 }
-// PARTS: partial sums are added first.  Only the weights (emb, norm_w, norm_b) are loaded as read-only data: a load of what
+// Partial sums, where there are any, are added first.  Only the weights (emb, norm_w, norm_b) are loaded as read-only data: a load of what
 // the preceding kernel produced must not become an invariant one, which the compiler may move above the dependency wait.
-template <typename T, bool PARTS>
-static __global__ void __launch_bounds__(PfNorm<PARTS>::kMaxThreads, PARTS ? 1 : 5) prefill_norm_kernel(const PrefillNormArgs a) {
-    constexpr int kPfNormPer = PfNorm<PARTS>::kPer;
-    __shared__ float red[2][PfNorm<PARTS>::kMaxThreads / 32];
+template <typename T, int MODE>
+static __global__ void __launch_bounds__(PfNorm<MODE>::kMaxThreads, PfNorm<MODE>::kResident) prefill_norm_kernel(const PrefillNormArgs a) {
+    constexpr int kPfNormPer = PfNorm<MODE>::kPer;
+    constexpr bool PARTS = MODE != kNormPlain;
+    __shared__ float red[2][PfNorm<MODE>::kMaxThreads / 32];
     pdl_launch_dependents();
     const int tid = threadIdx.x, D = a.D, nt = blockDim.x;
     const int nv4 = D >> 2;  // D is a multiple of 8
