@@ -2924,9 +2924,13 @@ static lpp_status prefill_latent_mixer(lpp_engine* e, int l, int n, int start_po
     f.st = e->st;
     f.lat = latent_args(e, y, r);
     f.lat.query = e->pf_lq;
-    const int q_sections = cache_only ? 0 : (y.q_plain_rows + y.q_rot_rows + 2 * kLatFinishThreads - 1) / (2 * kLatFinishThreads);
-    CU(launch_kernel(prefill_latent_finish_kernel<T>, dim3(n, 1 + q_sections), dim3(kLatFinishThreads), (size_t)y.latent_rows * 4, e->stream,
-                     true, f));
+    f.n_tokens = n;
+    const bool quads = y.d.dim % 4 == 0 && y.d.rot_dim % 4 == 0 && y.in_rows % 4 == 0 && n >= kLatFinishQuadTokens;
+    const int per_cta = (quads ? 4 : 2) * kLatFinishThreads;  // query rows
+    const int q_sections = cache_only ? 0 : (y.q_plain_rows + y.q_rot_rows + per_cta - 1) / per_cta;
+    const dim3 grid = quads ? dim3((n + kLatFinishTokens - 1) / kLatFinishTokens, kLatFinishTokens + q_sections) : dim3(n, 1 + q_sections);
+    CU(launch_kernel(quads ? prefill_latent_finish_kernel<T, true> : prefill_latent_finish_kernel<T, false>, grid, dim3(kLatFinishThreads),
+                     (size_t)y.latent_rows * 4, e->stream, true, f));
     if (cache_only) return LPP_OK;
     PrefillGemmArgs q = prefill_gemm_args(e, y.rank_pitch, y.dim_pitch, n, start_pos, 1, H);
     q.group_stride = y.rank_pitch;
@@ -2957,12 +2961,16 @@ static lpp_status prefill_shared_kv_mixer(lpp_engine* e, int l, int n, int start
     f.n_rows = y.in_rows;
     f.start_pos = start_pos;
     f.seq_len = e->c.seq_len;
+    f.n_tokens = n;
     f.keys_only = cache_only;
     f.st = e->st;
     f.kv = shared_kv_args(e, y, r);
     f.kv.query = e->pf_lq;
     f.kv.gate = e->pf_gate;
-    CU(launch_kernel(prefill_shared_kv_finish_kernel, dim3(n, (y.in_rows / 2 + 255) / 256), dim3(256), 0, e->stream, true, f));
+    if (y.d.dim % 4 == 0 && f.kv.rot % 4 == 0 && n >= kKvFinishQuadTokens)
+        CU(launch_kernel(prefill_shared_kv_finish4_kernel, dim3((n + kKvFinishTokens - 1) / kKvFinishTokens, (y.in_rows + 1023) / 1024), dim3(256), 0, e->stream, true, f));
+    else
+        CU(launch_kernel(prefill_shared_kv_finish_kernel, dim3(n, (y.in_rows / 2 + 255) / 256), dim3(256), 0, e->stream, true, f));
     return cache_only ? LPP_OK : prefill_row_attention(e, y, r, n, start_pos, e->pf_att);
 }
 

@@ -629,25 +629,72 @@ static __global__ void __launch_bounds__(128) prefill_latent_combine_kernel(cons
 // ---- prompt block: after the input GEMM (partial sums over ranges of K, added in range order): plain queries -> hi + lo
 // operands of the query GEMM, rotated parts turned into query and cache rows, latent normed into its cache row, gates
 // through the sigmoid.  The section layout of the rows is that of latent_in_rows.
-// grid: (tokens, 1 + query sections): y = 0 takes latent, rotated key part and gates, y >= 1 512 query rows each.
-constexpr int kLatFinishThreads = 256;
+// grid: (tokens, 1 + query sections): y = 0 takes latent, rotated key part and gates, y >= 1 512 query rows each.  QUADS: where every
+// section and head starts on a multiple of four rows, a thread takes four query rows of kLatFinishTokens tokens (one pair of one token a
+// thread made 7161 CTAs of 1023 tokens of the rutenex-1b shape, 21.7 us; now 11.6); grid (tokens / kLatFinishTokens, kLatFinishTokens +
+// query sections of 1024 rows), y < kLatFinishTokens takes one token's latent, rotated key part and gates.
+constexpr int kLatFinishThreads = 256, kLatFinishTokens = 4;
+constexpr int kLatFinishQuadTokens = 128;  // fewer tokens: more CTAs rather than more work in each (70 tokens of rutenex-300m: 1745 us, quads 1777)
 struct PrefillLatentFinishArgs {
     const float* part;  // [splits][part_tokens][n_rows]
     int part_tokens, cap, n_rows, splits;
-    int start_pos, seq_len;
+    int n_tokens, start_pos, seq_len;
     void* qn;           // plain queries: [2 planes][cap][heads * dim_pitch]
     float* gate;        // [tokens][heads]
     StepState* st;
     LatentArgs lat;     // query: [tokens * heads][row_width]
 };
-template <typename T>
+template <typename T, bool QUADS>
 static __global__ void __launch_bounds__(kLatFinishThreads) prefill_latent_finish_kernel(const PrefillLatentFinishArgs a) {
     extern __shared__ float fin_smem[];  // the raw latent
     __shared__ float red[kLatFinishThreads / 32];
     pdl_launch_dependents();
-    pdl_wait();
     const LatentArgs& L = a.lat;
-    const int t = blockIdx.x, tid = threadIdx.x, pos = a.start_pos + t;
+    if constexpr (QUADS) {
+        constexpr int N = kLatFinishTokens;
+        if ((int)blockIdx.y >= N) {
+            const int row = 4 * (((int)blockIdx.y - N) * kLatFinishThreads + (int)threadIdx.x), t0 = blockIdx.x * N;
+            const bool mine = row < L.q_plain_rows + L.q_rot_rows, plain = row < L.q_plain_rows;
+            const int r = plain ? row : row - L.q_plain_rows, per = plain ? L.dim : L.rot, h = r / per, j = r - h * per;
+            float4 cs[N];  // constants: ahead of the dependency wait
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const int pos = a.start_pos + t0 + i;
+                if (mine && !plain && pos >= 0 && pos < a.seq_len) cs[i] = __ldg(reinterpret_cast<const float4*>(L.rope + (size_t)pos * (L.rot >> 1) + (j >> 1)));
+            }
+            pdl_wait();
+            if (!mine) return;
+            float4 v[N];
+            prefill_sums<N>(a.part, a.part_tokens, a.n_rows, a.splits, a.n_tokens, t0, row, v);
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const int t = t0 + i, pos = a.start_pos + t;
+                if (t >= a.n_tokens || pos < 0 || pos >= a.seq_len) break;  // (the section of the latent reports a bad position)
+                if (plain) {
+                    T* qn = reinterpret_cast<T*>(a.qn) + ((size_t)t * L.heads + h) * L.dim_pitch + j;
+                    const float x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+                    __align__(8) T hi[4], lo[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) split_pair(x[k], hi[k], lo[k]);
+                    if (h < L.heads) {  // beyond: padding rows
+                        *reinterpret_cast<uint2*>(qn) = *reinterpret_cast<const uint2*>(hi);
+                        *reinterpret_cast<uint2*>(qn + (size_t)a.cap * L.heads * L.dim_pitch) = *reinterpret_cast<const uint2*>(lo);
+                    }
+                } else {
+                    __half* q = reinterpret_cast<__half*>(L.query) + ((size_t)t * L.heads + h) * L.row_width + L.rank_pitch + j;
+                    const float4 c = cs[i], y = v[i];
+                    __align__(8) __half2 o[2] = {
+                        __floats2half2_rn(__fsub_rn(__fmul_rn(y.x, c.x), __fmul_rn(y.y, c.y)), __fadd_rn(__fmul_rn(y.y, c.x), __fmul_rn(y.x, c.y))),
+                        __floats2half2_rn(__fsub_rn(__fmul_rn(y.z, c.z), __fmul_rn(y.w, c.w)), __fadd_rn(__fmul_rn(y.w, c.z), __fmul_rn(y.z, c.w)))};
+                    *reinterpret_cast<uint2*>(q) = *reinterpret_cast<const uint2*>(o);
+                }
+            }
+            return;
+        }
+    }
+    pdl_wait();
+    const int t = QUADS ? (int)(blockIdx.x * kLatFinishTokens + blockIdx.y) : (int)blockIdx.x, tid = threadIdx.x, pos = a.start_pos + t;
+    if (QUADS && t >= a.n_tokens) return;
     if (pos < 0 || pos >= a.seq_len) {
         if (tid == 0) atomicOr(&a.st->status, kStatusBadPos);
         return;
@@ -670,7 +717,7 @@ static __global__ void __launch_bounds__(kLatFinishThreads) prefill_latent_finis
         return make_float2(__fsub_rn(__fmul_rn(v.x, cs.x), __fmul_rn(v.y, cs.y)), __fadd_rn(__fmul_rn(v.y, cs.x), __fmul_rn(v.x, cs.y)));
     };
     const int q_rows = L.q_plain_rows + L.q_rot_rows;
-    if (blockIdx.y > 0) {
+    if (!QUADS && blockIdx.y > 0) {
         const int row = ((int)blockIdx.y - 1) * 2 * kLatFinishThreads + 2 * tid;
         if (row >= q_rows) return;
         float2 v = sum2(row);

@@ -22,12 +22,15 @@ __device__ __forceinline__ float2 prefill_sum2(const float* part, int part_token
 }
 
 // ---- attention whose values are its keys (shared_kv.cuh): after the input GEMM (partial sums over ranges of K, added in
-// range order), one row pair per thread.
-// grid: (tokens, ceil(row pairs / 256))
+// range order), one row pair per thread; grid: (tokens, ceil(row pairs / 256)).  Where every section, head and rotated part starts on a
+// multiple of four rows: four rows of kKvFinishTokens tokens a thread, as in prefill_latent_finish_kernel (517 tokens of the kolatar-1b
+// shape 19.2 -> 8.7 us); grid: (ceil(tokens / kKvFinishTokens), ceil(rows / 1024)).
+constexpr int kKvFinishTokens = 4;
+constexpr int kKvFinishQuadTokens = 192;  // fewer tokens: more CTAs rather than more work in each (130 tokens of kolatar-300m: 1514 us, quads 1527)
 struct PrefillSharedKvArgs {
     const float* part;  // [splits][part_tokens][n_rows]
     int part_tokens, n_rows, splits;
-    int start_pos, seq_len;
+    int n_tokens, start_pos, seq_len;
     int keys_only;      // only the cache rows are wanted
     StepState* st;
     SharedKvArgs kv;    // query: [tokens][heads][row_width] FP16, gate: [tokens][heads * dim]
@@ -51,6 +54,55 @@ static __global__ void __launch_bounds__(256) prefill_shared_kv_finish_kernel(co
     float* gate = s.gate + (size_t)t * s.heads * s.dim;
     shared_kv_row(s, query, gate, a.seq_len, pos, row, v.x, v.y, p0);
     shared_kv_row(s, query, gate, a.seq_len, pos, row + 1, v.y, v.x, p1);
+}
+
+static __global__ void __launch_bounds__(256) prefill_shared_kv_finish4_kernel(const PrefillSharedKvArgs a) {
+    constexpr int N = kKvFinishTokens;
+    pdl_launch_dependents();
+    const SharedKvArgs& s = a.kv;
+    const int t0 = blockIdx.x * N, row = 4 * ((int)blockIdx.y * 256 + (int)threadIdx.x);
+    const bool is_q = row < s.q_rows, is_k = !is_q && row < s.q_rows + s.k_rows;
+    const bool mine = row < a.n_rows && !(a.keys_only && !is_k);
+    const int r = is_q ? row : is_k ? row - s.q_rows : row - s.q_rows - s.k_rows, h = r / s.head_rows, j = r - h * s.head_rows;
+    const bool turns = (is_q || is_k) && j < s.rot;
+    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), cs[N];
+    if (mine) {  // constants: ahead of the dependency wait
+        if (is_q || is_k) bias = __ldg(reinterpret_cast<const float4*>(s.bias + row));
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const int pos = a.start_pos + t0 + i;
+            if (turns && pos >= 0 && pos < a.seq_len) cs[i] = __ldg(reinterpret_cast<const float4*>(s.rope + (size_t)pos * (s.rot >> 1) + (j >> 1)));
+        }
+    }
+    pdl_wait();
+    if (!mine) return;
+    float4 v[N];
+    prefill_sums<N>(a.part, a.part_tokens, a.n_rows, a.splits, a.n_tokens, t0, row, v);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int t = t0 + i, pos = a.start_pos + t;
+        if (t >= a.n_tokens) break;
+        if (pos < 0 || pos >= a.seq_len) {
+            atomicOr(&a.st->status, kStatusBadPos);
+            break;
+        }
+        float4 y = v[i];
+        if (!is_q && !is_k) {
+            *reinterpret_cast<float4*>(s.gate + ((size_t)t * s.heads + h) * s.dim + j) = make_float4(sigmoid_f(y.x), sigmoid_f(y.y), sigmoid_f(y.z), sigmoid_f(y.w));
+            continue;
+        }
+        y.x += bias.x; y.y += bias.y; y.z += bias.z; y.w += bias.w;
+        __half* at = is_q ? reinterpret_cast<__half*>(s.query) + ((size_t)t * s.heads + h) * s.row_width
+                          : reinterpret_cast<__half*>(s.cache) + ((size_t)h * a.seq_len + pos) * s.row_width;
+        const bool blank = is_q && turns;
+        *reinterpret_cast<uint2*>(at + j) = blank ? make_uint2(0u, 0u) : make_uint2(pack_half2(y.x, y.y), pack_half2(y.z, y.w));
+        if (turns) {
+            const float4 c = cs[i];
+            *reinterpret_cast<uint2*>(at + s.rank_pitch + j) =
+                make_uint2(pack_half2(__fsub_rn(__fmul_rn(y.x, c.x), __fmul_rn(y.y, c.y)), __fadd_rn(__fmul_rn(y.y, c.x), __fmul_rn(y.x, c.y))),
+                           pack_half2(__fsub_rn(__fmul_rn(y.z, c.z), __fmul_rn(y.w, c.w)), __fadd_rn(__fmul_rn(y.w, c.z), __fmul_rn(y.z, c.w))));
+        }
+    }
 }
 
 // ---- selective scan (mamba.cuh)
