@@ -36,6 +36,7 @@
 #include "common.cuh"
 #include "gemv.cuh"
 #include "latent_attention.cuh"
+#include "latent_head.cuh"
 #include "mamba.cuh"
 #include "ops.cuh"
 #include "prefill.cuh"
@@ -214,6 +215,7 @@ struct lpp_engine {
     float *scan_x = nullptr, *scan_z = nullptr, *scan_low = nullptr;
     unsigned int* row_counters = nullptr;
     std::vector<std::pair<lpp_layer_desc, float2*>> rope_tables;
+    bool head_clusters = false;  // a layer's step runs on latent_head_kernel: the GEMVs around it take the same split of the SM's memory
     float *lat_qplain = nullptr, *lat_raw = nullptr, *lat_gate = nullptr, *lat_part = nullptr;
     void* lat_query = nullptr;
     bool wcls_owned = false;
@@ -286,33 +288,41 @@ struct lpp_engine {
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// cluster_x: CTAs of a cluster along x, 0 = none.  max_shared: the SM's memory split in favour of shared memory (a kernel that wants another
+// split than the one running has to wait for the SM to be empty).
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                   bool pdl, int cluster_x, Args... args) {
+static cudaError_t launch_with(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl, int cluster_x, bool max_shared, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[3];
     cfg.attrs = attr;
     cfg.numAttrs = 0;
     if (pdl) {
         attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
-    if (cluster_x > 0) {  // CTAs of a cluster, along x
+    if (cluster_x > 0) {
         attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
         attr[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster_x;
         attr[cfg.numAttrs].val.clusterDim.y = 1;
         attr[cfg.numAttrs++].val.clusterDim.z = 1;
     }
+    if (max_shared) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[cfg.numAttrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+    }
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                 bool pdl, Args... args) {
-    return launch_clusters(kernel, grid, block, smem, s, pdl, 0, args...);
+static cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl, int cluster_x, Args... args) {
+    return launch_with(kernel, grid, block, smem, s, pdl, cluster_x, false, args...);
+}
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl, Args... args) {
+    return launch_with(kernel, grid, block, smem, s, pdl, 0, false, args...);
 }
 
 // ---- GEMV dispatch
@@ -388,7 +398,7 @@ static cudaError_t launch_gemv_t(lpp_engine* e, GemvArgsOf<EPI>& a, bool pdl, cu
         if (r != cudaSuccess) return r;
         attr_done[e->c.device & 63] = true;
     }
-    return launch_kernel(gemv_ring_kernel<WT, EPI, LN>, dim3(grid + extra), dim3(kGemvRingThreads), smem, s, pdl, a);
+    return launch_with(gemv_ring_kernel<WT, EPI, LN>, dim3(grid + extra), dim3(kGemvRingThreads), smem, s, pdl, 0, e->head_clusters, a);
 }
 
 static cudaError_t launch_gemv(lpp_engine* e, int epi, int w_dtype, GemvArgs& a, bool pdl, cudaStream_t s) {
@@ -1128,7 +1138,21 @@ static void record_mamba_mixer(Recorder& R, int l, float* cur) {
     });
 }
 
-// Latent attention: input GEMV, query GEMV, attention over the window, value GEMV (latent.cuh).
+// CTAs per head of latent_head_kernel in a step, 0 = query GEMV, attention and value GEMV as launches of their own: other types than BF16
+// weights over an FP16 cache, more heads than clusters of four have SMs for, a share of the window's rows that does not fit beside a GEMV's CTA.
+static int latent_head_rows(const lpp_engine* e, const ModelLayer& y, int ctas) {
+    const int keys = y.d.window > 0 ? std::min(e->c.seq_len, y.d.window) : e->c.seq_len;
+    return (keys + ctas - 1) / ctas;
+}
+static int latent_head_ctas(const lpp_engine* e, const ModelLayer& y) {
+    if (e->c.weight_dtype != LPP_BF16 || e->c.kv_dtype != LPP_F16 || (e->c.flags & (LPP_FLAG_GEMV_LDG | LPP_FLAG_LATENT_CUDA_CORES))) return 0;
+    if (y.rank_pitch > kLhMaxRank) return 0;
+    for (int ctas = kLhMaxCtas; ctas >= 4; ctas /= 2)
+        if (y.d.heads * ctas <= e->num_sms && latent_head_smem(y.row_width, y.rank_pitch, y.dim_pitch, y.vdim_rows, y.val_pitch, latent_head_rows(e, y, ctas), ctas) <= kLhSmemBytes)
+            return ctas;
+    return 0;
+}
+// Latent attention: input GEMV, then the head's clusters (latent_head.cuh), or query GEMV, attention over the window and value GEMV (latent.cuh).
 static void record_latent_mixer(Recorder& R, int l, float* cur) {
     lpp_engine* e = R.e;
     const LayerRun& r = e->runs[l];
@@ -1137,6 +1161,30 @@ static void record_latent_mixer(Recorder& R, int l, float* cur) {
     a.lat = latent_args(e, y, r);
     set_mixer_input(e, a, y, l, cur);
     record_gemv(R, kQkv, kEpiLatentIn, a);
+    if (const int ctas = latent_head_ctas(e, y)) {
+        LatentHeadArgs t = {};
+        t.lat = a.lat;
+        t.st = e->st;
+        t.w_uk = (const __nv_bfloat16*)y.w_uk;
+        t.w_uv = (const __nv_bfloat16*)y.w_uv;
+        t.out = e->att_out;
+        t.val_pitch = y.val_pitch;
+        t.seq_len = e->c.seq_len;
+        t.rows_cap = latent_head_rows(e, y, ctas);
+        t.early = step_early(e);
+        t.scale = y.d.scale;
+        record_launch(R, kAttn, "latent attention launch", [&](bool pdl) {
+            static bool attr_done[64] = {};
+            if (!attr_done[e->c.device & 63]) {
+                const cudaError_t r = cudaFuncSetAttribute(latent_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLhSmemBytes);
+                if (r != cudaSuccess) return r;
+                attr_done[e->c.device & 63] = true;
+            }
+            return launch_with(latent_head_kernel, dim3(y.d.heads * ctas), dim3(kLhThreads),
+                               latent_head_smem(y.row_width, y.rank_pitch, y.dim_pitch, y.vdim_rows, y.val_pitch, t.rows_cap, ctas), R.s, pdl, ctas, true, t);
+        });
+        return;
+    }
     GemvLatentArgs q = {};
     q.lat = a.lat;
     q.W = y.w_uk;
@@ -1160,6 +1208,8 @@ static void record_latent_mixer(Recorder& R, int l, float* cur) {
 
 static void record_step(Recorder& R, bool with_sampler) {
     lpp_engine* e = R.e;
+    e->head_clusters = false;
+    for (const ModelLayer& y : e->layers) e->head_clusters |= y.d.mixer == LPP_MIXER_LATENT && latent_head_ctas(e, y) > 0;
     const lpp_config& c = e->c;
     const int D = e->Dp, L = n_runs(e);
     const size_t esz = e->esz;
