@@ -124,6 +124,7 @@ __device__ __forceinline__ float float_of_ulps(unsigned long long S, int E) {
 }
 
 // ---- grid barrier for this kernel (all blocks co-resident; bounded wait) -------------------------
+// The block's writes are ordered by its own barrier and thread 0's release; a fence of every thread on top of that cost a microsecond a stage.
 
 __device__ __forceinline__ bool sampler_grid_barrier(unsigned int* counter, unsigned int target, StepState* st,
                                                      int* s_flag, int tid) {
@@ -645,7 +646,6 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_exact_kernel(con
         if (alive) {
             emit_entries(x, before_blocks + (incl - loc), base, n_quads, ea.entries + (size_t)blockIdx.x * kExactMaxEntries,
                          ea.entry_count + blockIdx.x, s_wm, s_wf, s_i, tid);
-            __threadfence();
         }
         alive = alive && sampler_grid_barrier(&ea.sync[0], ++bar * nb, st, &s_flag, tid);
 
@@ -675,7 +675,6 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_exact_kernel(con
         int* cdf_count = ea.entry_count + nb;
         if (alive) {
             emit_entries(x, pre_p, base, n_quads, cdf_entries + (size_t)blockIdx.x * kExactMaxEntries, cdf_count + blockIdx.x, s_wm, s_wf, s_i, tid);
-            __threadfence();
         }
         alive = alive && sampler_grid_barrier(&ea.sync[0], ++bar * nb, st, &s_flag, tid);
 
@@ -705,7 +704,6 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_exact_kernel(con
                 st->history_len = min(st->history_count, w);
             }
         }
-        __threadfence();
     }
     __syncthreads();
     if (tid == 0) {
