@@ -29,6 +29,9 @@
 //   Latency-bound: ceil(V/2048) blocks, a few microseconds per dependent stage.  A token of the
 //   Llama-3.2-1B shape whose distribution is confident (0.998 on one token): 3.35 ms with windows of
 //   whole blocks added one by one by one warp, of which this kernel took 2.7 ms; 0.66 ms now.
+//   128256 logits with 64 history entries: 48.8 us a call with maps of 64-bit words, carries and offsets
+//   found warp after warp, checks inside the walk's chain and the history searched per entry; 34.7 us with
+//   32-bit maps made by two additions, carries scanned by every warp, checks after the walk and counts.
 //
 // exp() is exp_repro (common.cuh): IEEE double arithmetic only, identical on host and device; it
 // differs from libm's expf in the last bit for about 0.06 % of arguments, which is the only source
@@ -72,55 +75,36 @@ struct SampleExactArgs {
 
 // ---- the integer map of one element -------------------------------------------------------------
 
+// Increments of a valid run are at most 2^23 (it ends inside its binade or on the next power of two); larger ones only have
+// to stay larger, so sums saturate here and a map is two 32-bit words.
+constexpr unsigned int kMapCap = 0x3fffffffu;
 struct Map2 {
-    unsigned long long d0, d1;  // increment of S when S is even / odd
+    unsigned int d0, d1;  // increment of S when S is even / odd
 };
-__device__ __forceinline__ Map2 map_identity() { return Map2{0ull, 0ull}; }
+__device__ __forceinline__ Map2 map_identity() { return Map2{0u, 0u}; }
 // b after a
 __device__ __forceinline__ Map2 map_compose(Map2 a, Map2 b) {
     Map2 c;
-    c.d0 = a.d0 + ((a.d0 & 1ull) ? b.d1 : b.d0);
-    c.d1 = a.d1 + (((1ull + a.d1) & 1ull) ? b.d1 : b.d0);
+    c.d0 = min(a.d0 + ((a.d0 & 1u) ? b.d1 : b.d0), kMapCap);
+    c.d1 = min(a.d1 + ((a.d1 & 1u) ? b.d0 : b.d1), kMapCap);
     return c;
 }
-// Map of adding x (a non-negative float) to a sum in binade E (ulp 2^(E-23)); requires x < 2^E.
+// Map of adding x (a non-negative float) to a sum in binade E (ulp 2^(E-23)); requires x < 2^E.  The two additions are
+// those to the binade's first even and first odd S: S + x/u stays below 2^24 + 1, and where it passes 2^24 (S = 2^23 + 1,
+// x = 2^E - u/2) the coarser rounding there gives 2^24 as the tie in this binade does.
 __device__ __forceinline__ Map2 map_of(float x, int E) {
-    const unsigned int bits = __float_as_uint(x);
-    int ex = (int)((bits >> 23) & 0xffu);
-    unsigned int mx = bits & 0x7fffffu;
-    if (ex == 0)
-        ex = 1;  // zero or subnormal: value = mx * 2^(1-150)
-    else
-        mx |= 0x800000u;
-    const int shift = (E + 127) - ex;  // x/ulp = mx / 2^shift, shift >= 1
-    if (mx == 0u || shift > 25) return map_identity();
-    const unsigned long long m = mx;
-    const unsigned long long n = m >> shift;
-    const unsigned long long rem = m & ((1ull << shift) - 1ull);
-    const unsigned long long half = 1ull << (shift - 1);
-    Map2 r;
-    if (rem < half) {
-        r.d0 = r.d1 = n;
-    } else if (rem > half) {
-        r.d0 = r.d1 = n + 1ull;
-    } else {  // tie: round so that S + increment is even
-        r.d0 = n + (n & 1ull);
-        r.d1 = n + ((n + 1ull) & 1ull);
-    }
-    return r;
+    const unsigned int b = (unsigned int)(E + 127) << 23;
+    return Map2{__float_as_uint(__fadd_rn(__uint_as_float(b), x)) - b, __float_as_uint(__fadd_rn(__uint_as_float(b + 1u), x)) - (b + 1u)};
 }
 
 __device__ __forceinline__ int binade_of(double v) {  // floor(log2(v)) for v > 0 (normal doubles)
     return (int)((__double_as_longlong(v) >> 52) & 0x7ff) - 1023;
 }
 
-// Increments of a valid run are at most 2^23; larger ones only have to stay invalid.
-__device__ __forceinline__ unsigned int map_word(unsigned long long d) { return (unsigned int)min(d, 0x7fffffffull); }
-
 // The float that S ulps of binade E are (S in [2^23, 2^24]).
-__device__ __forceinline__ float float_of_ulps(unsigned long long S, int E) {
-    return (S >= (1ull << 24)) ? __uint_as_float((unsigned int)(E + 128) << 23)
-                               : __uint_as_float(((unsigned int)(E + 127) << 23) | ((unsigned int)S & 0x7fffffu));
+__device__ __forceinline__ float float_of_ulps(unsigned int S, int E) {
+    return (S >= (1u << 24)) ? __uint_as_float((unsigned int)(E + 128) << 23)
+                               : __uint_as_float(((unsigned int)(E + 127) << 23) | (S & 0x7fffffu));
 }
 
 // ---- grid barrier for this kernel (all blocks co-resident; bounded wait) -------------------------
@@ -181,15 +165,29 @@ __device__ __forceinline__ Map2 block_segscan(Map2 v, bool start, Map2* s_warp_m
         s_warp_flag[warp] = f;
     }
     __syncthreads();
-    if (!f) {  // the run began in an earlier warp: prepend the carried maps of the warps before
-        Map2 carry = map_identity();
-        bool open = true;
-        for (int w = warp - 1; w >= 0 && open; --w) {
-            carry = map_compose(s_warp_map[w], carry);
-            if (s_warp_flag[w]) open = false;
-        }
-        v = map_compose(carry, v);
+    // the maps of the warps are scanned in the same way by every warp; one that is carried into this warp is prepended
+    constexpr int kWarps = kSampleThreads / 32;
+    Map2 c = map_identity();
+    int fc = 1;
+    if (lane < kWarps) {
+        c = s_warp_map[lane];
+        fc = s_warp_flag[lane];
     }
+#pragma unroll
+    for (int o = 1; o < kWarps; o <<= 1) {
+        Map2 u;
+        u.d0 = __shfl_up_sync(0xffffffffu, c.d0, o);
+        u.d1 = __shfl_up_sync(0xffffffffu, c.d1, o);
+        const int fu = __shfl_up_sync(0xffffffffu, fc, o);
+        if (lane >= o) {
+            if (!fc) c = map_compose(u, c);
+            fc |= fu;
+        }
+    }
+    Map2 carry;
+    carry.d0 = __shfl_sync(0xffffffffu, c.d0, (warp - 1) & 31);
+    carry.d1 = __shfl_sync(0xffffffffu, c.d1, (warp - 1) & 31);
+    if (!f && warp > 0) v = map_compose(carry, v);
     __syncthreads();
     return v;
 }
@@ -250,7 +248,7 @@ static __device__ __noinline__ void emit_entries(const float (&x)[4], double pre
     // runs: maximal sequences of threads of one class (mapped runs also share E)
     const int cls = !valid ? 5000 : zero ? 4000 : plain ? E : dual ? 1000 + E : 3000;  // binades lie in (-120, 119): no clash
     const int prev = __shfl_up_sync(0xffffffffu, cls, 1);
-    __shared__ int s_cls_last[kSampleThreads / 32];
+    __shared__ int s_cls_last[kSampleThreads / 32], s_cls_first[kSampleThreads / 32];
     if (lane == 31) s_cls_last[tid >> 5] = cls;
     __syncthreads();
     const int before = (tid == 0) ? 6000 : (lane == 0 ? s_cls_last[(tid >> 5) - 1] : prev);
@@ -271,26 +269,18 @@ static __device__ __noinline__ void emit_entries(const float (&x)[4], double pre
         run2 = block_segscan(mp2, start, s_wm, s_wf, tid);
     }
     // entry index = number of run starts up to and including this thread, minus one
-    int cnt = start ? 1 : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, cnt, o);
-        if (lane >= o) cnt += u;
-    }
-    if (lane == 31) s_i[tid >> 5] = cnt;
+    const unsigned int starts = __ballot_sync(0xffffffffu, start);
+    if (lane == 0) s_i[tid >> 5] = __popc(starts);
+    if (lane == 0) s_cls_first[tid >> 5] = cls;
     __syncthreads();
-    int off = 0;
-    for (int w = 0; w < (tid >> 5); ++w) off += s_i[w];
-    const int idx = cnt + off - 1;
-    int total = 0;
-    for (int w = 0; w < kSampleThreads / 32; ++w) total += s_i[w];
-    __syncthreads();
+    const int warp_starts = (lane < kSampleThreads / 32) ? s_i[lane] : 0;
+    const int off = __reduce_add_sync(0xffffffffu, lane < (tid >> 5) ? warp_starts : 0);
+    const int total = __reduce_add_sync(0xffffffffu, warp_starts);
+    const int idx = off + __popc(starts & (0xffffffffu >> (31 - lane))) - 1;
     const bool overflow = total > kExactMaxEntries;
     // is this thread the last of its run?
     const int nxt_cls = __shfl_down_sync(0xffffffffu, cls, 1);
-    if (lane == 0) s_cls_last[tid >> 5] = cls;  // reuse as "first class of warp"
-    __syncthreads();
-    const int after = (tid == kSampleThreads - 1) ? 6000 : (lane == 31 ? s_cls_last[(tid >> 5) + 1] : nxt_cls);
+    const int after = (tid == kSampleThreads - 1) ? 6000 : (lane == 31 ? s_cls_first[(tid >> 5) + 1] : nxt_cls);
     const bool last = valid && !zero && (cls != after || !mapped);
     if (!overflow) {
         if (start) {
@@ -302,7 +292,7 @@ static __device__ __noinline__ void emit_entries(const float (&x)[4], double pre
             out[idx].hi = first_elem + 4 * tid + 4;
             uint4 d;
             if (mapped)
-                d = make_uint4(map_word(run.d0), map_word(run.d1), map_word(run2.d0), map_word(run2.d1));
+                d = make_uint4(run.d0, run.d1, run2.d0, run2.d1);
             else  // a window carries its values, sparing the walker a memory round trip
                 d = make_uint4(__float_as_uint(x[0]), __float_as_uint(x[1]), __float_as_uint(x[2]), __float_as_uint(x[3]));
             *reinterpret_cast<uint4*>(out[idx].d) = d;
@@ -402,14 +392,14 @@ static __device__ __noinline__ void resolve_range(const float* x, int lo, int hi
             if (lane == 31) z->last_map[warp] = incl;
             __syncthreads();
             if (lane == 0) ex = (warp == 0) ? map_identity() : z->last_map[warp - 1];
-            const unsigned long long S0 = (bits & 0x7fffffu) | 0x800000u;
-            unsigned long long S = S0 + ((S0 & 1ull) ? ex.d1 : ex.d0), before[4];
+            const unsigned int S0 = (bits & 0x7fffffu) | 0x800000u;
+            unsigned int S = S0 + ((S0 & 1u) ? ex.d1 : ex.d0), before[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 before[k] = S;
-                S += (S & 1ull) ? m[k].d1 : m[k].d0;
+                S += (S & 1u) ? m[k].d1 : m[k].d0;
                 if (scan && i0 + k >= from && i0 + k < brk) {
-                    if (S > (1ull << 24))
+                    if (S > (1u << 24))
                         atomicMin(&z->cross, i0 + k);
                     else if (stop && r < float_of_ulps(S, E))
                         atomicMin(&z->found, i0 + k);
@@ -486,56 +476,61 @@ static __device__ __noinline__ void walk_all(const ExactEntry* entries, const in
             }
             const uint4* src = reinterpret_cast<const uint4*>(entries + (size_t)lo * kExactMaxEntries + (g - s_pref[lo]));
             uint4* dst = reinterpret_cast<uint4*>(s_list + j);
-            const uint4 v0 = __ldcg(src), v1 = __ldcg(src + 1);
+            uint4 v0 = __ldcg(src);
+            const uint4 v1 = __ldcg(src + 1);
+            v0.w = (v0.w + 128u) << 23;  // the binade as the bit pattern of its end
             dst[0] = v0;
             dst[1] = v1;
         }
         __syncthreads();
         for (int i0 = 0; i0 < m;) {
-            // pass 1 (warp 0, every lane the same): apply the entries from i0 on speculatively without a branch, keeping
-            // the sum before every entry; the first entry whose map does not hold is remembered.  A map moves the sum by
-            // an integer number of ulps inside one binade (or exactly onto the next power of two), which on the bit
-            // pattern of a positive float is a plain integer addition.
+            // pass 1 (warp 0, every lane the same): apply the entries from i0 on speculatively without a branch or a check,
+            // keeping the sum before every entry.  A map moves the sum by an integer number of ulps inside one binade (or
+            // exactly onto the next power of two), which on the bit pattern of a positive float is a plain integer addition.
+            // The chain from sum to sum bounds the walk: with the checks inside it took 70 clocks an entry, 3.3 us for the
+            // list of a 128 K vocabulary.
             if (tid < 32) {
                 unsigned int bits = __float_as_uint(out->s);
-                int bad = 0x7fffffff;
 #pragma unroll 4
                 for (int i = i0; i < m; ++i) {
-                    const int4 h = *reinterpret_cast<const int4*>(&s_list[i]);  // kind, lo, hi, e
+                    const int4 h = *reinterpret_cast<const int4*>(&s_list[i]);  // kind, lo, hi, end of the binade
                     const uint4 d = *reinterpret_cast<const uint4*>(s_list[i].d);
                     s_before[i] = bits;
-                    // as a map: of binade e, or of the next one when the sum of a dual entry is there
-                    const unsigned int ebase = (unsigned int)(h.w + 127) << 23;
-                    const bool next = h.x == kEntryDual && bits - ebase >= 0x800000u;
-                    const unsigned int from = next ? ebase + 0x800000u : ebase;
-                    const unsigned int dd = next ? ((bits & 1u) ? d.w : d.z) : ((bits & 1u) ? d.y : d.x);
-                    const unsigned int nb = bits + dd;
-                    const bool map_ok = bits - from < 0x800000u && dd <= 0x800000u && nb - from <= 0x800000u;
+                    // as a map: of the entry's binade, or of the next one (none there unless the entry is dual)
+                    const bool next = bits >= (unsigned int)h.w, odd = bits & 1u;
+                    const unsigned int even_d = next ? d.z : d.x, odd_d = next ? d.w : d.y;
+                    const unsigned int nb = bits + (odd ? odd_d : even_d);
                     // as four values
                     float q = __uint_as_float(bits);
                     q = __fadd_rn(q, __uint_as_float(d.x));
                     q = __fadd_rn(q, __uint_as_float(d.y));
                     q = __fadd_rn(q, __uint_as_float(d.z));
                     q = __fadd_rn(q, __uint_as_float(d.w));
-                    const bool is_quad = h.x == kEntryQuad;
-                    const bool fine = is_quad || (h.x != kEntrySeq && map_ok);
-                    bad = (!fine && bad == 0x7fffffff) ? i : bad;
-                    bits = is_quad ? __float_as_uint(q) : nb;
+                    bits = (h.x == kEntryQuad) ? __float_as_uint(q) : nb;
                 }
                 s_before[m] = bits;
-                if (lane == 0) {
-                    s_ctl[0] = bad;
-                    s_ctl[1] = 0x7fffffff;
+                if (lane == 0) s_ctl[0] = s_ctl[1] = 0x7fffffff;
+            }
+            __syncthreads();
+            // pass 2: the first entry whose map does not hold at the sum before it, so that everything before it is exact,
+            // and the first entry after which the running sum exceeds r (sums never decrease)
+            for (int i = i0 + tid - lane; i < m; i += kSampleThreads) {
+                int bad = 0x7fffffff, cross = 0x7fffffff;
+                if (i + lane < m) {
+                    const int kind = s_list[i + lane].kind;
+                    const unsigned int end = (unsigned int)s_list[i + lane].e, in = s_before[i + lane], after = s_before[i + lane + 1];
+                    const unsigned int from = (kind == kEntryDual && in >= end) ? end : end - 0x800000u;
+                    const bool holds = in - from < 0x800000u && after - in <= 0x800000u && after - from <= 0x800000u;
+                    if (kind == kEntrySeq || (kind != kEntryQuad && !holds)) bad = i + lane;
+                    if (stop && r < __uint_as_float(after)) cross = i + lane;
                 }
+                bad = __reduce_min_sync(0xffffffffu, bad);
+                cross = __reduce_min_sync(0xffffffffu, cross);
+                if (lane == 0 && bad != 0x7fffffff) atomicMin(&s_ctl[0], bad);
+                if (lane == 0 && cross != 0x7fffffff) atomicMin(&s_ctl[1], cross);
             }
             __syncthreads();
             const int good = min(m, s_ctl[0]);  // entries [i0, good) were applied exactly
-            // pass 2: the first entry after which the running sum exceeds r (sums never decrease)
-            if (stop) {
-                for (int i = i0 + tid; i < good; i += kSampleThreads)
-                    if (r < __uint_as_float(s_before[i + 1])) atomicMin(&s_ctl[1], i);
-                __syncthreads();
-            }
             const int redo = stop ? min(s_ctl[1], good) : good;  // entry to look at element by element, m = none
             if (tid == 0) {
                 out->s = __uint_as_float(s_before[redo]);
@@ -563,7 +558,7 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_exact_kernel(con
     __shared__ int s_pref[kSampleThreads + 1];
     __shared__ WalkState s_walk;
     __shared__ ResolveScratch s_res;
-    __shared__ int s_hist[kHistoryMax];
+    __shared__ int s_cnt[kSampleChunk];  // occurrences in the history
 
     pdl_launch_dependents();
     pdl_wait();
@@ -579,33 +574,18 @@ static __global__ void __launch_bounds__(kSampleThreads) sample_exact_kernel(con
     const bool greedy = (temperature == 0.0f);
     unsigned int bar = 0;  // barriers passed so far
     // ---- stage 0: penalty, temperature, block maximum (element i of the block lives in s_val[i])
-    for (int i = tid; i < kSampleChunk; i += kSampleThreads) s_val[i] = (i < n) ? __ldcg(a.logits + base + i) : 0.f;
-    __syncthreads();
-    if (penalty > 1.0f && hist_len > 0) {
-        // the history is scanned by every thread that owns one of its entries: keep it in shared memory
-        for (int i = tid; i < hist_len; i += kSampleThreads) s_hist[i] = st->history[i];
-        __syncthreads();
-        for (int i = tid; i < hist_len; i += kSampleThreads) {
-            const int tok = s_hist[i];
-            if (tok < base || tok >= base + n) continue;
-            bool first = true;
-            for (int j = 0; j < i; ++j)
-                if (s_hist[j] == tok) {
-                    first = false;
-                    break;
-                }
-            if (!first) continue;
-            int cnt = 1;
-            for (int j = i + 1; j < hist_len; ++j) cnt += (s_hist[j] == tok);
-            float v = s_val[tok - base];
-            for (int c = 0; c < cnt; ++c) v = (v > 0.f) ? __fdiv_rn(v, penalty) : __fmul_rn(v, penalty);
-            s_val[tok - base] = v;
-        }
-        __syncthreads();
+    const int h0 = st->history[tid];  // in bounds whatever the length
+    for (int i = tid; i < kSampleChunk; i += kSampleThreads) {
+        s_val[i] = (i < n) ? __ldcg(a.logits + base + i) : 0.f;
+        s_cnt[i] = 0;
     }
+    __syncthreads();
+    const bool penalised = penalty > 1.0f && hist_len > 0;
+    if (penalised) count_history(st->history, h0, hist_len, base, n, s_cnt, tid);
     MaxIdx best = {-INFINITY, 0x7fffffff};
     for (int i = tid; i < n; i += kSampleThreads) {
         float v = s_val[i];
+        if (penalised) v = penalise(v, s_cnt[i], penalty);
         if (!greedy) v = __fdiv_rn(v, temperature);
         s_val[i] = v;
         best = better(best, MaxIdx{v, base + i});
