@@ -400,13 +400,22 @@ __global__ void __launch_bounds__(kAttnKernelThreads) attn_decode_kernel(const A
 // The kernel above spends its time in FP32 shuffles and exponentials (1.7 TB/s at 32 K positions, and
 // slower than this one from a few dozen positions on).  Here the scores q.K^T and the product P.V run
 // as mma.sync.m16n8k16 (FP16 operands, FP32 accumulators): the up to 8 query heads of a KV head are the
-// rows of the 16-row operand (the rest is zero), a warp handles 16 positions per step and keeps the rows
-// of its next step in flight.  No shared memory is involved in the operands: the dot product over head
-// dimensions and the sum over positions do not care about order, so the dimension / position that an
-// operand register stands for is chosen such that every lane reads whole 16-byte pieces of the rows
-// straight from global memory (a quad of lanes covers one K row; lane quad-row g owns head dims
-// [g*HS/8, (g+1)*HS/8) of its V rows).  Same splits, partials and combine as above.  As there, the
+// rows of the 16-row operand (the rest is zero), a warp handles 16 positions per step.  The dot product over
+// head dimensions and the sum over positions do not care about order, so the dimension / position that an
+// operand register stands for is chosen such that every lane reads whole 16-byte pieces of the rows and
+// neighbouring lanes read neighbouring pieces.  Same splits, partials and combine as above.  As there, the
 // position and the rows of earlier positions are read before the dependency wait.
+//
+// Memory bounds it: a layer of the 8B shape at 32 K positions is 134 MB, 20.8 us at the measured copy rate.  How
+// the rows travel decides the rest.  Loaded to registers one step ahead, with L2 requests one step further, 16 K
+// more positions cost 13.6 us a layer (4.9 TB/s); copied by the lanes (cp.async) three steps ahead, in pieces of
+// 64 and 128 bytes, 15.7 us; in bulk, 4 KB of K and 4 KB of V at a time, 10.6 us (6.3 TB/s), although the operands
+// are then read from rows that share banks (K twice, V four times over, 0.8 us of the 1.5 us that a round's
+// 64 KB take to come).  Where a split never holds more than the ring, all of it is requested at once and latency
+// counts instead: there the lanes' own copies, read back without conflicts or barriers, are the faster ones (48
+// tokens of the 1B shape at 640: 32.0 ms with registers, 32.2 in bulk, 31.6 with these), so the capacity of the
+// cache decides between the two.  Both in one kernel, chosen by the split's length, took 32.5 ms and 3 % more at
+// 32 K: the instructions of this kernel come anew from L2 on every launch.
 __device__ __forceinline__ void mma_16816(float (&d)[4], unsigned int a0, unsigned int a1, unsigned int a2, unsigned int a3,
                                           unsigned int b0, unsigned int b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -418,9 +427,19 @@ __device__ __forceinline__ unsigned int pack_half2(float lo, float hi) {
     return *reinterpret_cast<const unsigned int*>(&h);
 }
 
-constexpr int kAttnPrefetchSteps = 1;  // how many steps past the next one the L2 prefetch runs ahead
+// The rows of the steps ahead are copied into a ring in shared memory.
+template <int HS>
+constexpr int kAttnStages = HS == 128 ? 3 : 4;
+template <int HS>
+constexpr int kAttnRingBytes = (kAttnKernelThreads / 32) * kAttnStages<HS> * 16 * HS * 4;  // 16 positions of K and V rows per warp and stage
+// Whether a split can never hold more positions than the ring, whatever the position.
+inline bool attn_split_fits_ring(const AttnArgs& a, int hs) {
+    const int room = (hs == 128 ? kAttnStages<128> : kAttnStages<64>) * (kAttnKernelThreads / 32) * 16;
+    const int min_chunk = a.min_chunk > 0 ? a.min_chunk : kAttnMinChunk;
+    return 2 * min_chunk <= room && (a.seq_len + a.n_splits - 1) / a.n_splits <= room;
+}
 
-template <int HS, int GQA>
+template <int HS, int GQA, bool BULK>
 __global__ void __launch_bounds__(kAttnKernelThreads) attn_mma_kernel(const AttnArgs a) {
     static_assert(HS == 64 || HS == 128, "head size");
     static_assert(GQA >= 1 && GQA <= 8, "query heads per KV head");
@@ -453,52 +472,88 @@ __global__ void __launch_bounds__(kAttnKernelThreads) attn_mma_kernel(const Attn
     for (int t = 0; t < NTL; ++t) o[t][0] = o[t][1] = o[t][2] = o[t][3] = 0.f;
     float m = -INFINITY, l = 0.f;  // running maximum / sum of head g (identical on the 4 lanes of a quad)
 
-    // K rows of one step: group 0 = positions base..base+7, group 1 = base+8..base+15; this lane reads the
-    // piece [j*HS/4, (j+1)*HS/4) of the rows base+g and base+8+g
-    auto load_k = [&](int base, unsigned int (&kr)[2][2 * KS], int lim) {
+    // One step of this warp is 16 positions: the 16 rows of K, then those of V, two bulk copies of what lies in one piece in the
+    // cache.  As operands, K group 0 = positions base..base+7, group 1 = base+8..base+15, this lane taking the 16-byte pieces
+    // 4*i + j of the rows base+g and base+8+g; V the rows base+2j, base+2j+1, base+8+2j, base+8+2j+1 (the order in which the
+    // probabilities sit in the A operand below), pieces 8*i + g.
+    // Without BULK every lane copies the pieces that it will read itself, to places of its own.
+    constexpr int kStages = kAttnStages<HS>;
+    constexpr int KP = KS / 2, VP = NTL / 8;  // pieces of a K row and of a V row per lane
+    constexpr int kRow = HS / 8;              // pieces of a row
+    extern __shared__ __align__(128) uint4 s_ring[];
+    __shared__ __align__(8) uint64_t s_full[NW * kStages];
+    uint4* ring = s_ring + (size_t)warp * kStages * 32 * kRow;
+    uint64_t* full = s_full + warp * kStages;
+    if constexpr (BULK) {
+        if (lane == 0) {
 #pragma unroll
-        for (int grp = 0; grp < 2; ++grp) {
-            const int t = base + grp * 8 + g;
-            if (t < lim) {
-                const uint4* p = reinterpret_cast<const uint4*>(kb + (size_t)t * HS + j * (HS / 4));
+            for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
+            mbar_fence_init();
+        }
+        __syncwarp();
+    }
+    auto k_row = [&](int base, int c) { return base + c / KP * 8 + g; };
+    auto v_row = [&](int base, int c) { return base + (c / VP >> 1) * 8 + 2 * j + (c / VP & 1); };
+    auto k_src = [&](int t, int c) { return reinterpret_cast<const uint4*>(kb + (size_t)t * HS) + 4 * (c % KP) + j; };
+    auto v_src = [&](int t, int c) { return reinterpret_cast<const uint4*>(vb + (size_t)t * HS) + 8 * (c % VP) + g; };
+    // this lane's pieces of the rows [base, base + 16) but the current position's; zeros from t1 on
+    auto request_own = [&](int base, int stage) {
+        uint4* d = ring + stage * 32 * kRow + lane;
 #pragma unroll
-                for (int i = 0; i < KS / 2; ++i) {
-                    const uint4 u = __ldcg(p + i);
-                    kr[grp][4 * i] = u.x; kr[grp][4 * i + 1] = u.y; kr[grp][4 * i + 2] = u.z; kr[grp][4 * i + 3] = u.w;
-                }
-            } else {
+        for (int c = 0; c < 2 * KP; ++c) {
+            const int t = k_row(base, c);
+            if (t != pos) cp_async_16(d + c * 32, k_src(t < t1 ? t : t0, c), t < t1);
+        }
 #pragma unroll
-                for (int i = 0; i < 2 * KS; ++i) kr[grp][i] = 0u;
+        for (int c = 0; c < 4 * VP; ++c) {
+            const int t = v_row(base, c);
+            if (t != pos) cp_async_16(d + (2 * KP + c) * 32, v_src(t < t1 ? t : t0, c), t < t1);
+        }
+    };
+    // rows [base, min(base + 16, t1)) but the current position's
+    auto request = [&](int base, int stage) {
+        const int n = min(min(base + 16, t1), pos) - base;
+        if (lane == 0) {
+            const uint32_t bytes = (uint32_t)max(n, 0) * HS * 2;
+            mbar_arrive_expect_tx(&full[stage], 2 * bytes);
+            if (n > 0) {
+                bulk_g2s(ring + stage * 32 * kRow, kb + (size_t)base * HS, bytes, &full[stage]);
+                bulk_g2s(ring + stage * 32 * kRow + 16 * kRow, vb + (size_t)base * HS, bytes, &full[stage]);
             }
         }
     };
-    // V rows of one step: positions base+2j, base+2j+1, base+8+2j, base+8+2j+1 (the order in which the
-    // probabilities sit in the A operand below), head dims [g*NTL, (g+1)*NTL)
-    auto load_v = [&](int base, unsigned int (&vr)[4][NTL / 2], int lim) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int t = base + (r >> 1) * 8 + 2 * j + (r & 1);
-            if (t < lim) {
-                const uint4* p = reinterpret_cast<const uint4*>(vb + (size_t)t * HS + g * NTL);
-#pragma unroll
-                for (int i = 0; i < NTL / 8; ++i) {
-                    const uint4 u = __ldcg(p + i);
-                    vr[r][4 * i] = u.x; vr[r][4 * i + 1] = u.y; vr[r][4 * i + 2] = u.z; vr[r][4 * i + 3] = u.w;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < NTL / 2; ++i) vr[r][i] = 0u;
+    auto holds_pos = [&](int base) { return pos >= base && pos < base + 16 && pos < t1; };
+    // the current position's rows, written by the QKV kernel of this step: no copy touches their places
+    auto place_pos = [&](int base, int stage) {
+        if constexpr (BULK) {
+            if (lane < 2 * kRow) {
+                const int v = lane / kRow, i = lane % kRow;
+                ring[stage * 32 * kRow + (v * 16 + pos - base) * kRow + i] = __ldcg(reinterpret_cast<const uint4*>((v ? vb : kb) + (size_t)pos * HS) + i);
             }
+            __syncwarp();
+        } else {
+            uint4* d = ring + stage * 32 * kRow + lane;
+#pragma unroll
+            for (int c = 0; c < 2 * KP; ++c)
+                if (k_row(base, c) == pos) d[c * 32] = __ldcg(k_src(pos, c));
+#pragma unroll
+            for (int c = 0; c < 4 * VP; ++c)
+                if (v_row(base, c) == pos) d[(2 * KP + c) * 32] = __ldcg(v_src(pos, c));
         }
     };
-    unsigned int kr[2][2 * KS], vr[4][NTL / 2];
     int base = t0 + warp * 16;
-    // first step: rows of earlier positions (written by earlier steps) are requested before the wait; the
+    // first steps: rows of earlier positions (written by earlier steps) are requested before the wait; the
     // row of the current position, like q, comes from the QKV kernel of this step and follows it
-    const int stable = min(t1, pos);
-    if (base < t1) {
-        load_k(base, kr, stable);
-        load_v(base, vr, stable);
+    const int base0 = base;
+#pragma unroll
+    for (int s = 0; s < kStages; ++s) {
+        if (base + s * NW * 16 < t1) {
+            if constexpr (BULK)
+                request(base + s * NW * 16, s);
+            else
+                request_own(base + s * NW * 16, s);
+        }
+        if constexpr (!BULK) cp_async_commit();
     }
     pdl_wait();
     // A operand of the score product: row g = head g (zero from GQA on), this lane's HS/4 dims, pre-scaled
@@ -508,53 +563,52 @@ __global__ void __launch_bounds__(kAttnKernelThreads) attn_mma_kernel(const Attn
 #pragma unroll
         for (int s = 0; s < KS; ++s) {
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (g < GQA) v = __ldcg(reinterpret_cast<const float4*>(a.q + (size_t)(hbase + g) * HS + j * (HS / 4) + 4 * s));
+            if (g < GQA) v = __ldcg(reinterpret_cast<const float4*>(a.q + (size_t)(hbase + g) * HS + (4 * (s >> 1) + j) * 8 + (s & 1) * 4));
             qa[s][0] = pack_half2(v.x * scale, v.y * scale);
             qa[s][1] = pack_half2(v.z * scale, v.w * scale);
         }
     }
-    if (pos < t1 && pos >= base && pos < base + 16) {
 #pragma unroll
-        for (int grp = 0; grp < 2; ++grp)
-            if (base + grp * 8 + g == pos) {
-                const uint4* p = reinterpret_cast<const uint4*>(kb + (size_t)pos * HS + j * (HS / 4));
+    for (int s = 0; s < kStages; ++s)
+        if (holds_pos(base + s * NW * 16)) place_pos(base + s * NW * 16, s);
+    uint32_t phase = 0;
+    bool alive = true;
+    for (int stage = 0; base < t1; base += NW * 16) {
+        unsigned int kr[2][2 * KS], vr[4][NTL / 2];
+        if constexpr (!BULK) {
+            cp_async_commit();  // an empty group a step, so that the oldest but kStages are always the ones to wait for
+            cp_async_wait<kStages>();
+            const uint4* d = ring + stage * 32 * kRow + lane;
 #pragma unroll
-                for (int i = 0; i < KS / 2; ++i) {
-                    const uint4 u = __ldcg(p + i);
-                    kr[grp][4 * i] = u.x; kr[grp][4 * i + 1] = u.y; kr[grp][4 * i + 2] = u.z; kr[grp][4 * i + 3] = u.w;
-                }
+            for (int c = 0; c < 2 * KP; ++c) {
+                const uint4 u = d[c * 32];
+                unsigned int* k = &kr[c / KP][4 * (c % KP)];
+                k[0] = u.x, k[1] = u.y, k[2] = u.z, k[3] = u.w;
             }
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-            if (base + (r >> 1) * 8 + 2 * j + (r & 1) == pos) {
-                const uint4* p = reinterpret_cast<const uint4*>(vb + (size_t)pos * HS + g * NTL);
-#pragma unroll
-                for (int i = 0; i < NTL / 8; ++i) {
-                    const uint4 u = __ldcg(p + i);
-                    vr[r][4 * i] = u.x; vr[r][4 * i + 1] = u.y; vr[r][4 * i + 2] = u.z; vr[r][4 * i + 3] = u.w;
-                }
+            for (int c = 0; c < 4 * VP; ++c) {
+                const uint4 u = d[(2 * KP + c) * 32];
+                unsigned int* v = &vr[c / VP][4 * (c % VP)];
+                v[0] = u.x, v[1] = u.y, v[2] = u.z, v[3] = u.w;
             }
-    }
-    for (; base < t1; base += NW * 16) {
-        // the rows of this warp's next step are requested before this step is computed
-        unsigned int krn[2][2 * KS], vrn[4][NTL / 2];
-        const int nbase = base + NW * 16;
-        if (nbase < t1) {
-            load_k(nbase, krn, t1);
-            load_v(nbase, vrn, t1);
-        }
-        // the rows of the step after that are pulled towards L2 (no registers to hold them yet), so that
-        // their loads, one iteration from now, take an L2 round trip instead of an HBM one
-        {
-            const int pbase = nbase + kAttnPrefetchSteps * NW * 16;
+        } else {
+            alive = __all_sync(0xffffffffu, mbar_wait_bounded(&full[stage], phase, const_cast<StepState*>(a.st)));
+            if (!alive) break;
+            const uint4* d = ring + stage * 32 * kRow;
 #pragma unroll
-            for (int grp = 0; grp < 2; ++grp)
-                if (pbase + grp * 8 + g < t1)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(kb + (size_t)(pbase + grp * 8 + g) * HS + j * (HS / 4)));
+            for (int c = 0; c < 2 * KP; ++c) {
+                const uint4 u = d[k_row(0, c) * kRow + 4 * (c % KP) + j];
+                unsigned int* k = &kr[c / KP][4 * (c % KP)];
+                k[0] = u.x, k[1] = u.y, k[2] = u.z, k[3] = u.w;
+            }
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
-                if (pbase + (r >> 1) * 8 + 2 * j + (r & 1) < t1)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(vb + (size_t)(pbase + (r >> 1) * 8 + 2 * j + (r & 1)) * HS + g * NTL));
+            for (int c = 0; c < 4 * VP; ++c) {
+                const int row = v_row(0, c);
+                uint4 u = d[(16 + row) * kRow + 8 * (c % VP) + g];
+                if (base + row >= t1) u = make_uint4(0u, 0u, 0u, 0u);  // nothing was copied there
+                unsigned int* v = &vr[c / VP][4 * (c % VP)];
+                v[0] = u.x, v[1] = u.y, v[2] = u.z, v[3] = u.w;
+            }
         }
         // scores of the two groups
         float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
@@ -590,28 +644,34 @@ __global__ void __launch_bounds__(kAttnKernelThreads) attn_mma_kernel(const Attn
         for (int t = 0; t < NTL; ++t) {
             o[t][0] *= alpha;
             o[t][1] *= alpha;
-            // B operand of n-tile t: column g = head dim g*NTL + t, rows = the four positions above
+            // B operand of n-tile t: column g = head dim (t/8)*64 + g*8 + t%8, rows = the four positions above
             const unsigned int sel = (t & 1) ? 0x7632u : 0x5410u;
             const unsigned int b0 = __byte_perm(vr[0][t >> 1], vr[1][t >> 1], sel);
             const unsigned int b1 = __byte_perm(vr[2][t >> 1], vr[3][t >> 1], sel);
             mma_16816(o[t], pa0, 0u, pa2, 0u, b0, b1);
         }
-        if (nbase < t1) {
-#pragma unroll
-            for (int i = 0; i < 2 * KS; ++i) kr[0][i] = krn[0][i], kr[1][i] = krn[1][i];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int i = 0; i < NTL / 2; ++i) vr[r][i] = vrn[r][i];
+        if constexpr (BULK) {  // the products have read the stage: the step kStages on takes its place
+            __syncwarp();
+            if (base + kStages * NW * 16 < t1) {
+                request(base + kStages * NW * 16, stage);
+                if (holds_pos(base + kStages * NW * 16)) place_pos(base + kStages * NW * 16, stage);
+            }
+        }
+        if (++stage == kStages) stage = 0, phase ^= 1u;
+    }
+    if (BULK && !alive) {  // a copy was lost: the others end before the block does
+        for (int s = 0, at = base; s < kStages && at < t1; ++s, at += NW * 16) {
+            const int k = (at - base0) / (NW * 16);
+            mbar_wait_bounded(&full[k % kStages], (uint32_t)(k / kStages) & 1u, const_cast<StepState*>(a.st));
         }
     }
-    // this warp's state: row g of n-tile t, columns 2j and 2j+1 = head dims (2j)*NTL + t and (2j+1)*NTL + t
+    // this warp's state: row g of n-tile t, columns 2j and 2j+1 = head dims as above
     float (*s_state)[GQA][HS + 2] = reinterpret_cast<float (*)[GQA][HS + 2]>(s_scratch);
     if (g < GQA) {
 #pragma unroll
         for (int t = 0; t < NTL; ++t) {
-            s_state[warp][g][(2 * j) * NTL + t] = o[t][0];
-            s_state[warp][g][(2 * j + 1) * NTL + t] = o[t][1];
+            s_state[warp][g][(t >> 3) * 64 + (2 * j) * 8 + (t & 7)] = o[t][0];
+            s_state[warp][g][(t >> 3) * 64 + (2 * j + 1) * 8 + (t & 7)] = o[t][1];
         }
         if (j == 0) {
             s_state[warp][g][HS] = m;

@@ -487,11 +487,17 @@ static cudaError_t launch_attn_t(lpp_engine* e, const AttnArgs& a, dim3 grid, bo
 static cudaError_t launch_attn_mma(lpp_engine* e, const AttnArgs& a, bool pdl, cudaStream_t s) {
     if (e->c.kv_dtype != LPP_F16) return cudaErrorNotSupported;
     const dim3 grid(a.n_splits, e->KVHl, 1), block(kAttnKernelThreads);
-#define LPP_MMA_CASE(HS_, G_) \
-    if (e->hs == HS_ && e->gqa == G_) return launch_kernel(attn_mma_kernel<HS_, G_>, grid, block, 0, s, pdl, a);
+    const bool bulk = !attn_split_fits_ring(a, e->hs);
+#define LPP_MMA_LAUNCH(HS_, G_, B_) \
+    if (e->hs == HS_ && e->gqa == G_ && bulk == B_) { \
+        const cudaError_t r = cudaFuncSetAttribute(attn_mma_kernel<HS_, G_, B_>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnRingBytes<HS_>); \
+        return r != cudaSuccess ? r : launch_kernel(attn_mma_kernel<HS_, G_, B_>, grid, block, kAttnRingBytes<HS_>, s, pdl, a); \
+    }
+#define LPP_MMA_CASE(HS_, G_) LPP_MMA_LAUNCH(HS_, G_, false) LPP_MMA_LAUNCH(HS_, G_, true)
     LPP_MMA_CASE(64, 1) LPP_MMA_CASE(64, 2) LPP_MMA_CASE(64, 4) LPP_MMA_CASE(64, 8)
     LPP_MMA_CASE(128, 1) LPP_MMA_CASE(128, 2) LPP_MMA_CASE(128, 4) LPP_MMA_CASE(128, 8)
 #undef LPP_MMA_CASE
+#undef LPP_MMA_LAUNCH
     return cudaErrorNotSupported;
 }
 static bool attn_mma_supported(const lpp_engine* e) {

@@ -861,16 +861,6 @@ static __global__ void __launch_bounds__(256) prefill_attention_kernel(const flo
         }
 }
 
-__device__ __forceinline__ void cp_async_16(void* dst_smem, const void* src, bool valid) {
-    const uint32_t d = smem_u32(dst_smem);
-    const int n = valid ? 16 : 0;  // 0 source bytes: the 16 destination bytes are filled with zeros
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
