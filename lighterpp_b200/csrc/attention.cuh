@@ -15,6 +15,8 @@
 // finish (ticket counter), in a fixed order, so results do not depend on scheduling.
 // HBM traffic: K and V rows 0..pos of the layer once (twice when gqa > 4).
 #pragma once
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace lpp {
@@ -413,9 +415,10 @@ __global__ void __launch_bounds__(kAttnKernelThreads) attn_decode_kernel(const A
 // are then read from rows that share banks (K twice, V four times over, 0.8 us of the 1.5 us that a round's
 // 64 KB take to come).  Where a split never holds more than the ring, all of it is requested at once and latency
 // counts instead: there the lanes' own copies, read back without conflicts or barriers, are the faster ones (48
-// tokens of the 1B shape at 640: 32.0 ms with registers, 32.2 in bulk, 31.6 with these), so the capacity of the
-// cache decides between the two.  Both in one kernel, chosen by the split's length, took 32.5 ms and 3 % more at
-// 32 K: the instructions of this kernel come anew from L2 on every launch.
+// tokens of the 1B shape at 640: 32.0 ms with registers, 32.2 in bulk, 31.6 with these), up to the last length whose
+// splits the ring holds (9000 positions of the 1B shape: 10.1 us a launch in bulk, 9.2 with these), so the length decides between
+// the two, on the host.  Both in one kernel, chosen by the split's length, took 32.5 ms and 3 % more at 32 K: the
+// instructions of this kernel come anew from L2 on every launch.
 __device__ __forceinline__ void mma_16816(float (&d)[4], unsigned int a0, unsigned int a1, unsigned int a2, unsigned int a3,
                                           unsigned int b0, unsigned int b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -432,11 +435,18 @@ template <int HS>
 constexpr int kAttnStages = HS == 128 ? 3 : 4;
 template <int HS>
 constexpr int kAttnRingBytes = (kAttnKernelThreads / 32) * kAttnStages<HS> * 16 * HS * 4;  // 16 positions of K and V rows per warp and stage
-// Whether a split can never hold more positions than the ring, whatever the position.
-inline bool attn_split_fits_ring(const AttnArgs& a, int hs) {
+// Splits of attn_mma_kernel at sequence length T.  One CTA per KV head up to two chunks of positions: below that a second split costs
+// more in the combine (partials, ticket, second pass) than it saves (measured: 602 against 620 us/token at 180-243).
+__host__ __device__ inline int attn_mma_splits(const AttnArgs& a, int T) {
+    const int min_chunk = a.min_chunk > 0 ? a.min_chunk : kAttnMinChunk;
+    return T <= 2 * min_chunk ? 1 : attn_effective_splits(T, a.n_splits, min_chunk);
+}
+// Whether the ring holds the splits of sequence length T and of every shorter one whole (they grow up to two chunks of one split, and
+// again once all splits are in use).
+inline bool attn_splits_fit_ring(const AttnArgs& a, int hs, int T) {
     const int room = (hs == 128 ? kAttnStages<128> : kAttnStages<64>) * (kAttnKernelThreads / 32) * 16;
     const int min_chunk = a.min_chunk > 0 ? a.min_chunk : kAttnMinChunk;
-    return 2 * min_chunk <= room && (a.seq_len + a.n_splits - 1) / a.n_splits <= room;
+    return std::min(T, 2 * min_chunk) <= room && (T + a.n_splits - 1) / a.n_splits <= room;
 }
 
 template <int HS, int GQA, bool BULK>
@@ -454,10 +464,7 @@ __global__ void __launch_bounds__(kAttnKernelThreads) attn_mma_kernel(const Attn
     // the position was written by the previous step's sampler, which completed before this step began
     const int pos = a.st->pos;
     const int T = (pos < 0 || pos >= a.seq_len) ? 0 : pos + 1;
-    // one CTA per KV head up to two chunks of positions: below that a second split costs more in the
-    // combine (partials, ticket, second pass) than it saves (measured: 602 against 620 us/token at 180-243)
-    const int min_chunk = a.min_chunk > 0 ? a.min_chunk : kAttnMinChunk;
-    const int n_eff = (T <= 2 * min_chunk) ? 1 : attn_effective_splits(T, a.n_splits, min_chunk);
+    const int n_eff = attn_mma_splits(a, T);
     const int split = blockIdx.x, kvh = blockIdx.y;
     if (split >= n_eff) return;
     const int chunk = (T + n_eff - 1) / n_eff;

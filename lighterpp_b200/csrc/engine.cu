@@ -484,10 +484,9 @@ static cudaError_t launch_attn_t(lpp_engine* e, const AttnArgs& a, dim3 grid, bo
 
 // Attention with the scores and P.V on the tensor cores (FP16 cache, head size 64 or 128, 1/2/4/8 query heads
 // per KV head); other shapes keep the CUDA-core kernel.
-static cudaError_t launch_attn_mma(lpp_engine* e, const AttnArgs& a, bool pdl, cudaStream_t s) {
+static cudaError_t launch_attn_mma(lpp_engine* e, const AttnArgs& a, bool bulk, bool pdl, cudaStream_t s) {
     if (e->c.kv_dtype != LPP_F16) return cudaErrorNotSupported;
     const dim3 grid(a.n_splits, e->KVHl, 1), block(kAttnKernelThreads);
-    const bool bulk = !attn_split_fits_ring(a, e->hs);
 #define LPP_MMA_LAUNCH(HS_, G_, B_) \
     if (e->hs == HS_ && e->gqa == G_ && bulk == B_) { \
         const cudaError_t r = cudaFuncSetAttribute(attn_mma_kernel<HS_, G_, B_>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnRingBytes<HS_>); \
@@ -499,6 +498,10 @@ static cudaError_t launch_attn_mma(lpp_engine* e, const AttnArgs& a, bool pdl, c
 #undef LPP_MMA_CASE
 #undef LPP_MMA_LAUNCH
     return cudaErrorNotSupported;
+}
+static int attn_min_chunk() {
+    const char* mc = aid_env("LPP_ATTN_CHUNK");  // timing experiments
+    return mc ? atoi(mc) : 0;
 }
 static bool attn_mma_supported(const lpp_engine* e) {
     return e->c.kv_dtype == LPP_F16 && (e->hs == 64 || e->hs == 128) && (e->gqa == 1 || e->gqa == 2 || e->gqa == 4 || e->gqa == 8);
@@ -744,7 +747,7 @@ struct Recorder {
     cudaStream_t s;
     bool prev_kernel = false;  // previous stream item was one of our kernels -> PDL edge allowed
     int kernels = 0;
-    bool long_ctx = false;  // record the long-context variant of the step (tensor-core attention kernel)
+    bool long_ctx = false;  // record the long-context variant of the step (step_long_ctx)
     cudaError_t err = cudaSuccess;
     std::string where;
 
@@ -1054,7 +1057,7 @@ static void record_gqa_mixer(Recorder& R, int l, float* cur) {
     at.gqa = e->gqa;
     at.n_splits = e->attn_splits;
     at.n_kv_heads = e->KVHl;
-    if (const char* mc = aid_env("LPP_ATTN_CHUNK")) at.min_chunk = atoi(mc);  // timing experiments
+    at.min_chunk = attn_min_chunk();
     set_prefetch(e, a, kQkv, l);
     record_gemv(R, kQkv, kEpiQkv, a);
     dim3 grid(e->attn_splits, e->KVHl, e->attn_z);
@@ -1063,7 +1066,7 @@ static void record_gqa_mixer(Recorder& R, int l, float* cur) {
     R.mark(kAttn);
     if (attn_mma_supported(e) && !aid_env("LPP_ATTN_CUDA_CORES")) {
         at.n_splits = e->attn_splits_long;
-        R.check(launch_attn_mma(e, at, R.pdl(), R.s), "attention (tensor-core) launch");
+        R.check(launch_attn_mma(e, at, R.long_ctx, R.pdl(), R.s), "attention (tensor-core) launch");
     } else {
         R.check(c.kv_dtype == LPP_F32 ? launch_attn_t<float>(e, at, grid, R.pdl(), R.s)
                                       : launch_attn_t<__half>(e, at, grid, R.pdl(), R.s),
@@ -1212,6 +1215,18 @@ static void record_latent_mixer(Recorder& R, int l, float* cur) {
     record_gemv(R, kLatValue, kEpiLatentValue, v);
 }
 
+// Whether the step at `pos` takes the long-context variant: attention whose splits outgrow the ring of attn_mma_kernel, so that their rows
+// come in bulk.  The host knows the position of every step, and each variant is a graph of its own.  By the cache's capacity instead,
+// a short conversation in a large window pays for a long one: 1B shape with a cache of 16 K, us a token by capacity / by position: at 3
+// 593 / 580, 640 619 / 609, 1900 636 / 629, 4000 658 / 654, 9000 699 / 690; from 9216 on both are the bulk kernel (15 000: 740).
+static bool step_long_ctx(const lpp_engine* e, int pos) {
+    if (!e->layers.empty() || !attn_mma_supported(e)) return false;
+    AttnArgs a = {};
+    a.n_splits = e->attn_splits_long;
+    a.min_chunk = attn_min_chunk();
+    return !attn_splits_fit_ring(a, e->hs, pos + 1);
+}
+
 static void record_step(Recorder& R, bool with_sampler) {
     lpp_engine* e = R.e;
     e->head_clusters = false;
@@ -1350,8 +1365,7 @@ static lpp_status capture(lpp_engine* e, bool with_sampler, bool long_ctx, cudaG
 
 // pos: the position this step runs at (known to the host in every mode); it selects the variant.
 static lpp_status run_step(lpp_engine* e, bool with_sampler, int pos) {
-    const int v = 0;  // a single graph variant serves every position
-    (void)pos;
+    const int v = step_long_ctx(e, pos);
     if (e->c.flags & LPP_FLAG_NO_GRAPH) {
         Recorder R{e, e->stream};
         R.long_ctx = v == 1;
@@ -2252,7 +2266,7 @@ extern "C" lpp_status lpp_finalize(lpp_engine* e) {
         CU(cudaMemset(e->gtrace, 0, (size_t)256 * e->num_sms * 8 * sizeof(unsigned long long)));
     }
     if (!(c.flags & LPP_FLAG_NO_GRAPH)) {
-        for (int v = 0; v < 1; ++v) {
+        for (int v = 0; v <= step_long_ctx(e, c.seq_len - 1); ++v) {
             TRY(capture(e, true, v == 1, &e->g_full[v], v == 0 ? &e->kernels_full : nullptr));
             TRY(capture(e, false, v == 1, &e->g_logits[v], nullptr));
         }
@@ -3586,7 +3600,7 @@ extern "C" lpp_status lpp_profile_kind(lpp_engine* e, int pos, int kind, int ite
     cudaGraphExec_t gx = nullptr;
     int n_kernels = 0;
     e->only_kind = kind;
-    lpp_status rs = capture(e, true, false, &gx, &n_kernels);
+    lpp_status rs = capture(e, true, step_long_ctx(e, pos), &gx, &n_kernels);
     e->only_kind = -1;
     if (rs != LPP_OK) return rs;
     if (n_kernels == 0 && kind != kAllReduce) {
@@ -3638,6 +3652,7 @@ extern "C" lpp_status lpp_profile_step(lpp_engine* e, int pos, int iters, const 
         CU(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
         e->profiling = e->profiling_capture = true;
         Recorder R{e, e->stream};
+        R.long_ctx = step_long_ctx(e, pos);
         record_step(R, true);
         e->profiling = e->profiling_capture = false;
         cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
