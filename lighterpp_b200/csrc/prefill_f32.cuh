@@ -320,9 +320,13 @@ static __global__ void __launch_bounds__(kTileWarps * 32, 2) prefill_f32_tile_ke
 
 // The decode attention of attn_decode_kernel for a block of tokens: token t attends to positions 0 .. start_pos + t with the
 // splits that a step at its position uses (a.n_splits: at least as many as the last token's); rows before block_pos are complete before the block's first kernel starts.  grid: (splits of the last token, kv heads, tokens x head batches)
-// (Bound by the latency of its stages: small head sizes give up registers for a third CTA an SM.)
+// Bound by the latency of its stages, so CTAs an SM count: as many as fit without spills to speak of.  800 tokens, whole prompts in us with the
+// compiler's own choice / with one CTA but three up to dpl * gb = 8 / with these: head size 128, 8 heads of 1024 7747 / 8713 / 7716; 64
+// with two query heads a KV head 3972 / 3882 / 3139; 32 with four 4100 / 5253 / 4098; 48 with two 1480 / 2055 / 1476; 16 heads of 16 2275 / 2628 /
+// 2310; 64 with one (three CTAs spill 144 bytes, 5571) 5478.
+constexpr int f32_attn_ctas(int dpl, int gb) { return dpl * gb <= 4 ? 4 : dpl * gb <= 8 && dpl < 8 ? 3 : dpl * gb <= 16 ? 2 : 1; }
 template <int DPL, int GB>
-static __global__ void __launch_bounds__(kAttnKernelThreads, DPL * GB <= 8 ? 3 : 1) prefill_f32_attn_kernel(AttnArgs a, int start_pos, int block_pos, int n_z, int q_rows,
+static __global__ void __launch_bounds__(kAttnKernelThreads, f32_attn_ctas(DPL, GB)) prefill_f32_attn_kernel(AttnArgs a, int start_pos, int block_pos, int n_z, int q_rows,
                                                                                       int part_row) {
     __shared__ float s_scratch[(kAttnKernelThreads / 32) * GB * (DPL * 8 + 2)];
     __shared__ int s_last;

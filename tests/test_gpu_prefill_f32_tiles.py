@@ -29,3 +29,38 @@ def test_bits_equal_the_token_loop(cfg):
     assert np.array_equal(batched.extend(toks[130:], 130, range(270)), ref[130:])
     for e in (batched, loop):
         e.close()
+
+
+def medians(cfg, sizes):
+    """Microseconds of prompts of these sizes (medians of 15)."""
+    import time
+
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from lighterpp_b200 import engine as E
+    e = E.Engine(cfg, "f32", "f32")
+    e.load_weights(synth.gen_model(cfg, 7, "f32", True))
+    toks, out = synth.prompt_tokens(cfg.vocab_size, max(sizes), 7), []
+    for n in sizes:
+        times = []
+        for _ in range(18):
+            t = time.perf_counter()
+            e.extend(toks[:n], 0, [n - 1])
+            times.append(time.perf_counter() - t)
+        out.append(sorted(times[3:])[7] * 1e6)
+    e.close()
+    return out
+
+
+def least(tries, bound):
+    """The smallest of up to three measured ratios: other work on the machine only makes them larger."""
+    ratios = []
+    while len(ratios) < 3 and (not ratios or ratios[-1] > bound):
+        ratios.append(tries())
+    assert min(ratios) <= bound, ratios
+
+
+def test_fewer_kv_heads_are_not_slower():
+    """Four query heads a KV head read half the rows that two do (with a single CTA an SM for them: 1.18 times as long, else 0.92)."""
+    least(lambda: medians(ModelConfig(512, 1376, 4, 16, 4, 1000, 900), [800])[0] / medians(ModelConfig(512, 1376, 4, 16, 8, 1000, 900), [800])[0], 1.05)
