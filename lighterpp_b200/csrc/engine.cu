@@ -3110,10 +3110,11 @@ static lpp_status prefill_gemm_f32(lpp_engine* e, const void* w, const void* x, 
     // Tiles in shared memory where the step sums a row up in one go (so that its order can be kept), they fit, and half of the SMs get
     // a CTA; else the kernel that reads both operands through L1, whose CTAs are smaller (whole prompts, tiles always / by this rule, us:
     // stories15M 17 tokens 238 / 227, 33 255 / 249; 4 layers of 512 x 1024 17 tokens 203 / 189, 64 236 / 210).  Four lanes to 16 outputs (32 rows a CTA) where that
-    // gives every SM a CTA, else eight (16 rows): half as many steps for a warp.
+    // gives every SM a CTA and fits, else eight (16 rows): half as many steps for a warp.  Rows of 909 to 1208 inputs fit 16 at a time only (6
+    // layers of 1024 x 2816, 64 tokens: row kernel 1203 us, 16 rows 901; 288 tokens 4322 / 3528).
     const int tiles = (n + kTileTokens - 1) / kTileTokens;
     if (a.kc >= K && n > kF32Tokens && (n_rows + kTileRows<8> - 1) / kTileRows<8> * tiles >= e->num_sms / 2) {
-        const bool wide = (n_rows + kTileRows<4> - 1) / kTileRows<4> * tiles >= e->num_sms;
+        const bool wide = (n_rows + kTileRows<4> - 1) / kTileRows<4> * tiles >= e->num_sms && f32_tile_smem(K, kTileRows<4>) <= e->smem_optin;
         const int rows = wide ? kTileRows<4> : kTileRows<8>;
         const size_t smem = f32_tile_smem(K, rows);
         if (smem <= e->smem_optin) {

@@ -1,6 +1,6 @@
 """FP32 prompts through tiles in shared memory, the attention of a block in one launch and the classifier of a few tokens: bit for bit
 the token loop's logits around the tiles' edges (tokens 32, rows 16 and 32, rows of fewer inputs than a warp has lanes and of every
-remainder of 128), with one and several splits of the positions, and for one, four, five and more wanted tokens."""
+remainder of 128, rows of which 32 do not fit beside the tokens), with one and several splits of the positions, and for one, four, five and more wanted tokens."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("cfg", [ModelConfig(96, 1192, 2, 6, 6, 1210, 400), ModelConfig(288, 768, 2, 6, 2, 1026, 400), ModelConfig(384, 1020, 1, 8, 8, 1202, 400),
-                                 ModelConfig(768, 100, 1, 12, 4, 1190, 400)], ids=str)
+                                 ModelConfig(768, 100, 1, 12, 4, 1190, 400), ModelConfig(1152, 908, 1, 9, 3, 1000, 400)], ids=str)
 def test_bits_equal_the_token_loop(cfg):
     import torch
     if not torch.cuda.is_available():
@@ -64,3 +64,12 @@ def least(tries, bound):
 def test_fewer_kv_heads_are_not_slower():
     """Four query heads a KV head read half the rows that two do (with a single CTA an SM for them: 1.18 times as long, else 0.92)."""
     least(lambda: medians(ModelConfig(512, 1376, 4, 16, 4, 1000, 900), [800])[0] / medians(ModelConfig(512, 1376, 4, 16, 8, 1000, 900), [800])[0], 1.05)
+
+
+def test_rows_of_which_sixteen_fit():
+    """1152 inputs: 96 tokens make as many CTAs as 32 rows each would be chosen for, but only 16 fit (row kernel instead of tiles from there on: 1.72
+    times as long as 64 tokens, else 1.40)."""
+    def ratio():
+        few, many = medians(ModelConfig(1152, 1152, 4, 18, 6, 1000, 200), [64, 96])
+        return many / few
+    least(ratio, 1.55)
