@@ -3107,14 +3107,18 @@ static lpp_status prefill_gemm_f32(lpp_engine* e, const void* w, const void* x, 
     gemv_geometry(g, 4, kStageTarget);
     a.kc = (e->c.flags & LPP_FLAG_GEMV_LDG) ? K : g.kc;
     a.st = e->st;
-    // Tiles in shared memory where the step sums a row up in one go (so that its order can be kept), they fit, and half of the SMs get
-    // a CTA; else the kernel that reads both operands through L1, whose CTAs are smaller (whole prompts, tiles always / by this rule, us:
-    // stories15M 17 tokens 238 / 227, 33 255 / 249; 4 layers of 512 x 1024 17 tokens 203 / 189, 64 236 / 210).  Four lanes to 16 outputs (32 rows a CTA) where that
-    // gives every SM a CTA and fits, else eight (16 rows): half as many steps for a warp.  Rows of 909 to 1208 inputs fit 16 at a time only (6
-    // layers of 1024 x 2816, 64 tokens: row kernel 1203 us, 16 rows 901; 288 tokens 4322 / 3528).
+    // Tiles in shared memory where the step sums a row up in one go (so that its order can be kept), they fit, and enough SMs get a CTA;
+    // else the kernel that reads both operands through L1, whose CTAs are smaller.  Enough: half of the SMs where there are many
+    // tokens or inputs (768 x 2048, 17 tokens: row kernel 491 us, tiles 449; 384 x 1024, 128 tokens: 396 / 369), else as many full tiles as SMs,
+    // since a short row's tile is bound by its latency (256 x 512, 33 tokens: 193 / 217; 256 x 688, 48 tokens, 172 tiles that are half
+    // empty: 210 / 213, 64 tokens: 223 / 215).  Four lanes to 16 outputs (32 rows a CTA) where that gives every SM a CTA and fits, else eight (16 rows): half
+    // as many steps for a warp.  Rows of 909 to 1208 inputs fit 16 at a time only
+    // (6 layers of 1024 x 2816, 64 tokens: row kernel 1203 us, 16 rows 901; 288 tokens 4322 / 3528).
     const int tiles = (n + kTileTokens - 1) / kTileTokens;
-    if (a.kc >= K && n > kF32Tokens && (n_rows + kTileRows<8> - 1) / kTileRows<8> * tiles >= e->num_sms / 2) {
-        const bool wide = (n_rows + kTileRows<4> - 1) / kTileRows<4> * tiles >= e->num_sms && f32_tile_smem(K, kTileRows<4>) <= e->smem_optin;
+    auto ctas = [&](int rows) { return (n_rows + rows - 1) / rows * tiles; };
+    const bool enough = n > 64 || K >= 512 ? ctas(kTileRows<8>) >= e->num_sms / 2 : (long long)n_rows * n >= (long long)e->num_sms * kTileRows<8> * kTileTokens;
+    if (a.kc >= K && n > kF32Tokens && enough) {
+        const bool wide = ctas(kTileRows<4>) >= e->num_sms && f32_tile_smem(K, kTileRows<4>) <= e->smem_optin;
         const int rows = wide ? kTileRows<4> : kTileRows<8>;
         const size_t smem = f32_tile_smem(K, rows);
         if (smem <= e->smem_optin) {

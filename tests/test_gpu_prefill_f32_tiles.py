@@ -73,3 +73,12 @@ def test_rows_of_which_sixteen_fit():
         few, many = medians(ModelConfig(1152, 1152, 4, 18, 6, 1000, 200), [64, 96])
         return many / few
     least(ratio, 1.55)
+
+
+def test_second_tile_of_few_tokens():
+    """One token more than a tile of 32, short rows: the second tile is all but empty (tiles for the query, key and value rows there all the same: 1.12
+    times as long as 32 tokens, else 1.0)."""
+    def ratio():
+        one, two = medians(ModelConfig(256, 512, 6, 16, 16, 4000, 100), [32, 33])
+        return two / one
+    least(ratio, 1.07)
