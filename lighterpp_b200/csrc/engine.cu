@@ -3106,7 +3106,6 @@ static lpp_status prefill_gemm_f32(lpp_engine* e, const void* w, const void* x, 
     g.K = K;
     gemv_geometry(g, 4, kStageTarget);
     a.kc = (e->c.flags & LPP_FLAG_GEMV_LDG) ? K : g.kc;
-    a.st = e->st;
     // Tiles in shared memory where the step sums a row up in one go (so that its order can be kept), they fit, and enough SMs get a CTA;
     // else the kernel that reads both operands through L1, whose CTAs are smaller.  Enough: half of the SMs where there are many
     // tokens or inputs (768 x 2048, 17 tokens: row kernel 491 us, tiles 449; 384 x 1024, 128 tokens: 396 / 369), else as many full tiles as SMs,

@@ -82,7 +82,6 @@ struct PrefillF32Args {
     int n_rows, K, kc, n_tokens;
     float* out;          // kPfResid: [tokens][out_pitch] += ; kPfSwiglu: [tokens][out_pitch], column row / 2; kPfStore: [tokens][out_pitch]
     int out_pitch, act;
-    StepState* st;
     PrefillGemmArgs qkv; // kPfQkv: what pf_qkv_store takes
 };
 template <int EPI, bool CHUNKS>
