@@ -634,7 +634,9 @@ static __global__ void __launch_bounds__(128) prefill_latent_combine_kernel(cons
 // thread made 7161 CTAs of 1023 tokens of the rutenex-1b shape, 21.7 us; now 11.6); grid (tokens / kLatFinishTokens, kLatFinishTokens +
 // query sections of 1024 rows), y < kLatFinishTokens takes one token's latent, rotated key part and gates.
 constexpr int kLatFinishThreads = 256, kLatFinishTokens = 4;
-constexpr int kLatFinishQuadTokens = 128;  // fewer tokens: more CTAs rather than more work in each (70 tokens of rutenex-300m: 1745 us, quads 1777)
+// Fewer tokens: more CTAs rather than more work in each (whole prompts, pairs / quads, us: rutenex-1b 128 tokens 1528 / 1555, 160 1893 / 1907, 200 1982 /
+// 1972, 224 1997 / 1988, 256 2039 / 1998; 300m 128 1612 / 1624, 144 1712 / 1705, 200 1897 / 1910, 224 1924 / 1915, 256 1988 / 1959).
+constexpr int kLatFinishQuadTokens = 224;
 struct PrefillLatentFinishArgs {
     const float* part;  // [splits][part_tokens][n_rows]
     int part_tokens, cap, n_rows, splits;

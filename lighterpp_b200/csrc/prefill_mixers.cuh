@@ -26,7 +26,9 @@ __device__ __forceinline__ float2 prefill_sum2(const float* part, int part_token
 // multiple of four rows: four rows of kKvFinishTokens tokens a thread, as in prefill_latent_finish_kernel (517 tokens of the kolatar-1b
 // shape 19.2 -> 8.7 us); grid: (ceil(tokens / kKvFinishTokens), ceil(rows / 1024)).
 constexpr int kKvFinishTokens = 4;
-constexpr int kKvFinishQuadTokens = 192;  // fewer tokens: more CTAs rather than more work in each (130 tokens of kolatar-300m: 1514 us, quads 1527)
+// Fewer tokens: more CTAs rather than more work in each (whole prompts, pairs / quads, us: kolatar-300m 192 tokens 2028 / 2038, 200 2147 / 2165, 224 2225 /
+// 2230, 240 2280 / 2278, 256 2330 / 2321; 1b 224 2142 / 2141, 240 2186 / 2164).
+constexpr int kKvFinishQuadTokens = 240;
 struct PrefillSharedKvArgs {
     const float* part;  // [splits][part_tokens][n_rows]
     int part_tokens, n_rows, splits;
