@@ -3189,8 +3189,10 @@ static lpp_status prefill_f32_attention(lpp_engine* e, const PrefillGemmArgs& g,
     return LPP_OK;
 }
 // Logits of up to this many tokens go through the step's classifier GEMV one by one: it streams the matrix where the block kernel, whose
-// warps take eight tokens whether there are as many or not, is bound by the loads of its tiles (32 000 x 288, one token: 69 us -> 10).
-constexpr int kF32GemvRows = 4;
+// warps take eight tokens whether there are as many or not, is bound by the loads of its tiles (32 000 x 288, one token: 69 us -> 10).  Several
+// tokens of a classifier of fewer elements than this: one launch instead (512 x 64, four tokens, whole prompts: 125 us one by one, 115
+// together; 1000 x 288: 251 and 251).
+constexpr int kF32GemvRows = 4, kF32GemvElements = 1 << 18;
 // prefill_block for engines with FP32 weights.
 static lpp_status prefill_block_f32(lpp_engine* e, int n, int start_pos, int n_want, float* h_logits) {
     const lpp_config& c = e->c;
@@ -3214,7 +3216,7 @@ static lpp_status prefill_block_f32(lpp_engine* e, int n, int start_pos, int n_w
     for (int i = 0; i < n_want; i += kPfTile) {
         const int m = std::min(kPfTile, n_want - i);
         TRY(prefill_f32_norm(e, m, e->rms_final, false, e->pf_rows + i));
-        if (m <= kF32GemvRows) {
+        if (m == 1 || (m <= kF32GemvRows && (size_t)e->Vp * D >= kF32GemvElements)) {
             for (int r = 0; r < m; ++r) {
                 GemvArgs a = {};
                 a.W = e->wcls;
