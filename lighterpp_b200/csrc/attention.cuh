@@ -503,18 +503,18 @@ __global__ void __launch_bounds__(kAttnKernelThreads) attn_mma_kernel(const Attn
     auto v_row = [&](int base, int c) { return base + (c / VP >> 1) * 8 + 2 * j + (c / VP & 1); };
     auto k_src = [&](int t, int c) { return reinterpret_cast<const uint4*>(kb + (size_t)t * HS) + 4 * (c % KP) + j; };
     auto v_src = [&](int t, int c) { return reinterpret_cast<const uint4*>(vb + (size_t)t * HS) + 8 * (c % VP) + g; };
-    // this lane's pieces of the rows [base, base + 16) but the current position's; zeros from t1 on
+    // this lane's pieces of the rows [base, base + 16) but the current position's, which may be a later split's; zeros from t1 on
     auto request_own = [&](int base, int stage) {
         uint4* d = ring + stage * 32 * kRow + lane;
 #pragma unroll
         for (int c = 0; c < 2 * KP; ++c) {
             const int t = k_row(base, c);
-            if (t != pos) cp_async_16(d + c * 32, k_src(t < t1 ? t : t0, c), t < t1);
+            if (t != pos || t >= t1) cp_async_16(d + c * 32, k_src(t < t1 ? t : t0, c), t < t1);
         }
 #pragma unroll
         for (int c = 0; c < 4 * VP; ++c) {
             const int t = v_row(base, c);
-            if (t != pos) cp_async_16(d + (2 * KP + c) * 32, v_src(t < t1 ? t : t0, c), t < t1);
+            if (t != pos || t >= t1) cp_async_16(d + (2 * KP + c) * 32, v_src(t < t1 ? t : t0, c), t < t1);
         }
     };
     // rows [base, min(base + 16, t1)) but the current position's
