@@ -5,11 +5,11 @@
 // Why: each of the three moves a few hundred KB and is bound by a launch, its dependency wait and a round trip or two (rutenex-300m: 3.0 + 3.8 +
 // 3.9 us back to back); per head they depend on nothing of the other heads.  The CTAs of a head share its work: rows of W_uk, keys
 // of the window, rows of W_uv.  What they owe each other, the query (rank floats) and the unnormalised results (rank floats a CTA),
-// is written straight into everybody's shared memory, and a hardware cluster barrier follows: two of them, where three kernel boundaries
-// were.  Weights and the cache rows of earlier positions are requested before the dependency wait.  Every head reads the shared cache rows by
+// is written straight into everybody's shared memory, and a hardware cluster barrier follows: two exchanges, and a meeting at the start
+// (a CTA has to run before it is written to), where three kernel boundaries were.  Weights and the cache rows of earlier positions are requested before the dependency wait.  Every head reads the shared cache rows by
 // itself (16 heads: 4.7 MB from L2 at the 300m shape), in exchange for as many SMs; query, scores and probabilities stay FP32.
 // Measured, 33 tokens of rutenex-300m at 700: 21.75 -> 20.1 ms, 18.9 with the SM's memory split as the GEMVs have it.  What is left is latency:
-// launch and dependency wait, three cluster barriers, and code that is fetched once a launch (loops are kept short; 98 registers of
+// launch and dependency wait, the three barriers, and code that is fetched once a launch (loops are kept short; 98 registers of
 // prefetched weights instead of shared memory: 0.3 ms more at position 3).
 #pragma once
 #include "latent.cuh"
@@ -19,7 +19,7 @@ namespace lpp {
 
 constexpr int kLhThreads = 256, kLhMaxCtas = 8, kLhMaxRank = 2048;
 // Shared memory beside which a GEMV's CTA finds room on an SM.  A CTA with more waits for the input GEMV's CTA to leave and clusters then
-// for whole groups of free SMs (rutenex-1b, 156 KB, 33 tokens: 30.4 instead of 25.2 ms; its rows left in L2: 27.5).
+// for whole groups of free SMs (rutenex-1b, 208 KB, of which 150 are cache rows: a token at 3 771 us instead of 695, at 700 906 instead of 762).
 constexpr size_t kLhSmemBytes = 80 * 1024;
 
 struct LatentHeadArgs {

@@ -631,7 +631,7 @@ static __global__ void __launch_bounds__(256) prefill_qkv_finish_kernel(const Pr
 // that the rows of a block are all resident at once (one or two pieces on 512 threads, two or three rows an SM: 13 us for 1023
 // rows of 2048 and 22 us for 1000 of 4096; now 6 and 11).  With partial sums of a few rows the latency counts: one
 // or two pieces a thread, all ranges in flight (47 rows of 2048 with 8 ranges: 4.5 us, four pieces a thread 8.3), one row an SM.  Many
-// rows become waves that way: half the threads and registers for four rows an SM instead (517 rows of 2048 with partial sums: 12.3 -> 7.9
+// rows become waves that way: half the threads and registers for four rows an SM instead (64 registers, 88 bytes of spills; 517 rows of 2048 with partial sums: 12.3 -> 7.9
 // us), from 384 rows of 512 threads on (whole prompts of the TinyLlama shape, few / many rows' kernel: 200 tokens 1878 / 1946 us, 350
 // 2127 / 2169, 400 2554 / 2501; kolatar-300m, rows of 256 threads: 400 tokens 2739 / 2788, 900 4080 / 3938).
 enum PfNormMode : int { kNormPlain = 0, kNormFewParts = 1, kNormManyParts = 2 };

@@ -29,9 +29,10 @@
 //   Latency-bound: ceil(V/2048) blocks, a few microseconds per dependent stage.  A token of the
 //   Llama-3.2-1B shape whose distribution is confident (0.998 on one token): 3.35 ms with windows of
 //   whole blocks added one by one by one warp, of which this kernel took 2.7 ms; 0.66 ms now.
-//   128256 logits with 64 history entries: 48.8 us a call with maps of 64-bit words, carries and offsets
-//   found warp after warp, checks inside the walk's chain and the history searched per entry; 34.7 us with
-//   32-bit maps made by two additions, carries scanned by every warp, checks after the walk and counts.
+//   128256 logits with 64 history entries, calls behind one another on one box: 43.5 us with maps of 64-bit words,
+//   carries and offsets found warp after warp, checks inside the walk's chain and the history searched per entry;
+//   32.6 us with 32-bit maps made by two additions, carries scanned by every warp, checks after the walk and
+//   counts; 31.2 us with the registers of one CTA an SM.
 //
 // exp() is exp_repro (common.cuh): IEEE double arithmetic only, identical on host and device; it
 // differs from libm's expf in the last bit for about 0.06 % of arguments, which is the only source
