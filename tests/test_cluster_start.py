@@ -8,8 +8,8 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lighterpp_b200", "csrc")
-REMOTE = re.compile(r"\bmapa\.|\bcluster_load4?\(|\bcluster_map\(|\bcluster_addr\(")
-MET = re.compile(r"barrier\.cluster\.wait|\bpair_sync\(\)|\bcluster_barrier\(\)")
+REMOTE = re.compile(r"\bmapa\.|\bcluster_load4?\(|\bcluster_store\(|\bcluster_map\(|\bcluster_addr\(")
+MET = re.compile(r"barrier\.cluster\.wait|\bpair_sync\(\)|\bcluster_barrier\(\)|\bcluster_wait\(\)")
 
 
 def kernels():
@@ -31,7 +31,8 @@ REMOTE_KERNELS = [k for k in kernels() if REMOTE.search(k[2])]
 
 
 def test_finds_the_kernels_there_are():
-    assert {name for _, name, _ in REMOTE_KERNELS} >= {"aggregation_kernel", "prefill_gemm_pair_kernel", "prefill_attention_umma_kernel", "latent_attn_mma_kernel"}
+    assert {name for _, name, _ in REMOTE_KERNELS} >= {"aggregation_kernel", "prefill_gemm_pair_kernel", "prefill_attention_umma_kernel", "latent_attn_mma_kernel",
+                                                            "latent_head_kernel"}
 
 
 @pytest.mark.parametrize("file,name,body", REMOTE_KERNELS, ids=[k[1] for k in REMOTE_KERNELS])

@@ -38,7 +38,7 @@ def test_step_at_edges(oracle, heads, kv_heads, hs):
 
 def test_large_cache_with_a_short_context():
     """The kernel follows the position, not the capacity of the cache: at short contexts the attention of an engine whose cache outgrows the
-    ring takes as long as with a small cache.  (Chosen by capacity: 1.09 to 1.12 times as long at these positions.  Medians, the best of three
+    ring takes as long as with a small cache.  (Chosen by capacity: 1.09 to 1.13 times as long at these positions.  Medians, the best of five
     tries: other work on the GPU only makes it slower.)"""
     import torch
     if not torch.cuda.is_available():
@@ -57,7 +57,7 @@ def test_large_cache_with_a_short_context():
         engines.append(e)
     for pos in (100, 1900):
         ratios = []
-        for _ in range(3):
+        for _ in range(5):
             small, large = [sorted(e.profile_kind(pos, "attention", 3)["ms_per_launch"] for _ in range(9))[4] for e in engines]
             ratios.append(large / small)
             if ratios[-1] <= 1.04:

@@ -54,9 +54,9 @@ def medians(cfg, sizes):
 
 
 def least(tries, bound):
-    """The smallest of up to three measured ratios: other work on the machine only makes them larger."""
+    """The smallest of up to five measured ratios: other work on the machine only makes them larger."""
     ratios = []
-    while len(ratios) < 3 and (not ratios or ratios[-1] > bound):
+    while len(ratios) < 5 and (not ratios or ratios[-1] > bound):
         ratios.append(tries())
     assert min(ratios) <= bound, ratios
 
